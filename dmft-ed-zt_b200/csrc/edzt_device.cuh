@@ -29,6 +29,7 @@ struct DevSpin {
     const double* amp;      // [namp] amplitude of a slot: +V at 2c, -V at 2c+1, c = iorb*nbath + jbath
     const uint8_t* imp;     // [count] impurity bits (sites 1..norb)
     const int32_t* sub;     // [count][P] rank after replacing the impurity bits (norb > 1)
+    const int32_t* nat;     // [count] rank in the reference's order (tables in internal order, else null)
 };
 
 // Packed hop entry: target rank in the low 20 bits (C(20,10) < 2^20), the
@@ -163,32 +164,29 @@ struct ApplyCArgs {
     const int32_t* in_dn_rank;
 };
 
-// Element i of apply_c's output, row-wise over the output sector
-// (ed_operator.f90:31-54).  The bit of the full state is
-// q = (ispin-1)*nsite + iorb - 1 and the sign is (-1)^{popcount of the output
-// state's bits 0..q-1} (ed_operator.f90:34,59-76); for a down-spin operator
-// that count includes every up electron.
+// apply_c's output at the state with strings (u, d) (ed_operator.f90:31-54).
+// The bit of the full state is q = (ispin-1)*nsite + iorb - 1 and the sign is
+// (-1)^{popcount of the output state's bits 0..q-1} (ed_operator.f90:34,59-76);
+// for a down-spin operator that count includes every up electron.
+__device__ __forceinline__ double apply_c_at(const ApplyCArgs& A, const double* __restrict__ in, uint32_t u, uint32_t d)
+{
+    const uint32_t bit = 1u << (A.iorb - 1);
+    const uint32_t s = (A.ispin == 1) ? u : d;
+    if ((A.pm == 1) != ((s & bit) != 0u)) return 0.0;
+    const int par = (A.ispin == 1) ? __popc(u & (bit - 1u)) : __popc(u) + __popc(d & (bit - 1u));
+    const int ju = __ldg(A.in_up_rank + (A.ispin == 1 ? u ^ bit : u));
+    const int jd = __ldg(A.in_dn_rank + (A.ispin == 1 ? d : d ^ bit));
+    EDZT_OK_OR(ju >= 0 && jd >= 0, 41, u, d, bit, return 0.0)
+    const double v = __ldg(in + (long long)jd * A.in_nup + ju);
+    return (par & 1) ? -v : v;
+}
+
+// Element i of apply_c's output, row-wise over the output sector.
 __device__ __forceinline__ double apply_c_value(const ApplyCArgs& A, const double* __restrict__ in,
                                                 long long i)
 {
     const int iu = (int)(i % A.out_nup), id = (int)(i / A.out_nup);
-    const uint32_t u = __ldg(A.out_up_str + iu), d = __ldg(A.out_dn_str + id);
-    const uint32_t bit = 1u << (A.iorb - 1);
-    int par;
-    long long j;
-    if (A.ispin == 1) {
-        if ((A.pm == 1) != ((u & bit) != 0u)) return 0.0;
-        par = __popc(u & (bit - 1u));
-        j = (long long)id * A.in_nup + __ldg(A.in_up_rank + (u ^ bit));   // down rank unchanged
-        EDZT_OK_OR(__ldg(A.in_up_rank + (u ^ bit)) >= 0, 41, i, u, bit, return 0.0)
-    } else {
-        if ((A.pm == 1) != ((d & bit) != 0u)) return 0.0;
-        par = __popc(u) + __popc(d & (bit - 1u));
-        j = (long long)__ldg(A.in_dn_rank + (d ^ bit)) * A.in_nup + iu;   // up rank unchanged
-        EDZT_OK_OR(__ldg(A.in_dn_rank + (d ^ bit)) >= 0, 42, i, d, bit, return 0.0)
-    }
-    const double v = __ldg(in + j);
-    return (par & 1) ? -v : v;
+    return apply_c_at(A, in, __ldg(A.out_up_str + iu), __ldg(A.out_dn_str + id));
 }
 
 // Error codes written by kernels into a device status word.

@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <deque>
 #include <thread>
+#include <tuple>
 #include <cuda_runtime.h>
 #include "../../include/edzt.h"
 #include "edzt_internal.h"
@@ -162,6 +163,7 @@ bool is_device_ptr(const void* p, int device)
 struct StrTable {
     int n = 0, count = 0;
     std::unique_ptr<DevBuf> str, rank;
+    std::unique_ptr<DevBuf> nat;            // internal order only: ranks in the reference's order
 };
 
 struct OpsTable {
@@ -177,7 +179,8 @@ struct ModelTables {
     DevModel model{};
     int P = 1;
     bool has_j = false;
-    std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> ops;
+    std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> ops;    // strings in the reference's order
+    std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> iops;   // strings in internal order
     std::unique_ptr<DevBuf> wint, jcnt, jt;
 };
 
@@ -194,6 +197,8 @@ struct edzt_ctx {
     ModelTables mt;                         // the model of the single-model entry points
     // bit strings and rank tables by (nsite, electron count): model-independent, shared
     std::map<std::pair<int, int>, std::unique_ptr<StrTable>> str_tables;
+    // the same in internal order, by (nsite, electron count, norb)
+    std::map<std::tuple<int, int, int>, std::unique_ptr<StrTable>> int_tables;
     Pool pool;
     // resident ground state
     bool has_gs = false;
@@ -216,7 +221,7 @@ struct edzt_ctx {
     unsigned long long dbg_wait_ns = 0;
     int dbg_stall_cta = -1;
     // tile shapes chosen by edzt_tune_sector, by (up strings, down strings)
-    struct Tuned { int wc, r, block; double ms_per_step; };
+    struct Tuned { LzShape shape; double ms_per_step; };
     std::map<std::pair<int, int>, Tuned> tuned;
     // per launch since the last statistics reset: device ms, algorithmic
     // bytes, states in the launch (the last kLaunchLog)
@@ -227,34 +232,46 @@ namespace {
 
 int nsite_of(const edzt_ctx* c) { return c->mt.model.nsite; }
 
-StrTable& str_table_ns(edzt_ctx* c, int ns, int n)
+std::unique_ptr<StrTable> build_str_table(edzt_ctx* c, int ns, int n, int norb)
 {
-    const auto key = std::make_pair(ns, n);
-    auto it = c->str_tables.find(key);
-    if (it != c->str_tables.end()) return *it->second;
     auto t = std::make_unique<StrTable>();
     t->n = n;
     t->count = (int)edzt_binom(ns, n);
-    t->str = std::make_unique<DevBuf>(sizeof(uint32_t) * (size_t)std::max(t->count, 1));
+    const size_t cnt = (size_t)std::max(t->count, 1);
+    t->str = std::make_unique<DevBuf>(sizeof(uint32_t) * cnt);
     t->rank = std::make_unique<DevBuf>(sizeof(int32_t) * ((size_t)1 << ns));
-    launch_build_strings(ns, n, t->str->as<uint32_t>(), t->rank->as<int32_t>(), c->stream);
+    if (norb > 0) t->nat = std::make_unique<DevBuf>(sizeof(int32_t) * cnt);
+    launch_build_strings(ns, n, t->str->as<uint32_t>(), t->rank->as<int32_t>(), c->stream, norb,
+                         t->nat ? t->nat->as<int32_t>() : nullptr);
     c->launches += 2;
     CKLAUNCH();
-    StrTable& ref = *t;
-    c->str_tables.emplace(key, std::move(t));
-    return ref;
+    return t;
+}
+
+StrTable& str_table_ns(edzt_ctx* c, int ns, int n)
+{
+    auto& t = c->str_tables[std::make_pair(ns, n)];
+    if (!t) t = build_str_table(c, ns, n, 0);
+    return *t;
+}
+
+StrTable& int_table_ns(edzt_ctx* c, int ns, int n, int norb)
+{
+    auto& t = c->int_tables[std::make_tuple(ns, n, norb)];
+    if (!t) t = build_str_table(c, ns, n, norb);
+    return *t;
 }
 
 StrTable& str_table(edzt_ctx* c, int n) { return str_table_ns(c, nsite_of(c), n); }
 
-OpsTable& ops_table_mt(edzt_ctx* c, ModelTables& mt, int n, int sigma)
+// The operator tables of (n, sigma), strings in the reference's order or (internal) in internal order.
+OpsTable& ops_table_mt(edzt_ctx* c, ModelTables& mt, int n, int sigma, bool internal)
 {
-    auto key = std::make_pair(n, sigma);
-    auto it = mt.ops.find(key);
-    if (it != mt.ops.end()) return *it->second;
-    StrTable& st = str_table_ns(c, mt.model.nsite, n);
-    auto t = std::make_unique<OpsTable>();
+    auto& ref = (internal ? mt.iops : mt.ops)[std::make_pair(n, sigma)];
+    if (ref) return *ref;
     const int norb = mt.model.norb, nbath = mt.model.nbath;
+    StrTable& st = internal ? int_table_ns(c, mt.model.nsite, n, norb) : str_table_ns(c, mt.model.nsite, n);
+    auto t = std::make_unique<OpsTable>();
     // hop slots per string: the largest hop count of any string, rounded up to whole uint4s
     const int maxh = edzt_max_hops(mt.model, sigma, n);
     t->hw = std::max(4, (maxh + 3) / 4 * 4);
@@ -272,9 +289,8 @@ OpsTable& ops_table_mt(edzt_ctx* c, ModelTables& mt, int n, int sigma)
                           c->stream);
     c->launches += 1;
     CKLAUNCH();
-    OpsTable& ref = *t;
-    mt.ops.emplace(key, std::move(t));
-    return ref;
+    ref = std::move(t);
+    return *ref;
 }
 
 bool sector_valid_ns(int ns, int nu, int nd) { return nu >= 0 && nd >= 0 && nu <= ns && nd <= ns; }
@@ -289,14 +305,16 @@ bool sector_valid(const edzt_ctx* c, int nu, int nd) { return sector_valid_ns(ns
 
 long long sector_dim(const edzt_ctx* c, int nu, int nd) { return sector_dim_ns(nsite_of(c), nu, nd); }
 
-DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd)
+// The sector of (nu, nd) with its tables in the reference's string order, or
+// (internal) in the internal order of the Lanczos runs.
+DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd, bool internal)
 {
     DevSector S{};
-    const int ns = mt.model.nsite;
-    StrTable& su = str_table_ns(c, ns, nu);
-    StrTable& sd = str_table_ns(c, ns, nd);
-    OpsTable& ou = ops_table_mt(c, mt, nu, 0);
-    OpsTable& od = ops_table_mt(c, mt, nd, 1);
+    const int ns = mt.model.nsite, norb = mt.model.norb;
+    StrTable& su = internal ? int_table_ns(c, ns, nu, norb) : str_table_ns(c, ns, nu);
+    StrTable& sd = internal ? int_table_ns(c, ns, nd, norb) : str_table_ns(c, ns, nd);
+    OpsTable& ou = ops_table_mt(c, mt, nu, 0, internal);
+    OpsTable& od = ops_table_mt(c, mt, nd, 1, internal);
     auto fill = [&](DevSpin& sp, StrTable& st, OpsTable& o) {
         sp.count = st.count;
         sp.hw = o.hw;
@@ -309,6 +327,7 @@ DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd)
         sp.amp = o.amp->as<double>();
         sp.imp = o.imp->as<uint8_t>();
         sp.sub = o.sub ? o.sub->as<int32_t>() : nullptr;
+        sp.nat = st.nat ? st.nat->as<int32_t>() : nullptr;
     };
     fill(S.up, su, ou);
     fill(S.dn, sd, od);
@@ -325,7 +344,14 @@ DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd)
     return S;
 }
 
-DevSector make_sector(edzt_ctx* c, int nu, int nd) { return make_sector_mt(c, c->mt, nu, nd); }
+// A sector of the context's model, the reference's string order; the tables
+// in internal order are built too, as edzt_lanczos_iteration_noalloc, which
+// builds none, may be called on any sector that another call has prepared.
+DevSector make_sector(edzt_ctx* c, int nu, int nd)
+{
+    make_sector_mt(c, c->mt, nu, nd, true);
+    return make_sector_mt(c, c->mt, nu, nd, false);
+}
 
 // Interaction tables over impurity occupation patterns (pu, pd).
 // wint: impurity_hamiltonian.f90:119-141 without the em-mu terms (those are
@@ -421,6 +447,7 @@ DevModel model_from(int norb, int nbath, const double* em, const double* ek, con
 void set_tables_model(ModelTables& mt, const DevModel& m, cudaStream_t stream)
 {
     mt.ops.clear();
+    mt.iops.clear();
     mt.model = m;
     build_model_tables(mt, stream);
     mt.valid = true;
@@ -489,30 +516,25 @@ struct JobSpec {
     double* eig = nullptr;           // device, EIGVEC
     double* a = nullptr;             // device [maxnstep]
     double* b = nullptr;             // device [maxnstep]
-    double2* keep = nullptr;         // device [maxnstep + 1][dim]: keep every step's pair (else ping-pong)
+    double* keep = nullptr;          // device [maxnstep] vectors: keep every step's v (else ping-pong)
     // results
     int nstep = 0;
     double norm0 = 0.0;
 };
 
-// Widths preset on the jobs from the context's tuning table (the widest
-// tuned job decides the block size), or forced (force_* > 0, the tuner).
-int preset_widths(edzt_ctx* c, std::vector<LzJob>& jobs, int force_wc, int force_r, int force_block)
+// The tile shape that the autotuner chose for the widest tuned run of a
+// launch (null: none tuned).
+const LzShape* tuned_shape(edzt_ctx* c, const std::vector<LzJob>& jobs)
 {
-    if (force_block > 0) {
-        for (LzJob& J : jobs) { J.ph[0].width = force_wc; J.ph[1].width = force_r; }
-        return force_block;
-    }
-    int block = 0;
+    const LzShape* best = nullptr;
     long long widest = -1;
-    for (LzJob& J : jobs) {
+    for (const LzJob& J : jobs) {
         auto it = c->tuned.find({J.S.up.count, J.S.dn.count});
-        if (it == c->tuned.end()) continue;
-        J.ph[0].width = it->second.wc;
-        J.ph[1].width = it->second.r;
-        if (J.S.dim > widest) { widest = J.S.dim; block = it->second.block; }
+        if (it == c->tuned.end() || J.S.dim <= widest) continue;
+        widest = J.S.dim;
+        best = &it->second.shape;
     }
-    return block;
+    return best;
 }
 
 constexpr size_t kLaunchLog = 256;
@@ -525,63 +547,64 @@ void log_launch(edzt_ctx* c, double ms, double bytes, double states)
     c->log_states.push_back(states);
 }
 
-void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, int force_wc = 0, int force_r = 0, int force_block = 0)
+// The run's descriptor but for its vectors and state.
+void fill_job(LzJob& J, const JobSpec& s, const DevSector& S)
+{
+    std::memset(&J, 0, sizeof(J));
+    J.S = S;
+    J.eig = s.eig;
+    J.coeff = s.coeff;
+    J.a = s.a;
+    J.b = s.b;
+    J.maxnstep = s.maxnstep;
+    J.mode = s.mode;
+    J.init = s.init;
+    J.key = s.key;
+    J.ac = s.ac;
+    J.src = s.ac_src;
+}
+
+void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = nullptr)
 {
     const int nj = (int)specs.size();
     if (nj == 0) return;
     std::vector<LzJob> jobs(nj);
-    std::vector<Lease<double2>> bufs;
-    std::vector<Lease<double>> dbufs;
-    bufs.reserve((size_t)nj * 2);
-    dbufs.reserve((size_t)nj);
+    std::vector<Lease<double>> bufs;
+    bufs.reserve((size_t)nj * 3);
     int max_steps = 0;
     for (int j = 0; j < nj; j++) {
         JobSpec& s = specs[j];
         LzJob& J = jobs[j];
-        std::memset(&J, 0, sizeof(J));
-        J.S = make_sector_mt(c, s.mt ? *s.mt : c->mt, s.nu, s.nd);
-        const long long dim = J.S.dim;
+        fill_job(J, s, make_sector_mt(c, s.mt ? *s.mt : c->mt, s.nu, s.nd, true));
+        auto vec = [&] {
+            bufs.emplace_back(c->pool, (size_t)lz_vec_size(J.S.up.count, J.S.dn.count));
+            return bufs.back().p;
+        };
+        J.Y = vec();
         if (s.keep) {
             J.keep = 1;
-            J.YW[0] = s.keep;
-            J.YW[1] = nullptr;
+            J.V[0] = s.keep;
         } else {
-            for (int q = 0; q < 2; q++) {
-                bufs.emplace_back(c->pool, (size_t)dim);
-                J.YW[q] = bufs.back().p;
-            }
+            J.V[0] = vec();
+            J.V[1] = vec();
         }
-        dbufs.emplace_back(c->pool, (size_t)lz_d_size(J.S.up.count, J.S.dn.count));
-        J.D = dbufs.back().p;
-        J.eig = s.eig;
-        J.coeff = s.coeff;
-        J.a = s.a;
-        J.b = s.b;
-        J.maxnstep = s.maxnstep;
-        J.mode = s.mode;
-        J.init = s.init;
-        J.key = s.key;
-        J.ac = s.ac;
-        J.src = s.ac_src;
         max_steps = std::max(max_steps, J.maxnstep);
         if (s.mode == LZ_COEFF) {
             CK(cudaMemsetAsync(s.a, 0, sizeof(double) * s.maxnstep, c->stream));
             CK(cudaMemsetAsync(s.b, 0, sizeof(double) * s.maxnstep, c->stream));
         }
     }
-    // rows per tile and columns per slab of every job (tuned, else by
-    // lz_plan's rule), tile lists of both phases, grid and shared memory
-    const int prefer = preset_widths(c, jobs, force_wc, force_r, force_block);
+    // the tile shape (tuned, else by lz_plan's rule), the lists of both
+    // phases, grid and shared memory
     std::vector<long long> prefix;
-    const LzPlan P = lz_plan(c->device, jobs.data(), nj, prefix, prefer);
+    const LzPlan P = lz_plan(c->device, jobs.data(), nj, prefix, force ? force : tuned_shape(c, jobs));
     if (P.grid <= 0) throw EdztError{EDZT_ERR_CUDA, "persistent kernel cannot be resident (shared memory too large)"};
-    const int G = P.grid;
     std::vector<LzState> st(2 * (size_t)nj);
     std::memset(st.data(), 0, sizeof(LzState) * st.size());
     for (int j = 0; j < nj; j++) st[2 * (size_t)j + 1].active = 1;   // the state before phase 0 (parity 1)
     const size_t bytes_jobs = sizeof(LzJob) * nj, bytes_st = sizeof(LzState) * st.size();
-    const size_t bytes_pre = sizeof(long long) * prefix.size(), bytes_slots = sizeof(double) * 2 * (size_t)P.slots;
-    const size_t bytes_sw = lz_sync_bytes(G);
+    const size_t bytes_pre = sizeof(long long) * prefix.size(), bytes_slots = sizeof(double) * (size_t)P.slots;
+    const size_t bytes_sw = lz_sync_bytes(nj);
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t total = al(bytes_jobs) + al(bytes_st) + al(bytes_pre) + al(bytes_slots) + al(bytes_sw);
     Lease<char> blob(c->pool, total);
@@ -591,28 +614,21 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, int force_wc = 0, int fo
     long long* d_pre = reinterpret_cast<long long*>(base + al(bytes_jobs) + al(bytes_st));
     double* d_slots = reinterpret_cast<double*>(base + al(bytes_jobs) + al(bytes_st) + al(bytes_pre));
     unsigned* d_sw = reinterpret_cast<unsigned*>(base + al(bytes_jobs) + al(bytes_st) + al(bytes_pre) + al(bytes_slots));
-    std::vector<unsigned> sw(bytes_sw / sizeof(unsigned), 0u);
-    sw[64] = (unsigned)nj;   // runs still going
     for (int j = 0; j < nj; j++) jobs[j].st = d_st + 2 * (size_t)j;
     CK(cudaMemcpyAsync(d_jobs, jobs.data(), bytes_jobs, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(d_st, st.data(), bytes_st, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(d_pre, prefix.data(), bytes_pre, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(d_sw, sw.data(), bytes_sw, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(d_sw, 0, bytes_sw, c->stream));
     CK(cudaMemsetAsync(c->status->p, 0, sizeof(int), c->stream));
     LzBatch B;
     std::memset(&B, 0, sizeof(B));
     B.njobs = nj;
-    B.grid = G;
-    B.block = P.block;
-    B.smem = P.smem;
-    B.total[0] = P.total[0];
-    B.total[1] = P.total[1];
     B.max_phases = 2 * max_steps + 4;   // two phases per step and the phase that closes the last one
     if (c->dbg_pass_cap > 0) B.max_phases = std::min(B.max_phases, c->dbg_pass_cap);
     B.wait_ns = c->dbg_wait_ns;
     B.stall_cta = c->dbg_stall_cta;
     CK(cudaEventRecord(c->ev0, c->stream));
-    CK(launch_lanczos_persistent(B, d_jobs, d_pre, d_slots, d_sw, c->status->as<int>(), c->stream));
+    CK(launch_lanczos_persistent(P, B, d_jobs, d_pre, d_slots, d_sw, c->status->as<int>(), c->stream));
     CK(cudaEventRecord(c->ev1, c->stream));
     c->launches += 1;
     int status = 0;
@@ -656,9 +672,9 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, int force_wc = 0, int fo
 // ---------------------------------------------------------------------------
 edzt_ctx::Tuned tune_sector(edzt_ctx* c, int nu, int nd, int steps)
 {
-    const DevSector S = make_sector(c, nu, nd);
+    const DevSector S = make_sector_mt(c, c->mt, nu, nd, true);
     Lease<double> ab(c->pool, (size_t)2 * steps);
-    auto run = [&](int wc, int r, int block) {
+    auto run = [&](const LzShape& q) {
         std::vector<JobSpec> specs(1);
         specs[0].nu = nu; specs[0].nd = nd;
         specs[0].mode = LZ_COEFF;
@@ -668,24 +684,18 @@ edzt_ctx::Tuned tune_sector(edzt_ctx* c, int nu, int nd, int steps)
         specs[0].a = ab.p;
         specs[0].b = ab.p + steps;
         const double ms0 = c->st_ms;
-        run_jobs(c, specs, wc, r, block);
+        run_jobs(c, specs, &q);
         return (c->st_ms - ms0) / std::max(1, specs[0].nstep);
     };
-    const size_t fixed = lz_fixed_smem();
-    edzt_ctx::Tuned best{0, 0, 0, HUGE_VAL};
-    run(2, 1, 512);                                       // warm-up
-    for (int block : {256, 512}) {
-        const size_t budget = (block == 256 ? 108 * 1024 : kLzSmemMax) - fixed;
-        for (int wc : {8, 4, 2}) {
-            if (lz_col_smem(S.dn.count, wc) > budget) continue;
-            for (int r : {4, 2, 1}) {
-                if (lz_row_smem(S.up.count, r) > budget) continue;
-                const double ms = run(wc, r, block);
-                if (ms < best.ms_per_step) best = {wc, r, block, ms};
-            }
-        }
+    edzt_ctx::Tuned best{{0, 0, 0}, HUGE_VAL};
+    run({2, 2, 512});                                     // warm-up
+    for (const LzShape q : {LzShape{16, 8, 256}, LzShape{16, 8, 512}, LzShape{8, 8, 256}, LzShape{8, 8, 512}, LzShape{8, 4, 256},
+                            LzShape{8, 4, 512}, LzShape{4, 4, 256}, LzShape{4, 4, 512}, LzShape{2, 2, 256}, LzShape{2, 2, 512}}) {
+        if (!lz_shape_fits(S, q)) continue;
+        const double ms = run(q);
+        if (ms < best.ms_per_step) best = {q, ms};
     }
-    if (best.wc == 0) throw EdztError{EDZT_ERR_ARG, "no tile shape of this sector fits shared memory"};
+    if (best.shape.wc == 0) throw EdztError{EDZT_ERR_ARG, "no tile shape of this sector fits shared memory"};
     c->tuned[{S.up.count, S.dn.count}] = best;
     return best;
 }
@@ -970,6 +980,7 @@ void diag_arpack_impl(edzt_ctx* c, const DevSector& S, uint64_t key, double* vec
 
 struct SectorResult {
     int nstep = 0;
+    double norm0 = 0.0;
     double e = HUGE_VAL;
     std::vector<double> a, b, coeff;
     bool ok = false;
@@ -1024,18 +1035,20 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
         return;
     }
     std::vector<SectorResult> res(nsector);
-    // The scan keeps every step's (y, w) pairs when they fit in half of the
+    const int ns = nsite_of(c);
+    auto vec_size = [&](int nu, int nd) { return lz_vec_size((int)edzt_binom(ns, nu), (int)edzt_binom(ns, nd)); };
+    // The scan keeps every step's v_k when they fit in half of the
     // device memory that was free when the context was created (queried once:
     // a query per solve can wait on the driver behind other processes'
-    // queries): the winner's eigenvector is then one pass over its kept w_k
+    // queries): the winner's eigenvector is then one pass over its kept v_k
     // instead of a second run of the recurrence (the same sum, in the same
     // order, of the same vectors).  The pool keeps the blocks for the next solve.
-    std::vector<Lease<double2>> kept(nsector);
+    std::vector<Lease<double>> kept(nsector);
     bool keep = false;
     if (c->engine == EDZT_ENGINE_FUSED && c->keep_vectors) {
         long long states = 0;
-        for (int i = 0; i < nsector; i++) states += std::max(0LL, sector_dim(c, sectors[2 * i], sectors[2 * i + 1]));
-        keep = (double)states * (maxnstep + 1) * sizeof(double2) <= 0.5 * (double)c->free_at_create;
+        for (int i = 0; i < nsector; i++) states += vec_size(sectors[2 * i], sectors[2 * i + 1]);
+        keep = (double)states * maxnstep * sizeof(double) <= 0.5 * (double)c->free_at_create;
     }
     if (c->engine == EDZT_ENGINE_FUSED) {
         std::vector<JobSpec> specs;
@@ -1053,7 +1066,7 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             s.a = ab.p + (size_t)(2 * i) * maxnstep;
             s.b = ab.p + (size_t)(2 * i + 1) * maxnstep;
             if (keep) {
-                kept[i] = Lease<double2>(c->pool, (size_t)(maxnstep + 1) * sector_dim(c, nu, nd));
+                kept[i] = Lease<double>(c->pool, (size_t)maxnstep * vec_size(nu, nd));
                 s.keep = kept[i].p;
             }
             specs.push_back(s);
@@ -1067,6 +1080,7 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             const int i = which[q];
             SectorResult& r = res[i];
             r.nstep = specs[q].nstep;
+            r.norm0 = specs[q].norm0;
             r.a.assign(hab.begin() + (size_t)(2 * i) * maxnstep, hab.begin() + (size_t)(2 * i + 1) * maxnstep);
             r.b.assign(hab.begin() + (size_t)(2 * i + 1) * maxnstep, hab.begin() + (size_t)(2 * i + 2) * maxnstep);
             if (r.nstep >= 1) {
@@ -1092,15 +1106,20 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
         const long long dim = sector_dim(c, nu, nd);
         c->gs_vec = Lease<double>(c->pool, (size_t)dim);
         SectorResult& r = res[best];
-        Lease<double> cf(c->pool, (size_t)r.nstep), ab(c->pool, (size_t)2 * maxnstep);
-        CK(cudaMemcpyAsync(cf.p, r.coeff.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemcpyAsync(ab.p, r.a.data(), sizeof(double) * maxnstep, cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemcpyAsync(ab.p + maxnstep, r.b.data(), sizeof(double) * maxnstep, cudaMemcpyHostToDevice, c->stream));
+        const DevSector Si = make_sector_mt(c, c->mt, nu, nd, true);
+        Lease<double> cf(c->pool, (size_t)r.nstep);
         if (keep) {
-            launch_keep_combine(kept[best].p, dim, r.nstep, cf.p, c->gs_vec.p, c->stream);
+            std::vector<double> hc(r.nstep);              // sum_k coeff_k w_k, w_k = v_k / b_k
+            for (int k = 0; k < r.nstep; k++) hc[k] = r.coeff[k] / (k == 0 ? r.norm0 : r.b[k]);
+            CK(cudaMemcpyAsync(cf.p, hc.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
+            launch_keep_combine(kept[best].p, Si, r.nstep, cf.p, c->gs_vec.p, c->stream);
             c->launches += 1;
             CKLAUNCH();
         } else {
+            Lease<double> ab(c->pool, (size_t)2 * maxnstep), eig(c->pool, (size_t)vec_size(nu, nd));
+            CK(cudaMemcpyAsync(cf.p, r.coeff.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
+            CK(cudaMemcpyAsync(ab.p, r.a.data(), sizeof(double) * maxnstep, cudaMemcpyHostToDevice, c->stream));
+            CK(cudaMemcpyAsync(ab.p + maxnstep, r.b.data(), sizeof(double) * maxnstep, cudaMemcpyHostToDevice, c->stream));
             std::vector<JobSpec> ev(1);
             ev[0].nu = nu; ev[0].nd = nd;
             ev[0].mode = LZ_EIGVEC;
@@ -1108,12 +1127,15 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             ev[0].key = edzt_stream_key(seed, stream_of(best));
             ev[0].maxnstep = r.nstep;
             ev[0].coeff = cf.p;
-            ev[0].eig = c->gs_vec.p;
+            ev[0].eig = eig.p;
             ev[0].a = ab.p;
             ev[0].b = ab.p + maxnstep;
             run_jobs(c, ev);
+            launch_to_natural(eig.p, Si, c->gs_vec.p, c->stream);
+            c->launches += 1;
+            CKLAUNCH();
         }
-        for (auto& k : kept) k = Lease<double2>();
+        for (auto& k : kept) k = Lease<double>();
         DevSector S = make_sector(c, nu, nd);
         c->gs_residual = finish_eigvec(c, S, c->gs_vec.p, r.e);
         c->gs_up = nu; c->gs_dn = nd; c->gs_isector = best; c->gs_e0 = r.e;
@@ -1254,7 +1276,7 @@ void green_runs(edzt_ctx* c, std::vector<GreenRun>& runs, int maxnstep, int nw, 
             GreenRun& g = runs[r];
             const int ns = g.mt->model.nsite;
             if (sector_dim_ns(ns, g.nu, g.nd) <= 0) continue;
-            DevSector S = make_sector_mt(c, *g.mt, g.nu, g.nd);
+            DevSector S = make_sector_mt(c, *g.mt, g.nu, g.nd, false);
             Lease<double> vin(c->pool, (size_t)S.dim);
             if (g.start) {
                 launch_copy(vin.p, g.start, S.dim, c->stream);
@@ -1597,6 +1619,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     }
     // ---- eigenvector pass of every winner (lanczos_solver.f90:213-300)
     std::vector<JobSpec> ev;
+    std::vector<Lease<double>> eigs;          // the eigenvectors in internal order
     Lease<double> coeffs(c->pool, (size_t)std::max(i1 - i0, 1) * maxnstep);
     std::vector<double> hcoef((size_t)std::max(i1 - i0, 1) * maxnstep, 0.0);
     for (int i = i0; i < i1; i++) {
@@ -1607,6 +1630,8 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
         I.gs_up = specs[q].nu; I.gs_dn = specs[q].nd;
         I.e0 = res[q].e;
         I.gsvec = Lease<double>(c->pool, (size_t)sector_dim_ns(I.model.nsite, I.gs_up, I.gs_dn));
+        const int ns = I.model.nsite;
+        eigs.emplace_back(c->pool, (size_t)lz_vec_size((int)edzt_binom(ns, I.gs_up), (int)edzt_binom(ns, I.gs_dn)));
         std::copy(res[q].coeff.begin(), res[q].coeff.end(), hcoef.begin() + (size_t)(i - i0) * maxnstep);
         JobSpec j;
         j.mt = I.mt.get();
@@ -1616,7 +1641,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
         j.key = specs[q].key;
         j.maxnstep = res[q].nstep;
         j.coeff = coeffs.p + (size_t)(i - i0) * maxnstep;
-        j.eig = I.gsvec.p;
+        j.eig = eigs.back().p;
         j.a = specs[q].a;            // the coefficients of the scan, still on the device
         j.b = specs[q].b;
         ev.push_back(j);
@@ -1625,10 +1650,13 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     run_jobs(c, ev);
     for (int i = i0; i < i1; i++) {   // normalise (lanczos_solver.f90:291)
         const long long n = sector_dim_ns(B[i].model.nsite, B[i].gs_up, B[i].gs_dn);
+        const DevSector Si = make_sector_mt(c, *B[i].mt, B[i].gs_up, B[i].gs_dn, true);
+        launch_to_natural(eigs[i - i0].p, Si, B[i].gsvec.p, c->stream);
         launch_dot(B[i].gsvec.p, B[i].gsvec.p, n, c->dot_part->as<double>(), c->scal->as<double>(), c->stream);
         launch_scale_inv_sqrt(B[i].gsvec.p, n, c->scal->as<double>(), c->stream);
-        c->launches += 3;
+        c->launches += 4;
     }
+    eigs.clear();
     CKLAUNCH();
     // ---- Green's function runs of every instance (dmft_green.f90:47-126)
     std::vector<GreenRun> runs;
@@ -1657,7 +1685,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
 }
 
 // Validate one instance and estimate the device memory it holds at its peak
-// (sector scan: 32 B per state of every sector; Green's runs: 4*norb runs of
+// (sector scan: 24 B per state of every sector; Green's runs: 4*norb runs of
 // the largest neighbouring sector plus the ground state).
 void init_inst(const edzt_instance& in, BatchInst& I)
 {
@@ -1673,14 +1701,15 @@ void init_inst(const edzt_instance& in, BatchInst& I)
         const int nu = I.sec[2 * s], nd = I.sec[2 * s + 1];
         arg_check(sector_valid_ns(ns, nu, nd), "electron counts outside [0, nsite]");
         const long long d = sector_dim_ns(ns, nu, nd);
-        gsb += 40 * d + 56 * sector_dim_ns(ns, 0, nd);   // two pair buffers and D (slab padding) per run
+        gsb += 24 * lz_vec_size((int)edzt_binom(ns, nu), (int)edzt_binom(ns, nd));   // y and two v per run
         maxd = std::max(maxd, d);
         for (int du = -1; du <= 1; du++)
             for (int dd = -1; dd <= 1; dd++)
-                if ((du == 0) != (dd == 0)) maxe = std::max(maxe, sector_dim_ns(ns, nu + du, nd + dd));
+                if (((du == 0) != (dd == 0)) && sector_valid_ns(ns, nu + du, nd + dd))
+                    maxe = std::max(maxe, lz_vec_size((int)edzt_binom(ns, nu + du), (int)edzt_binom(ns, nd + dd)));
     }
-    const long long cfb = 4LL * I.model.norb * (40 * maxe + 56 * sector_dim_ns(ns, 0, ns / 2)) + 8 * maxd;
-    I.footprint = std::max(gsb, cfb) + 56 * maxd;
+    const long long cfb = 4LL * I.model.norb * 24 * maxe + 8 * maxd;
+    I.footprint = std::max(gsb, cfb) + 64 * maxd;
 }
 
 void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int maxnstep, int nw, const double* omega,
@@ -1735,8 +1764,7 @@ void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int max
 struct LiveJob {
     JobSpec spec;
     DevSector S{};
-    Lease<double2> yw0, yw1;
-    Lease<double> d;
+    Lease<double> y, v0, v1;
     Lease<LzState> st;                     // [2] by phase parity, on the device
     int k = 0;                             // steps done (host view, from the last slice)
     bool done = false;
@@ -1754,6 +1782,7 @@ struct ServReq {
     std::vector<SectorResult> res;
     int win = -1;                          // winning sector
     Lease<double> coef;                    // tridiagonal eigenvector of the winner (device)
+    Lease<double> eig;                     // the winner's eigenvector in internal order
     std::vector<GreenRun> runs;
     Lease<double> gab;                     // [nruns][2][maxnstep] Green's-run coefficients (device)
     std::vector<double> G;                 // G_cl(nw, norb, nspin), complex interleaved
@@ -1785,10 +1814,11 @@ std::unique_ptr<LiveJob> make_live(edzt_ctx* c, const JobSpec& spec)
 {
     auto L = std::make_unique<LiveJob>();
     L->spec = spec;
-    L->S = make_sector_mt(c, spec.mt ? *spec.mt : c->mt, spec.nu, spec.nd);
-    L->yw0 = Lease<double2>(c->pool, (size_t)L->S.dim);
-    L->yw1 = Lease<double2>(c->pool, (size_t)L->S.dim);
-    L->d = Lease<double>(c->pool, (size_t)lz_d_size(L->S.up.count, L->S.dn.count));
+    L->S = make_sector_mt(c, spec.mt ? *spec.mt : c->mt, spec.nu, spec.nd, true);
+    const size_t n = (size_t)lz_vec_size(L->S.up.count, L->S.dn.count);
+    L->y = Lease<double>(c->pool, n);
+    L->v0 = Lease<double>(c->pool, n);
+    L->v1 = Lease<double>(c->pool, n);
     L->st = Lease<LzState>(c->pool, 2);
     LzState init[2];
     std::memset(init, 0, sizeof(init));
@@ -1812,56 +1842,37 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases)
     for (int j = 0; j < nj; j++) {
         LiveJob& L = *v[j];
         LzJob& J = jobs[j];
-        std::memset(&J, 0, sizeof(J));
-        J.S = L.S;
-        J.YW[0] = L.yw0.p;
-        J.YW[1] = L.yw1.p;
-        J.D = L.d.p;
-        J.eig = L.spec.eig;
-        J.coeff = L.spec.coeff;
-        J.a = L.spec.a;
-        J.b = L.spec.b;
-        J.maxnstep = L.spec.maxnstep;
-        J.mode = L.spec.mode;
-        J.init = L.spec.init;
-        J.key = L.spec.key;
-        J.ac = L.spec.ac;
-        J.src = L.spec.ac_src;
+        fill_job(J, L.spec, L.S);
+        J.Y = L.y.p;
+        J.V[0] = L.v0.p;
+        J.V[1] = L.v1.p;
         J.st = L.st.p;
     }
-    const int prefer = preset_widths(c, jobs, 0, 0, 0);
     std::vector<long long> prefix;
-    const LzPlan P = lz_plan(c->device, jobs.data(), nj, prefix, prefer);
+    const LzPlan P = lz_plan(c->device, jobs.data(), nj, prefix, tuned_shape(c, jobs));
     if (P.grid <= 0) throw EdztError{EDZT_ERR_CUDA, "persistent kernel cannot be resident (shared memory too large)"};
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t bytes_jobs = sizeof(LzJob) * nj, bytes_pre = sizeof(long long) * prefix.size();
-    const size_t bytes_slots = sizeof(double) * 2 * (size_t)P.slots, bytes_sw = lz_sync_bytes(P.grid);
+    const size_t bytes_slots = sizeof(double) * (size_t)P.slots, bytes_sw = lz_sync_bytes(nj);
     Lease<char> blob(c->pool, al(bytes_jobs) + al(bytes_pre) + al(bytes_slots) + al(bytes_sw));
     LzJob* d_jobs = reinterpret_cast<LzJob*>(blob.p);
     long long* d_pre = reinterpret_cast<long long*>(blob.p + al(bytes_jobs));
     double* d_slots = reinterpret_cast<double*>(blob.p + al(bytes_jobs) + al(bytes_pre));
     unsigned* d_sw = reinterpret_cast<unsigned*>(blob.p + al(bytes_jobs) + al(bytes_pre) + al(bytes_slots));
-    std::vector<unsigned> sw(bytes_sw / sizeof(unsigned), 0u);
-    sw[64] = (unsigned)nj;
     CK(cudaMemcpyAsync(d_jobs, jobs.data(), bytes_jobs, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(d_pre, prefix.data(), bytes_pre, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(d_sw, sw.data(), bytes_sw, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(d_sw, 0, bytes_sw, c->stream));
     CK(cudaMemsetAsync(c->status->p, 0, sizeof(int), c->stream));
     LzBatch B;
     std::memset(&B, 0, sizeof(B));
     B.njobs = nj;
-    B.grid = P.grid;
-    B.block = P.block;
-    B.smem = P.smem;
-    B.total[0] = P.total[0];
-    B.total[1] = P.total[1];
     B.max_phases = std::max(2, phases & ~1);
     if (c->dbg_pass_cap > 0) B.max_phases = std::min(B.max_phases, std::max(2, c->dbg_pass_cap & ~1));
     B.wait_ns = c->dbg_wait_ns;
     B.stall_cta = c->dbg_stall_cta;
     B.slice = 1;
     CK(cudaEventRecord(c->ev0, c->stream));
-    CK(launch_lanczos_persistent(B, d_jobs, d_pre, d_slots, d_sw, c->status->as<int>(), c->stream));
+    CK(launch_lanczos_persistent(P, B, d_jobs, d_pre, d_slots, d_sw, c->status->as<int>(), c->stream));
     CK(cudaEventRecord(c->ev1, c->stream));
     c->launches += 1;
     std::vector<LzState> st(2 * (size_t)nj);
@@ -1989,7 +2000,9 @@ void after_scan(edzt_server* sv, ServReq& q)
     j.key = edzt_stream_key(q.I.seed, (uint64_t)w);
     j.maxnstep = q.res[w].nstep;
     j.coeff = q.coef.p;
-    j.eig = q.I.gsvec.p;
+    q.eig = Lease<double>(c->pool, (size_t)lz_vec_size((int)edzt_binom(q.I.model.nsite, q.I.gs_up),
+                                                       (int)edzt_binom(q.I.model.nsite, q.I.gs_dn)));
+    j.eig = q.eig.p;
     j.a = q.ab.p + (size_t)(2 * w) * maxnstep;
     j.b = q.ab.p + (size_t)(2 * w + 1) * maxnstep;
     q.jobs.push_back(make_live(c, j));
@@ -2004,10 +2017,13 @@ void after_eigvec(edzt_server* sv, ServReq& q)
     const int maxnstep = sv->maxnstep;
     BatchInst& I = q.I;
     const long long n = sector_dim_ns(I.model.nsite, I.gs_up, I.gs_dn);
+    const DevSector Si = make_sector_mt(c, *I.mt, I.gs_up, I.gs_dn, true);
+    launch_to_natural(q.eig.p, Si, I.gsvec.p, c->stream);
     launch_dot(I.gsvec.p, I.gsvec.p, n, c->dot_part->as<double>(), c->scal->as<double>(), c->stream);
     launch_scale_inv_sqrt(I.gsvec.p, n, c->scal->as<double>(), c->stream);
-    c->launches += 3;
+    c->launches += 4;
     CKLAUNCH();
+    q.eig.reset();
     const bool even = !(I.nspin == 2 || I.gs_up != I.gs_dn);
     q.runs = cluster_runs(I.model.norb, even, I.gs_up, I.gs_dn);
     q.gab = Lease<double>(c->pool, std::max<size_t>(q.runs.size(), 1) * 2 * maxnstep);
@@ -2136,7 +2152,7 @@ int server_step(edzt_server* sv)
         if ((*it)->phase == 4) {
             ServReq& q = **it;
             q.jobs.clear();
-            q.I.gsvec.reset(); q.I.mt.reset(); q.ab.reset(); q.coef.reset(); q.gab.reset();
+            q.I.gsvec.reset(); q.I.mt.reset(); q.ab.reset(); q.coef.reset(); q.eig.reset(); q.gab.reset();
             sv->reserved -= q.I.footprint;
             sv->finished[q.id] = std::move(*it);
             it = sv->active.erase(it);
@@ -2185,14 +2201,16 @@ int edzt_ctx_ready_sector(edzt_ctx* c, int nu, int nd, DevSector* S, const char*
     if (!c->mt.valid) { *why = "no model: call edzt_set_model first"; return EDZT_ERR_STATE; }
     if (!sector_valid(c, nu, nd)) { *why = "electron counts outside [0, nsite]"; return EDZT_ERR_ARG; }
     const int ns = nsite_of(c);
-    const bool ready = c->str_tables.count(std::make_pair(ns, nu)) && c->str_tables.count(std::make_pair(ns, nd)) &&
-                       c->mt.ops.count(std::make_pair(nu, 0)) && c->mt.ops.count(std::make_pair(nd, 1));
+    const int norb = c->mt.model.norb;
+    const bool ready = c->int_tables.count(std::make_tuple(ns, nu, norb)) &&
+                       c->int_tables.count(std::make_tuple(ns, nd, norb)) &&
+                       c->mt.iops.count(std::make_pair(nu, 0)) && c->mt.iops.count(std::make_pair(nd, 1));
     if (!ready) {
         *why = "the sector's tables are not built on this context: make one allocating call on the sector "
                "first (edzt_hx or edzt_lanczos_iteration)";
         return EDZT_ERR_STATE;
     }
-    *S = make_sector(c, nu, nd);   // only looks the tables up
+    *S = make_sector_mt(c, c->mt, nu, nd, true);   // only looks the tables up
     return EDZT_OK;
 }
 
@@ -2644,9 +2662,9 @@ int edzt_tune_sector(edzt_ctx* c, int ne_up, int ne_dn, int steps, int* wc, int*
         arg_check(steps >= 2 && steps <= 1000, "steps in [2, 1000]");
         arg_check(sector_dim(c, ne_up, ne_dn) > 0, "empty sector");
         const edzt_ctx::Tuned t = tune_sector(c, ne_up, ne_dn, steps);
-        if (wc) *wc = t.wc;
-        if (rows) *rows = t.r;
-        if (block) *block = t.block;
+        if (wc) *wc = t.shape.wc;
+        if (rows) *rows = t.shape.r;
+        if (block) *block = t.shape.block;
         if (ms_per_step) *ms_per_step = t.ms_per_step;
     });
 }

@@ -32,8 +32,12 @@ inline bool edzt_once_per_device(std::atomic<unsigned long long>& done)
 // ---- tables.cu -------------------------------------------------------------
 void edzt_init_binomials(int device);
 uint64_t edzt_binom(int n, int k);
-// Fills str[C(nsite,n)] (ascending) and rank[2^nsite] on the device.
-void launch_build_strings(int nsite, int n, uint32_t* str, int32_t* rank, cudaStream_t s);
+// Fills str[C(nsite,n)] (ascending) and rank[2^nsite] on the device.  With
+// norb > 0 the strings come in internal order instead: ascending with the
+// norb impurity bits moved above the bath bits (hv_plane.cuh), and nat
+// (nullable) gets each string's rank in the plain order.
+void launch_build_strings(int nsite, int n, uint32_t* str, int32_t* rank, cudaStream_t s, int norb = 0,
+                          int32_t* nat = nullptr);
 // Per-string tables of one spin species (sigma = 0 up, 1 down) for a model.
 // hpk: [hw/4][count] uint4 (packed hop entries, see edzt_hop_pack); amp:
 // [2*norb*nbath] (at least 2) amplitude slots.
@@ -44,11 +48,14 @@ void launch_build_spin_ops(const DevModel& m, int sigma, int count, const uint32
 int edzt_max_hops(const DevModel& m, int sigma, int n);
 
 // ---- kernels.cu: standalone (non-persistent) kernels ------------------------
-// Ground-state vector from the kept pairs of a coefficient run: out =
-// sum_{k=1..nstep} coeff[k-1] w_k, w_k the second value of step k's pair,
-// accumulated in step order as the eigenvector pass does.
-void launch_keep_combine(const double2* keep, long long dim, int nstep, const double* coeff, double* out,
+// Ground-state vector from the kept vectors of a coefficient run (step k at
+// (k - 1) * lz_vec_size): out (the reference's order) =
+// sum_{k=1..nstep} coeff[k-1] v_k, accumulated in step order as the
+// eigenvector pass does.
+void launch_keep_combine(const double* keep, const DevSector& S, int nstep, const double* coeff, double* out,
                          cudaStream_t s);
+// out (the reference's order) = v (a run's vector).
+void launch_to_natural(const double* v, const DevSector& S, double* out, cudaStream_t s);
 // H.v in two phases (hv_phase.cuh); scratch: hx_scratch_size doubles of
 // device memory (the down-hop part, slab-major, slabs of up to 16 columns).
 void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, double* scratch, cudaStream_t s);
@@ -106,17 +113,18 @@ void launch_rl_div(double* out, const double* w, double beta, long long n, cudaS
 enum LzMode { LZ_COEFF = 0, LZ_EIGVEC = 1 };
 enum LzInit { LZ_INIT_HASH = 0, LZ_INIT_APPLYC = 1, LZ_INIT_COPY = 2 };
 
-// The tiles of one job in one phase (0: column phase, 1: row phase): tiles
-// [tile0, tile0 + ntiles) of that phase's list; its participants are CTAs
-// (tile0 + q) mod G, q < npart, and participant q owns partial-sum slot
-// slot0 + q.
+// The list positions of one job in one phase (0: column phase, slabs of
+// `width` columns; 1: row phase, groups of `width` rows): [tile0, tile0 +
+// ntiles) of that phase's list.  Its participants are the CTAs part0, part0 +
+// 1, ... (npart of them); participant q owns partial-sum slot slot0 + q.
 struct LzPhase {
-    long long tile0;      // first tile in the launch's tile list of the phase
+    long long tile0;      // first position in the launch's list of the phase
     long long slot0;      // first partial-sum slot
     int ntiles;
     int npart;            // participating CTAs: part0, part0 + 1, ..., one slot each
-    int width;            // columns per slab (column phase) or rows per tile (row phase)
+    int width;            // columns (column phase) or rows (row phase) of a list position
     int part0;
+    int planes;           // list positions staged together as one tile
 };
 
 // Recurrence state of one run between phases (every participating CTA
@@ -127,18 +135,21 @@ struct LzState {
     int nstep;            // result: number of valid Lanczos steps
     int opened;           // step k already opened (a_{k-1} derived) by the closing pass of a slice
     double a_prev;        // a_{k-1}
-    double b_cur;         // b_k, the normaliser of the step (||v_init|| for k = 1)
+    double b_cur;         // the last norm known: b_{k-1} in a column phase, b_k in a row phase (||v_init|| for k = 1)
+    double b_prev;        // b_{k-1} in a row phase
     double norm0;         // ||v_init||
-    double spare;
 };
 
-// The Lanczos vectors of a run live as interleaved pairs (y_k, w_k), one
-// 16-byte access each: step k writes YW[k & 1] and reads YW[(k - 1) & 1].
+// A run's vectors, in the internal string order (S.up.nat, S.dn.nat), are
+// stored as 4 x 4 blocks of 128 bytes, the four rows of a column adjacent:
+// slab of four columns, then group of four rows, column, row (lz_index).  A
+// slab of columns is one contiguous stream, a group of rows is a 128-byte
+// line per slab, and two rows of a column are one 16-byte access.  Rows and
+// columns are padded to whole blocks; the padding is never read as values.
 struct LzJob {
-    DevSector S;
-    double2* YW[2];       // ping-pong pair buffers [dim]; keep: YW[0] holds every step's pair, step k at k * dim
-    double* D;            // [lz_d_size] down-hop part of H v_k, column phase -> row phase, slab-major:
-                          // the slab of columns [c0, c0 + WC) is the block [ndn][WC] at c0 * ndn
+    DevSector S;          // spin tables in internal order
+    double* Y;            // y_k; between a step's phases D, the down-hop part of H v_k
+    double* V[2];         // v_k, unnormalised: step k at V[k & 1]; keep: step k at V[0] + (k - 1) * lz_vec_size
     double* eig;          // EIGVEC: output eigenvector (unnormalised)
     const double* coeff;  // EIGVEC: ground eigenvector of the tridiagonal [nstep]
     double* a;            // [maxnstep] a(1..), written as steps are accepted
@@ -146,75 +157,83 @@ struct LzJob {
     int maxnstep;         // COEFF: LanczosSteps; EIGVEC: nstep of the coefficient pass
     int mode;
     int init;
-    int keep;             // 1: the pairs of every step are kept ([maxnstep + 1][dim] at YW[0])
+    int keep;             // 1: every step's v is kept ([maxnstep] vectors at V[0])
     LzPhase ph[2];
     LzState* st;          // [2] the run's state by phase parity (kept across launches of a sliced run)
     uint64_t key;         // LZ_INIT_HASH
     ApplyCArgs ac;        // LZ_INIT_APPLYC
-    const double* src;    // LZ_INIT_APPLYC: the ground state; LZ_INIT_COPY: the start vector
+    const double* src;    // LZ_INIT_APPLYC: the ground state; LZ_INIT_COPY: the start vector (the reference's order)
 };
 
-// The pair buffer step k of a run writes (and step k + 1 reads).
-__host__ __device__ inline double2* lz_pairs(const LzJob& J, int k)
+__host__ __device__ constexpr int lz_pad(int count) { return (count + 3) / 4 * 4; }
+
+// Where element (id, iu) of a run's vector lies; ndp = lz_pad(down strings).
+__host__ __device__ inline unsigned lz_index(int id, int iu, int ndp)
 {
-    return J.keep ? J.YW[0] + (long long)k * J.S.dim : J.YW[k & 1];
+    return (unsigned)(((iu >> 2) * ndp + (id & ~3)) * 4 + (iu & 3) * 4 + (id & 3));
 }
 
-// Doubles of a job's D buffer (slabs of up to 8 columns).
-inline long long lz_d_size(int nup, int ndn) { return (long long)((nup + 7) / 8) * 8 * ndn; }
+// Doubles of one vector of a run.
+__host__ __device__ inline long long lz_vec_size(int nup, int ndn) { return (long long)lz_pad(nup) * lz_pad(ndn); }
+
+// v_k of a run (k = 0: never read).
+__host__ __device__ inline double* lz_v(const LzJob& J, int k)
+{
+    return J.keep ? J.V[0] + (k > 0 ? k - 1 : 0) * lz_vec_size(J.S.up.count, J.S.dn.count) : J.V[k & 1];
+}
 
 struct LzBatch {
     int njobs;
-    int grid;
-    int block;
+    int grid;                     // set by the launch
+    size_t fixed;                 // shared memory before the staged tile; set by the launch
     int max_phases;               // phase budget of the launch (even for a slice)
-    size_t smem;
-    long long total[2];           // tiles of the column and the row phase
-    unsigned long long wait_ns;   // grid-barrier wait limit (0: the default 5 s)
+    unsigned long long wait_ns;   // wait limit of a job's arrivals (0: the default 5 s)
     int stall_cta;                // fault test: this CTA leaves without arriving (-1: none)
     int slice;                    // 1: a slice of longer runs; at the end of the budget every run
                                   // still going opens its next step, so a later launch resumes it
 };
 
 // Largest dynamic shared memory of one persistent CTA.
-constexpr size_t kLzSmemMax = 220 * 1024;
-// CTAs of block threads that can be resident with smem bytes each.
-int lz_grid_size(int device, size_t smem, int block);
-// jobs[j].st: the job's state by phase parity; prefix: [2][njobs + 1] tile
-// prefix sums of the column and row phases; slots: [slots][2] partial sums
-// by step parity.
-cudaError_t launch_lanczos_persistent(const LzBatch& B, const LzJob* jobs, const long long* prefix, double* slots,
-                                      unsigned* sync_words, int* status, cudaStream_t s);
-// Shared memory of a row tile of R rows, of a column slab of WC columns, and
-// of the fixed tables.
-size_t lz_row_smem(int nup, int R);
-size_t lz_col_smem(int ndn, int WC);
-size_t lz_fixed_smem();
-// Sync-word buffer size (bytes) for a grid of G CTAs.
-size_t lz_sync_bytes(int G);
-// Tile shapes of the jobs of one launch: every job's rows per tile and
-// columns per slab (a nonzero jobs[j].ph[].width on entry is a preset, kept
-// when it fits), the launch's block size (prefer_block 512: one CTA of 512
-// threads per SM; 256: two of 256 whenever they fit; 0: two of 256 unless a
-// job has long lines or needs more shared memory), grid and shared memory;
-// the phases' tile lists, participants and slots are filled in.  prefix
-// receives, per phase, the jobs' first tiles [njobs + 1], then per phase
-// every CTA's first tile [grid + 1] (CTA b takes the contiguous tiles
-// [range[b], range[b + 1]), cut by tile cost so the CTAs finish together),
-// then the slab of each column-phase tile position [total[0]].
+constexpr size_t kLzSmemMax = 227 * 1024;
+// A tile shape of the persistent kernel: columns per slab tile, rows per row
+// tile, threads per CTA.
+struct LzShape {
+    int wc, r, block;
+};
+// Plan of a launch: its kernel (tile shape, exchange terms), block, grid and
+// shared memory; the jobs' phases are filled in.  prefix receives, per phase,
+// the jobs' first list positions [njobs + 1], then per phase every CTA's first
+// position [grid + 1] (CTA b takes the contiguous positions [range[b],
+// range[b + 1]), cut by cost so the CTAs finish together), then the slab of
+// each column-phase position [total[0]].  force: use this shape when every job
+// fits it.
 struct LzPlan {
-    int block = 256;
+    int wc = 0, r = 0;
+    bool exchange = false;
+    int block = 0;
     int grid = 0;
     size_t smem = 0;
+    size_t fixed = 0;             // shared memory before the staged tile
     long long total[2] = {0, 0};
     long long slots = 0;
 };
-LzPlan lz_plan(int device, LzJob* jobs, int njobs, std::vector<long long>& prefix, int prefer_block = 0);
+LzPlan lz_plan(int device, LzJob* jobs, int njobs, std::vector<long long>& prefix, const LzShape* force = nullptr);
+// CTAs of a plan's kernel that can be resident.
+int lz_grid_size(int device, const LzPlan& P);
+bool lz_shape_fits(const DevSector& S, const LzShape& q);
+// jobs[j].st: the job's state by phase parity; prefix: as lz_plan fills it;
+// slots: [P.slots] partial sums; sync_words: lz_sync_bytes(njobs), zeroed.
+cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const LzJob* jobs, const long long* prefix,
+                                      double* slots, unsigned* sync_words, int* status, cudaStream_t s);
+// Sync-word buffer size (bytes) for a launch of njobs runs.
+size_t lz_sync_bytes(int njobs);
 // The device-free part of lz_plan: given every job's widths (ph[].width) and
 // the grid G, the phases' tile lists, CTA ranges, participants and the column
 // phase's slab order (prefix as lz_plan describes it), the tiles per phase
 // (total) and the number of partial-sum slots (returned).
 long long lz_cut(LzJob* jobs, int njobs, int G, std::vector<long long>& prefix, long long total[2]);
+// The slab order regrouped so that the slabs of a tile of several planes are neighbours.
+void lz_group_slabs(const LzJob* jobs, int njobs, int G, std::vector<long long>& prefix);
 
 // ---- edzt_host.cu: context accessors (no table building, no allocation) -----
 struct edzt_ctx;

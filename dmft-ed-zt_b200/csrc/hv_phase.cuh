@@ -28,16 +28,11 @@
 // differs (diagonal, up hops in table order, then the down-hop sum, then
 // the exchange terms).
 #pragma once
-#include "edzt_device.cuh"
+#include "hv_plane.cuh"
 
 // Padded stride of a staged line of n doubles: n rounded up to 2 (mod 4)
 // (n = 1 stays 1: a single value, loaded as a scalar).
 __host__ __device__ constexpr int phase_stride(int n) { return n <= 1 ? 1 : ((n + 1) / 4) * 4 + 2; }
-
-__device__ __forceinline__ void stage_table(const double* __restrict__ src, int n, double* dst)
-{
-    for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(src + i);
-}
 
 // Asynchronous 8-byte copy global -> shared (cp.async, no register holds the
 // value in flight, so a thread can have its whole share of a tile in flight
@@ -48,9 +43,6 @@ __device__ __forceinline__ void copy_async8(double* dst, const double* src, bool
     const int bytes = valid ? 8 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
-
-// Wait for every asynchronous copy this thread issued (the caller then syncs the CTA).
-__device__ __forceinline__ void copy_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // acc[q] += a * line[q] for q < N, two at a time (16-byte shared loads).
 template <int N>
@@ -66,25 +58,6 @@ __device__ __forceinline__ void axpy_line(double a, const double* __restrict__ l
             acc[q + 1] = fma(a, v.y, acc[q + 1]);
         }
     }
-}
-
-// The packed hop list of string t (table [hw/4][count] of uint4): its count
-// and first eight entries, loaded as one byte and two 16-byte words.  A
-// loop over strings loads the next string's list before it uses the current
-// one, so the table's latency overlaps the current string's arithmetic.
-struct HopList {
-    int hc;
-    uint4 q0, q1;
-};
-
-__device__ __forceinline__ HopList hop_list(const DevSpin& sp, int t)
-{
-    HopList L;
-    const uint4* __restrict__ hp = sp.hpk + t;
-    L.hc = __ldg(sp.hcnt + t);
-    L.q0 = (sp.hw > 0) ? __ldg(hp) : make_uint4(0u, 0u, 0u, 0u);
-    L.q1 = (sp.hw > 4) ? __ldg(hp + sp.count) : make_uint4(0u, 0u, 0u, 0u);
-    return L;
 }
 
 // Hop sum of string t over staged lines: acc[q] += amp(h) * lines[rank(h) *
@@ -200,22 +173,3 @@ __device__ __forceinline__ void col_part(const DevSector& S, const double* __res
     hop_sum<WC, WS>(S.dn, id, L, amp, ws, d, 72);
 }
 
-// Spin-flip and pair-hopping terms (impurity_hamiltonian.f90:179-226) of
-// element (id, iu) with up impurity pattern pu and down pattern pd;
-// fetch(index) returns the vector at a global index.
-template <class Fetch>
-__device__ __forceinline__ double exchange_part(const DevSector& S, int id, int iu, int pu, int pd, double acc,
-                                                Fetch fetch)
-{
-    const int P = S.P, nup = S.up.count;
-    const int pp = pu * P + pd;
-    const int nj = __ldg(S.jcnt + pp);
-    for (int t = 0; t < nj; t++) {
-        const JTrans tr = S.jt[pp * EDZT_MAX_JT + t];
-        const int iu2 = __ldg(S.up.sub + iu * P + tr.pu2);
-        const int id2 = __ldg(S.dn.sub + id * P + tr.pd2);
-        EDZT_OK_OR(iu2 >= 0 && iu2 < nup && id2 >= 0 && id2 < S.dn.count, 73, iu2, id2, pp, continue)
-        acc = fma(tr.c, fetch((long long)id2 * nup + iu2), acc);
-    }
-    return acc;
-}

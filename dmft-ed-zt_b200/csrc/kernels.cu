@@ -93,10 +93,7 @@ __global__ void __launch_bounds__(NT) k_hx_row(DevSector S, const double* __rest
     }
     copy_async_wait_all();
     __syncthreads();
-    auto fetch = [&](long long idx) {
-        EDZT_OK_OR(idx >= 0 && idx < S.dim, 61, idx, S.dim, blockIdx.x, return 0.0)
-        return __ldg(x + idx);
-    };
+    auto fetch = [&](int id2, int iu2) { return __ldg(x + (long long)id2 * nup + iu2); };
     RowCol<R> nxt{};
     if ((int)threadIdx.x < nup) nxt = row_col<R>(S, D, wsh, threadIdx.x, r0, nr);
     for (int iu = threadIdx.x; iu < nup; iu += blockDim.x) {
@@ -286,30 +283,64 @@ void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, d
 }
 
 // ---------------------------------------------------------------------------
-// Ground-state vector from kept Lanczos pairs (the eigenvector pass's sum,
+// Ground-state vector from kept Lanczos vectors (the eigenvector pass's sum,
 // src/lanczos_solver.f90:213-300, without rerunning the recurrence).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_keep_combine(const double2* __restrict__ keep, long long dim, int nstep,
-                                                      const double* __restrict__ coeff, double* __restrict__ out)
+// A run's vectors are read in storage order (lz_index), coalesced, eight of
+// them in flight per thread; the results go to the reference's order.
+// Storage position e of a run's vector as its place in the reference's order (-1: padding).
+__device__ __forceinline__ long long natural_of(unsigned e, int nup, int ndn, const int32_t* __restrict__ natu,
+                                                const int32_t* __restrict__ natd)
 {
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < dim; e += (long long)gridDim.x * blockDim.x) {
-        const double* w = reinterpret_cast<const double*>(keep + dim + e) + 1;   // w_1
-        double acc = __ldg(coeff) * __ldcs(w);
+    const unsigned ndp = (unsigned)lz_pad(ndn);
+    const unsigned slab = e / (4 * ndp), rem = e - slab * 4 * ndp;
+    const int iu = (int)(slab * 4 + ((rem >> 2) & 3)), id = (int)((rem >> 4) * 4 + (rem & 3));
+    return (iu < nup && id < ndn) ? (long long)__ldg(natd + id) * nup + __ldg(natu + iu) : -1;
+}
+
+__global__ void __launch_bounds__(256) k_keep_combine(const double* __restrict__ keep, int nup, int ndn, int nstep,
+                                                      const double* __restrict__ coeff,
+                                                      const int32_t* __restrict__ natu,
+                                                      const int32_t* __restrict__ natd, double* __restrict__ out)
+{
+    const long long stride = lz_vec_size(nup, ndn);
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < stride; e += (long long)gridDim.x * blockDim.x) {
+        const double* v = keep + e;                      // v_1
+        double acc = 0.0;
 #pragma unroll 8
-        for (int k = 2; k <= nstep; k++) acc = fma(__ldg(coeff + k - 1), __ldcs(w + 2 * (k - 1) * dim), acc);
-        out[e] = acc;
+        for (int k = 0; k < nstep; k++) acc = fma(__ldg(coeff + k), __ldcs(v + k * stride), acc);
+        const long long o = natural_of((unsigned)e, nup, ndn, natu, natd);
+        if (o >= 0) out[o] = acc;
     }
 }
 
-void launch_keep_combine(const double2* keep, long long dim, int nstep, const double* coeff, double* out,
+void launch_keep_combine(const double* keep, const DevSector& S, int nstep, const double* coeff, double* out,
                          cudaStream_t s)
 {
-    if (dim <= 0 || nstep <= 0) return;
+    if (S.dim <= 0 || nstep <= 0) return;
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const long long blocks = std::min<long long>((dim + 255) / 256, 8LL * nsm);
-    k_keep_combine<<<(unsigned)blocks, 256, 0, s>>>(keep, dim, nstep, coeff, out);
+    const long long blocks = std::min<long long>((S.dim + 255) / 256, 8LL * nsm);
+    k_keep_combine<<<(unsigned)blocks, 256, 0, s>>>(keep, S.up.count, S.dn.count, nstep, coeff, S.up.nat, S.dn.nat, out);
+}
+
+__global__ void __launch_bounds__(256) k_to_natural(const double* __restrict__ v, int nup, int ndn,
+                                                    const int32_t* __restrict__ natu, const int32_t* __restrict__ natd,
+                                                    double* __restrict__ out)
+{
+    const long long size = lz_vec_size(nup, ndn);
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < size; e += (long long)gridDim.x * blockDim.x) {
+        const long long o = natural_of((unsigned)e, nup, ndn, natu, natd);
+        if (o >= 0) out[o] = v[e];
+    }
+}
+
+void launch_to_natural(const double* v, const DevSector& S, double* out, cudaStream_t s)
+{
+    if (S.dim <= 0) return;
+    const long long blocks = std::min<long long>((S.dim + 255) / 256, 148LL * 16);
+    k_to_natural<<<(unsigned)blocks, 256, 0, s>>>(v, S.up.count, S.dn.count, S.up.nat, S.dn.nat, out);
 }
 
 // ---------------------------------------------------------------------------

@@ -10,29 +10,46 @@
 //   y_k = H w_k - b_k w_{k-1},  a_k = <w_k, y_k>,
 // with a(1..), b(1) = 0, b(k) = ||v_k|| (k >= 2) stored as they are accepted.
 //
-// A step is two phases of the whole grid, separated by grid barriers; H.v
-// is split as in hv_phase.cuh:
-//   column phase  each CTA stages slabs of whole columns of v_k (formed from
-//                 the stored pair (y_{k-1}, w_{k-1}) element by element),
-//                 sums ||v_k||^2 exactly and writes D = the down-hop part of
-//                 H v_k (not yet normalised);
+// A step is two phases; H.v is split as in hv_plane.cuh:
+//   column phase  each CTA stages slabs of whole columns of
+//                 v_k = y_{k-1} - a_{k-1} w_{k-1}, stores v_k, sums
+//                 ||v_k||^2 exactly and writes D = the down-hop part of
+//                 H v_k over y_{k-1} (its own columns);
 //   row phase     with b_k known from those sums, each CTA stages tiles of
-//                 whole rows of w_k = v_k / b_k, adds the diagonal, up-hop and
-//                 exchange parts to D / b_k, subtracts b_k w_{k-1}, stores the
-//                 pair (y_k, w_k) and sums <w_k, y_k> exactly.
-// Every neighbour value comes from shared memory, every global access is a
-// coalesced stream (pair buffers, D, the eigenvector), and both reductions
-// are exact sums, as in the reference.  The tiles of all jobs of a phase
-// form one list, cut into one contiguous range per CTA at equal modelled
-// cost (lz_plan); within a job the column slabs are numbered by round, so
-// the CTAs stage neighbouring slabs at the same time.  A job's participants
-// in a phase (the CTAs whose range meets its tiles) write one partial sum
-// each into their slot (double-buffered by step parity).  Every
-// participating CTA re-derives a job's scalars from the slots in a fixed
-// order, so all of them get the same bits; the first participant also
-// stores them.
+//                 whole rows of v_k, adds the diagonal, up-hop and exchange
+//                 parts to D, scales by 1 / b_k, subtracts b_k w_{k-1},
+//                 stores y_k over D (its own rows) and sums <w_k, y_k>.
+// Vectors are stored unnormalised (w_k = v_k / b_k is formed where it is
+// read), in the internal string order of hv_plane.cuh, as 4 x 4 blocks of
+// 128 bytes (lz_index), so that both phases move whole lines.  A run holds y
+// and the last two v: 24 bytes a state.  Every neighbour value comes from
+// shared memory, every global access is a stream, and both reductions are
+// exact sums, as in the reference.
 //
-// The pairs of a run are ping-pong buffers, or (LzJob::keep) one slot per
+// What bounds it: the load/store pipe (hop values from shared memory, 2 x 8
+// bytes a hop and state, 1.1-1.2 times the conflict-free wavefronts) and the
+// latency of staging and of the arrivals, then DRAM (64 bytes a state and
+// step once the vectors exceed L2).  Registers decide the rest: with 128 of
+// them nothing spills; 80 for half as many threads again spilled and lost a
+// sixth, tile functions called instead of inlined a third.  Measured per step
+// against slabs of the reference's string order staged as (y, w) pairs under
+// grid-wide barriers: 9 sectors of nsite 12 146 -> 124 us, 4 sectors of nsite
+// 13 280 -> 196 us, one sector of nsite 14 279 -> 212 us, of nsite 15
+// 1,092 -> 930 us, of nsite 8 13.6 -> 9.4 us.
+//
+// The tiles of all jobs of a phase form one list, cut into one contiguous
+// range per CTA at equal modelled cost (lz_plan); within a job the column
+// slabs are numbered by round, so the CTAs stage neighbouring slabs at the
+// same time.  A job's participants in a phase are the CTAs whose range meets
+// its list positions.  Jobs are synchronised one by one: a participant that has
+// finished its tiles of a phase writes its partial sum into its slot and
+// arrives on the job's counter; a participant of the next phase waits for
+// all arrivals of the earlier ones and derives the run's scalars from the
+// slots in a fixed order, so all get the same bits.  Runs do not wait for
+// one another, and a small run's phases are synchronised over its own few
+// CTAs.
+//
+// The v_k of a run are ping-pong buffers, or (LzJob::keep) one slot per
 // step, so that the eigenvector can be summed from them afterwards.  The
 // eigenvector pass (LZ_EIGVEC) instead reruns the recurrence with the stored
 // a, b (src/lanczos_solver.f90:213-300) and accumulates sum_k coeff_k w_k.
@@ -42,30 +59,20 @@
 // (derives a(k-1) and the finish test) and stores the state marked opened,
 // so a later launch, with any mix of other runs, resumes it.
 #include <algorithm>
-#include <type_traits>
 #include <cuda_runtime.h>
 #include "edzt_internal.h"
-#include "hv_phase.cuh"
+#include "hv_plane.cuh"
 
 static constexpr unsigned long long kBarrierTimeoutNs = 5ull * 1000ull * 1000ull * 1000ull;
-static constexpr int kRedDoubles = 64;
-static constexpr int kWintDoubles = EDZT_MAX_P * EDZT_MAX_P;
-static constexpr int kFixedDoubles = kRedDoubles + kWintDoubles + 2 * EDZT_MAX_AMP;
-static constexpr int kBarGroup = 16;                    // CTAs per barrier group
-static constexpr int kStageDepth = 16;                  // pair loads a thread keeps in flight when staging
+static constexpr int kMaxPlanes = 4;                    // planes of a tile
+static constexpr int kMaxRows = 8;                      // rows of a row tile
+static constexpr int kLzThreads = 512;                  // threads per SM: one CTA, or two of half as many
+static constexpr unsigned kDone = 0x80000000u;          // a job's counter word: the run has finished
 
-// sync words (unsigned), each counter on its own 128-byte line; SW_GEN is a
-// 64-bit word (barrier count << 32 | runs still going)
-#define SW_GEN 0
-#define SW_TOP 32
-#define SW_ACTIVE 64
-#define SW_GROUP(g) (128 + 32 * (g))
+size_t lz_sync_bytes(int njobs) { return sizeof(unsigned) * 32 * (size_t)njobs; }   // one 128-byte line per job
 
-size_t lz_sync_bytes(int G) { return sizeof(unsigned) * (128 + 32 * (size_t)((G + kBarGroup - 1) / kBarGroup)); }
-
-size_t lz_row_smem(int nup, int R) { return (size_t)nup * phase_stride(R) * sizeof(double); }
-size_t lz_col_smem(int ndn, int WC) { return (size_t)ndn * phase_stride(WC) * sizeof(double); }
-size_t lz_fixed_smem() { return kFixedDoubles * sizeof(double); }
+static size_t lz_row_smem(int nup, int R) { return (size_t)nup * R * sizeof(double); }
+static size_t lz_col_smem(int ndn, int WC) { return (size_t)lz_pad(ndn) * WC * sizeof(double); }
 
 __device__ __forceinline__ unsigned long long globaltimer_ns()
 {
@@ -74,72 +81,9 @@ __device__ __forceinline__ unsigned long long globaltimer_ns()
     return t;
 }
 
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p)
+__device__ __forceinline__ void red_release_add(unsigned* p, unsigned v)
 {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v)
-{
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-// Hierarchical grid barrier with a bounded wait.  Counters only grow: the
-// k-th barrier of a launch is complete on a group counter at k * (group
-// size) arrivals and on the top counter at k * (number of groups), so no
-// counter is read before arriving or reset after.  CTAs arrive on the counter
-// of their group of 16, the last of each group on the top counter, and the
-// last of all publishes (k << 32 | runs still going) in the 64-bit
-// generation word, which the others wait for.  Returns false (and the kernel
-// stops) when the wait ran out or another CTA reported an error; snap
-// receives the number of runs still going.
-__device__ bool grid_barrier(unsigned* sw, int* status, unsigned& nbar, unsigned& snap, const LzBatch& B)
-{
-    if ((int)blockIdx.x == B.stall_cta) return false;   // fault test: leave without arriving
-    const unsigned long long limit = B.wait_ns ? B.wait_ns : kBarrierTimeoutNs;
-    __shared__ int s_ok;
-    __shared__ unsigned s_snap;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const unsigned k1 = nbar + 1u;
-        const int G = gridDim.x;
-        const int g = blockIdx.x / kBarGroup;
-        const unsigned ngroups = (unsigned)((G + kBarGroup - 1) / kBarGroup);
-        const unsigned gsize = (unsigned)min(kBarGroup, G - g * kBarGroup);
-        unsigned long long* genw = reinterpret_cast<unsigned long long*>(sw + SW_GEN);
-        __threadfence();                                  // this CTA's sums and states before its arrival
-        bool last = false;
-        if (atomicAdd(sw + SW_GROUP(g), 1u) == k1 * gsize - 1u)
-            last = atomicAdd(sw + SW_TOP, 1u) == k1 * ngroups - 1u;
-        unsigned long long w;
-        if (last) {
-            const unsigned act = atomicAdd(sw + SW_ACTIVE, 0u);   // every arrival's decrements are in
-            w = ((unsigned long long)k1 << 32) | act;
-            st_release_u64(genw, w);
-        } else {
-            const unsigned long long t0 = globaltimer_ns();
-            unsigned it = 0;
-            while ((unsigned)((w = ld_acquire_u64(genw)) >> 32) < k1) {
-                if (ld_acquire_s32(status) != EDZT_DEV_OK) { ok = 0; break; }
-                if ((++it & 255u) == 0u && globaltimer_ns() - t0 > limit) {
-                    atomicCAS(status, EDZT_DEV_OK, EDZT_DEV_BARRIER_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(20);
-            }
-        }
-        __threadfence();
-        s_snap = (unsigned)w;
-        s_ok = ok && (ld_acquire_s32(status) == EDZT_DEV_OK);
-    }
-    __syncthreads();
-    nbar++;
-    snap = s_snap;
-    return s_ok != 0;
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 __device__ __forceinline__ int find_job(const long long* __restrict__ prefix, int njobs, long long t)
@@ -152,352 +96,489 @@ __device__ __forceinline__ int find_job(const long long* __restrict__ prefix, in
     return lo;
 }
 
-// Element e of the start vector of a job.
-__device__ __forceinline__ double init_value(const LzJob& J, long long e)
+// x / d from r = 1 / d, rounded as a division is: one correction of x * r by
+// its remainder (P. Markstein, IBM J. Res. Dev. 34 (1990) 111-119).
+__device__ __forceinline__ double div_by(double x, double d, double r)
 {
-    if (J.init == LZ_INIT_HASH) return edzt_u01(J.key, (uint64_t)e);
-    if (J.init == LZ_INIT_APPLYC) return apply_c_value(J.ac, J.src, e);
-    return __ldg(J.src + e);
+    const double q = x * r;
+    return fma(fma(-q, d, x), r, q);
 }
 
-// v_k at element e: the start vector for k = 1, else y_{k-1} - a_{k-1} w_{k-1}
-// from the stored pair.  Every phase and every CTA forms it with this one
-// expression, so all get the same bits.
-__device__ __forceinline__ double form_v(const LzJob& J, int k, const double2* __restrict__ pin, double am,
-                                         long long e)
+// Element (jd, ju) (internal order) of the start vector of a job.
+__device__ __forceinline__ double init_value(const LzJob& J, int jd, int ju)
 {
-    if (k == 1) return init_value(J, e);
-    const double2 pr = __ldcg(pin + e);
-    return fma(am, pr.y, pr.x);
+    if (J.init == LZ_INIT_APPLYC) return apply_c_at(J.ac, J.src, __ldg(J.S.up.str + ju), __ldg(J.S.dn.str + jd));
+    const long long e = (long long)__ldg(J.S.dn.nat + jd) * J.S.up.count + __ldg(J.S.up.nat + ju);
+    return (J.init == LZ_INIT_HASH) ? edzt_u01(J.key, (uint64_t)e) : __ldg(J.src + e);
 }
 
 // ---------------------------------------------------------------------------
 // the persistent kernel
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(512) k_lanczos(LzBatch B, const LzJob* __restrict__ jobs,
-                                                 const long long* __restrict__ prefix, double* __restrict__ slots,
-                                                 unsigned* __restrict__ sw, int* __restrict__ status)
+// A CTA's shared memory: this, the model tables, the staged tile.
+struct LzShared {
+    double red[32];                          // reduction scratch
+    double* wint;                            // [P * P] interaction energies by impurity patterns
+    double* amp_up;                          // [namp] hop amplitudes by slot
+    double* amp_dn;
+    double* dg;                              // [kMaxRows * P] a row tile's diagonal by row and up impurity pattern, less e1 of the column
+    double* chunk;                           // the staged tile
+    LzJob J;                                 // the current run
+    LzState S;                               // its state in the current phase
+    const LzJob* jobs;                       // the launch
+    const long long* slab_of;
+    double* slots;
+    unsigned* sync;
+    int* status;
+    unsigned long long wait_ns;
+    int job, phase;                          // what J and S hold
+    int ok;
+    int pd[kMaxRows];                        // a row tile's down impurity patterns
+    int c0[kMaxPlanes];                      // first column of a column tile's planes
+};
+
+// Doubles of the tables of a model: P impurity patterns a spin, namp amplitude slots.
+static int table_doubles(int P, int namp) { return P * P + 2 * namp + kMaxRows * P; }
+static size_t fixed_bytes(int tables) { return (sizeof(LzShared) + sizeof(double) * tables + 127) / 128 * 128; }
+
+extern __shared__ __align__(128) unsigned char lz_smem[];
+__device__ __forceinline__ LzShared& lz_shared() { return *reinterpret_cast<LzShared*>(lz_smem); }
+
+// Wait until a job's counter word reaches `need` arrivals or is marked done
+// (bounded: on a timeout, or when another CTA reported an error, false).
+__device__ __forceinline__ bool wait_arrivals(const unsigned* sw, unsigned need, LzShared& C, bool& done)
 {
-    extern __shared__ __align__(16) double smem[];
-    double* red = smem;                                  // reduction scratch
-    double* wint = red + kRedDoubles;                    // interaction energies by impurity patterns
-    double* amp_up = wint + kWintDoubles;                // up-spin hop amplitudes by slot
-    double* amp_dn = amp_up + EDZT_MAX_AMP;              // down-spin hop amplitudes by slot
-    double* chunk = smem + kFixedDoubles;                // the staged row tile or column slab
-    __shared__ LzJob sJ;
-    __shared__ LzState sS;
-    __shared__ int s_job;
-    __shared__ int s_resumed;
-
-    const int G = gridDim.x;
-    const int T = blockDim.x;
-    unsigned nbar = 0u;                                  // grid barriers this CTA has passed
-    if (threadIdx.x == 0) s_job = -1;
-    __syncthreads();
-
-    // participant index of this CTA in phase ph of the current job
-    auto my_q = [&](int ph) { return (int)blockIdx.x - sJ.ph[ph].part0; };
-    // this CTA's tiles of phase ph: [range[0], range[1])
-    auto my_range = [&](int ph) { return prefix + 2 * (size_t)(B.njobs + 1) + (size_t)ph * (G + 1) + blockIdx.x; };
-    // the slab that column-phase tile position t stages
-    const long long* __restrict__ slab_of = prefix + 2 * (size_t)(B.njobs + 1) + 2 * (size_t)(G + 1);
-
-
-    // Enter job j in phase p: load it if needed and derive its state.  The
-    // closing pass of a slice (closing) opens the next step only: it derives
-    // a(k-1) and the finish test of a column phase and stores the state,
-    // marked opened, under both parities for the launch that resumes it.
-    auto begin_job = [&](int j, int p, bool closing) {
-        __syncthreads();
-        if (j != s_job) {
-            const int* src = reinterpret_cast<const int*>(jobs + j);
-            int* dst = reinterpret_cast<int*>(&sJ);
-            for (int i = threadIdx.x; i < (int)(sizeof(LzJob) / sizeof(int)); i += T) dst[i] = __ldg(src + i);
-            __syncthreads();
-            stage_table(sJ.S.wint, sJ.S.P * sJ.S.P, wint);
-            stage_table(sJ.S.up.amp, sJ.S.up.namp, amp_up);
-            stage_table(sJ.S.dn.amp, sJ.S.dn.namp, amp_dn);
-            if (threadIdx.x == 0) s_job = j;
-        }
-        const int ph = p & 1;
-        // The sums of the other phase's partial-sum slots, both parities, in
-        // participant order (every thread gets them), loaded while thread 0
-        // loads the run's state: which parity applies depends on the step.
-        double ps2[2] = {0.0, 0.0};
-        {
-            const LzPhase& O = sJ.ph[ph ^ 1];
-            const double2* sl = reinterpret_cast<const double2*>(slots) + O.slot0;
-            for (int i = threadIdx.x; i < O.npart; i += T) {
-                const double2 q = __ldcg(sl + i);
-                ps2[0] += q.x;
-                ps2[1] += q.y;
+    unsigned w = ld_acquire_u32(sw);
+    if (!(w & kDone) && w < need) {
+        const unsigned long long t0 = globaltimer_ns();
+        unsigned it = 0;
+        while (w = ld_acquire_u32(sw), !(w & kDone) && w < need) {
+            if ((++it & 63u) == 0u) {
+                if (ld_acquire_s32(C.status) != EDZT_DEV_OK) return false;
+                if (globaltimer_ns() - t0 > C.wait_ns) {
+                    atomicCAS(C.status, EDZT_DEV_OK, EDZT_DEV_BARRIER_TIMEOUT);
+                    return false;
+                }
             }
         }
+    }
+    done = (w & kDone) != 0u;
+    return true;
+}
+
+// Enter job j in phase p: wait for the earlier phases' arrivals and derive
+// the run's state (one warp; the rest of the CTA waits at the barrier).
+// The closing pass of a slice (closing) opens the next step only: it derives
+// a(k-1) and the finish test of a column phase and stores the state, marked
+// opened, under both parities for the launch that resumes it.  False: an
+// error, leave the kernel.
+__device__ __forceinline__ bool begin_job(int j, int p, bool closing)
+{
+    LzShared& C = lz_shared();
+    __syncthreads();                                     // nobody reads the previous job's state any more
+    const bool same = (j == C.job);
+    if (!same) {
+        const int* src = reinterpret_cast<const int*>(C.jobs + j);
+        int* dst = reinterpret_cast<int*>(&C.J);
+        for (int i = threadIdx.x; i < (int)(sizeof(LzJob) / sizeof(int)); i += blockDim.x) dst[i] = __ldg(src + i);
+        __syncthreads();
         if (threadIdx.x == 0) {
-            const int* ss = reinterpret_cast<const int*>(sJ.st + ((p + 1) & 1));
-            int* sd = reinterpret_cast<int*>(&sS);
-            for (int i = 0; i < (int)(sizeof(LzState) / sizeof(int)); i++) sd[i] = __ldcg(ss + i);
-            s_resumed = (ph == 0 && sS.opened);          // step already opened by a closing pass
-            if (ph == 0 && !sS.opened) sS.k += 1;        // the column phase opens the next step
-            sS.opened = 0;
+            C.wint = reinterpret_cast<double*>(&C + 1);
+            C.amp_up = C.wint + C.J.S.P * C.J.S.P;
+            C.amp_dn = C.amp_up + C.J.S.up.namp;
+            C.dg = C.amp_dn + C.J.S.dn.namp;
         }
-        block_sum<2>(ps2, red);                          // ends with a CTA barrier: sS is visible
-        if (s_resumed) {
-            if (threadIdx.x == 0 && my_q(0) == 0) sJ.st[p & 1] = sS;
-            __syncthreads();
-            return;
+        __syncthreads();
+        stage_table(C.J.S.wint, C.J.S.P * C.J.S.P, C.wint);
+        stage_table(C.J.S.up.amp, C.J.S.up.namp, C.amp_up);
+        stage_table(C.J.S.dn.amp, C.J.S.dn.namp, C.amp_dn);
+    }
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x, ph = p & 1;
+        const LzPhase& O = C.J.ph[ph ^ 1];
+        unsigned* word = C.sync + 32 * (size_t)j;
+        int ok = 1, done = 0;
+        if (lane == 0 && p > 0) {
+            bool d = false;
+            const unsigned need = (unsigned)((p + 1) / 2) * C.J.ph[0].npart + (unsigned)(p / 2) * C.J.ph[1].npart;
+            ok = wait_arrivals(word, need, C, d);
+            done = d;
         }
-        const int k = sS.k;
-        const bool coeff = (sJ.mode == LZ_COEFF);
-        // sums needed: a(k-1) before a column phase, ||v_k||^2 before a row
-        // phase (the eigenvector pass takes a and b from the coefficient pass
-        // but sums ||v_init|| itself)
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        done = __shfl_sync(0xffffffffu, done, 0);
+        // the partial sums of the previous phase, in participant order
         double sum = 0.0;
-        if (sS.active && ((ph == 0 && k >= 2 && coeff) || (ph == 1 && (coeff || k == 1))))
-            sum = (ph == 0) ? ps2[(k - 1) & 1] : ps2[k & 1];
-        if (threadIdx.x == 0) {
-            const bool out = (my_q(ph) == 0);
-            LzState n = sS;
+        if (ok && !done && p > 0)
+            for (int i = lane; i < O.npart; i += 32) sum += __ldcg(C.slots + O.slot0 + i);
+        sum = warp_sum(sum);
+        if (lane == 0) {
+            if (!(same && C.phase == p - 1)) {           // else derived here in the previous phase
+                const int* ss = reinterpret_cast<const int*>(C.J.st + ((p + 1) & 1));
+                int* sd = reinterpret_cast<int*>(&C.S);
+                for (int i = 0; i < (int)(sizeof(LzState) / sizeof(int)); i++) sd[i] = __ldcg(ss + i);
+            }
+            LzState& n = C.S;
+            const bool out = ((int)blockIdx.x == C.J.ph[ph].part0);   // the job's first participant
+            const bool coeff = (C.J.mode == LZ_COEFF);
+            const bool resumed = (ph == 0 && n.opened);  // step already opened by a closing pass
+            if (ph == 0 && !n.opened) n.k += 1;          // the column phase opens the next step
+            n.opened = 0;
+            const int k = n.k;
+            if (done) n.active = 0;
             auto finish = [&](int nstep) {
                 n.active = 0;
                 n.nstep = nstep;
-                if (out) atomicSub(sw + SW_ACTIVE, 1u);
             };
-            if (n.active) {
+            if (n.active && !resumed) {
                 if (ph == 0) {
                     if (k >= 2) {                        // a(k-1) = <w, y> of the last row phase (:134,159)
-                        const double a = coeff ? sum : sJ.a[k - 2];
-                        if (out && coeff) sJ.a[k - 2] = a;
+                        const double a = coeff ? sum : C.J.a[k - 2];
+                        if (out && coeff) C.J.a[k - 2] = a;
                         n.a_prev = a;
-                        if (k - 1 >= sJ.maxnstep) finish(k - 1);          // :137-141, :161-164
+                        if (k - 1 >= C.J.maxnstep) finish(k - 1);             // :137-141, :161-164
                     } else {
                         n.a_prev = 0.0;
                     }
-                } else if (k == 1) {                     // ||v_init|| (:128-130); b(1) = 0 (:135)
-                    const double nrm = sqrt(sum);
-                    n.norm0 = nrm;
-                    n.b_cur = nrm;
-                    if (out && coeff) sJ.b[0] = 0.0;
-                    if (!(nrm > 0.0)) finish(0);         // zero start vector
-                } else {                                 // b(k) = ||v_k|| (:144,167), breakdown (:161)
-                    const double bk = coeff ? sqrt(sum) : sJ.b[k - 1];
-                    if (coeff && bk < 1.0e-16) {
-                        if (out) sJ.b[k - 1] = 0.0;
-                        finish(k - 1);
-                    } else {
-                        if (out && coeff) sJ.b[k - 1] = bk;
-                        n.b_cur = bk;
-                    }
-                }
-            }
-            if (closing && n.active) n.opened = 1;
-            if (out) {                                   // published by the barrier's fence (or the launch's end)
-                sJ.st[p & 1] = n;
-                if (closing) sJ.st[(p + 1) & 1] = n;
-            }
-            sS = n;
-        }
-        __syncthreads();
-    };
-
-    auto flush = [&](int ph, double acc) {
-        double v[1] = {acc};
-        block_sum<1>(v, red);
-        if (threadIdx.x == 0) {
-            EDZT_OK_OR(my_q(ph) < sJ.ph[ph].npart, 24, blockIdx.x, sJ.ph[ph].tile0, sJ.ph[ph].npart, return)
-            slots[(sJ.ph[ph].slot0 + my_q(ph)) * 2 + (sS.k & 1)] = v[0];
-        }
-    };
-
-    // Column phase of step k on slab tl: stage v_k on columns [c0, c0 + WC)
-    // of every row, sum v^2, write the down-hop part of H v_k into D.
-    auto col_tile = [&](auto wc_tag, int tl, double& acc) {
-        constexpr int WC = decltype(wc_tag)::value;
-        constexpr int WS = phase_stride(WC);
-        const int nup = sJ.S.up.count, ndn = sJ.S.dn.count, k = sS.k;
-        const double2* __restrict__ pin = lz_pairs(sJ, k - 1);
-        const double am = -sS.a_prev;
-        const int c0 = tl * WC;
-        double* ws = chunk;
-        const int n = ndn * WC;
-        if (k == 1) {
-            for (int i = threadIdx.x; i < n; i += T) {
-                const int id = i / WC, c = i - id * WC;
-                const double v = (c0 + c < nup) ? init_value(sJ, (long long)id * nup + c0 + c) : 0.0;
-                ws[id * WS + c] = v;
-                acc = fma(v, v, acc);
-            }
-        } else {
-            // kStageDepth pair loads in flight per thread before the first is used
-            for (int i0 = threadIdx.x; i0 < n; i0 += kStageDepth * T) {
-                double2 pr[kStageDepth];
-#pragma unroll
-                for (int q = 0; q < kStageDepth; q++) {
-                    const int i = i0 + q * T;
-                    const int id = i / WC, c = i - id * WC;
-                    pr[q] = (i < n && c0 + c < nup) ? __ldcg(pin + (long long)id * nup + c0 + c) : make_double2(0.0, 0.0);
-                }
-#pragma unroll
-                for (int q = 0; q < kStageDepth; q++) {
-                    const int i = i0 + q * T;
-                    const int id = i / WC, c = i - id * WC;
-                    if (i < n) {
-                        const double v = fma(am, pr[q].y, pr[q].x);   // form_v of the stored pair
-                        ws[id * WS + c] = v;
-                        acc = fma(v, v, acc);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        HopList nxt{};
-        if ((int)threadIdx.x < ndn) nxt = hop_list(sJ.S.dn, threadIdx.x);
-        for (int id = threadIdx.x; id < ndn; id += T) {
-            const HopList cur = nxt;                     // this row's hop list; the next one's in flight
-            if (id + T < ndn) nxt = hop_list(sJ.S.dn, id + T);
-            double d[WC];
-            col_part<WC, WS>(sJ.S, ws, amp_dn, id, cur, d);
-            store_slab_row<WC>(sJ.D, c0, ndn, id, d);   // columns past nup hold 0 (staged as 0)
-        }
-        __syncthreads();
-    };
-
-    // Row phase of step k on tile tl: stage w_k = v_k / b_k (and w_{k-1}) on
-    // rows [r0, r0 + R), finish y_k = H w_k - b_k w_{k-1}, store (y_k, w_k),
-    // sum <w_k, y_k> (or accumulate the eigenvector).
-    auto row_tile = [&](auto r_tag, int tl, double& acc) {
-        constexpr int R = decltype(r_tag)::value;
-        constexpr int RS = phase_stride(R);
-        const int nup = sJ.S.up.count, ndn = sJ.S.dn.count, k = sS.k;
-        const double2* __restrict__ pin = lz_pairs(sJ, k - 1);
-        double2* __restrict__ pout = lz_pairs(sJ, k);
-        const double am = -sS.a_prev, bk = sS.b_cur, rb = 1.0 / bk, n0 = sS.norm0;
-        const bool first = (k == 1);
-        const bool coeff = (sJ.mode == LZ_COEFF);
-        const double ck = coeff ? 0.0 : sJ.coeff[k - 1];
-        const int r0 = tl * R, nr = min(R, ndn - r0);
-        const int wsh = __ffs(sJ.ph[0].width) - 1;       // D's slab width, log2
-        double* xs = chunk;                              // [nup][RS] w_k
-        const double2* prev = first ? nullptr : pin;     // w_{k-1}: read with each column's data
-        // w at a global index, as its owner forms it (exchange terms)
-        auto fetch_w = [&](long long idx) {
-            EDZT_OK_OR(idx >= 0 && idx < sJ.S.dim, 21, idx, sJ.S.dim, k, return 0.0)
-            const double v = form_v(sJ, k, pin, am, idx);
-            return first ? v / n0 : v * rb;
-        };
-        if (first) {
-            for (int iu = threadIdx.x; iu < nup; iu += T) {
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    const long long e = (long long)(r0 + r) * nup + iu;
-                    xs[iu * RS + r] = (r < nr) ? init_value(sJ, e) / n0 : 0.0;   // the reference divides (:130)
-                }
-            }
-        } else {
-            // U columns of R rows per thread: U * R pair loads in flight before the first is used
-            constexpr int U = (kStageDepth / R) > 0 ? kStageDepth / R : 1;
-            for (int iu0 = threadIdx.x; iu0 < nup; iu0 += U * T) {
-                double2 pr[U][R];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int iu = iu0 + u * T;
-#pragma unroll
-                    for (int r = 0; r < R; r++)
-                        pr[u][r] = (iu < nup && r < nr) ? __ldcg(pin + (long long)(r0 + r) * nup + iu)
-                                                        : make_double2(0.0, 0.0);
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const int iu = iu0 + u * T;
-                    if (iu >= nup) break;
-#pragma unroll
-                    for (int r = 0; r < R; r++) xs[iu * RS + r] = fma(am, pr[u][r].y, pr[u][r].x) * rb;
-                }
-            }
-        }
-        double e1d[R];
-        int pd[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int id = min(r0 + r, ndn - 1);
-            e1d[r] = __ldg(sJ.S.dn.e1 + id);
-            pd[r] = __ldg(sJ.S.dn.imp + id);
-        }
-        __syncthreads();
-        RowCol<R> nxt{};
-        if ((int)threadIdx.x < nup) nxt = row_col<R>(sJ.S, sJ.D, wsh, threadIdx.x, r0, nr, prev);
-        for (int iu = threadIdx.x; iu < nup; iu += T) {
-            const RowCol<R> cur = nxt;                   // this column's data; the next one's in flight
-            if (iu + T < nup) nxt = row_col<R>(sJ.S, sJ.D, wsh, iu + T, r0, nr, prev);
-            double hv[R];
-            row_part<R, RS>(sJ.S, xs, wint, amp_up, iu, cur, e1d, pd, hv);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                if (r >= nr) break;
-                const long long e = (long long)(r0 + r) * nup + iu;
-                double y = hv[r] + (first ? cur.dd[r] / n0 : cur.dd[r] * rb);
-                if (sJ.S.has_j) y = exchange_part(sJ.S, r0 + r, iu, cur.pu, pd[r], y, fetch_w);
-                const double w = xs[iu * RS + r];
-                if (!first) y = fma(-bk, cur.wp[r], y);
-                __stcg(pout + e, make_double2(y, w));
-                if (coeff) {
-                    acc = fma(w, y, acc);
                 } else {
-                    double* ep = sJ.eig + e;
-                    __stcg(ep, first ? ck * w : fma(ck, w, __ldcg(ep)));
+                    n.b_prev = n.b_cur;
+                    if (k == 1) {                        // ||v_init|| (:128-130); b(1) = 0 (:135)
+                        const double nrm = sqrt(sum);
+                        n.norm0 = nrm;
+                        n.b_cur = nrm;
+                        if (out && coeff) C.J.b[0] = 0.0;
+                        if (!(nrm > 0.0)) finish(0);     // zero start vector
+                    } else {                             // b(k) = ||v_k|| (:144,167), breakdown (:161)
+                        const double bk = coeff ? sqrt(sum) : C.J.b[k - 1];
+                        if (coeff && bk < 1.0e-16) {
+                            if (out) C.J.b[k - 1] = 0.0;
+                            finish(k - 1);
+                        } else {
+                            if (out && coeff) C.J.b[k - 1] = bk;
+                            n.b_cur = bk;
+                        }
+                    }
+                }
+                if (closing && n.active) n.opened = 1;
+            }
+            if (out && !done) {                          // published by the arrival (or the launch's end)
+                C.J.st[p & 1] = n;
+                if (closing) C.J.st[(p + 1) & 1] = n;
+                if (!n.active) {
+                    __threadfence();
+                    atomicOr(word, kDone);
                 }
             }
+            C.job = j;
+            C.phase = p;
+            C.ok = ok;
         }
-        __syncthreads();
-    };
+    }
+    __syncthreads();
+    return C.ok != 0;
+}
 
-    unsigned running = 1u;
-    int p = 0;
+// Leave the current job in phase ph with this thread's share acc of the sum.
+__device__ __forceinline__ void end_job(int ph, double acc)
+{
+    LzShared& C = lz_shared();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    acc = warp_sum(acc);
+    if (lane == 0) C.red[wid] = acc;
+    __syncthreads();                                     // this CTA's stores of the phase are before it
+    if (wid == 0) {
+        double s = (lane < (int)(blockDim.x >> 5)) ? C.red[lane] : 0.0;
+        s = warp_sum(s);
+        if (lane == 0) {
+            const int q = (int)blockIdx.x - C.J.ph[ph].part0;
+            EDZT_OK_OR(q >= 0 && q < C.J.ph[ph].npart, 24, blockIdx.x, C.J.ph[ph].tile0, C.J.ph[ph].npart, return)
+            __stcg(C.slots + C.J.ph[ph].slot0 + q, s);
+            __threadfence();
+            red_release_add(C.sync + 32 * (size_t)C.job, 1u);
+        }
+    }
+}
+
+// Column phase of step k on the NP slabs of PW columns at list positions
+// t, t + 1, ...: stage v_k on their columns of every row, store it, sum v^2,
+// write the down-hop part of H v_k over y.  Returns this thread's share of
+// the sum.
+template <int PW>
+__device__ __noinline__ double col_init(int np)
+{
+    constexpr int H = PW / 2;
+    LzShared& C = lz_shared();
+    const int nup = C.J.S.up.count, ndn = C.J.S.dn.count, ndp = lz_pad(ndn), ps = ndp * PW, n = ndp * H;
+    double* ws = C.chunk;
+    double* vk = lz_v(C.J, 1);
+    double acc = 0.0;
+    for (int q = 0; q < np; q++)
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const int id = i / (4 * H) * 4 + 2 * (i & 1), cc = (i >> 1) & (PW - 1), c = C.c0[q] + cc;
+            double2 v = make_double2(0.0, 0.0);
+            if (c < nup && id < ndn) v.x = init_value(C.J, id, c);
+            if (c < nup && id + 1 < ndn) v.y = init_value(C.J, id + 1, c);
+            double* d = ws + q * ps + id * PW + cc;
+            d[0] = v.x;
+            d[PW] = v.y;
+            const unsigned o = (unsigned)(C.c0[q] / 4 * 4 * ndp) + (H == 2 ? 2u * i : (unsigned)(i / 4 * 16 + (C.c0[q] & 2) * 4 + i % 4 * 2));
+            __stcg(reinterpret_cast<double2*>(vk + o), v);
+            acc = fma(v.x, v.x, acc);
+            acc = fma(v.y, v.y, acc);
+        }
+    return acc;
+}
+
+template <int NP, int PW, int T>
+__device__ __forceinline__ double col_tile(long long t, int np)
+{
+    constexpr int H = PW / 2;
+    LzShared& C = lz_shared();
+    
+    double acc = 0.0;
+    const DevSpin& dn = C.J.S.dn;
+    const int nup = C.J.S.up.count, ndn = dn.count, k = C.S.k, ndp = lz_pad(ndn), ps = ndp * PW;
+    double* ws = C.chunk;                              // [NP][ndp][PW]
+    double* __restrict__ vk = lz_v(C.J, k);
+    double* __restrict__ yd = C.J.Y;
+    if ((int)threadIdx.x < np) C.c0[threadIdx.x] = (int)__ldg(C.slab_of + t + threadIdx.x) * PW;
+    __syncthreads();
+    // Staged item i of plane q: 16 bytes, two rows of one column.  A slab of
+    // four columns is one contiguous run of blocks (a slab of two the halves
+    // of its blocks), read and written in storage order: whole lines per warp.
+    const int n = ndp * H;
+    auto off = [&](int q, int i) {
+        return (unsigned)(C.c0[q] / 4 * 4 * ndp) + (H == 2 ? 2u * i : (unsigned)(i / 4 * 16 + (C.c0[q] & 2) * 4 + i % 4 * 2));
+    };
+    auto put = [&](int q, int i, unsigned o, double2 v) {
+        const int id = i / (4 * H) * 4 + 2 * (i & 1), cc = (i >> 1) & (PW - 1), c = C.c0[q] + cc;
+        if (c >= nup) v = make_double2(0.0, 0.0);        // the padding holds nothing
+        if (id + 1 >= ndn) {
+            v.y = 0.0;
+            if (id >= ndn) v.x = 0.0;
+        }
+        double* d = ws + q * ps + id * PW + cc;
+        d[0] = v.x;
+        d[PW] = v.y;
+        __stcg(reinterpret_cast<double2*>(vk + o), v);
+        acc = fma(v.x, v.x, acc);
+        acc = fma(v.y, v.y, acc);
+    };
+    if (k == 1) {
+        acc = col_init<PW>(np);
+    } else {
+        const double* __restrict__ vp = lz_v(C.J, k - 1);
+        const double am = -C.S.a_prev, bp = C.S.b_cur, rp = 1.0 / bp;
+        constexpr int U = 4;                     // pairs of y and of v_{k-1} in flight per thread
+#pragma unroll 1
+        for (int q = 0; q < np; q++)
+            for (int i0 = threadIdx.x; i0 < n; i0 += U * T) {
+                double2 yy[U], vv[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int i = i0 + u * T;
+                    if (i < n) {
+                        yy[u] = __ldcg(reinterpret_cast<const double2*>(yd + off(q, i)));
+                        vv[u] = __ldcg(reinterpret_cast<const double2*>(vp + off(q, i)));
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int i = i0 + u * T;
+                    if (i < n)
+                        put(q, i, off(q, i), make_double2(fma(am, div_by(vv[u].x, bp, rp), yy[u].x),
+                                                          fma(am, div_by(vv[u].y, bp, rp), yy[u].y)));
+                }
+            }
+    }
+    __syncthreads();
+    HopList nxt{};
+    const int m = ndn * H;
+    if ((int)threadIdx.x < m) nxt = hop_list(dn, threadIdx.x / H);
+    for (int i = threadIdx.x; i < m; i += T) {
+        const HopList cur = nxt;                     // this row's hop list; the next one's in flight
+        const int id = i / H;
+        if (i + T < m) nxt = hop_list(dn, (i + T) / H);
+        double2 d[NP];
+#pragma unroll
+        for (int q = 0; q < NP; q++) d[q] = make_double2(0.0, 0.0);
+        plane_hops<NP, PW>(dn, id, cur, C.amp_dn, ws + 2 * (i % H), ps, d, 72);
+#pragma unroll
+        for (int q = 0; q < NP; q++) {
+            if (q < np) {
+                double* o = yd + lz_index(id, C.c0[q] + 2 * (i % H), ndp);
+                __stcg(o, d[q].x);
+                __stcg(o + 4, d[q].y);
+            }
+        }
+    }
+    __syncthreads();
+    return acc;
+}
+
+// Row phase of step k on rows [r0, r0 + NP * PW): stage v_k, finish
+// y_k = H w_k - b_k w_{k-1}, store it over D (or also accumulate the
+// eigenvector).  Returns this thread's share of <w_k, y_k>.  X: the model has
+// exchange terms.
+template <int NP, int PW, bool X, int T>
+__device__ __forceinline__ double row_tile(int r0, int np)
+{
+    constexpr int W = NP * PW, H = PW / 2;
+    LzShared& C = lz_shared();
+    
+    double acc = 0.0;
+    const DevSpin& up = C.J.S.up;
+    const int nup = up.count, ndn = C.J.S.dn.count, k = C.S.k, ndp = lz_pad(ndn), P = C.J.S.P;
+    const double* __restrict__ vk = lz_v(C.J, k);
+    const double* __restrict__ vp = lz_v(C.J, k - 1);
+    double* __restrict__ yd = C.J.Y;
+    const double bk = C.S.b_cur, rb = 1.0 / bk, bp = C.S.b_prev, rp = (k >= 2) ? 1.0 / bp : 0.0;
+    const bool first = (k == 1);
+    const int nr = min(W, ndn - r0), ps = nup * PW;
+    double* xs = C.chunk;                              // [NP][nup][PW]
+    const int m = nup * H;
+    for (int i = threadIdx.x; i < W * P; i += T) {
+        const int r = i / P, pu = i - r * P;
+        const bool in = r < nr;
+        const int pd = in ? __ldg(C.J.S.dn.imp + r0 + r) : 0;
+        C.dg[i] = in ? __ldg(C.J.S.dn.e1 + r0 + r) + C.wint[pu * P + pd] : 0.0;
+        if (pu == 0) C.pd[r] = pd;
+    }
+    // item i: column i / H, rows r0 + 2 * (i % H) and the next of every plane
+    auto at = [&](int i) { return lz_index(r0 + 2 * (i % H), i / H, ndp); };
+    for (int i = threadIdx.x; i < m; i += T) {       // the whole tile in flight at once
+        const unsigned o = at(i);
+#pragma unroll
+        for (int p = 0; p < NP; p++)
+            if (p < np) copy_async16(xs + (size_t)p * ps + 2 * i, vk + o + 16 * p);
+    }
+    HopList nxt{};
+    double2 sn[NP], wn[NP];                          // D and v_{k-1} of the next item
+    auto load_next = [&](int i) {
+        nxt = hop_list(up, i / H);
+        const unsigned o = at(i);
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            sn[p] = wn[p] = make_double2(0.0, 0.0);
+            if (p >= np) break;
+            sn[p] = __ldcg(reinterpret_cast<const double2*>(yd + o + 16 * p));
+            wn[p] = first ? make_double2(0.0, 0.0) : __ldcg(reinterpret_cast<const double2*>(vp + o + 16 * p));
+        }
+    };
+    copy_async_wait_all();
+    __syncthreads();
+    if (C.J.mode != LZ_COEFF) {                       // eigenvector pass: += coeff_k w_k
+        const double ck = C.J.coeff[k - 1];
+        for (int i = threadIdx.x; i < m; i += T) {
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                if (p >= np) break;
+                const double2 v = *reinterpret_cast<const double2*>(xs + (size_t)p * ps + 2 * i);
+                double2* e = reinterpret_cast<double2*>(C.J.eig + at(i) + 16 * p);
+                double2 z = first ? make_double2(0.0, 0.0) : __ldcg(e);
+                z.x = fma(ck, div_by(v.x, bk, rb), z.x);
+                z.y = fma(ck, div_by(v.y, bk, rb), z.y);
+                __stcg(e, z);
+            }
+        }
+    }
+    auto fetch = [&](int id2, int iu2) { return __ldcg(vk + lz_index(id2, iu2, ndp)); };
+    for (int i = threadIdx.x; i < m; i += T) {
+        load_next(i);
+        const HopList cur = nxt;
+        double2 s[NP], e[NP];                            // e: D / b_k - b_k w_{k-1}
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            s[p] = make_double2(0.0, 0.0);
+            e[p].x = fma(-bk, div_by(wn[p].x, bp, rp), div_by(sn[p].x, bk, rb));
+            e[p].y = fma(-bk, div_by(wn[p].y, bp, rp), div_by(sn[p].y, bk, rb));
+        }
+        const int iu = i / H, h = i - iu * H;
+        const double e1u = __ldg(up.e1 + iu);
+        const int pu = __ldg(up.imp + iu);
+
+        plane_hops<NP, PW>(up, iu, cur, C.amp_up, xs + 2 * h, ps, s, 71);
+        double* out = yd + at(i);
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            if (p >= np) break;
+            const int r = p * PW + 2 * h;
+            const double2 v = *reinterpret_cast<const double2*>(xs + (size_t)p * ps + 2 * i);
+            auto row = [&](int rr, double sum, double vv, double ee) {
+                double y = fma(e1u + C.dg[rr * P + pu], vv, sum);
+                if constexpr (X) { if (C.J.S.has_j && rr < nr) y = exchange_part(C.J.S, r0 + rr, iu, pu, C.pd[rr], y, fetch); }
+                y = div_by(y, bk, rb) + ee;
+                if (rr < nr) acc = fma(div_by(vv, bk, rb), y, acc);
+                return y;
+            };
+            double2 y;
+            y.x = row(r, s[p].x, v.x, e[p].x);
+            y.y = row(r + 1, s[p].y, v.y, e[p].y);
+            __stcg(reinterpret_cast<double2*>(out + 16 * p), y);
+        }
+    }
+    __syncthreads();
+    return acc;
+}
+
+// NC, NR: planes of PW lines of a column and of a row tile; X: a model of the
+// launch has exchange terms.
+template <int NC, int NR, int PW, bool X, int T>
+__global__ void __launch_bounds__(T, kLzThreads / T) k_lanczos(LzBatch B, const LzJob* __restrict__ jobs,
+                                                           const long long* __restrict__ prefix, double* slots,
+                                                           unsigned* sync, int* status)
+{
+    LzShared& C = lz_shared();
+    const int G = gridDim.x;
+    if (threadIdx.x == 0) {
+        C.jobs = jobs;
+        C.slab_of = prefix + 2 * (size_t)(B.njobs + 1) + 2 * (size_t)(G + 1);
+        C.slots = slots;
+        C.sync = sync;
+        C.status = status;
+        C.wait_ns = B.wait_ns ? B.wait_ns : kBarrierTimeoutNs;
+        C.job = C.phase = -1;
+        C.chunk = reinterpret_cast<double*>(lz_smem + B.fixed);
+    }
+    __syncthreads();
+    // this CTA's tiles of phase ph: [range[0], range[1])
+    auto my_range = [&](int ph) { return prefix + 2 * (size_t)(B.njobs + 1) + (size_t)ph * (G + 1) + blockIdx.x; };
+    const bool stalled = (int)blockIdx.x == B.stall_cta;
+    int p = 0, idle = 0;
     for (; p < B.max_phases; p++) {
         const int ph = p & 1;
         const long long* pre = prefix + (size_t)ph * (B.njobs + 1);
-        const long long* rg = my_range(ph);
-        const long long t_end = __ldg(rg + 1);
-        int cur = -1;
-        double acc = 0.0;
-        for (long long t = __ldg(rg); t < t_end; t++) {
-            if (cur < 0 || t >= __ldg(pre + cur + 1)) {
-                if (cur >= 0 && sS.active) flush(ph, acc);
-                cur = find_job(pre, B.njobs, t);
-                begin_job(cur, p, false);
-                acc = 0.0;
-            }
-            if (!sS.active) continue;
-            const int tl = (ph == 0) ? (int)__ldg(slab_of + t) : (int)(t - sJ.ph[ph].tile0);
-            const int wdt = sJ.ph[ph].width;
-            if (ph == 0) {
-                switch (wdt) {
-                case 8: col_tile(std::integral_constant<int, 8>{}, tl, acc); break;
-                case 4: col_tile(std::integral_constant<int, 4>{}, tl, acc); break;
-                default: col_tile(std::integral_constant<int, 2>{}, tl, acc); break;
+        const long long t_end = __ldg(my_range(ph) + 1);
+        bool alive = false;
+        for (long long t = __ldg(my_range(ph)); t < t_end;) {
+            const int j = find_job(pre, B.njobs, t);
+            const long long j_end = min(t_end, __ldg(pre + j + 1));
+            if (!begin_job(j, p, false)) return;
+            if (C.S.active) {
+                alive = true;
+                const long long tile0 = C.J.ph[ph].tile0;
+                double acc = 0.0;
+                if (ph == 0) {
+#pragma unroll 1
+                    for (; t < j_end; t += NC) acc += col_tile<NC, PW, T>(t, (int)min((long long)NC, j_end - t));
+                } else {
+#pragma unroll 1
+                    for (; t < j_end; t += NR) acc += row_tile<NR, PW, X, T>((int)(t - tile0) * PW, (int)min((long long)NR, j_end - t));
                 }
-            } else {
-                switch (wdt) {
-                case 4: row_tile(std::integral_constant<int, 4>{}, tl, acc); break;
-                case 2: row_tile(std::integral_constant<int, 2>{}, tl, acc); break;
-                default: row_tile(std::integral_constant<int, 1>{}, tl, acc); break;
-                }
+                if (stalled) return;                     // fault test: leave without arriving
+                end_job(ph, acc);
             }
+            t = j_end;
         }
-        if (cur >= 0 && sS.active) flush(ph, acc);
-        if (!grid_barrier(sw, status, nbar, running, B)) return;
-        if (running == 0u) break;
+        // every run of both phases' lists has finished
+        idle = alive ? 0 : idle + 1;
+        if (idle >= 2) return;
     }
-    if (B.slice && running != 0u && p == B.max_phases) {  // budget spent: open every run's next step
-        const long long* pre = prefix;
-        const long long* rg = my_range(0);
-        const long long t_end = __ldg(rg + 1);
-        int cur = -1;
-        for (long long t = __ldg(rg); t < t_end; t++) {
-            if (cur < 0 || t >= __ldg(pre + cur + 1)) {
-                cur = find_job(pre, B.njobs, t);
-                begin_job(cur, p, true);
-            }
+    if (B.slice) {                                       // budget spent: open every run's next step
+        const long long t_end = __ldg(my_range(0) + 1);
+        for (long long t = __ldg(my_range(0)); t < t_end;) {
+            const int j = find_job(prefix, B.njobs, t);
+            if (!begin_job(j, p, true)) return;
+            t = __ldg(prefix + j + 1);
         }
     }
 }
@@ -509,98 +590,134 @@ int lz_debug_bad(long long* out4)
 }
 #endif
 
-int lz_grid_size(int device, size_t smem, int block)
+using LzKernel = void (*)(LzBatch, const LzJob*, const long long*, double*, unsigned*, int*);
+
+// The kernel of a tile shape: wc columns by r rows.
+static LzKernel lz_kernel(const LzPlan& P)
 {
-    static std::atomic<unsigned long long> attr{0};
-    if (edzt_once_per_device(attr))
-        cudaFuncSetAttribute(k_lanczos, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLzSmemMax);
+#define EDZT_LZ(c, w, nc, nr, pw)                                                                        \
+    if (P.wc == c && P.r == w) {                                                                         \
+        if (P.block == kLzThreads)                                                                       \
+            return P.exchange ? k_lanczos<nc, nr, pw, true, kLzThreads> : k_lanczos<nc, nr, pw, false, kLzThreads>; \
+        return P.exchange ? k_lanczos<nc, nr, pw, true, kLzThreads / 2> : k_lanczos<nc, nr, pw, false, kLzThreads / 2>; \
+    }
+    EDZT_LZ(16, 8, 4, 2, 4)
+    EDZT_LZ(8, 8, 2, 2, 4)
+    EDZT_LZ(8, 4, 2, 1, 4)
+    EDZT_LZ(4, 4, 1, 1, 4)
+    EDZT_LZ(2, 2, 1, 1, 2)
+#undef EDZT_LZ
+    return nullptr;
+}
+
+int lz_grid_size(int device, const LzPlan& P)
+{
     int per_sm = 0, nsm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lanczos, block, smem);
+    const LzKernel k = lz_kernel(P);
+    cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLzSmemMax);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, P.block, P.smem);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
     return per_sm * nsm;
 }
 
-cudaError_t launch_lanczos_persistent(const LzBatch& B, const LzJob* jobs, const long long* prefix, double* slots,
-                                      unsigned* sync_words, int* status, cudaStream_t s)
+cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const LzJob* jobs, const long long* prefix,
+                                      double* slots, unsigned* sync_words, int* status, cudaStream_t s)
 {
     LzBatch b = B;
+    b.grid = P.grid;
+    b.fixed = P.fixed;
     void* args[] = {(void*)&b, (void*)&jobs, (void*)&prefix, (void*)&slots, (void*)&sync_words, (void*)&status};
-    return cudaLaunchCooperativeKernel((const void*)k_lanczos, dim3(B.grid), dim3(B.block), args, B.smem, s);
+    return cudaLaunchCooperativeKernel((const void*)lz_kernel(P), dim3(P.grid), dim3(P.block), args,
+                                       P.smem, s);
 }
 
 // ---------------------------------------------------------------------------
 // launch plan
 // ---------------------------------------------------------------------------
-// Per-CTA dynamic shared memory: two CTAs of 256 threads per SM when every
-// job fits, else one CTA of 512 threads per SM.
-static constexpr size_t kLzSmemTwoPerSm = 108 * 1024;
-static constexpr int kLzLongLine = 1500;
+// Per-CTA dynamic shared memory: two 512-thread CTAs per SM when every job
+// fits, else one.
+static constexpr size_t kLzSmemTwoPerSm = 113 * 1024;
 // Fixed cost of a tile in states, for cutting the tile list into CTA ranges
-static constexpr double kLzTileCost = 1024.0;
+static constexpr double kLzTileCost = 256.0;
 
-// Width (of opts, descending) for `count` lines, each tile needing need(w)
-// bytes of the budget: with few tiles in the launch, the one that minimises
-// the lines one CTA sweeps when the job runs alone, ceil(tiles / G) * w
-// (ties to the wider); with many, the widest that fits.
-template <class Need>
-static int pick_width(const int* opts, int nopt, int count, size_t budget, int G, bool many, Need need)
-{
-    int best = -1;
-    long long best_cost = -1;
-    for (int i = 0; i < nopt; i++) {
-        const int w = opts[i];
-        if (need(w) > budget) continue;
-        if (many) return w;
-        const long long tiles = (count + w - 1) / w;
-        const long long cost = ((tiles + G - 1) / G) * w;
-        if (best < 0 || cost < best_cost) { best = w; best_cost = cost; }
-    }
-    return best < 0 ? opts[nopt - 1] : best;
-}
-
-LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, int prefer_block)
+LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, const LzShape* force)
 {
     LzPlan P;
-    int nsm = 148;
+    int tables = 0, lines_up = 0, lines_dn = 0, nsm = 148;
+    long long slabs = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-    const size_t fixed = lz_fixed_smem();
-    size_t need_min = 0;
-    long long lines8 = 0;
-    int longest = 0;
     for (int j = 0; j < nj; j++) {
-        const int nup = jobs[j].S.up.count, ndn = jobs[j].S.dn.count;
-        need_min = std::max(need_min, std::max(lz_row_smem(nup, 1), lz_col_smem(ndn, 2)));
-        lines8 += (ndn + 7) / 8 + (nup + 15) / 16;
-        longest = std::max(longest, std::max(nup, ndn));
+        const DevSector& S = jobs[j].S;
+        lines_up = std::max(lines_up, S.up.count);
+        slabs += (S.up.count + 3) / 4;
+        lines_dn = std::max(lines_dn, S.dn.count);
+        tables = std::max(tables, table_doubles(S.P, std::max(S.up.namp, S.dn.namp)));
+        P.exchange = P.exchange || S.has_j;
     }
-    // Lines of kLzLongLine strings or more (nsite >= 13 near half filling)
-    // run faster as one 512-thread CTA per SM with twice the shared memory
-    // for wider tiles (measured with the tuner: 5-35% per step at nsite
-    // 13-15, equal at 16); shorter lines as two 256-thread CTAs.
-    const bool two = fixed + need_min <= kLzSmemTwoPerSm &&
-                     (prefer_block == 256 || (longest < kLzLongLine && prefer_block != 512));
-    P.block = two ? 256 : 512;
-    const size_t budget = (two ? kLzSmemTwoPerSm : kLzSmemMax) - fixed;
-    const int G_est = (two ? 2 : 1) * nsm;
-    const bool many = lines8 >= 4LL * G_est;
-    const int ropts[3] = {4, 2, 1}, copts[3] = {8, 4, 2};
-    size_t chunk = 0;
+    P.fixed = fixed_bytes(tables);
+    auto chunk = [&](int wc, int r) { return std::max(lz_col_smem(lines_dn, wc), lz_row_smem(lines_up, r)); };
+    // The first shape that fits.  Two CTAs per SM overlap one's staging with
+    // the other's hop sums, so they come first when there are slabs enough to
+    // go round (9 sectors of nsite 12: 124 us a step, one CTA per SM 132); with
+    // few slabs one CTA per SM halves the arrivals (one sector of nsite 12: 24
+    // against 32 us, nsite 10: 11.6 against 14.4).  Wide tiles come before two
+    // CTAs: a hop is decoded once for the eight lines of a tile.
+    struct Option { int wc, r, per_sm; };
+    static const Option opts[4] = {{8, 8, 2}, {8, 8, 1}, {4, 4, 1}, {2, 2, 1}};
+    for (int i = (slabs < 4LL * nsm) ? 1 : 0; i < 4; i++) {
+        const Option& o = opts[i];
+        P.wc = o.wc;
+        P.r = o.r;
+        P.block = kLzThreads / o.per_sm;
+        P.smem = P.fixed + chunk(o.wc, o.r);
+        if (P.smem <= (o.per_sm == 2 ? kLzSmemTwoPerSm : kLzSmemMax)) break;
+    }
+    if (force && P.fixed + chunk(force->wc, force->r) <= (force->block < kLzThreads ? kLzSmemTwoPerSm : kLzSmemMax)) {
+        P.wc = force->wc;
+        P.r = force->r;
+        P.block = force->block;
+        P.smem = P.fixed + chunk(force->wc, force->r);
+    }
     for (int j = 0; j < nj; j++) {
-        LzJob& J = jobs[j];
-        const int nup = J.S.up.count, ndn = J.S.dn.count;
-        // a width preset by the tuner is kept when it fits this launch's budget
-        const int wc = J.ph[0].width, r = J.ph[1].width;
-        J.ph[0].width = (wc > 0 && lz_col_smem(ndn, wc) <= budget)
-                            ? wc : pick_width(copts, 3, nup, budget, G_est, many, [&](int w) { return lz_col_smem(ndn, w); });
-        J.ph[1].width = (r > 0 && lz_row_smem(nup, r) <= budget)
-                            ? r : pick_width(ropts, 3, ndn, budget, G_est, many, [&](int w) { return lz_row_smem(nup, w); });
-        chunk = std::max(chunk, std::max(lz_col_smem(ndn, J.ph[0].width), lz_row_smem(nup, J.ph[1].width)));
+        jobs[j].ph[0].width = jobs[j].ph[1].width = P.wc >= 4 ? 4 : 2;
+        jobs[j].ph[0].planes = P.wc / jobs[j].ph[0].width;
+        jobs[j].ph[1].planes = P.r / jobs[j].ph[1].width;
     }
-    P.smem = fixed + chunk;
-    P.grid = lz_grid_size(device, P.smem, P.block);
+    P.grid = lz_grid_size(device, P);
     if (P.grid <= 0) return P;
     P.slots = lz_cut(jobs, nj, P.grid, prefix, P.total);
+    lz_group_slabs(jobs, nj, P.grid, prefix);
     return P;
+}
+
+bool lz_shape_fits(const DevSector& S, const LzShape& q)
+{
+    const size_t need = fixed_bytes(table_doubles(S.P, std::max(S.up.namp, S.dn.namp))) +
+                        std::max(lz_col_smem(S.dn.count, q.wc), lz_row_smem(S.up.count, q.r));
+    return need <= (q.block < kLzThreads ? kLzSmemTwoPerSm : kLzSmemMax);
+}
+
+// lz_cut numbers a job's slabs by round (the r-th list position of every
+// participant side by side).  A tile of n planes takes n positions at once:
+// in every group of n full rounds the slabs are renumbered so that a
+// participant's n slabs are neighbours, and the participants' groups still
+// follow one another.
+void lz_group_slabs(const LzJob* jobs, int nj, int G, std::vector<long long>& prefix)
+{
+    const long long* range = prefix.data() + 2 * (size_t)(nj + 1);
+    long long* slab = prefix.data() + 2 * (size_t)(nj + 1) + 2 * (size_t)(G + 1);
+    for (int j = 0; j < nj; j++) {
+        const LzPhase& Q = jobs[j].ph[0];
+        const int n = Q.planes;
+        if (n <= 1) continue;
+        const long long lo = Q.tile0, hi = Q.tile0 + Q.ntiles;
+        long long full = hi - lo;                        // rounds that every participant takes part in
+        for (int q = 0; q < Q.npart; q++)
+            full = std::min(full, std::min(range[Q.part0 + q + 1], hi) - std::max(range[Q.part0 + q], lo));
+        for (long long r = 0; r < full / n * n; r++)
+            for (int q = 0; q < Q.npart; q++)
+                slab[std::max(range[Q.part0 + q], lo) + r] = r / n * n * Q.npart + (long long)q * n + r % n;
+    }
 }
 
 long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, long long total[2])

@@ -43,16 +43,14 @@ constexpr size_t kOffPrefix = kOffState + al(2 * sizeof(LzState));
 // (at most one slab per two up strings)
 constexpr size_t kOffStatus = kOffPrefix + al((4 + 2 * (kMaxGrid + 1) + EDZT_NOALLOC_MAX_DIM / 2) * sizeof(long long));
 constexpr size_t kOffSync = kOffStatus + al(sizeof(int));
-constexpr size_t kSyncBytes = al(sizeof(unsigned) * (128 + 32 * ((kMaxGrid + 15) / 16)));
-constexpr size_t kOffSlots = kOffSync + kSyncBytes;     // [2 phases * kMaxGrid][2] doubles
+constexpr size_t kSyncBytes = al(128);                  // one run's counter line
+constexpr size_t kOffSlots = kOffSync + kSyncBytes;     // [2 phases * kMaxGrid] doubles
 constexpr size_t kOffAB = kOffSlots + al(sizeof(double) * 4 * kMaxGrid);
-constexpr size_t kOffYW = kOffAB + al(sizeof(double) * 2 * EDZT_NOALLOC_MAX_STEPS);
-constexpr size_t kYWBytes = sizeof(double2) * (size_t)EDZT_NOALLOC_MAX_DIM;
-constexpr size_t kOffD = kOffYW + 2 * kYWBytes;
-// D is slab-major with slabs of up to 8 columns: up to 7 padding columns of
-// every row past the sector's own states
-constexpr size_t kDDoubles = 2 * (size_t)EDZT_NOALLOC_MAX_DIM;
-constexpr size_t kNoAllocScratchBytes = kOffD + sizeof(double) * kDDoubles;
+constexpr size_t kOffVec = kOffAB + al(sizeof(double) * 2 * EDZT_NOALLOC_MAX_STEPS);
+// y and two v, rows padded to a multiple of four columns (at most twice the
+// states, but for sectors of a single up string, which have few)
+constexpr size_t kVecDoubles = 2 * (size_t)EDZT_NOALLOC_MAX_DIM;
+constexpr size_t kNoAllocScratchBytes = kOffVec + 3 * sizeof(double) * kVecDoubles;
 
 static_assert(sizeof(LzJob) <= 2048, "job descriptor outgrew its scratch slot");
 
@@ -140,16 +138,14 @@ void run(edzt_ctx* c, int ne_up, int ne_dn, const double* v_init, int maxnstep, 
     double* d_slots = reinterpret_cast<double*>(base + kOffSlots);
     double* d_a = reinterpret_cast<double*>(base + kOffAB);
     double* d_b = d_a + EDZT_NOALLOC_MAX_STEPS;
-    double2* d_yw0 = reinterpret_cast<double2*>(base + kOffYW);
-    double2* d_yw1 = reinterpret_cast<double2*>(base + kOffYW + kYWBytes);
-    double* d_d = reinterpret_cast<double*>(base + kOffD);
+    double* d_vec = reinterpret_cast<double*>(base + kOffVec);
 
     LzJob J;
     std::memset(&J, 0, sizeof(J));
     J.S = S;
-    J.YW[0] = d_yw0;
-    J.YW[1] = d_yw1;
-    J.D = d_d;
+    J.V[0] = d_vec;
+    J.V[1] = d_vec + kVecDoubles;
+    J.Y = d_vec + 2 * kVecDoubles;
     J.a = d_a;
     J.b = d_b;
     J.maxnstep = maxnstep;
@@ -161,24 +157,21 @@ void run(edzt_ctx* c, int ne_up, int ne_dn, const double* v_init, int maxnstep, 
     const LzPlan P = lz_plan(device, &J, 1, prefix);
     if (P.grid <= 0) throw Fail{EDZT_ERR_CUDA, "persistent kernel cannot be resident (shared memory too large)"};
     if (P.grid > kMaxGrid) throw Fail{EDZT_ERR_CUDA, "persistent grid larger than the no-allocation sync area"};
-    if ((size_t)((S.up.count + J.ph[0].width - 1) / J.ph[0].width) * J.ph[0].width * S.dn.count > kDDoubles)
-        throw Fail{EDZT_ERR_ARG, "sector's column slabs exceed the no-allocation scratch"};
-    // The start vector is read in the first step only (both phases), which
-    // writes YW[1]; a host vector is staged in YW[0], first written by step 2.
+    if ((size_t)lz_vec_size(S.up.count, S.dn.count) > kVecDoubles)
+        throw Fail{EDZT_ERR_ARG, "sector's padded rows exceed the no-allocation scratch"};
+    // The start vector is read in the first column phase only, which writes
+    // V[1] and y; a host vector is staged in V[0], first written by step 2.
     if (is_device_ptr(v_init, device)) {
         J.src = v_init;
     } else {
-        NA_CK(cudaMemcpyAsync(d_yw0, v_init, sizeof(double) * S.dim, cudaMemcpyHostToDevice, st));
-        J.src = reinterpret_cast<const double*>(d_yw0);
+        NA_CK(cudaMemcpyAsync(J.V[0], v_init, sizeof(double) * S.dim, cudaMemcpyHostToDevice, st));
+        J.src = J.V[0];
     }
     LzState hs[2];
     std::memset(hs, 0, sizeof(hs));
     hs[1].active = 1;                                    // the state before phase 0 (parity 1)
-    // what must start at zero: the barrier's sync words (but the count of
-    // runs still going, one), status, a, b
-    const unsigned runs_going = 1u;
-    NA_CK(cudaMemsetAsync(d_sync, 0, lz_sync_bytes(P.grid), st));
-    NA_CK(cudaMemcpyAsync(d_sync + 64, &runs_going, sizeof(unsigned), cudaMemcpyHostToDevice, st));
+    // what must start at zero: the run's counter line, status, a, b
+    NA_CK(cudaMemsetAsync(d_sync, 0, lz_sync_bytes(1), st));
     NA_CK(cudaMemsetAsync(d_status, 0, sizeof(int), st));
     NA_CK(cudaMemsetAsync(d_a, 0, sizeof(double) * 2 * EDZT_NOALLOC_MAX_STEPS, st));
     NA_CK(cudaMemcpyAsync(d_job, &J, sizeof(J), cudaMemcpyHostToDevice, st));
@@ -187,14 +180,9 @@ void run(edzt_ctx* c, int ne_up, int ne_dn, const double* v_init, int maxnstep, 
     LzBatch B;
     std::memset(&B, 0, sizeof(B));
     B.njobs = 1;
-    B.grid = P.grid;
-    B.block = P.block;
-    B.smem = P.smem;
-    B.total[0] = P.total[0];
-    B.total[1] = P.total[1];
     B.max_phases = 2 * maxnstep + 4;
     B.stall_cta = -1;
-    NA_CK(launch_lanczos_persistent(B, d_job, d_prefix, d_slots, d_sync, d_status, st));
+    NA_CK(launch_lanczos_persistent(P, B, d_job, d_prefix, d_slots, d_sync, d_status, st));
     edzt_count_launches(c, 1);
     int status = 0;
     NA_CK(cudaMemcpyAsync(hs, d_state, sizeof(hs), cudaMemcpyDeviceToHost, st));

@@ -78,16 +78,32 @@ __device__ __forceinline__ int32_t rank_colex(uint32_t s)
     return r;
 }
 
-__global__ void k_build_strings(int nsite, int n, int count, uint32_t* __restrict__ str)
+// Internal order: the string with its norb impurity bits moved above the
+// bath bits, and back (norb = 0: the reference's order).
+__device__ __forceinline__ uint32_t imp_on_top(uint32_t u, int norb, int nsite)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < count) str[t] = unrank_colex((uint32_t)t, n, nsite);
+    return (u >> norb) | ((u & ((1u << norb) - 1u)) << (nsite - norb));
+}
+__device__ __forceinline__ uint32_t imp_below(uint32_t k, int norb, int nsite)
+{
+    const int nb = nsite - norb;
+    return ((k & ((1u << nb) - 1u)) << norb) | (k >> nb);
 }
 
-__global__ void k_build_rank(int nsite, int n, int32_t* __restrict__ rank)
+__global__ void k_build_strings(int nsite, int n, int count, int norb, uint32_t* __restrict__ str,
+                                int32_t* __restrict__ nat)
+{
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count) return;
+    const uint32_t u = imp_below(unrank_colex((uint32_t)t, n, nsite), norb, nsite);
+    str[t] = u;
+    if (nat) nat[t] = rank_colex(u);
+}
+
+__global__ void k_build_rank(int nsite, int n, int norb, int32_t* __restrict__ rank)
 {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < (1u << nsite)) rank[s] = (__popc(s) == n) ? rank_colex(s) : -1;
+    if (s < (1u << nsite)) rank[s] = (__popc(s) == n) ? rank_colex(imp_on_top(s, norb, nsite)) : -1;
 }
 
 // Per string of one spin species: one-body energy, hop list, impurity bits
@@ -153,12 +169,12 @@ int tables_debug_bad(long long* out4)
 }
 #endif
 
-void launch_build_strings(int nsite, int n, uint32_t* str, int32_t* rank, cudaStream_t s)
+void launch_build_strings(int nsite, int n, uint32_t* str, int32_t* rank, cudaStream_t s, int norb, int32_t* nat)
 {
     int count = (int)edzt_binom(nsite, n);
-    if (count > 0) k_build_strings<<<(count + 255) / 256, 256, 0, s>>>(nsite, n, count, str);
+    if (count > 0) k_build_strings<<<(count + 255) / 256, 256, 0, s>>>(nsite, n, count, norb, str, nat);
     int nst = 1 << nsite;
-    k_build_rank<<<(nst + 255) / 256, 256, 0, s>>>(nsite, n, rank);
+    k_build_rank<<<(nst + 255) / 256, 256, 0, s>>>(nsite, n, norb, rank);
 }
 
 void launch_build_spin_ops(const DevModel& m, int sigma, int count, const uint32_t* str, const int32_t* rank,
