@@ -205,7 +205,7 @@ struct LzShape {
 // the jobs' first list positions [njobs + 1], then per phase every CTA's first
 // position [grid + 1] (CTA b takes the contiguous positions [range[b],
 // range[b + 1]), cut by cost so the CTAs finish together), then the slab of
-// each column-phase position [total[0]].  force: use this shape when every job
+// each column-phase position [total[0]] and padding.  force: use this shape when every job
 // fits it.
 struct LzPlan {
     int wc = 0, r = 0;

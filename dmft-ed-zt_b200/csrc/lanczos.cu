@@ -35,7 +35,10 @@
 // against slabs of the reference's string order staged as (y, w) pairs under
 // grid-wide barriers: 9 sectors of nsite 12 146 -> 124 us, 4 sectors of nsite
 // 13 280 -> 196 us, one sector of nsite 14 279 -> 212 us, of nsite 15
-// 1,092 -> 930 us, of nsite 8 13.6 -> 9.4 us.
+// 1,092 -> 930 us, of nsite 8 13.6 -> 9.4 us.  With the hop lists of the row
+// phase loaded ahead, a CTA serving one run where that comes out even (lz_cut)
+// and no look-up of its range left in a phase: 100, 185, 202, 809 and 8.9 us,
+// 9 sectors of nsite 10 30 -> 15.
 //
 // The tiles of all jobs of a phase form one list, cut into one contiguous
 // range per CTA at equal modelled cost (lz_plan); within a job the column
@@ -59,6 +62,8 @@
 // (derives a(k-1) and the finish test) and stores the state marked opened,
 // so a later launch, with any mix of other runs, resumes it.
 #include <algorithm>
+#include <cmath>
+#include <queue>
 #include <cuda_runtime.h>
 #include "edzt_internal.h"
 #include "hv_plane.cuh"
@@ -131,6 +136,8 @@ struct LzShared {
     unsigned* sync;
     int* status;
     unsigned long long wait_ns;
+    double sum;                              // this CTA's partial sum of the last phase
+    double rb, rp;                           // 1 / S.b_cur, 1 / S.b_prev (0 before the second step)
     int job, phase;                          // what J and S hold
     int ok;
     int pd[kMaxRows];                        // a row tile's down impurity patterns
@@ -198,7 +205,10 @@ __device__ __forceinline__ bool begin_job(int j, int p, bool closing)
         const LzPhase& O = C.J.ph[ph ^ 1];
         unsigned* word = C.sync + 32 * (size_t)j;
         int ok = 1, done = 0;
-        if (lane == 0 && p > 0) {
+        // a run that only this CTA takes part in: nothing to wait for, its sum is here
+        const bool alone = same && C.phase == p - 1 && C.J.ph[0].npart == 1 && C.J.ph[1].npart == 1 &&
+                           C.J.ph[0].part0 == C.J.ph[1].part0;
+        if (lane == 0 && p > 0 && !alone) {
             bool d = false;
             const unsigned need = (unsigned)((p + 1) / 2) * C.J.ph[0].npart + (unsigned)(p / 2) * C.J.ph[1].npart;
             ok = wait_arrivals(word, need, C, d);
@@ -208,7 +218,8 @@ __device__ __forceinline__ bool begin_job(int j, int p, bool closing)
         done = __shfl_sync(0xffffffffu, done, 0);
         // the partial sums of the previous phase, in participant order
         double sum = 0.0;
-        if (ok && !done && p > 0)
+        if (alone) sum = (lane == 0) ? C.sum : 0.0;
+        else if (ok && !done && p > 0)
             for (int i = lane; i < O.npart; i += 32) sum += __ldcg(C.slots + O.slot0 + i);
         sum = warp_sum(sum);
         if (lane == 0) {
@@ -268,6 +279,8 @@ __device__ __forceinline__ bool begin_job(int j, int p, bool closing)
                     atomicOr(word, kDone);
                 }
             }
+            C.rb = 1.0 / n.b_cur;
+            C.rp = (k >= 2 && ph == 1) ? 1.0 / n.b_prev : 0.0;
             C.job = j;
             C.phase = p;
             C.ok = ok;
@@ -292,8 +305,8 @@ __device__ __forceinline__ void end_job(int ph, double acc)
             const int q = (int)blockIdx.x - C.J.ph[ph].part0;
             EDZT_OK_OR(q >= 0 && q < C.J.ph[ph].npart, 24, blockIdx.x, C.J.ph[ph].tile0, C.J.ph[ph].npart, return)
             __stcg(C.slots + C.J.ph[ph].slot0 + q, s);
-            __threadfence();
             red_release_add(C.sync + 32 * (size_t)C.job, 1u);
+            C.sum = s;
         }
     }
 }
@@ -329,7 +342,7 @@ __device__ __noinline__ double col_init(int np)
 }
 
 template <int NP, int PW, int T>
-__device__ __forceinline__ double col_tile(long long t, int np)
+__device__ __forceinline__ double col_tile(int np, int t_next)
 {
     constexpr int H = PW / 2;
     LzShared& C = lz_shared();
@@ -340,8 +353,6 @@ __device__ __forceinline__ double col_tile(long long t, int np)
     double* ws = C.chunk;                              // [NP][ndp][PW]
     double* __restrict__ vk = lz_v(C.J, k);
     double* __restrict__ yd = C.J.Y;
-    if ((int)threadIdx.x < np) C.c0[threadIdx.x] = (int)__ldg(C.slab_of + t + threadIdx.x) * PW;
-    __syncthreads();
     // Staged item i of plane q: 16 bytes, two rows of one column.  A slab of
     // four columns is one contiguous run of blocks (a slab of two the halves
     // of its blocks), read and written in storage order: whole lines per warp.
@@ -367,8 +378,8 @@ __device__ __forceinline__ double col_tile(long long t, int np)
         acc = col_init<PW>(np);
     } else {
         const double* __restrict__ vp = lz_v(C.J, k - 1);
-        const double am = -C.S.a_prev, bp = C.S.b_cur, rp = 1.0 / bp;
-        constexpr int U = 4;                     // pairs of y and of v_{k-1} in flight per thread
+        const double am = -C.S.a_prev, bp = C.S.b_cur, rp = C.rb;
+        constexpr int U = T > 256 ? 4 : 3;       // pairs of y and of v_{k-1} in flight per thread
 #pragma unroll 1
         for (int q = 0; q < np; q++)
             for (int i0 = threadIdx.x; i0 < n; i0 += U * T) {
@@ -391,6 +402,8 @@ __device__ __forceinline__ double col_tile(long long t, int np)
             }
     }
     __syncthreads();
+    // the next tile's slabs, on their way during this one's hop sums
+    const int c_next = ((int)threadIdx.x < NP) ? (int)__ldg(C.slab_of + t_next + threadIdx.x) * PW : 0;
     HopList nxt{};
     const int m = ndn * H;
     if ((int)threadIdx.x < m) nxt = hop_list(dn, threadIdx.x / H);
@@ -412,6 +425,8 @@ __device__ __forceinline__ double col_tile(long long t, int np)
         }
     }
     __syncthreads();
+    if ((int)threadIdx.x < NP) C.c0[threadIdx.x] = c_next;
+    __syncthreads();
     return acc;
 }
 
@@ -431,7 +446,7 @@ __device__ __forceinline__ double row_tile(int r0, int np)
     const double* __restrict__ vk = lz_v(C.J, k);
     const double* __restrict__ vp = lz_v(C.J, k - 1);
     double* __restrict__ yd = C.J.Y;
-    const double bk = C.S.b_cur, rb = 1.0 / bk, bp = C.S.b_prev, rp = (k >= 2) ? 1.0 / bp : 0.0;
+    const double bk = C.S.b_cur, rb = C.rb, bp = C.S.b_prev, rp = C.rp;
     const bool first = (k == 1);
     const int nr = min(W, ndn - r0), ps = nup * PW;
     double* xs = C.chunk;                              // [NP][nup][PW]
@@ -454,7 +469,6 @@ __device__ __forceinline__ double row_tile(int r0, int np)
     HopList nxt{};
     double2 sn[NP], wn[NP];                          // D and v_{k-1} of the next item
     auto load_next = [&](int i) {
-        nxt = hop_list(up, i / H);
         const unsigned o = at(i);
 #pragma unroll
         for (int p = 0; p < NP; p++) {
@@ -464,6 +478,7 @@ __device__ __forceinline__ double row_tile(int r0, int np)
             wn[p] = first ? make_double2(0.0, 0.0) : __ldcg(reinterpret_cast<const double2*>(vp + o + 16 * p));
         }
     };
+    if ((int)threadIdx.x < m) nxt = hop_list(up, threadIdx.x / H);
     copy_async_wait_all();
     __syncthreads();
     if (C.J.mode != LZ_COEFF) {                       // eigenvector pass: += coeff_k w_k
@@ -483,15 +498,12 @@ __device__ __forceinline__ double row_tile(int r0, int np)
     }
     auto fetch = [&](int id2, int iu2) { return __ldcg(vk + lz_index(id2, iu2, ndp)); };
     for (int i = threadIdx.x; i < m; i += T) {
-        load_next(i);
         const HopList cur = nxt;
-        double2 s[NP], e[NP];                            // e: D / b_k - b_k w_{k-1}
+        load_next(i);
+        if (i + T < m) nxt = hop_list(up, (i + T) / H);
+        double2 s[NP];
 #pragma unroll
-        for (int p = 0; p < NP; p++) {
-            s[p] = make_double2(0.0, 0.0);
-            e[p].x = fma(-bk, div_by(wn[p].x, bp, rp), div_by(sn[p].x, bk, rb));
-            e[p].y = fma(-bk, div_by(wn[p].y, bp, rp), div_by(sn[p].y, bk, rb));
-        }
+        for (int p = 0; p < NP; p++) s[p] = make_double2(0.0, 0.0);
         const int iu = i / H, h = i - iu * H;
         const double e1u = __ldg(up.e1 + iu);
         const int pu = __ldg(up.imp + iu);
@@ -503,16 +515,16 @@ __device__ __forceinline__ double row_tile(int r0, int np)
             if (p >= np) break;
             const int r = p * PW + 2 * h;
             const double2 v = *reinterpret_cast<const double2*>(xs + (size_t)p * ps + 2 * i);
-            auto row = [&](int rr, double sum, double vv, double ee) {
+            auto row = [&](int rr, double sum, double vv, double dd, double ww) {
                 double y = fma(e1u + C.dg[rr * P + pu], vv, sum);
                 if constexpr (X) { if (C.J.S.has_j && rr < nr) y = exchange_part(C.J.S, r0 + rr, iu, pu, C.pd[rr], y, fetch); }
-                y = div_by(y, bk, rb) + ee;
+                y = fma(-bk, div_by(ww, bp, rp), div_by(y + dd, bk, rb));
                 if (rr < nr) acc = fma(div_by(vv, bk, rb), y, acc);
                 return y;
             };
             double2 y;
-            y.x = row(r, s[p].x, v.x, e[p].x);
-            y.y = row(r + 1, s[p].y, v.y, e[p].y);
+            y.x = row(r, s[p].x, v.x, sn[p].x, wn[p].x);
+            y.y = row(r + 1, s[p].y, v.y, sn[p].y, wn[p].y);
             __stcg(reinterpret_cast<double2*>(out + 16 * p), y);
         }
     }
@@ -540,45 +552,58 @@ __global__ void __launch_bounds__(T, kLzThreads / T) k_lanczos(LzBatch B, const 
         C.chunk = reinterpret_cast<double*>(lz_smem + B.fixed);
     }
     __syncthreads();
-    // this CTA's tiles of phase ph: [range[0], range[1])
-    auto my_range = [&](int ph) { return prefix + 2 * (size_t)(B.njobs + 1) + (size_t)ph * (G + 1) + blockIdx.x; };
+    // This CTA's positions of each phase, [t0, t1), and the job of the first:
+    // looked up once, since every arrival that is waited for empties the L1.
+    const long long* range = prefix + 2 * (size_t)(B.njobs + 1);
+    const int t0c = (int)__ldg(range + blockIdx.x), t1c = (int)__ldg(range + blockIdx.x + 1);
+    const int t0r = (int)__ldg(range + G + 1 + blockIdx.x), t1r = (int)__ldg(range + G + 2 + blockIdx.x);
+    const int j0c = find_job(prefix, B.njobs, t0c), j0r = find_job(prefix + B.njobs + 1, B.njobs, t0r);
+    const int e0c = min(t1c, (int)__ldg(prefix + j0c + 1)), e0r = min(t1r, (int)__ldg(prefix + B.njobs + 2 + j0r));
+    if (threadIdx.x < NC && t0c < t1c) C.c0[threadIdx.x] = (int)__ldg(C.slab_of + t0c + threadIdx.x) * PW;
     const bool stalled = (int)blockIdx.x == B.stall_cta;
     int p = 0, idle = 0;
     for (; p < B.max_phases; p++) {
         const int ph = p & 1;
-        const long long* pre = prefix + (size_t)ph * (B.njobs + 1);
-        const long long t_end = __ldg(my_range(ph) + 1);
+        const int t_end = ph ? t1r : t1c;
+        int t = ph ? t0r : t0c, j = ph ? j0r : j0c, j_end = ph ? e0r : e0c;
         bool alive = false;
-        for (long long t = __ldg(my_range(ph)); t < t_end;) {
-            const int j = find_job(pre, B.njobs, t);
-            const long long j_end = min(t_end, __ldg(pre + j + 1));
+        while (t < t_end) {
             if (!begin_job(j, p, false)) return;
             if (C.S.active) {
                 alive = true;
-                const long long tile0 = C.J.ph[ph].tile0;
                 double acc = 0.0;
+                // a tile: the job's next list positions, one per plane
                 if (ph == 0) {
 #pragma unroll 1
-                    for (; t < j_end; t += NC) acc += col_tile<NC, PW, T>(t, (int)min((long long)NC, j_end - t));
+                    while (t < j_end) {
+                        const int np = min(NC, j_end - t);
+                        t += np;
+                        acc += col_tile<NC, PW, T>(np, t < t_end ? t : t0c);
+                    }
                 } else {
 #pragma unroll 1
-                    for (; t < j_end; t += NR) acc += row_tile<NR, PW, X, T>((int)(t - tile0) * PW, (int)min((long long)NR, j_end - t));
+                    for (; t < j_end; t += NR) acc += row_tile<NR, PW, X, T>((t - (int)C.J.ph[1].tile0) * PW, min(NR, j_end - t));
                 }
                 if (stalled) return;                     // fault test: leave without arriving
                 end_job(ph, acc);
+            } else if (ph == 0) {                        // a finished run's slabs are passed over
+                __syncthreads();
+                const int tn = j_end < t_end ? j_end : t0c;
+                if (threadIdx.x < NC) C.c0[threadIdx.x] = (int)__ldg(C.slab_of + tn + threadIdx.x) * PW;
             }
             t = j_end;
+            j++;
+            if (t < t_end) j_end = min(t_end, (int)__ldg(prefix + (ph ? B.njobs + 1 : 0) + j + 1));
         }
         // every run of both phases' lists has finished
         idle = alive ? 0 : idle + 1;
         if (idle >= 2) return;
     }
     if (B.slice) {                                       // budget spent: open every run's next step
-        const long long t_end = __ldg(my_range(0) + 1);
-        for (long long t = __ldg(my_range(0)); t < t_end;) {
-            const int j = find_job(prefix, B.njobs, t);
+        int j = j0c, j_end = e0c;
+        for (int t = t0c; t < t1c; t = j_end, j++) {
+            j_end = min(t1c, (int)__ldg(prefix + j + 1));
             if (!begin_job(j, p, true)) return;
-            t = __ldg(prefix + j + 1);
         }
     }
 }
@@ -639,54 +664,92 @@ cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const L
 static constexpr size_t kLzSmemTwoPerSm = 113 * 1024;
 // Fixed cost of a tile in states, for cutting the tile list into CTA ranges
 static constexpr double kLzTileCost = 256.0;
+// A CTA that serves two jobs in a phase reloads tables and waits twice: worth
+// this much work in states, or an uneven share of the whole
+static constexpr double kLzSwitchCost = 2000.0;
+static constexpr double kLzUneven = 1.15;
+// Time of a tile with two CTAs on the SM over its time with one
+static constexpr double kLzPairSlowdown = 1.75;
+
+// Load of the busiest CTA, both phases: passes over a tile times its lines,
+// a partly filled tile 0.8 of a pass.
+static double lz_load(const LzJob* jobs, int nj, int G, const std::vector<long long>& prefix)
+{
+    double sum = 0.0;
+    for (int ph = 0; ph < 2; ph++) {
+        const long long* range = prefix.data() + 2 * (size_t)(nj + 1) + (size_t)ph * (G + 1);
+        std::vector<double> load((size_t)G, 0.0);
+        for (int j = 0; j < nj; j++) {
+            const LzPhase& Q = jobs[j].ph[ph];
+            const int lines = (ph == 0) ? jobs[j].S.dn.count : jobs[j].S.up.count;
+            for (int b = Q.part0; b < Q.part0 + Q.npart; b++) {
+                const long long n = std::min(range[b + 1], Q.tile0 + Q.ntiles) - std::max(range[b], Q.tile0);
+                load[b] += lines * ((double)(n / Q.planes) + (n % Q.planes ? 0.8 : 0.0));
+            }
+        }
+        sum += *std::max_element(load.begin(), load.end());
+    }
+    return sum;
+}
 
 LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, const LzShape* force)
 {
     LzPlan P;
-    int tables = 0, lines_up = 0, lines_dn = 0, nsm = 148;
-    long long slabs = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+    int tables = 0, lines_up = 0, lines_dn = 0;
     for (int j = 0; j < nj; j++) {
         const DevSector& S = jobs[j].S;
         lines_up = std::max(lines_up, S.up.count);
-        slabs += (S.up.count + 3) / 4;
         lines_dn = std::max(lines_dn, S.dn.count);
         tables = std::max(tables, table_doubles(S.P, std::max(S.up.namp, S.dn.namp)));
         P.exchange = P.exchange || S.has_j;
     }
     P.fixed = fixed_bytes(tables);
     auto chunk = [&](int wc, int r) { return std::max(lz_col_smem(lines_dn, wc), lz_row_smem(lines_up, r)); };
-    // The first shape that fits.  Two CTAs per SM overlap one's staging with
-    // the other's hop sums, so they come first when there are slabs enough to
-    // go round (9 sectors of nsite 12: 124 us a step, one CTA per SM 132); with
-    // few slabs one CTA per SM halves the arrivals (one sector of nsite 12: 24
-    // against 32 us, nsite 10: 11.6 against 14.4).  Wide tiles come before two
-    // CTAs: a hop is decoded once for the eight lines of a tile.
-    struct Option { int wc, r, per_sm; };
-    static const Option opts[4] = {{8, 8, 2}, {8, 8, 1}, {4, 4, 1}, {2, 2, 1}};
-    for (int i = (slabs < 4LL * nsm) ? 1 : 0; i < 4; i++) {
-        const Option& o = opts[i];
-        P.wc = o.wc;
-        P.r = o.r;
-        P.block = kLzThreads / o.per_sm;
-        P.smem = P.fixed + chunk(o.wc, o.r);
-        if (P.smem <= (o.per_sm == 2 ? kLzSmemTwoPerSm : kLzSmemMax)) break;
+    auto shape = [&](LzPlan& Q, int wc, int r, int block) {
+        Q.wc = wc;
+        Q.r = r;
+        Q.block = block;
+        Q.smem = Q.fixed + chunk(wc, r);
+        return Q.smem <= (block < kLzThreads ? kLzSmemTwoPerSm : kLzSmemMax);
+    };
+    auto cut = [&](LzPlan& Q, std::vector<long long>& pre) {
+        for (int j = 0; j < nj; j++) {
+            jobs[j].ph[0].width = jobs[j].ph[1].width = Q.wc >= 4 ? 4 : 2;
+            jobs[j].ph[0].planes = Q.wc / jobs[j].ph[0].width;
+            jobs[j].ph[1].planes = Q.r / jobs[j].ph[1].width;
+        }
+        Q.grid = lz_grid_size(device, Q);
+        if (Q.grid <= 0) return;
+        Q.slots = lz_cut(jobs, nj, Q.grid, pre, Q.total);
+        lz_group_slabs(jobs, nj, Q.grid, pre);
+        pre.resize(pre.size() + kMaxPlanes, 0);          // the kernel reads whole tiles of slab numbers
+    };
+    LzPlan F = P;
+    if (force && shape(F, force->wc, force->r, force->block)) {
+        cut(F, prefix);
+        return F;
     }
-    if (force && P.fixed + chunk(force->wc, force->r) <= (force->block < kLzThreads ? kLzSmemTwoPerSm : kLzSmemMax)) {
-        P.wc = force->wc;
-        P.r = force->r;
-        P.block = force->block;
-        P.smem = P.fixed + chunk(force->wc, force->r);
+    // The widest tiles that fit one CTA per SM: a hop is decoded once for the
+    // lines of a tile (nsite 14: eight lines 202 us a step, four 250).  Tiles
+    // of eight lines may also run two CTAs per SM, which overlap one's staging
+    // with the other's hop sums but halve what a CTA gets through: taken when
+    // the busiest CTA's load, in passes over a tile, times kLzPairSlowdown is
+    // less than one CTA per SM has (us a step, one / two CTAs: 9 sectors of
+    // nsite 12 106 / 99, of nsite 10 18.2 / 15.5; one sector of nsite 12
+    // 23 / 31; 2 sectors of nsite 13 92 / 110).
+    if (!shape(P, 8, 8, kLzThreads) && !shape(P, 4, 4, kLzThreads)) shape(P, 2, 2, kLzThreads);
+    cut(P, prefix);
+    LzPlan Q = P;
+    if (P.wc == 8 && shape(Q, 8, 8, kLzThreads / 2)) {
+        const double one = lz_load(jobs, nj, P.grid, prefix);
+        std::vector<long long> pre;
+        cut(Q, pre);
+        if (Q.grid > P.grid && kLzPairSlowdown * lz_load(jobs, nj, Q.grid, pre) < one) {
+            prefix.swap(pre);
+            return Q;
+        }
+        cut(P, prefix);                                  // the jobs' phases of the plan that is kept
     }
-    for (int j = 0; j < nj; j++) {
-        jobs[j].ph[0].width = jobs[j].ph[1].width = P.wc >= 4 ? 4 : 2;
-        jobs[j].ph[0].planes = P.wc / jobs[j].ph[0].width;
-        jobs[j].ph[1].planes = P.r / jobs[j].ph[1].width;
-    }
-    P.grid = lz_grid_size(device, P);
-    if (P.grid <= 0) return P;
-    P.slots = lz_cut(jobs, nj, P.grid, prefix, P.total);
-    lz_group_slabs(jobs, nj, P.grid, prefix);
     return P;
 }
 
@@ -737,14 +800,18 @@ long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, lon
         const long long T = pre[nj];
         total[ph] = T;
         // CTA ranges: with no more tiles than CTAs, CTA b takes tile b; else
-        // the list is cut where the running cost crosses b/G of the total
-        // (a tile costs its states plus a fixed amount for its staging round
-        // and barriers), every CTA keeping at least one tile.
+        // each job gets CTAs in proportion to its cost (a tile costs its
+        // states plus a fixed amount for its staging round and barriers),
+        // so that a CTA serves one job and need not reload its tables or
+        // wait for two; where that leaves some CTA with much more than its
+        // share, and with more jobs than CTAs, the list is cut where the
+        // running cost crosses b/G of the total, every CTA keeping at least
+        // one tile.
         long long* range = prefix.data() + 2 * (size_t)(nj + 1) + (size_t)ph * (G + 1);
         if (T <= G) {
             for (int b = 0; b <= G; b++) range[b] = std::min<long long>(b, T);
         } else {
-            std::vector<double> cum((size_t)T + 1, 0.0);
+            std::vector<double> cost((size_t)nj, 0.0), cum((size_t)T + 1, 0.0);
             for (int j = 0; j < nj; j++) {
                 const LzPhase& Q = jobs[j].ph[ph];
                 const long long lines = (ph == 0) ? jobs[j].S.dn.count : jobs[j].S.up.count;
@@ -753,15 +820,54 @@ long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, lon
                     const int w = std::min(Q.width, count - i * Q.width);
                     cum[Q.tile0 + i + 1] = cum[Q.tile0 + i] + (double)lines * w + kLzTileCost;
                 }
+                cost[j] = cum[Q.tile0 + Q.ntiles] - cum[Q.tile0];
             }
-            range[0] = 0;
-            range[G] = T;
-            long long t = 0;
-            for (int b = 1; b < G; b++) {
-                const double target = cum[T] * b / G;
-                while (t < T && cum[t + 1] <= target) t++;
-                range[b] = std::min(std::max(t, range[b - 1] + 1), T - (G - b));
-                t = range[b];
+            std::vector<int> share;
+            double worst = HUGE_VAL;
+            if (nj <= G) {                               // CTAs one by one to the job whose CTAs have the most to do
+                share.assign((size_t)nj, 1);
+                std::priority_queue<std::pair<double, int>> load;
+                for (int j = 0; j < nj; j++) load.push({cost[j], j});
+                for (int left = G - nj; left > 0; left--) {
+                    int j = -1;
+                    std::vector<std::pair<double, int>> full;   // jobs with a CTA for every tile
+                    while (!load.empty()) {
+                        j = load.top().second;
+                        if (share[j] < jobs[j].ph[ph].ntiles) break;
+                        full.push_back(load.top());
+                        load.pop();
+                        j = -1;
+                    }
+                    if (j >= 0) {
+                        load.pop();
+                        share[j]++;
+                        load.push({cost[j] / share[j], j});
+                    }
+                    for (const auto& f : full) load.push(f);
+                    if (j < 0) break;
+                }
+                worst = 0.0;
+                for (int j = 0; j < nj; j++) {
+                    const int nt = jobs[j].ph[ph].ntiles;
+                    worst = std::max(worst, cost[j] / nt * ((nt + share[j] - 1) / share[j]));
+                }
+            }
+            if (worst <= kLzUneven * cum[T] / G + kLzSwitchCost) {
+                int b = 0;
+                for (int j = 0; j < nj; j++)
+                    for (int q = 0; q < share[j]; q++)
+                        range[b++] = jobs[j].ph[ph].tile0 + (long long)jobs[j].ph[ph].ntiles * q / share[j];
+                range[G] = T;
+            } else {
+                range[0] = 0;
+                range[G] = T;
+                long long t = 0;
+                for (int b = 1; b < G; b++) {
+                    const double target = cum[T] * b / G;
+                    while (t < T && cum[t + 1] <= target) t++;
+                    range[b] = std::min(std::max(t, range[b - 1] + 1), T - (G - b));
+                    t = range[b];
+                }
             }
         }
         // participants of a job: the CTAs whose range meets its tiles (a contiguous run)
