@@ -89,10 +89,18 @@ class Pool {
         free_.emplace(it->second, p);
         used_.erase(it);
     }
-    void trim()
+    void trim() { trim_to(0); }
+    // Give cached blocks back, the largest first, until at most `keep` bytes stay cached.
+    void trim_to(size_t keep)
     {
-        for (auto& kv : free_) cudaFree(kv.second);
-        free_.clear();
+        size_t cached = 0;
+        for (const auto& kv : free_) cached += kv.first;
+        while (cached > keep && !free_.empty()) {
+            auto it = std::prev(free_.end());
+            cached -= it->first;
+            cudaFree(it->second);
+            free_.erase(it);
+        }
     }
     void release_all()
     {
@@ -166,9 +174,15 @@ struct StrTable {
     std::unique_ptr<DevBuf> nat;            // internal order only: ranks in the reference's order
 };
 
+// One block of the context's pool per table (a cudaMalloc and cudaFree of six
+// buffers a table made up half of a small solve's time).
 struct OpsTable {
     int hw = 0, namp = 0;
-    std::unique_ptr<DevBuf> e1, hcnt, hpk, amp, imp, sub;
+    Lease<char> block;
+    double *e1 = nullptr, *amp = nullptr;
+    uint4* hpk = nullptr;
+    int32_t* sub = nullptr;
+    uint8_t *hcnt = nullptr, *imp = nullptr;
 };
 
 // The model-dependent tables of one impurity model: per-spin operator tables
@@ -181,7 +195,11 @@ struct ModelTables {
     bool has_j = false;
     std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> ops;    // strings in the reference's order
     std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> iops;   // strings in internal order
-    std::unique_ptr<DevBuf> wint, jcnt, jt;
+    std::vector<char> host;                 // wint, jcnt and jt as uploaded
+    Lease<char> block;                      // the same on the device
+    double* wint = nullptr;
+    int* jcnt = nullptr;
+    JTrans* jt = nullptr;
 };
 
 }  // namespace
@@ -205,8 +223,9 @@ struct edzt_ctx {
     int gs_up = 0, gs_dn = 0, gs_isector = -1;
     double gs_e0 = 0.0, gs_residual = 0.0;
     Lease<double> gs_vec;
-    // persistent-kernel scratch
-    std::unique_ptr<DevBuf> sync_words, status;
+    // pinned host buffer for what a launch of the persistent kernel copies in and out
+    char* stage = nullptr;
+    size_t stage_bytes = 0;
     // persistent-kernel statistics
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     long long st_launches = 0;
@@ -277,16 +296,25 @@ OpsTable& ops_table_mt(edzt_ctx* c, ModelTables& mt, int n, int sigma, bool inte
     t->hw = std::max(4, (maxh + 3) / 4 * 4);
     t->namp = std::max(2, 2 * norb * nbath);
     const size_t cnt = (size_t)std::max(st.count, 1);
-    t->e1 = std::make_unique<DevBuf>(sizeof(double) * cnt);
-    t->hcnt = std::make_unique<DevBuf>(cnt);
-    t->hpk = std::make_unique<DevBuf>(sizeof(uint32_t) * cnt * t->hw);
-    t->amp = std::make_unique<DevBuf>(sizeof(double) * t->namp);
-    t->imp = std::make_unique<DevBuf>(cnt);
-    if (mt.has_j) t->sub = std::make_unique<DevBuf>(sizeof(int32_t) * cnt * mt.P);
-    launch_build_spin_ops(mt.model, sigma, st.count, st.str->as<uint32_t>(), st.rank->as<int32_t>(), t->hw,
-                          t->e1->as<double>(), t->hcnt->as<uint8_t>(), t->hpk->as<uint32_t>(),
-                          t->amp->as<double>(), t->imp->as<uint8_t>(), t->sub ? t->sub->as<int32_t>() : nullptr,
-                          c->stream);
+    size_t size = 0;
+    auto part = [&](size_t bytes) {
+        const size_t o = size;
+        size += (bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    const size_t o_e1 = part(sizeof(double) * cnt), o_hpk = part(sizeof(uint32_t) * cnt * t->hw);
+    const size_t o_amp = part(sizeof(double) * t->namp), o_hcnt = part(cnt), o_imp = part(cnt);
+    const size_t o_sub = part(mt.has_j ? sizeof(int32_t) * cnt * mt.P : 0);
+    t->block = Lease<char>(c->pool, size);
+    char* d = t->block.p;
+    t->e1 = reinterpret_cast<double*>(d + o_e1);
+    t->hpk = reinterpret_cast<uint4*>(d + o_hpk);
+    t->amp = reinterpret_cast<double*>(d + o_amp);
+    t->hcnt = reinterpret_cast<uint8_t*>(d + o_hcnt);
+    t->imp = reinterpret_cast<uint8_t*>(d + o_imp);
+    t->sub = mt.has_j ? reinterpret_cast<int32_t*>(d + o_sub) : nullptr;
+    launch_build_spin_ops(mt.model, sigma, st.count, st.str->as<uint32_t>(), st.rank->as<int32_t>(), t->hw, t->e1,
+                          t->hcnt, reinterpret_cast<uint32_t*>(t->hpk), t->amp, t->imp, t->sub, c->stream);
     c->launches += 1;
     CKLAUNCH();
     ref = std::move(t);
@@ -321,12 +349,12 @@ DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd, bool inte
         sp.namp = o.namp;
         sp.str = st.str->as<uint32_t>();
         sp.rank = st.rank->as<int32_t>();
-        sp.e1 = o.e1->as<double>();
-        sp.hcnt = o.hcnt->as<uint8_t>();
-        sp.hpk = o.hpk->as<uint4>();
-        sp.amp = o.amp->as<double>();
-        sp.imp = o.imp->as<uint8_t>();
-        sp.sub = o.sub ? o.sub->as<int32_t>() : nullptr;
+        sp.e1 = o.e1;
+        sp.hcnt = o.hcnt;
+        sp.hpk = o.hpk;
+        sp.amp = o.amp;
+        sp.imp = o.imp;
+        sp.sub = o.sub;
         sp.nat = st.nat ? st.nat->as<int32_t>() : nullptr;
     };
     fill(S.up, su, ou);
@@ -338,9 +366,9 @@ DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd, bool inte
               "beyond nsite 16 at half filling)");
     S.P = mt.P;
     S.has_j = mt.has_j ? 1 : 0;
-    S.wint = mt.wint->as<double>();
-    S.jcnt = mt.jcnt->as<int>();
-    S.jt = mt.jt->as<JTrans>();
+    S.wint = mt.wint;
+    S.jcnt = mt.jcnt;
+    S.jt = mt.jt;
     return S;
 }
 
@@ -356,7 +384,7 @@ DevSector make_sector(edzt_ctx* c, int nu, int nd)
 // Interaction tables over impurity occupation patterns (pu, pd).
 // wint: impurity_hamiltonian.f90:119-141 without the em-mu terms (those are
 // one-body and live in e1).  Exchange transitions: :179-226.
-void build_model_tables(ModelTables& mt, cudaStream_t stream)
+void build_model_tables(edzt_ctx* c, ModelTables& mt)
 {
     const DevModel& m = mt.model;
     const int norb = m.norb, P = 1 << norb;
@@ -408,13 +436,16 @@ void build_model_tables(ModelTables& mt, cudaStream_t stream)
             any_j = any_j || cnt > 0;
         }
     mt.has_j = any_j;
-    mt.wint = std::make_unique<DevBuf>(sizeof(double) * P * P);
-    mt.jcnt = std::make_unique<DevBuf>(sizeof(int) * P * P);
-    mt.jt = std::make_unique<DevBuf>(sizeof(JTrans) * jt.size());
-    CK(cudaMemcpyAsync(mt.wint->p, w.data(), sizeof(double) * P * P, cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(mt.jcnt->p, jc.data(), sizeof(int) * P * P, cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(mt.jt->p, jt.data(), sizeof(JTrans) * jt.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));      // the host vectors go out of scope
+    const size_t nw = sizeof(double) * P * P, nj = sizeof(JTrans) * jt.size();   // 8-byte multiples, jcnt last
+    mt.host.resize(nw + nj + sizeof(int) * P * P);
+    std::memcpy(mt.host.data(), w.data(), nw);
+    std::memcpy(mt.host.data() + nw, jt.data(), nj);
+    std::memcpy(mt.host.data() + nw + nj, jc.data(), sizeof(int) * P * P);
+    mt.block = Lease<char>(c->pool, mt.host.size());
+    mt.wint = reinterpret_cast<double*>(mt.block.p);
+    mt.jt = reinterpret_cast<JTrans*>(mt.block.p + nw);
+    mt.jcnt = reinterpret_cast<int*>(mt.block.p + nw + nj);
+    CK(cudaMemcpyAsync(mt.block.p, mt.host.data(), mt.host.size(), cudaMemcpyHostToDevice, c->stream));
 }
 
 // The reference's em(norb,2), ek(nbath,2), vmk(norb,nbath,2) (column-major) as a DevModel.
@@ -444,12 +475,12 @@ DevModel model_from(int norb, int nbath, const double* em, const double* ek, con
     return m;
 }
 
-void set_tables_model(ModelTables& mt, const DevModel& m, cudaStream_t stream)
+void set_tables_model(edzt_ctx* c, ModelTables& mt, const DevModel& m)
 {
     mt.ops.clear();
     mt.iops.clear();
     mt.model = m;
-    build_model_tables(mt, stream);
+    build_model_tables(c, mt);
     mt.valid = true;
 }
 
@@ -493,6 +524,14 @@ struct OutVec {
         }
     }
 };
+
+// Host data to a caller's host or device buffer.
+void put_out(edzt_ctx* c, void* dst, const void* src, size_t bytes)
+{
+    if (!dst || bytes == 0) return;
+    if (is_device_ptr(dst, c->device)) CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, c->stream));
+    else std::memcpy(dst, src, bytes);
+}
 
 void copy_out(edzt_ctx* c, void* dst, const void* src, size_t bytes)
 {
@@ -564,6 +603,90 @@ void fill_job(LzJob& J, const JobSpec& s, const DevSector& S)
     J.src = s.ac_src;
 }
 
+// At least `bytes` of the context's pinned staging buffer; its last use is over
+// (every launch ends with a stream synchronisation).
+char* stage_buffer(edzt_ctx* c, size_t bytes)
+{
+    if (bytes > c->stage_bytes) {
+        if (c->stage) cudaFreeHost(c->stage);
+        c->stage = nullptr;
+        c->stage_bytes = 0;
+        const size_t want = std::max<size_t>(bytes + bytes / 2, 64 * 1024);
+        CK(cudaMallocHost((void**)&c->stage, want));
+        c->stage_bytes = want;
+    }
+    return c->stage;
+}
+
+// One launch of the persistent kernel over `jobs`, whose states st [2 per job]
+// go in and come back.  Everything the launch needs goes up in one copy, and
+// states and status come back in one.  Returns the device time in ms.
+float launch_jobs(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& st, const LzShape* shape,
+                  int max_phases, bool slice)
+{
+    const int nj = (int)jobs.size();
+    std::vector<long long> prefix;
+    const LzPlan P = lz_plan(c->device, jobs.data(), nj, prefix, shape);
+    if (P.grid <= 0) throw EdztError{EDZT_ERR_CUDA, "persistent kernel cannot be resident (shared memory too large)"};
+    size_t size = 0;
+    auto part = [&](size_t bytes) {
+        const size_t o = size;
+        size += (bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    const size_t bytes_jobs = sizeof(LzJob) * nj, bytes_st = sizeof(LzState) * st.size();
+    const size_t bytes_pre = sizeof(long long) * prefix.size(), bytes_sw = lz_sync_bytes(nj);
+    const size_t o_jobs = part(bytes_jobs), o_pre = part(bytes_pre), o_sw = part(bytes_sw);
+    const size_t o_st = part(bytes_st + sizeof(int)), o_status = o_st + bytes_st, up = size;
+    const size_t o_slots = part(sizeof(double) * (size_t)P.slots);
+    Lease<char> blob(c->pool, size);
+    char* d = blob.p;
+    for (int j = 0; j < nj; j++) jobs[j].st = reinterpret_cast<LzState*>(d + o_st) + 2 * (size_t)j;
+    char* h = stage_buffer(c, up);
+    std::memcpy(h + o_jobs, jobs.data(), bytes_jobs);
+    std::memcpy(h + o_pre, prefix.data(), bytes_pre);
+    std::memset(h + o_sw, 0, bytes_sw);
+    std::memcpy(h + o_st, st.data(), bytes_st);
+    std::memset(h + o_status, 0, sizeof(int));
+    CK(cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, c->stream));
+    LzBatch B;
+    std::memset(&B, 0, sizeof(B));
+    B.njobs = nj;
+    B.max_phases = max_phases;
+    B.wait_ns = c->dbg_wait_ns;
+    B.stall_cta = c->dbg_stall_cta;
+    B.slice = slice ? 1 : 0;
+    CK(cudaEventRecord(c->ev0, c->stream));
+    CK(launch_lanczos_persistent(P, B, reinterpret_cast<LzJob*>(d + o_jobs), reinterpret_cast<long long*>(d + o_pre),
+                                 reinterpret_cast<double*>(d + o_slots), reinterpret_cast<unsigned*>(d + o_sw),
+                                 reinterpret_cast<int*>(d + o_status), c->stream));
+    CK(cudaEventRecord(c->ev1, c->stream));
+    c->launches += 1;
+    CK(cudaMemcpyAsync(h + o_st, d + o_st, bytes_st + sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    int status = 0;
+    std::memcpy(st.data(), h + o_st, bytes_st);
+    std::memcpy(&status, h + o_status, sizeof(int));
+    if (status == EDZT_DEV_BARRIER_TIMEOUT)
+        throw EdztError{EDZT_ERR_TIMEOUT, "persistent Lanczos kernel: the wait for a run's arrivals timed out"};
+    if (status != 0) throw EdztError{EDZT_ERR_CUDA, "persistent Lanczos kernel reported status " + std::to_string(status)};
+    float ms = 0.0f;
+    CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+    return ms;
+}
+
+void book_launch(edzt_ctx* c, const std::vector<LzJob>& jobs, double ms, double bytes)
+{
+    c->st_launches += 1;
+    c->st_ms += ms;
+    c->st_bytes += bytes;
+    double states = 0.0;
+    for (const LzJob& J : jobs) states += (double)J.S.dim;
+    log_launch(c, ms, bytes, states);
+}
+
+// All runs of specs from start to finish.  Coefficient runs write a and b up
+// to their last step only: the caller zeroes them.
 void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = nullptr)
 {
     const int nj = (int)specs.size();
@@ -589,55 +712,13 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
             J.V[1] = vec();
         }
         max_steps = std::max(max_steps, J.maxnstep);
-        if (s.mode == LZ_COEFF) {
-            CK(cudaMemsetAsync(s.a, 0, sizeof(double) * s.maxnstep, c->stream));
-            CK(cudaMemsetAsync(s.b, 0, sizeof(double) * s.maxnstep, c->stream));
-        }
     }
-    // the tile shape (tuned, else by lz_plan's rule), the lists of both
-    // phases, grid and shared memory
-    std::vector<long long> prefix;
-    const LzPlan P = lz_plan(c->device, jobs.data(), nj, prefix, force ? force : tuned_shape(c, jobs));
-    if (P.grid <= 0) throw EdztError{EDZT_ERR_CUDA, "persistent kernel cannot be resident (shared memory too large)"};
     std::vector<LzState> st(2 * (size_t)nj);
     std::memset(st.data(), 0, sizeof(LzState) * st.size());
     for (int j = 0; j < nj; j++) st[2 * (size_t)j + 1].active = 1;   // the state before phase 0 (parity 1)
-    const size_t bytes_jobs = sizeof(LzJob) * nj, bytes_st = sizeof(LzState) * st.size();
-    const size_t bytes_pre = sizeof(long long) * prefix.size(), bytes_slots = sizeof(double) * (size_t)P.slots;
-    const size_t bytes_sw = lz_sync_bytes(nj);
-    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t total = al(bytes_jobs) + al(bytes_st) + al(bytes_pre) + al(bytes_slots) + al(bytes_sw);
-    Lease<char> blob(c->pool, total);
-    char* base = blob.p;
-    LzJob* d_jobs = reinterpret_cast<LzJob*>(base);
-    LzState* d_st = reinterpret_cast<LzState*>(base + al(bytes_jobs));
-    long long* d_pre = reinterpret_cast<long long*>(base + al(bytes_jobs) + al(bytes_st));
-    double* d_slots = reinterpret_cast<double*>(base + al(bytes_jobs) + al(bytes_st) + al(bytes_pre));
-    unsigned* d_sw = reinterpret_cast<unsigned*>(base + al(bytes_jobs) + al(bytes_st) + al(bytes_pre) + al(bytes_slots));
-    for (int j = 0; j < nj; j++) jobs[j].st = d_st + 2 * (size_t)j;
-    CK(cudaMemcpyAsync(d_jobs, jobs.data(), bytes_jobs, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(d_st, st.data(), bytes_st, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(d_pre, prefix.data(), bytes_pre, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemsetAsync(d_sw, 0, bytes_sw, c->stream));
-    CK(cudaMemsetAsync(c->status->p, 0, sizeof(int), c->stream));
-    LzBatch B;
-    std::memset(&B, 0, sizeof(B));
-    B.njobs = nj;
-    B.max_phases = 2 * max_steps + 4;   // two phases per step and the phase that closes the last one
-    if (c->dbg_pass_cap > 0) B.max_phases = std::min(B.max_phases, c->dbg_pass_cap);
-    B.wait_ns = c->dbg_wait_ns;
-    B.stall_cta = c->dbg_stall_cta;
-    CK(cudaEventRecord(c->ev0, c->stream));
-    CK(launch_lanczos_persistent(P, B, d_jobs, d_pre, d_slots, d_sw, c->status->as<int>(), c->stream));
-    CK(cudaEventRecord(c->ev1, c->stream));
-    c->launches += 1;
-    int status = 0;
-    CK(cudaMemcpyAsync(st.data(), d_st, bytes_st, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(&status, c->status->p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (status == EDZT_DEV_BARRIER_TIMEOUT)
-        throw EdztError{EDZT_ERR_TIMEOUT, "persistent Lanczos kernel: grid barrier wait timed out"};
-    if (status != 0) throw EdztError{EDZT_ERR_CUDA, "persistent Lanczos kernel reported status " + std::to_string(status)};
+    int phases = 2 * max_steps + 4;     // two phases per step and the phase that closes the last one
+    if (c->dbg_pass_cap > 0) phases = std::min(phases, c->dbg_pass_cap);
+    const float ms = launch_jobs(c, jobs, st, force ? force : tuned_shape(c, jobs), phases, false);
     double bytes = 0.0;
     for (int j = 0; j < nj; j++) {
         // the final state is the finished one of the two parity copies
@@ -652,14 +733,7 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
         const double per_step = (specs[j].mode == LZ_COEFF) ? 24.0 : 40.0;
         bytes += dim * (init + per_step * specs[j].nstep);
     }
-    float ms = 0.0f;
-    CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-    c->st_launches += 1;
-    c->st_ms += ms;
-    c->st_bytes += bytes;
-    double states = 0.0;
-    for (int j = 0; j < nj; j++) states += (double)jobs[j].S.dim;
-    log_launch(c, ms, bytes, states);
+    book_launch(c, jobs, ms, bytes);
 }
 
 // ---------------------------------------------------------------------------
@@ -778,16 +852,22 @@ void check_sector(edzt_ctx* c, int nu, int nd)
 }
 
 // Normalise the eigenvector and compute |H g - E g|^2 (lanczos_solver.f90:291-297).
-double finish_eigvec(edzt_ctx* c, const DevSector& S, double* vec, double e0)
+void normalise(edzt_ctx* c, double* vec, long long n)
 {
-    const long long n = S.dim;
     double* sc = c->scal->as<double>();
     launch_dot(vec, vec, n, c->dot_part->as<double>(), sc, c->stream);
     launch_scale_inv_sqrt(vec, n, sc, c->stream);                              // :291
+    c->launches += 3;
+}
+
+double finish_eigvec(edzt_ctx* c, const DevSector& S, double* vec, double e0)
+{
+    const long long n = S.dim;
+    normalise(c, vec, n);
     Lease<double> v(c->pool, (size_t)n), hs(c->pool, (size_t)hx_scratch_size(S.up.count, S.dn.count));
     launch_hx(S, vec, v.p, 0, hs.p, c->stream);
     launch_axpy(v.p, vec, n, nullptr, e0, -1.0, c->stream);
-    c->launches += 7;
+    c->launches += 3;
     CKLAUNCH();
     return plain_dot(c, v.p, v.p, n);
 }
@@ -978,6 +1058,24 @@ void diag_arpack_impl(edzt_ctx* c, const DevSector& S, uint64_t key, double* vec
     R.eigval = theta[0];
 }
 
+// f(0) ... f(n - 1) on the host's threads, a thread for every per_thread of them.
+template <class F>
+void parallel_for(int n, int per_thread, F&& f)
+{
+    const int nt = std::max(1, std::min(n / per_thread, (int)std::thread::hardware_concurrency()));
+    if (nt == 1) {
+        for (int i = 0; i < n; i++) f(i);
+        return;
+    }
+    std::atomic<int> next{0};
+    std::vector<std::thread> th;
+    for (int t = 0; t < nt; t++)
+        th.emplace_back([&] {
+            for (int i = next++; i < n; i = next++) f(i);
+        });
+    for (auto& x : th) x.join();
+}
+
 struct SectorResult {
     int nstep = 0;
     double norm0 = 0.0;
@@ -1021,8 +1119,10 @@ void ground_state_arpack(edzt_ctx* c, int nsector, const int* sectors, uint64_t 
 }
 
 // streams (nullable): start-vector stream of each sector; default stream i for sector i.
+// want_residual: also |H g - E g|^2 of the result (only diag_lanczos returns it).
 void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnstep, uint64_t seed, int* isector,
-                       double* e0, double* gsvec, double* e_sector, const uint64_t* streams = nullptr)
+                       double* e0, double* gsvec, double* e_sector, const uint64_t* streams = nullptr,
+                       bool want_residual = false)
 {
     auto stream_of = [&](int i) { return streams ? streams[i] : (uint64_t)i; };
     require_model(c);
@@ -1054,6 +1154,7 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
         std::vector<JobSpec> specs;
         std::vector<int> which;
         Lease<double> ab(c->pool, (size_t)nsector * 2 * maxnstep);
+        CK(cudaMemsetAsync(ab.p, 0, sizeof(double) * (size_t)nsector * 2 * maxnstep, c->stream));
         for (int i = 0; i < nsector; i++) {
             const int nu = sectors[2 * i], nd = sectors[2 * i + 1];
             if (sector_dim(c, nu, nd) <= 0) continue;
@@ -1073,21 +1174,22 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             which.push_back(i);
         }
         run_jobs(c, specs);
-        std::vector<double> hab((size_t)nsector * 2 * maxnstep);
-        CK(cudaMemcpyAsync(hab.data(), ab.p, sizeof(double) * hab.size(), cudaMemcpyDeviceToHost, c->stream));
+        const size_t n_ab = (size_t)nsector * 2 * maxnstep;
+        double* hab = reinterpret_cast<double*>(stage_buffer(c, sizeof(double) * n_ab));
+        CK(cudaMemcpyAsync(hab, ab.p, sizeof(double) * n_ab, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
-        for (size_t q = 0; q < specs.size(); q++) {
+        parallel_for((int)specs.size(), 1 + 2000 / maxnstep, [&](int q) {
             const int i = which[q];
             SectorResult& r = res[i];
             r.nstep = specs[q].nstep;
             r.norm0 = specs[q].norm0;
-            r.a.assign(hab.begin() + (size_t)(2 * i) * maxnstep, hab.begin() + (size_t)(2 * i + 1) * maxnstep);
-            r.b.assign(hab.begin() + (size_t)(2 * i + 1) * maxnstep, hab.begin() + (size_t)(2 * i + 2) * maxnstep);
+            r.a.assign(hab + (size_t)(2 * i) * maxnstep, hab + (size_t)(2 * i + 1) * maxnstep);
+            r.b.assign(hab + (size_t)(2 * i + 1) * maxnstep, hab + (size_t)(2 * i + 2) * maxnstep);
             if (r.nstep >= 1) {
                 r.coeff.resize(r.nstep);
                 r.ok = edzt::lowest_eigenpair(r.nstep, r.a.data(), r.b.data(), &r.e, r.coeff.data()) == 0;
             }
-        }
+        });
     }
     // selection (ground_state.f90:62-68), strict with a 1e-10 relative tie band
     int best = -1;
@@ -1136,8 +1238,9 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             CKLAUNCH();
         }
         for (auto& k : kept) k = Lease<double>();
-        DevSector S = make_sector(c, nu, nd);
-        c->gs_residual = finish_eigvec(c, S, c->gs_vec.p, r.e);
+        if (want_residual) c->gs_residual = finish_eigvec(c, make_sector(c, nu, nd), c->gs_vec.p, r.e);
+        else normalise(c, c->gs_vec.p, dim);
+        CKLAUNCH();
         c->gs_up = nu; c->gs_dn = nd; c->gs_isector = best; c->gs_e0 = r.e;
     } else {
         // plain engine: diag_lanczos per sector, eigenvector for every sector
@@ -1293,8 +1396,9 @@ void green_runs(edzt_ctx* c, std::vector<GreenRun>& runs, int maxnstep, int nw, 
         }
     }
     // b(1) = |c^(+)|gs>| (dmft_green.f90:219,249); continued fractions on the device
-    Lease<double> g(c->pool, (size_t)std::max(nr, 1) * 2 * nw);
-    CK(cudaMemsetAsync(g.p, 0, sizeof(double) * (size_t)std::max(nr, 1) * 2 * nw, c->stream));
+    const size_t n_g = (size_t)std::max(nr, 1) * 2 * nw, n_ab = (size_t)std::max(nr, 1) * 2 * maxnstep;
+    Lease<double> g(c->pool, n_g);
+    CK(cudaMemsetAsync(g.p, 0, sizeof(double) * n_g, c->stream));
     std::vector<CFJob> cj;
     for (int r = 0; r < nr; r++) {
         GreenRun& gr = runs[r];
@@ -1309,23 +1413,27 @@ void green_runs(edzt_ctx* c, std::vector<GreenRun>& runs, int maxnstep, int nw, 
         J.g = g.p + (size_t)r * 2 * nw;
         cj.push_back(J);
     }
+    // pinned: the fractions' descriptors up, their values and the coefficients back
+    const size_t bytes_cj = (sizeof(CFJob) * cj.size() + 255) & ~(size_t)255;
+    char* stage = stage_buffer(c, bytes_cj + sizeof(double) * (n_g + n_ab));
+    double* hg = reinterpret_cast<double*>(stage + bytes_cj);
+    double* hab = hg + n_g;
+    Lease<CFJob> dj(c->pool, std::max<size_t>(cj.size(), 1));
     if (!cj.empty()) {
-        Lease<CFJob> dj(c->pool, cj.size());
-        CK(cudaMemcpyAsync(dj.p, cj.data(), sizeof(CFJob) * cj.size(), cudaMemcpyHostToDevice, c->stream));
+        std::memcpy(stage, cj.data(), sizeof(CFJob) * cj.size());
+        CK(cudaMemcpyAsync(dj.p, stage, sizeof(CFJob) * cj.size(), cudaMemcpyHostToDevice, c->stream));
         launch_cf(dj.p, (int)cj.size(), omega_dev, nw, c->stream, real_axis, eta);
         c->launches += 1;
         CKLAUNCH();
-        CK(cudaStreamSynchronize(c->stream));
     }
-    std::vector<double> hg((size_t)std::max(nr, 1) * 2 * nw), hab((size_t)std::max(nr, 1) * 2 * maxnstep);
-    CK(cudaMemcpyAsync(hg.data(), g.p, sizeof(double) * hg.size(), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(hab.data(), ab.p, sizeof(double) * hab.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(hg, g.p, sizeof(double) * n_g, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(hab, ab.p, sizeof(double) * n_ab, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     g_out.assign(nr, {});
     ab_out.assign(nr, {});
     for (int r = 0; r < nr; r++) {
-        g_out[r].assign(hg.begin() + (size_t)r * 2 * nw, hg.begin() + (size_t)(r + 1) * 2 * nw);
-        ab_out[r].assign(hab.begin() + (size_t)(2 * r) * maxnstep, hab.begin() + (size_t)(2 * r + 2) * maxnstep);
+        g_out[r].assign(hg + (size_t)r * 2 * nw, hg + (size_t)(r + 1) * 2 * nw);
+        ab_out[r].assign(hab + (size_t)(2 * r) * maxnstep, hab + (size_t)(2 * r + 2) * maxnstep);
         if (runs[r].nstep >= 1) ab_out[r][maxnstep] = runs[r].norm0;       // b(1) (:219, :249)
     }
 }
@@ -1412,8 +1520,8 @@ void cluster_green_impl(edzt_ctx* c, int nspin, int maxnstep, int nw, const doub
     std::vector<double> Gh((size_t)2 * nw * norb * nspin, 0.0);
     std::vector<double> ch((size_t)norb * 2 * 4 * maxnstep, 0.0);
     assemble_cluster(norb, nspin, even, maxnstep, nw, gs, abs_, 0, Gh.data(), ch.data());
-    if (G_cl) copy_out(c, G_cl, Gh.data(), sizeof(double) * Gh.size());
-    if (coeffs) copy_out(c, coeffs, ch.data(), sizeof(double) * ch.size());
+    if (G_cl) put_out(c, G_cl, Gh.data(), sizeof(double) * Gh.size());
+    if (coeffs) put_out(c, coeffs, ch.data(), sizeof(double) * ch.size());
     CK(cudaStreamSynchronize(c->stream));
 }
 
@@ -1436,11 +1544,11 @@ void green_diag_impl(edzt_ctx* c, int iorb, int ispin, int maxnstep, int nw, con
     std::vector<double> gsum(2 * nw, 0.0);
     for (int r = 0; r < 2; r++)
         for (int q = 0; q < 2 * nw; q++) gsum[q] += gs[r][q];
-    copy_out(c, ap, abs_[0].data(), sizeof(double) * maxnstep);
-    copy_out(c, bp, abs_[0].data() + maxnstep, sizeof(double) * maxnstep);
-    copy_out(c, am, abs_[1].data(), sizeof(double) * maxnstep);
-    copy_out(c, bm, abs_[1].data() + maxnstep, sizeof(double) * maxnstep);
-    copy_out(c, g, gsum.data(), sizeof(double) * 2 * nw);
+    put_out(c, ap, abs_[0].data(), sizeof(double) * maxnstep);
+    put_out(c, bp, abs_[0].data() + maxnstep, sizeof(double) * maxnstep);
+    put_out(c, am, abs_[1].data(), sizeof(double) * maxnstep);
+    put_out(c, bm, abs_[1].data() + maxnstep, sizeof(double) * maxnstep);
+    put_out(c, g, gsum.data(), sizeof(double) * 2 * nw);
     CK(cudaStreamSynchronize(c->stream));
 }
 
@@ -1528,7 +1636,7 @@ void cluster_green_matrix_impl(edzt_ctx* c, int nspin, int maxnstep, int nw, con
                     }
                     Gh[o] = re; Gh[o + 1] = im;
                 }
-    copy_out(c, G, Gh.data(), sizeof(double) * Gh.size());
+    put_out(c, G, Gh.data(), sizeof(double) * Gh.size());
     CK(cudaStreamSynchronize(c->stream));
 }
 
@@ -1549,25 +1657,12 @@ struct BatchInst {
     Lease<double> gsvec;
 };
 
-template <class F>
-void parallel_for(int n, F&& f)
-{
-    const int nt = std::max(1, std::min(n, (int)std::thread::hardware_concurrency()));
-    std::atomic<int> next{0};
-    std::vector<std::thread> th;
-    for (int t = 0; t < nt; t++)
-        th.emplace_back([&] {
-            for (int i = next++; i < n; i = next++) f(i);
-        });
-    for (auto& x : th) x.join();
-}
-
 void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxnstep, int nw,
                 const double* omega_dev, std::vector<double>& Gall, const std::vector<size_t>& goff)
 {
     for (int i = i0; i < i1; i++) {
         B[i].mt = std::make_unique<ModelTables>();
-        set_tables_model(*B[i].mt, B[i].model, c->stream);
+        set_tables_model(c, *B[i].mt, B[i].model);
     }
     // ---- ground-state scan: every sector of every instance (ground_state.f90:28-73)
     struct Owner { int inst, sector; };
@@ -1591,6 +1686,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     }
     const int nj = (int)specs.size();
     Lease<double> ab(c->pool, (size_t)std::max(nj, 1) * 2 * maxnstep);
+    CK(cudaMemsetAsync(ab.p, 0, sizeof(double) * (size_t)std::max(nj, 1) * 2 * maxnstep, c->stream));
     for (int q = 0; q < nj; q++) {
         specs[q].a = ab.p + (size_t)(2 * q) * maxnstep;
         specs[q].b = ab.p + (size_t)(2 * q + 1) * maxnstep;
@@ -1600,7 +1696,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     CK(cudaMemcpyAsync(hab.data(), ab.p, sizeof(double) * hab.size(), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     std::vector<SectorResult> res(nj);
-    parallel_for(nj, [&](int q) {
+    parallel_for(nj, 1 + 2000 / maxnstep, [&](int q) {   // a thread costs about 2,000 rows of tridiagonals
         SectorResult& r = res[q];
         r.nstep = specs[q].nstep;
         if (r.nstep < 1) return;
@@ -1712,6 +1808,10 @@ void init_inst(const edzt_instance& in, BatchInst& I)
     I.footprint = std::max(gsb, cfb) + 64 * maxd;
 }
 
+// Device memory a batch leaves cached for the next call: allocating and freeing
+// it anew took most of a small batch's time.
+constexpr size_t kBatchKeep = (size_t)2 << 30;
+
 void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int maxnstep, int nw, const double* omega,
                       int* isector, double* e0, double* G_cl, size_t budget)
 {
@@ -1723,7 +1823,11 @@ void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int max
         init_inst(inst[i], B[i]);
         goff[i + 1] = goff[i] + (size_t)2 * nw * B[i].model.norb * B[i].nspin;
     }
-    if (budget == 0) {
+    long long all = 0;
+    for (const BatchInst& I : B) all += I.footprint;
+    if (budget == 0 && all <= (long long)kBatchKeep) {
+        budget = kBatchKeep;                              // one wave; no need to ask what is free
+    } else if (budget == 0) {
         size_t fr = 0, tot = 0;
         CK(cudaMemGetInfo(&fr, &tot));
         budget = fr / 10 * 8;
@@ -1735,14 +1839,14 @@ void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int max
         long long sum = 0;
         while (i1 < ninst && (i1 == i0 || sum + B[i1].footprint <= (long long)budget)) sum += B[i1++].footprint;
         solve_wave(c, B, i0, i1, maxnstep, nw, om.d, Gall, goff);
-        c->pool.trim();
+        c->pool.trim_to(kBatchKeep);
         i0 = i1;
     }
     for (int i = 0; i < ninst; i++) {
         if (isector) isector[i] = B[i].best;
         if (e0) e0[i] = B[i].e0;
     }
-    if (G_cl && goff[ninst] > 0) copy_out(c, G_cl, Gall.data(), sizeof(double) * goff[ninst]);
+    if (G_cl && goff[ninst] > 0) put_out(c, G_cl, Gall.data(), sizeof(double) * goff[ninst]);
     CK(cudaStreamSynchronize(c->stream));
 }
 
@@ -1765,7 +1869,7 @@ struct LiveJob {
     JobSpec spec;
     DevSector S{};
     Lease<double> y, v0, v1;
-    Lease<LzState> st;                     // [2] by phase parity, on the device
+    LzState st[2] = {};                    // by phase parity, between slices
     int k = 0;                             // steps done (host view, from the last slice)
     bool done = false;
 };
@@ -1819,12 +1923,7 @@ std::unique_ptr<LiveJob> make_live(edzt_ctx* c, const JobSpec& spec)
     L->y = Lease<double>(c->pool, n);
     L->v0 = Lease<double>(c->pool, n);
     L->v1 = Lease<double>(c->pool, n);
-    L->st = Lease<LzState>(c->pool, 2);
-    LzState init[2];
-    std::memset(init, 0, sizeof(init));
-    init[1].active = 1;                                  // the state before the first phase (parity 1)
-    CK(cudaMemcpyAsync(L->st.p, init, sizeof(init), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));                // init (host memory) consumed
+    L->st[1].active = 1;                                 // the state before the first phase (parity 1)
     if (spec.mode == LZ_COEFF) {
         CK(cudaMemsetAsync(spec.a, 0, sizeof(double) * spec.maxnstep, c->stream));
         CK(cudaMemsetAsync(spec.b, 0, sizeof(double) * spec.maxnstep, c->stream));
@@ -1846,44 +1945,13 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases)
         J.Y = L.y.p;
         J.V[0] = L.v0.p;
         J.V[1] = L.v1.p;
-        J.st = L.st.p;
     }
-    std::vector<long long> prefix;
-    const LzPlan P = lz_plan(c->device, jobs.data(), nj, prefix, tuned_shape(c, jobs));
-    if (P.grid <= 0) throw EdztError{EDZT_ERR_CUDA, "persistent kernel cannot be resident (shared memory too large)"};
-    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t bytes_jobs = sizeof(LzJob) * nj, bytes_pre = sizeof(long long) * prefix.size();
-    const size_t bytes_slots = sizeof(double) * (size_t)P.slots, bytes_sw = lz_sync_bytes(nj);
-    Lease<char> blob(c->pool, al(bytes_jobs) + al(bytes_pre) + al(bytes_slots) + al(bytes_sw));
-    LzJob* d_jobs = reinterpret_cast<LzJob*>(blob.p);
-    long long* d_pre = reinterpret_cast<long long*>(blob.p + al(bytes_jobs));
-    double* d_slots = reinterpret_cast<double*>(blob.p + al(bytes_jobs) + al(bytes_pre));
-    unsigned* d_sw = reinterpret_cast<unsigned*>(blob.p + al(bytes_jobs) + al(bytes_pre) + al(bytes_slots));
-    CK(cudaMemcpyAsync(d_jobs, jobs.data(), bytes_jobs, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(d_pre, prefix.data(), bytes_pre, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemsetAsync(d_sw, 0, bytes_sw, c->stream));
-    CK(cudaMemsetAsync(c->status->p, 0, sizeof(int), c->stream));
-    LzBatch B;
-    std::memset(&B, 0, sizeof(B));
-    B.njobs = nj;
-    B.max_phases = std::max(2, phases & ~1);
-    if (c->dbg_pass_cap > 0) B.max_phases = std::min(B.max_phases, std::max(2, c->dbg_pass_cap & ~1));
-    B.wait_ns = c->dbg_wait_ns;
-    B.stall_cta = c->dbg_stall_cta;
-    B.slice = 1;
-    CK(cudaEventRecord(c->ev0, c->stream));
-    CK(launch_lanczos_persistent(P, B, d_jobs, d_pre, d_slots, d_sw, c->status->as<int>(), c->stream));
-    CK(cudaEventRecord(c->ev1, c->stream));
-    c->launches += 1;
     std::vector<LzState> st(2 * (size_t)nj);
-    for (int j = 0; j < nj; j++)
-        CK(cudaMemcpyAsync(&st[2 * (size_t)j], v[j]->st.p, 2 * sizeof(LzState), cudaMemcpyDeviceToHost, c->stream));
-    int status = 0;
-    CK(cudaMemcpyAsync(&status, c->status->p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (status == EDZT_DEV_BARRIER_TIMEOUT)
-        throw EdztError{EDZT_ERR_TIMEOUT, "persistent Lanczos kernel: grid barrier wait timed out"};
-    if (status != 0) throw EdztError{EDZT_ERR_CUDA, "persistent Lanczos kernel reported status " + std::to_string(status)};
+    for (int j = 0; j < nj; j++) std::memcpy(&st[2 * (size_t)j], v[j]->st, 2 * sizeof(LzState));
+    int budget = std::max(2, phases & ~1);
+    if (c->dbg_pass_cap > 0) budget = std::min(budget, std::max(2, c->dbg_pass_cap & ~1));
+    const float ms = launch_jobs(c, jobs, st, tuned_shape(c, jobs), budget, true);
+    for (int j = 0; j < nj; j++) std::memcpy(v[j]->st, &st[2 * (size_t)j], 2 * sizeof(LzState));
     double bytes = 0.0;
     for (int j = 0; j < nj; j++) {
         LiveJob& L = *v[j];
@@ -1901,14 +1969,7 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases)
             L.spec.norm0 = fin->norm0;
         }
     }
-    float ms = 0.0f;
-    CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-    c->st_launches += 1;
-    c->st_ms += ms;
-    c->st_bytes += bytes;
-    double states = 0.0;
-    for (int j = 0; j < nj; j++) states += (double)jobs[j].S.dim;
-    log_launch(c, ms, bytes, states);
+    book_launch(c, jobs, ms, bytes);
     return ms;
 }
 
@@ -1920,7 +1981,7 @@ void server_admit(edzt_server* sv)
         if (!sv->active.empty() && sv->reserved + q.I.footprint > sv->budget) break;
         sv->reserved += q.I.footprint;
         q.I.mt = std::make_unique<ModelTables>();
-        set_tables_model(*q.I.mt, q.I.model, c->stream);
+        set_tables_model(c, *q.I.mt, q.I.model);
         const int ns = (int)q.I.sec.size() / 2;
         q.ab = Lease<double>(c->pool, (size_t)std::max(ns, 1) * 2 * sv->maxnstep);
         q.cls = size_class(q.I);
@@ -2235,8 +2296,6 @@ int edzt_ctx_create(int device, edzt_ctx** out)
     int rc = guarded(c, [&] {
         CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
         edzt_init_binomials(device);
-        c->sync_words = std::make_unique<DevBuf>(64);
-        c->status = std::make_unique<DevBuf>(64);
         c->scal = std::make_unique<DevBuf>(sizeof(double) * 32);
         c->dot_part = std::make_unique<DevBuf>(sizeof(double) * dot_partials_size());
         CK(cudaMallocHost((void**)&c->pinned, sizeof(double) * 32));
@@ -2259,8 +2318,10 @@ void edzt_ctx_destroy(edzt_ctx* c)
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->gs_vec.reset();
+    c->mt = ModelTables();
     c->pool.release_all();
     if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->stage) cudaFreeHost(c->stage);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -2342,7 +2403,7 @@ int edzt_set_model(edzt_ctx* c, int norb, int nbath, const double* em, const dou
     return guarded(c, [&] {
         const DevModel m = model_from(norb, nbath, em, ek, vmk, U, Up, Jex, Jp, mu);
         c->has_gs = false;
-        set_tables_model(c->mt, m, c->stream);
+        set_tables_model(c, c->mt, m);
     });
 }
 
@@ -2432,6 +2493,7 @@ int edzt_lanczos_iteration(edzt_ctx* c, int ne_up, int ne_dn, const double* v_in
         std::vector<double> ha(maxnstep, 0.0), hb(maxnstep, 0.0);
         if (c->engine == EDZT_ENGINE_FUSED) {
             Lease<double> ab(c->pool, (size_t)2 * maxnstep);
+            CK(cudaMemsetAsync(ab.p, 0, sizeof(double) * 2 * maxnstep, c->stream));
             std::vector<JobSpec> specs(1);
             JobSpec& s = specs[0];
             s.nu = ne_up; s.nd = ne_dn;
@@ -2449,8 +2511,8 @@ int edzt_lanczos_iteration(edzt_ctx* c, int ne_up, int ne_dn, const double* v_in
             DevSector S = make_sector(c, ne_up, ne_dn);
             *nstep = plain_lanczos(c, S, vi.d, maxnstep, ha.data(), hb.data(), nullptr, nullptr, nullptr);
         }
-        copy_out(c, a, ha.data(), sizeof(double) * maxnstep);
-        copy_out(c, b, hb.data(), sizeof(double) * maxnstep);
+        put_out(c, a, ha.data(), sizeof(double) * maxnstep);
+        put_out(c, b, hb.data(), sizeof(double) * maxnstep);
         CK(cudaStreamSynchronize(c->stream));
     });
 }
@@ -2474,7 +2536,7 @@ int edzt_diag_lanczos(edzt_ctx* c, int ne_up, int ne_dn, int maxnstep, uint64_t 
             ~Keep() { c->diag_solver = solver; }
         } keep{c, c->diag_solver};
         c->diag_solver = EDZT_DIAG_LANCZOS;
-        ground_state_impl(c, 1, sec.data(), maxnstep, seed, &is, &e0, nullptr, nullptr, &stream);
+        ground_state_impl(c, 1, sec.data(), maxnstep, seed, &is, &e0, nullptr, nullptr, &stream, residual != nullptr);
         *eigval = e0;
         if (eigvec) copy_out(c, eigvec, c->gs_vec.p, sizeof(double) * dim);
         if (residual) *residual = c->gs_residual;
@@ -2700,7 +2762,7 @@ int edzt_server_result(edzt_server* sv, long long id, int* done, int* isector, d
         *done = 1;
         if (isector) *isector = q.I.best;
         if (e0) *e0 = q.I.e0;
-        if (G_cl && !q.G.empty()) copy_out(sv->c, G_cl, q.G.data(), sizeof(double) * q.G.size());
+        if (G_cl && !q.G.empty()) put_out(sv->c, G_cl, q.G.data(), sizeof(double) * q.G.size());
         CK(cudaStreamSynchronize(sv->c->stream));
         sv->finished.erase(it);
     });

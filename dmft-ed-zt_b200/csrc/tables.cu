@@ -8,6 +8,7 @@
 // sum_k C(p_k, k) (0-based here) and the r-th string is recovered greedily
 // from the top bit down.  The fermion signs of src/impurity_hamiltonian.f90:
 // 251-260 are popcounts of the bits strictly between the two sites.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <mutex>
@@ -185,23 +186,29 @@ void launch_build_spin_ops(const DevModel& m, int sigma, int count, const uint32
     k_build_spin_ops<<<(n + 127) / 128, 128, 0, s>>>(m, sigma, count, str, rank, hw, e1, hcnt, hpk, amp, imp, sub);
 }
 
+// For an impurity pattern, bath site l gives e_l hops when it is empty (the
+// filled orbitals coupled to it) and o_l when it is filled (the empty ones);
+// the electrons left for the bath go where o_l - e_l is largest.
 int edzt_max_hops(const DevModel& m, int sigma, int n)
 {
-    const int ns = m.nsite;
-    if (n < 0 || n > ns) return 0;
+    if (n < 0 || n > m.nsite) return 0;
     int best = 0;
-    // every string with popcount n (Gosper's hack; the empty and full strings directly)
-    uint64_t u = (n == 0) ? 0ull : ((1ull << n) - 1ull);
-    const uint64_t end = 1ull << ns;
-    while (u < end) {
-        int h = 0;
-        for (int a = 0; a < m.norb; a++)
-            for (int l = 0; l < m.nbath; l++)
-                if (std::fabs(m.vmk[a][l][sigma]) >= 1.0e-16 && (((u >> a) ^ (u >> (m.norb + l))) & 1ull)) h++;
-        if (h > best) best = h;
-        if (n == 0) break;
-        const uint64_t c = u & (0ull - u), r = u + c;
-        u = (((r ^ u) >> 2) / c) | r;
+    for (int p = 0; p < (1 << m.norb); p++) {
+        int filled = 0;
+        for (int a = 0; a < m.norb; a++) filled += (p >> a) & 1;
+        const int left = n - filled;
+        if (left < 0 || left > m.nbath) continue;
+        int hops = 0, gain[EDZT_MAX_NSITE];
+        for (int l = 0; l < m.nbath; l++) {
+            int e = 0, o = 0;
+            for (int a = 0; a < m.norb; a++)
+                if (std::fabs(m.vmk[a][l][sigma]) >= 1.0e-16) ((p >> a) & 1 ? e : o)++;
+            hops += e;
+            gain[l] = o - e;
+        }
+        std::sort(gain, gain + m.nbath, [](int x, int y) { return x > y; });
+        for (int i = 0; i < left; i++) hops += gain[i];
+        best = std::max(best, hops);
     }
     return best;
 }

@@ -39,23 +39,42 @@ inline int lowest_eigenpair(int n, const double* d, const double* e, double* lam
     const double pivmin = tiny * std::fmax(1.0, e2max);
     lo -= 2.0 * ulp * tn + pivmin;
     hi += 2.0 * ulp * tn + pivmin;
-    // count of eigenvalues < x
-    auto below = [&](double x) {
-        int c = 0;
-        double q = d[0] - x;
-        if (std::fabs(q) < pivmin) q = -pivmin;
-        c += q < 0.0;
-        for (int i = 1; i < n; i++) {
-            q = d[i] - x - e2[i] / q;
-            if (std::fabs(q) < pivmin) q = -pivmin;
-            c += q < 0.0;
-        }
-        return c;
-    };
+    // Bisection to neighbouring numbers, eight parts at a time: the Sturm
+    // sequences of seven points run side by side, so a pass costs little more
+    // than one point's chain of divisions.  An eigenvalue lies below x when a
+    // q_i(x) is negative.
+    constexpr int M = 7;
     for (int it = 0; it < 256; it++) {
-        const double mid = 0.5 * (lo + hi);
-        if (!(mid > lo && mid < hi)) break;
-        if (below(mid) >= 1) hi = mid; else lo = mid;
+        double x[M + 1], q[M + 1];
+        bool neg[M + 1];
+        int np = 0;
+        for (int j = 1; j <= M; j++) {
+            const double t = (j == 4) ? 0.5 * (lo + hi) : lo + (hi - lo) * (0.125 * j);
+            if (t > lo && t < hi && (np == 0 || t > x[np - 1])) x[np++] = t;
+        }
+        if (np == 0) break;
+        for (int j = np; j <= M; j++) x[j] = x[np - 1];
+        for (int j = 0; j <= M; j++) {
+            q[j] = d[0] - x[j];
+            if (std::fabs(q[j]) < pivmin) q[j] = -pivmin;
+            neg[j] = q[j] < 0.0;
+        }
+        for (int i = 1; i < n; i++)
+            for (int j = 0; j <= M; j++) {
+                q[j] = d[i] - x[j] - e2[i] / q[j];
+                q[j] = (std::fabs(q[j]) < pivmin) ? -pivmin : q[j];
+                neg[j] |= q[j] < 0.0;
+            }
+        double nlo = lo, nhi = hi;
+        for (int j = 0; j < np; j++) {
+            if (neg[j]) {
+                nhi = x[j];
+                break;
+            }
+            nlo = x[j];
+        }
+        lo = nlo;
+        hi = nhi;
     }
     const double lam = 0.5 * (lo + hi);
     *lambda = lam;
