@@ -195,6 +195,7 @@ struct ModelTables {
     bool has_j = false;
     std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> ops;    // strings in the reference's order
     std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> iops;   // strings in internal order
+    std::map<std::pair<int, int>, DevSector> hx;                     // sectors looked up for H.v
     std::vector<char> host;                 // wint, jcnt and jt as uploaded
     Lease<char> block;                      // the same on the device
     double* wint = nullptr;
@@ -372,13 +373,16 @@ DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd, bool inte
     return S;
 }
 
-// A sector of the context's model, the reference's string order; the tables
-// in internal order are built too, as edzt_lanczos_iteration_noalloc, which
-// builds none, may be called on any sector that another call has prepared.
-DevSector make_sector(edzt_ctx* c, int nu, int nd)
+// A sector of the context's model, the reference's string order, looked up
+// once per model.  The tables in internal order are built too, as
+// edzt_lanczos_iteration_noalloc, which builds none, may be called on any
+// sector that another call has prepared.
+const DevSector& make_sector(edzt_ctx* c, int nu, int nd)
 {
+    auto it = c->mt.hx.find(std::make_pair(nu, nd));
+    if (it != c->mt.hx.end()) return it->second;
     make_sector_mt(c, c->mt, nu, nd, true);
-    return make_sector_mt(c, c->mt, nu, nd, false);
+    return c->mt.hx.emplace(std::make_pair(nu, nd), make_sector_mt(c, c->mt, nu, nd, false)).first->second;
 }
 
 // Interaction tables over impurity occupation patterns (pu, pd).
@@ -479,6 +483,7 @@ void set_tables_model(edzt_ctx* c, ModelTables& mt, const DevModel& m)
 {
     mt.ops.clear();
     mt.iops.clear();
+    mt.hx.clear();
     mt.model = m;
     build_model_tables(c, mt);
     mt.valid = true;
@@ -762,9 +767,9 @@ edzt_ctx::Tuned tune_sector(edzt_ctx* c, int nu, int nd, int steps)
         return (c->st_ms - ms0) / std::max(1, specs[0].nstep);
     };
     edzt_ctx::Tuned best{{0, 0, 0}, HUGE_VAL};
-    run({2, 2, 512});                                     // warm-up
+    run({2, 1, 512});                                     // warm-up
     for (const LzShape q : {LzShape{16, 8, 256}, LzShape{16, 8, 512}, LzShape{8, 8, 256}, LzShape{8, 8, 512}, LzShape{8, 4, 256},
-                            LzShape{8, 4, 512}, LzShape{4, 4, 256}, LzShape{4, 4, 512}, LzShape{2, 2, 256}, LzShape{2, 2, 512}}) {
+                            LzShape{8, 4, 512}, LzShape{4, 4, 256}, LzShape{4, 4, 512}, LzShape{2, 2, 256}, LzShape{2, 2, 512}, LzShape{2, 1, 512}}) {
         if (!lz_shape_fits(S, q)) continue;
         const double ms = run(q);
         if (ms < best.ms_per_step) best = {q, ms};
@@ -792,8 +797,7 @@ int plain_lanczos(edzt_ctx* c, const DevSector& S, const double* v_init, int max
                   double* norm_out, const double* coeff, double* eig)
 {
     const long long n = S.dim;
-    Lease<double> v(c->pool, (size_t)n), w(c->pool, (size_t)n),
-        hs(c->pool, (size_t)hx_scratch_size(S.up.count, S.dn.count));
+    Lease<double> v(c->pool, (size_t)n), w(c->pool, (size_t)n);
     if (coeff == nullptr)
         for (int i = 0; i < maxnstep; i++) { a[i] = 0.0; b[i] = 0.0; }
     const double norm_v = std::sqrt(plain_dot(c, v_init, v_init, n));          // :128
@@ -808,8 +812,8 @@ int plain_lanczos(edzt_ctx* c, const DevSector& S, const double* v_init, int max
         launch_axpy(eig, w.p, n, nullptr, coeff[0], 1.0, c->stream);
         c->launches += 1;
     }
-    launch_hx(S, w.p, v.p, 0, hs.p, c->stream);                                // :132
-    c->launches += 2;
+    launch_hx(S, w.p, v.p, 0, c->stream);                                      // :132
+    c->launches += 1;
     CKLAUNCH();
     int nstep;
     if (!coeff) a[0] = plain_dot(c, w.p, v.p, n);                              // :134
@@ -826,7 +830,7 @@ int plain_lanczos(edzt_ctx* c, const DevSector& S, const double* v_init, int max
             launch_axpy(eig, w.p, n, nullptr, coeff[k - 1], 1.0, c->stream);
             c->launches += 1;
         }
-        launch_hx(S, w.p, v.p, 1, hs.p, c->stream);                            // :158
+        launch_hx(S, w.p, v.p, 1, c->stream);                            // :158
         c->launches += 2;
         if (!coeff) a[k - 1] = plain_dot(c, w.p, v.p, n);                      // :159
         if (k >= maxnstep) { nstep = k; break; }                               // :161-164
@@ -864,10 +868,10 @@ double finish_eigvec(edzt_ctx* c, const DevSector& S, double* vec, double e0)
 {
     const long long n = S.dim;
     normalise(c, vec, n);
-    Lease<double> v(c->pool, (size_t)n), hs(c->pool, (size_t)hx_scratch_size(S.up.count, S.dn.count));
-    launch_hx(S, vec, v.p, 0, hs.p, c->stream);
+    Lease<double> v(c->pool, (size_t)n);
+    launch_hx(S, vec, v.p, 0, c->stream);
     launch_axpy(v.p, vec, n, nullptr, e0, -1.0, c->stream);
-    c->launches += 3;
+    c->launches += 2;
     CKLAUNCH();
     return plain_dot(c, v.p, v.p, n);
 }
@@ -908,7 +912,7 @@ void diag_arpack_impl(edzt_ctx* c, const DevSector& S, uint64_t key, double* vec
     const int m = kArNcv, kmax = kArNev + (kArNcv - kArNev) / 2;
     const double eps = 0x1p-53, eps23 = std::pow(eps, 2.0 / 3.0), tol = eps;
     cudaStream_t st = c->stream;
-    Lease<double> buf(c->pool, (size_t)(m + 1 + kmax) * n), hxs(c->pool, (size_t)hx_scratch_size(S.up.count, S.dn.count));
+    Lease<double> buf(c->pool, (size_t)(m + 1 + kmax) * n);
     Lease<double> small(c->pool, (size_t)rl_partials_size() + 32 + EDZT_RL_MAXV * EDZT_RL_MAXV);
     double* part = small.p;
     double* hd = small.p + rl_partials_size();          // [0, 8) pass 1, [8, 16) pass 2, [16] |w|^2
@@ -962,8 +966,8 @@ void diag_arpack_impl(edzt_ctx* c, const DevSector& S, uint64_t key, double* vec
         for (int j = k; j < m; j++) {                    // extend the factorisation to m vectors
             if (!V[j + 1]) V[j + 1] = take();
             double* w = V[j + 1];
-            launch_hx(S, V[j], w, 0, hxs.p, st);
-            c->launches += 2;
+            launch_hx(S, V[j], w, 0, st);
+            c->launches += 1;
             R.nmult++;
             const double nrm2 = orth(w, j + 1);
             T[j][j] = hh[j] + hh[8 + j];
@@ -1049,9 +1053,9 @@ void diag_arpack_impl(edzt_ctx* c, const DevSector& S, uint64_t key, double* vec
         c->launches += 1;
         if (with_resid) {
             double* w = spare.back();
-            launch_hx(S, O.p[i], w, 0, hxs.p, st);
+            launch_hx(S, O.p[i], w, 0, st);
             launch_axpy(w, O.p[i], n, nullptr, theta[i], -1.0, st);
-            c->launches += 3;
+            c->launches += 2;
             R.resid[i] = std::sqrt(std::max(orth(w, 0), 0.0));
         }
     }
@@ -2445,13 +2449,18 @@ int edzt_hx(edzt_ctx* c, int ne_up, int ne_dn, const double* x, double* y, int a
         require_model(c);
         check_sector(c, ne_up, ne_dn);
         arg_check(x != nullptr && y != nullptr, "x and y required");
-        DevSector S = make_sector(c, ne_up, ne_dn);
+        const DevSector& S = make_sector(c, ne_up, ne_dn);
         InVec xi(c, x, S.dim);
         OutVec yo(c, y, S.dim);
         if (accumulate) yo.preload();
-        Lease<double> hs(c->pool, (size_t)std::max(hx_scratch_size(S.up.count, S.dn.count), 1LL));
-        launch_hx(S, xi.d, yo.d, accumulate ? 1 : 0, hs.p, c->stream);
-        c->launches += 2;
+        Lease<double> xc;                                 // y over x: from a copy, as other rows' x is read throughout
+        if (xi.d < yo.d + S.dim && yo.d < xi.d + S.dim) {
+            xc = Lease<double>(c->pool, (size_t)S.dim);
+            launch_copy(xc.p, xi.d, S.dim, c->stream);
+            xi.d = xc.p;
+        }
+        launch_hx(S, xi.d, yo.d, accumulate ? 1 : 0, c->stream);
+        c->launches += 1;
         CKLAUNCH();
         yo.finish();
         CK(cudaStreamSynchronize(c->stream));

@@ -56,10 +56,8 @@ void launch_keep_combine(const double* keep, const DevSector& S, int nstep, cons
                          cudaStream_t s);
 // out (the reference's order) = v (a run's vector).
 void launch_to_natural(const double* v, const DevSector& S, double* out, cudaStream_t s);
-// H.v in two phases (hv_phase.cuh); scratch: hx_scratch_size doubles of
-// device memory (the down-hop part, slab-major, slabs of up to 16 columns).
-void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, double* scratch, cudaStream_t s);
-inline long long hx_scratch_size(int nup, int ndn) { return (long long)((nup + 15) / 16) * 16 * ndn; }
+// y = H x, or y += H x (accumulate), of a sector in the reference's string order.
+void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, cudaStream_t s);
 // Whether a sector's staged row and column slab fit in shared memory.
 bool hx_fits(int nup, int ndn);
 // Deterministic dot product: result written to *out (device).  partials needs

@@ -27,6 +27,16 @@ __device__ __forceinline__ void stage_table(const double* __restrict__ src, int 
     for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(src + i);
 }
 
+// Asynchronous 8-byte copy global -> shared (cp.async, no register holds the
+// value in flight, so a thread can have its whole share of a tile in flight
+// at once); when `valid` is false nothing is read and the destination gets 0.
+__device__ __forceinline__ void copy_async8(double* dst, const double* src, bool valid)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int bytes = valid ? 8 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
 // Asynchronous 16-byte copy global -> shared through L2 (no register holds the data in flight).
 __device__ __forceinline__ void copy_async16(double* dst, const double* src)
 {

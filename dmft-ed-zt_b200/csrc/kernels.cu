@@ -4,8 +4,7 @@
 #include <algorithm>
 #include <cuda_runtime.h>
 #include "edzt_internal.h"
-#include "hv_phase.cuh"
-#include "hv_gather.cuh"
+#include "hv_tile.cuh"
 
 static constexpr int kWintDoubles = EDZT_MAX_P * EDZT_MAX_P;
 static constexpr int kAmpDoubles = EDZT_MAX_AMP;
@@ -19,267 +18,107 @@ int kernels_debug_bad(long long* out4)
 
 // ---------------------------------------------------------------------------
 // H.v: y = H x (accumulate = 0) or y = y + H x (accumulate = 1), the `py`
-// flag of src/impurity_hamiltonian.f90:241-245, in the two phases of
-// hv_phase.cuh: k_hx_col writes the down-hop part of every element into a
-// scratch vector D, then k_hx_row adds the diagonal, up-hop and exchange
-// parts.  Both stream their data once; all neighbour values come from
-// shared memory.
+// flag of src/impurity_hamiltonian.f90:241-245, in one pass over row tiles
+// (hv_tile.cuh): CTA b of G takes rows [b ndn / G, (b + 1) ndn / G), at most
+// R of them.  Bounded by the load/store pipe (hop values and gathers, 2.7
+// wavefronts a state, the pipe 74% busy at nsite 14) and, from nsite 16, by
+// L2.  Measured against the two launches of a column and a row phase that
+// this replaces (nsite <= 13) and the single pass by element (from nsite 14):
+// (7,5) of nsite 13 56.7 -> 48.6 us, nsite 12 38.2 -> 30.4, nsite 14
+// 209 -> 162, nsite 15 798 -> 610, nsite 16 2,870 -> 2,680, nsite 8
+// 24.4 -> 20.9 (device and launch, events around the call).
 // ---------------------------------------------------------------------------
-static constexpr int kHxThreads = 256;
-static constexpr int kHxThreadsLong = 1024;          // lines of kHxLongLine strings or more
-static constexpr int kHxLongLine = 1500;
-static constexpr int kHxGatherLine = 3000;            // single-pass form from here (nsite >= 14 near half filling)
-static constexpr size_t kHxSmemSoft = 100 * 1024;    // two CTAs per SM
-static constexpr size_t kHxSmemHard = 210 * 1024;    // one CTA per SM
-
-// Column phase: CTA b stages columns [b*WC, b*WC + WC) of every row.
-template <int WC, int NT>
-__global__ void __launch_bounds__(NT) k_hx_col(DevSector S, const double* __restrict__ x,
-                                                      double* __restrict__ D)
+template <bool ACC, int R, int PL, int T, int NB>
+__global__ void __launch_bounds__(T, NB) k_hx_tile(DevSector S, const double* __restrict__ x, double* __restrict__ y)
 {
-    constexpr int WS = phase_stride(WC);
-    extern __shared__ __align__(16) double smem[];
-    double* amp = smem;                                    // down-hop amplitudes
-    double* ws = smem + kAmpDoubles;                       // [ndn][WS]
-    const int nup = S.up.count, ndn = S.dn.count;
-    const int c0 = blockIdx.x * WC;
-    stage_table(S.dn.amp, S.dn.namp, amp);
-    const int n = ndn * WC;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {   // the whole slab in flight at once
-        const int id = i / WC, c = i - id * WC;
-        const bool in = c0 + c < nup;
-        copy_async8(ws + id * WS + c, x + (in ? (size_t)id * nup + c0 + c : 0), in);
-    }
-    copy_async_wait_all();
-    __syncthreads();
-    HopList nxt{};
-    if ((int)threadIdx.x < ndn) nxt = hop_list(S.dn, threadIdx.x);
-    for (int id = threadIdx.x; id < ndn; id += blockDim.x) {
-        const HopList cur = nxt;
-        if (id + (int)blockDim.x < ndn) nxt = hop_list(S.dn, id + blockDim.x);
-        double d[WC];
-        col_part<WC, WS>(S, ws, amp, id, cur, d);
-        store_slab_row<WC>(D, c0, ndn, id, d);          // columns past nup hold 0 (staged as 0)
-    }
-}
-
-// Row phase: CTA b stages rows [b*R, b*R + R), thread per column.
-template <bool ACC, int R, int NT>
-__global__ void __launch_bounds__(NT) k_hx_row(DevSector S, const double* __restrict__ x,
-                                                      const double* __restrict__ D, int wsh, double* __restrict__ y)
-{
-    constexpr int RS = phase_stride(R);
     extern __shared__ __align__(16) double smem[];
     double* wint = smem;
     double* amp = smem + kWintDoubles;
-    double* xs = amp + kAmpDoubles;                        // [nup][RS]
     const int nup = S.up.count, ndn = S.dn.count;
-    const int r0 = blockIdx.x * R;
-    const int nr = min(R, ndn - r0);
+    const RowTile t = tile_layout(amp + kAmpDoubles, R, S.dn.hw);
+    const int r0 = (int)((long long)blockIdx.x * ndn / gridDim.x);
+    const int nr = (int)((long long)(blockIdx.x + 1) * ndn / gridDim.x) - r0;
+    const double* __restrict__ x0 = x + (size_t)r0 * nup;
+    for (int iu = threadIdx.x; iu < nup; iu += T) {        // the whole tile in flight at once
+#pragma unroll
+        for (int r = 0; r < (R + PL - 1) / PL * PL; r++)
+            copy_async8(t.xs + ((size_t)(r / PL) * nup + iu) * PL + r % PL, x0 + (r < nr ? (size_t)r * nup + iu : 0), r < nr);
+    }
+    stage_row_tables<R>(S.dn, t, r0, nr, nup, x);
     stage_table(S.wint, S.P * S.P, wint);
     stage_table(S.up.amp, S.up.namp, amp);
-    for (int iu = threadIdx.x; iu < nup; iu += blockDim.x) {   // the whole tile in flight at once
-#pragma unroll
-        for (int r = 0; r < R; r++)
-            copy_async8(xs + iu * RS + r, x + (r < nr ? (size_t)(r0 + r) * nup + iu : 0), r < nr);
-    }
-    double e1d[R];
-    int pd[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int id = min(r0 + r, ndn - 1);
-        e1d[r] = __ldg(S.dn.e1 + id);
-        pd[r] = __ldg(S.dn.imp + id);
-    }
+    UpCol nxt{};
+    if ((int)threadIdx.x < nup) nxt = up_col(S.up, threadIdx.x);
     copy_async_wait_all();
     __syncthreads();
     auto fetch = [&](int id2, int iu2) { return __ldg(x + (long long)id2 * nup + iu2); };
-    RowCol<R> nxt{};
-    if ((int)threadIdx.x < nup) nxt = row_col<R>(S, D, wsh, threadIdx.x, r0, nr);
-    for (int iu = threadIdx.x; iu < nup; iu += blockDim.x) {
-        const RowCol<R> cur = nxt;                          // this column's data; the next one's in flight
-        if (iu + (int)blockDim.x < nup) nxt = row_col<R>(S, D, wsh, iu + blockDim.x, r0, nr);
+    for (int iu = threadIdx.x; iu < nup; iu += T) {
+        const UpCol cur = nxt;                             // this column's up string; the next one's in flight
+        if (iu + T < nup) nxt = up_col(S.up, iu + T);
         double acc[R];
-        row_part<R, RS>(S, xs, wint, amp, iu, cur, e1d, pd, acc);
+        tile_col<R, PL>(S, t, wint, amp, iu, nr, cur, acc, [](const double* p) { return __ldg(p); });
+        double* __restrict__ yo = y + (size_t)r0 * nup + iu;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            if (r >= nr) break;
-            const size_t g = (size_t)(r0 + r) * nup + iu;
-            double v = acc[r] + cur.dd[r];
-            if (S.has_j) v = exchange_part(S, r0 + r, iu, cur.pu, pd[r], v, fetch);
-            y[g] = ACC ? y[g] + v : v;
+            if (r < nr) {
+                double v = acc[r];
+                if (S.has_j) v = exchange_part(S, r0 + r, iu, cur.pu, t.pd[r], v, fetch);
+                yo[(size_t)r * nup] = ACC ? yo[(size_t)r * nup] + v : v;
+            }
         }
     }
 }
 
-// Rows per tile: the most (of 8, 4, 2, 1) that fit two CTAs per SM and still
-// give every SM two tiles; columns per slab likewise (16, 8, 4, 2).  A
-// sector too large for that takes one CTA per SM.
-static int hx_rows_of(int nup, int ndn, int nsm)
+static constexpr size_t kTileSmemMax = 227 * 1024 - 64;
+static constexpr size_t kHxSmemLimit = 210 * 1024;      // of a sector's staged lines (hx_fits)
+
+// Dynamic shared memory of a tile of R rows.
+static size_t hx_tile_smem(const DevSector& S, int R, int PL)
 {
-    const int opts[4] = {8, 4, 2, 1};
-    for (int R : opts) {
-        const size_t sm = (kWintDoubles + kAmpDoubles + (size_t)nup * phase_stride(R)) * sizeof(double);
-        if (sm <= kHxSmemSoft && (ndn + R - 1) / R >= 2 * nsm) return R;
-    }
-    for (int R : {2, 1}) {
-        const size_t sm = (kWintDoubles + kAmpDoubles + (size_t)nup * phase_stride(R)) * sizeof(double);
-        if (sm <= kHxSmemSoft) return R;
-    }
-    return 1;
+    return (kWintDoubles + kAmpDoubles + (size_t)S.up.count * ((R + PL - 1) / PL * PL)) * sizeof(double) +
+           tile_fixed_bytes(R, S.dn.hw);
 }
 
-static int hx_cols_of(int nup, int ndn, int nsm)
+template <int R, int PL, int T, int NB>
+static void launch_hx_tile(const DevSector& S, const double* x, double* y, int accumulate, int grid, cudaStream_t s)
 {
-    const int opts[4] = {16, 8, 4, 2};
-    for (int W : opts) {
-        const size_t sm = (kAmpDoubles + (size_t)ndn * phase_stride(W)) * sizeof(double);
-        if (sm <= kHxSmemSoft && (nup + W - 1) / W >= 2 * nsm) return W;
+    static std::atomic<unsigned long long> attr_set{0};
+    if (edzt_once_per_device(attr_set)) {
+        cudaFuncSetAttribute(k_hx_tile<false, R, PL, T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax);
+        cudaFuncSetAttribute(k_hx_tile<true, R, PL, T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax);
     }
-    return 2;
+    const size_t sm = hx_tile_smem(S, R, PL);
+    if (accumulate) k_hx_tile<true, R, PL, T, NB><<<grid, T, sm, s>>>(S, x, y);
+    else k_hx_tile<false, R, PL, T, NB><<<grid, T, sm, s>>>(S, x, y);
 }
-
 bool hx_fits(int nup, int ndn)
 {
-    const size_t row = (kWintDoubles + kAmpDoubles + (size_t)nup * phase_stride(1)) * sizeof(double);
-    const size_t col = (kAmpDoubles + (size_t)ndn * phase_stride(2)) * sizeof(double);
-    return row <= kHxSmemHard && col <= kHxSmemHard;
+    return (kWintDoubles + kAmpDoubles + (size_t)nup) * sizeof(double) <= kHxSmemLimit &&
+           (kAmpDoubles + 2 * (size_t)ndn) * sizeof(double) <= kHxSmemLimit;
 }
 
-template <int R, int NT>
-static void launch_hx_row(const DevSector& S, const double* x, const double* D, int wc, double* y, int accumulate,
-                          cudaStream_t s)
-{
-    const int wsh = __builtin_ctz((unsigned)wc);
-    static std::atomic<unsigned long long> attr_set{0};
-    if (edzt_once_per_device(attr_set)) {
-        cudaFuncSetAttribute(k_hx_row<false, R, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHxSmemHard);
-        cudaFuncSetAttribute(k_hx_row<true, R, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHxSmemHard);
-    }
-    const int tiles = (S.dn.count + R - 1) / R;
-    const size_t sm = (kWintDoubles + kAmpDoubles + (size_t)S.up.count * phase_stride(R)) * sizeof(double);
-    if (accumulate) k_hx_row<true, R, NT><<<tiles, NT, sm, s>>>(S, x, D, wsh, y);
-    else k_hx_row<false, R, NT><<<tiles, NT, sm, s>>>(S, x, D, wsh, y);
-}
-
-template <int W, int NT>
-static void launch_hx_col(const DevSector& S, const double* x, double* D, cudaStream_t s)
-{
-    static std::atomic<unsigned long long> attr_set{0};
-    if (edzt_once_per_device(attr_set))
-        cudaFuncSetAttribute(k_hx_col<W, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHxSmemHard);
-    const int slabs = (S.up.count + W - 1) / W;
-    const size_t sm = (kAmpDoubles + (size_t)S.dn.count * phase_stride(W)) * sizeof(double);
-    k_hx_col<W, NT><<<slabs, NT, sm, s>>>(S, x, D);
-}
-
-// ---------------------------------------------------------------------------
-// Single-pass H.v for long lines (hv_gather.cuh): one CTA per tile of R full
-// rows staged in shared memory with their down-hop records; the up hops read
-// the staged rows, the down hops gather coalesced slices of other rows from
-// global memory.  T threads per CTA, 64 registers (32 warps per SM).
-// ---------------------------------------------------------------------------
-static constexpr size_t kGatherTileBytes = 24 * 1024;
-
-template <bool ACC, int T>
-__global__ void __launch_bounds__(T, T == 512 ? 2 : 1) k_hx_gather(DevSector S, const double* __restrict__ x,
-                                                                  double* __restrict__ y, int R)
-{
-    extern __shared__ __align__(16) double smem[];
-    double* wint = smem;
-    double* amp = smem + kWintDoubles;
-    const int nup = S.up.count, ndn = S.dn.count;
-    Chunk C = chunk_layout(smem + kWintDoubles + kAmpDoubles, R, nup, S.dn.hw);
-    const int r0 = blockIdx.x * R;
-    const int rows = min(R, ndn - r0);
-    const int n = rows * nup;
-    const long long g0 = (long long)r0 * nup;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) C.xs[e] = __ldg(x + g0 + e);
-    stage_rows(S.dn, C, r0, rows);
-    stage_table(S.wint, S.P * S.P, wint);
-    stage_table(S.up.amp, S.up.namp, amp);
-    __syncthreads();
-    auto fetch = [&](long long idx) {
-        EDZT_OK_OR(idx >= 0 && idx < S.dim, 61, idx, S.dim, blockIdx.x, return 0.0)
-        return __ldg(x + idx);
-    };
-    const SrcVec src{x};
-    int r = threadIdx.x / nup, iu = threadIdx.x - r * nup;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        double du, dn;
-        hv_elem(S, C, wint, amp, src, r, iu, C.xs[e], du, dn);
-        double acc = du + dn;
-        if (S.has_j) acc = hv_exchange(S, C, r, iu, acc, fetch);
-        const long long g = g0 + e;
-        y[g] = ACC ? y[g] + acc : acc;
-        iu += blockDim.x;
-        while (iu >= nup) { iu -= nup; ++r; }
-    }
-}
-
-template <int T>
-static void launch_hx_gather(const DevSector& S, const double* x, double* y, int accumulate, cudaStream_t s)
-{
-    static std::atomic<unsigned long long> attr_set{0};
-    if (edzt_once_per_device(attr_set)) {
-        cudaFuncSetAttribute(k_hx_gather<false, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHxSmemHard);
-        cudaFuncSetAttribute(k_hx_gather<true, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHxSmemHard);
-    }
-    const int nup = S.up.count, ndn = S.dn.count;
-    const size_t row = staged_row_bytes(nup, S.dn.hw);
-    const int R = std::max(1, std::min(ndn, (int)(kGatherTileBytes / row)));
-    const int tiles = (ndn + R - 1) / R;
-    const size_t smem = (kWintDoubles + kAmpDoubles) * sizeof(double) + (size_t)R * row;
-    if (accumulate) k_hx_gather<true, T><<<tiles, T, smem, s>>>(S, x, y, R);
-    else k_hx_gather<false, T><<<tiles, T, smem, s>>>(S, x, y, R);
-}
-
-// Whether H.v of a sector takes the single-pass form: lines of
-// kHxGatherLine strings or more (measured faster there: the two-phase
-// slabs and tiles are too narrow).
-bool hx_single_pass(int nup, int ndn) { return std::max(nup, ndn) >= kHxGatherLine; }
-
-void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, double* scratch, cudaStream_t s)
+// Rows per tile: as many of 4, 2, 1 as leave every SM a tile and two CTAs (one
+// from 8,000 strings) room in shared memory: the hop decode is shared by the
+// tile's rows, but wide tiles of long rows leave too few warps (us at nsite 13
+// with 4 / 2 / 1 rows 48.6 / 50.4 / 50.3, nsite 14 166 / 162 / 174, nsite 15
+// 859 / 610 / 594).  Threads: 512, two CTAs per SM; four rows of 1,500 strings
+// or more run 256 threads three times (80 registers: 48.6 against 53.1), rows
+// of 8,000 or more 1,024 (2,677 against 2,732).
+void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, cudaStream_t s)
 {
     const int nup = S.up.count, ndn = S.dn.count;
     if (nup <= 0 || ndn <= 0) return;
-    if (hx_single_pass(nup, ndn)) {
-        // 1024 threads from 32 M states, else 512 (two CTAs per SM)
-        if (S.dim >= (32LL << 20)) launch_hx_gather<1024>(S, x, y, accumulate, s);
-        else launch_hx_gather<512>(S, x, y, accumulate, s);
-        return;
-    }
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    // long lines (1500 strings or more) take 1024-thread CTAs, so the SM has
-    // 32 or more warps to overlap the hop lists' and neighbours' latency
-    // (measured: 17% faster at nsite 13, 6% at 14)
-    const int wc = (ndn > kHxLongLine) ? (hx_cols_of(nup, ndn, nsm) == 4 ? 4 : 2) : hx_cols_of(nup, ndn, nsm);
-    if (ndn > kHxLongLine) {
-        if (wc == 4) launch_hx_col<4, kHxThreadsLong>(S, x, scratch, s);
-        else launch_hx_col<2, kHxThreadsLong>(S, x, scratch, s);
-    } else {
-        switch (wc) {
-        case 16: launch_hx_col<16, kHxThreads>(S, x, scratch, s); break;
-        case 8: launch_hx_col<8, kHxThreads>(S, x, scratch, s); break;
-        case 4: launch_hx_col<4, kHxThreads>(S, x, scratch, s); break;
-        default: launch_hx_col<2, kHxThreads>(S, x, scratch, s); break;
-        }
-    }
-    if (nup > kHxLongLine) {
-        const int r = hx_rows_of(nup, ndn, nsm);
-        if (r >= 4) launch_hx_row<4, kHxThreadsLong>(S, x, scratch, wc, y, accumulate, s);
-        else if (r == 2) launch_hx_row<2, kHxThreadsLong>(S, x, scratch, wc, y, accumulate, s);
-        else launch_hx_row<1, kHxThreadsLong>(S, x, scratch, wc, y, accumulate, s);
-    } else {
-        switch (hx_rows_of(nup, ndn, nsm)) {
-        case 8: launch_hx_row<8, kHxThreads>(S, x, scratch, wc, y, accumulate, s); break;
-        case 4: launch_hx_row<4, kHxThreads>(S, x, scratch, wc, y, accumulate, s); break;
-        case 2: launch_hx_row<2, kHxThreads>(S, x, scratch, wc, y, accumulate, s); break;
-        default: launch_hx_row<1, kHxThreads>(S, x, scratch, wc, y, accumulate, s); break;
-        }
-    }
+    int R = std::min(nup >= 8000 ? 1 : nup >= 3000 ? 2 : 4, std::max(1, ndn / nsm));
+    if (R == 3) R = 2;
+    const int grid = (ndn + R - 1) / R;
+    if (R == 4 && nup >= 1500) launch_hx_tile<4, 2, 256, 3>(S, x, y, accumulate, grid, s);
+    else if (R == 4) launch_hx_tile<4, 2, 512, 2>(S, x, y, accumulate, grid, s);
+    else if (R == 2) launch_hx_tile<2, 2, 512, 2>(S, x, y, accumulate, grid, s);
+    else if (nup >= 8000) launch_hx_tile<1, 1, 1024, 1>(S, x, y, accumulate, grid, s);
+    else launch_hx_tile<1, 1, 512, 2>(S, x, y, accumulate, grid, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -532,9 +532,51 @@ __device__ __forceinline__ double row_tile(int r0, int np)
     return acc;
 }
 
-// NC, NR: planes of PW lines of a column and of a row tile; X: a model of the
-// launch has exchange terms.
-template <int NC, int NR, int PW, bool X, int T>
+// Row phase of one row, for lines so long that two do not fit (13,400 up
+// strings or more: nsite 17 and beyond).
+template <bool X, int T>
+__device__ __forceinline__ double long_row(int r0)
+{
+    LzShared& C = lz_shared();
+    const DevSpin& up = C.J.S.up;
+    const int nup = up.count, k = C.S.k, ndp = lz_pad(C.J.S.dn.count), P = C.J.S.P;
+    const double* __restrict__ vk = lz_v(C.J, k);
+    const double* __restrict__ vp = lz_v(C.J, k - 1);
+    const double bk = C.S.b_cur, rb = C.rb, bp = C.S.b_prev, rp = C.rp;
+    double* xs = C.chunk;                                // [nup]
+    double acc = 0.0;
+    for (int iu = threadIdx.x; iu < nup; iu += T) copy_async8(xs + iu, vk + lz_index(r0, iu, ndp), true);
+    const int pd = __ldg(C.J.S.dn.imp + r0);
+    const double e1d = __ldg(C.J.S.dn.e1 + r0);
+    copy_async_wait_all();
+    __syncthreads();
+    auto fetch = [&](int id2, int iu2) { return __ldcg(vk + lz_index(id2, iu2, ndp)); };
+    for (int iu = threadIdx.x; iu < nup; iu += T) {
+        const unsigned o = lz_index(r0, iu, ndp);
+        const int hc = __ldg(up.hcnt + iu), pu = __ldg(up.imp + iu);
+        const double v = xs[iu];
+        double y = fma(__ldg(up.e1 + iu) + e1d + C.wint[pu * P + pd], v, __ldcg(C.J.Y + o));
+        for (int h = 0; h < hc; h++) {
+            const uint32_t e = __ldg(reinterpret_cast<const uint32_t*>(up.hpk) + ((size_t)(h >> 2) * nup + iu) * 4 + (h & 3));
+            y = fma(C.amp_up[edzt_hop_slot(e)], xs[edzt_hop_rank(e)], y);
+        }
+        if constexpr (X) { if (C.J.S.has_j) y = exchange_part(C.J.S, r0, iu, pu, pd, y, fetch); }
+        const double w = div_by(v, bk, rb);
+        y = fma(-bk, k == 1 ? 0.0 : div_by(__ldcg(vp + o), bp, rp), div_by(y, bk, rb));
+        __stcg(C.J.Y + o, y);
+        acc = fma(w, y, acc);
+        if (C.J.mode != LZ_COEFF) {
+            const double z = (k == 1) ? 0.0 : __ldcg(C.J.eig + o);
+            __stcg(C.J.eig + o, fma(C.J.coeff[k - 1], w, z));
+        }
+    }
+    __syncthreads();
+    return acc;
+}
+
+// NC planes of PW columns of a column tile; NR planes of PR rows of a row
+// tile (PR 1: one row); X: a model of the launch has exchange terms.
+template <int NC, int NR, int PW, int PR, bool X, int T>
 __global__ void __launch_bounds__(T, kLzThreads / T) k_lanczos(LzBatch B, const LzJob* __restrict__ jobs,
                                                            const long long* __restrict__ prefix, double* slots,
                                                            unsigned* sync, int* status)
@@ -582,7 +624,11 @@ __global__ void __launch_bounds__(T, kLzThreads / T) k_lanczos(LzBatch B, const 
                     }
                 } else {
 #pragma unroll 1
-                    for (; t < j_end; t += NR) acc += row_tile<NR, PW, X, T>((t - (int)C.J.ph[1].tile0) * PW, min(NR, j_end - t));
+                    for (; t < j_end; t += NR) {
+                        const int r0 = (t - (int)C.J.ph[1].tile0) * PR;
+                        if constexpr (PR == 1) acc += long_row<X, T>(r0);
+                        else acc += row_tile<NR, PR, X, T>(r0, min(NR, j_end - t));
+                    }
                 }
                 if (stalled) return;                     // fault test: leave without arriving
                 end_job(ph, acc);
@@ -620,17 +666,20 @@ using LzKernel = void (*)(LzBatch, const LzJob*, const long long*, double*, unsi
 // The kernel of a tile shape: wc columns by r rows.
 static LzKernel lz_kernel(const LzPlan& P)
 {
-#define EDZT_LZ(c, w, nc, nr, pw)                                                                        \
+#define EDZT_LZ(c, w, nc, nr, pw, pr)                                                                    \
     if (P.wc == c && P.r == w) {                                                                         \
         if (P.block == kLzThreads)                                                                       \
-            return P.exchange ? k_lanczos<nc, nr, pw, true, kLzThreads> : k_lanczos<nc, nr, pw, false, kLzThreads>; \
-        return P.exchange ? k_lanczos<nc, nr, pw, true, kLzThreads / 2> : k_lanczos<nc, nr, pw, false, kLzThreads / 2>; \
+            return P.exchange ? k_lanczos<nc, nr, pw, pr, true, kLzThreads>                              \
+                              : k_lanczos<nc, nr, pw, pr, false, kLzThreads>;                            \
+        return P.exchange ? k_lanczos<nc, nr, pw, pr, true, kLzThreads / 2>                              \
+                          : k_lanczos<nc, nr, pw, pr, false, kLzThreads / 2>;                            \
     }
-    EDZT_LZ(16, 8, 4, 2, 4)
-    EDZT_LZ(8, 8, 2, 2, 4)
-    EDZT_LZ(8, 4, 2, 1, 4)
-    EDZT_LZ(4, 4, 1, 1, 4)
-    EDZT_LZ(2, 2, 1, 1, 2)
+    EDZT_LZ(16, 8, 4, 2, 4, 4)
+    EDZT_LZ(8, 8, 2, 2, 4, 4)
+    EDZT_LZ(8, 4, 2, 1, 4, 4)
+    EDZT_LZ(4, 4, 1, 1, 4, 4)
+    EDZT_LZ(2, 2, 1, 1, 2, 2)
+    EDZT_LZ(2, 1, 1, 1, 2, 1)
 #undef EDZT_LZ
     return nullptr;
 }
@@ -714,7 +763,8 @@ LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, 
     };
     auto cut = [&](LzPlan& Q, std::vector<long long>& pre) {
         for (int j = 0; j < nj; j++) {
-            jobs[j].ph[0].width = jobs[j].ph[1].width = Q.wc >= 4 ? 4 : 2;
+            jobs[j].ph[0].width = std::min(Q.wc, 4);
+            jobs[j].ph[1].width = std::min(Q.r, 4);
             jobs[j].ph[0].planes = Q.wc / jobs[j].ph[0].width;
             jobs[j].ph[1].planes = Q.r / jobs[j].ph[1].width;
         }
@@ -737,7 +787,8 @@ LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, 
     // less than one CTA per SM has (us a step, one / two CTAs: 9 sectors of
     // nsite 12 106 / 99, of nsite 10 18.2 / 15.5; one sector of nsite 12
     // 23 / 31; 2 sectors of nsite 13 92 / 110).
-    if (!shape(P, 8, 8, kLzThreads) && !shape(P, 4, 4, kLzThreads)) shape(P, 2, 2, kLzThreads);
+    if (!shape(P, 8, 8, kLzThreads) && !shape(P, 4, 4, kLzThreads) && !shape(P, 2, 2, kLzThreads))
+        shape(P, 2, 1, kLzThreads);
     cut(P, prefix);
     LzPlan Q = P;
     if (P.wc == 8 && shape(Q, 8, 8, kLzThreads / 2)) {
