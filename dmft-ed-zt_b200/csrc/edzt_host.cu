@@ -240,6 +240,7 @@ struct edzt_ctx {
     int dbg_pass_cap = 0;
     unsigned long long dbg_wait_ns = 0;
     int dbg_stall_cta = -1;
+    double dbg_keep_limit = 0.0;            // test: bytes of kept vectors (0: the rules')
     // tile shapes chosen by edzt_tune_sector, by (up strings, down strings)
     struct Tuned { LzShape shape; double ms_per_step; };
     std::map<std::pair<int, int>, Tuned> tuned;
@@ -560,7 +561,12 @@ struct JobSpec {
     double* eig = nullptr;           // device, EIGVEC
     double* a = nullptr;             // device [maxnstep]
     double* b = nullptr;             // device [maxnstep]
-    double* keep = nullptr;          // device [maxnstep] vectors: keep every step's v (else ping-pong)
+    double* keep = nullptr;          // device, lz_keep_slots vectors: keep the v of the first keep_steps steps
+    int keep_steps = 0;
+    int resume = 0;                  // EIGVEC: go on at this step (>= 2) from
+    double* v_at = nullptr;          // its v, which is kept, and
+    double* v_before = nullptr;      // the one before (overwritten by later ones),
+    double b_before = 0.0;           // and the norm of that
     // results
     int nstep = 0;
     double norm0 = 0.0;
@@ -606,6 +612,7 @@ void fill_job(LzJob& J, const JobSpec& s, const DevSector& S)
     J.key = s.key;
     J.ac = s.ac;
     J.src = s.ac_src;
+    J.resume = s.resume;
 }
 
 // At least `bytes` of the context's pinned staging buffer; its last use is over
@@ -710,8 +717,11 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
         };
         J.Y = vec();
         if (s.keep) {
-            J.keep = 1;
+            J.keep = s.keep_steps;
             J.V[0] = s.keep;
+        } else if (s.resume) {
+            J.V[s.resume & 1] = s.v_at;
+            J.V[(s.resume & 1) ^ 1] = s.v_before;
         } else {
             J.V[0] = vec();
             J.V[1] = vec();
@@ -720,7 +730,14 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     }
     std::vector<LzState> st(2 * (size_t)nj);
     std::memset(st.data(), 0, sizeof(LzState) * st.size());
-    for (int j = 0; j < nj; j++) st[2 * (size_t)j + 1].active = 1;   // the state before phase 0 (parity 1)
+    for (int j = 0; j < nj; j++) {                                   // the state before phase 0 (parity 1)
+        LzState& n = st[2 * (size_t)j + 1];
+        n.active = 1;
+        if (specs[j].resume) {
+            n.k = specs[j].resume - 1;
+            n.b_cur = specs[j].b_before;
+        }
+    }
     int phases = 2 * max_steps + 4;     // two phases per step and the phase that closes the last one
     if (c->dbg_pass_cap > 0) phases = std::min(phases, c->dbg_pass_cap);
     const float ms = launch_jobs(c, jobs, st, force ? force : tuned_shape(c, jobs), phases, false);
@@ -1080,6 +1097,33 @@ void parallel_for(int n, int per_thread, F&& f)
     for (auto& x : th) x.join();
 }
 
+// How many of its maxnstep steps a scan over `states` states (as stored) may
+// keep the v_k of within `limit` bytes: all, or, with two buffers for the
+// others, at least half (a rerun from the last kept step then takes at most
+// half of one from the start), else 0.  300 steps of nsite 15, one sector:
+// 568 ms with none kept, 300 ms with the 285 that fit half of the memory.
+int keep_steps(const edzt_ctx* c, long long states, int maxnstep, double limit)
+{
+    if (!c->keep_vectors || states <= 0) return 0;
+    if (c->dbg_keep_limit > 0.0) limit = std::min(limit, c->dbg_keep_limit);
+    const double n = limit / ((double)states * sizeof(double));
+    if (n >= maxnstep) return maxnstep;
+    const int k = (int)n - 2;
+    return (k >= 2 && 2 * k >= maxnstep) ? k : 0;
+}
+
+// Device memory for kept vectors; nothing if there is none to be had (the
+// recurrence is rerun then).
+Lease<double> keep_lease(edzt_ctx* c, size_t n)
+{
+    try {
+        return Lease<double>(c->pool, n);
+    } catch (const EdztError& e) {
+        if (e.code != EDZT_ERR_OOM) throw;
+        return Lease<double>();
+    }
+}
+
 struct SectorResult {
     int nstep = 0;
     double norm0 = 0.0;
@@ -1087,6 +1131,14 @@ struct SectorResult {
     std::vector<double> a, b, coeff;
     bool ok = false;
 };
+
+// Weights of the kept v_k in sum_k coeff_k w_k, w_k = v_k / b_k (b = b(1..)).
+std::vector<double> keep_weights(const SectorResult& r, const double* b)
+{
+    std::vector<double> w(r.nstep);
+    for (int k = 0; k < r.nstep; k++) w[k] = r.coeff[k] / (k == 0 ? r.norm0 : b[k]);
+    return w;
+}
 
 // ground_state with diag_solver = 2: diag_arpack on every sector, the lowest
 // kept with the same strict rule and tie band as the Lanczos path.
@@ -1141,18 +1193,27 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
     std::vector<SectorResult> res(nsector);
     const int ns = nsite_of(c);
     auto vec_size = [&](int nu, int nd) { return lz_vec_size((int)edzt_binom(ns, nu), (int)edzt_binom(ns, nd)); };
-    // The scan keeps every step's v_k when they fit in half of the
-    // device memory that was free when the context was created (queried once:
-    // a query per solve can wait on the driver behind other processes'
-    // queries): the winner's eigenvector is then one pass over its kept v_k
-    // instead of a second run of the recurrence (the same sum, in the same
-    // order, of the same vectors).  The pool keeps the blocks for the next solve.
+    // The scan keeps the v_k of every step, or of as many first steps as fit,
+    // in at most half of the device memory that was free when the context was
+    // created (queried once: a query per solve can wait on the driver behind
+    // other processes' queries): the winner's eigenvector is then one pass over
+    // its kept v_k instead of a second run of the recurrence (the same sum, in
+    // the same order, of the same vectors), and a run only of the steps that
+    // were not kept.  The pool keeps the blocks for the next solve.
     std::vector<Lease<double>> kept(nsector);
-    bool keep = false;
-    if (c->engine == EDZT_ENGINE_FUSED && c->keep_vectors) {
+    int keep = 0;
+    if (c->engine == EDZT_ENGINE_FUSED) {
         long long states = 0;
         for (int i = 0; i < nsector; i++) states += vec_size(sectors[2 * i], sectors[2 * i + 1]);
-        keep = (double)states * maxnstep * sizeof(double) <= 0.5 * (double)c->free_at_create;
+        keep = keep_steps(c, states, maxnstep, 0.5 * (double)c->free_at_create);
+        for (int i = 0; i < nsector && keep; i++) {
+            const int nu = sectors[2 * i], nd = sectors[2 * i + 1];
+            if (sector_dim(c, nu, nd) <= 0) continue;
+            kept[i] = keep_lease(c, (size_t)lz_keep_slots(keep, maxnstep) * vec_size(nu, nd));
+            if (!kept[i].p) keep = 0;
+        }
+        if (!keep)
+            for (auto& k : kept) k = Lease<double>();
     }
     if (c->engine == EDZT_ENGINE_FUSED) {
         std::vector<JobSpec> specs;
@@ -1171,8 +1232,8 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             s.a = ab.p + (size_t)(2 * i) * maxnstep;
             s.b = ab.p + (size_t)(2 * i + 1) * maxnstep;
             if (keep) {
-                kept[i] = Lease<double>(c->pool, (size_t)maxnstep * vec_size(nu, nd));
                 s.keep = kept[i].p;
+                s.keep_steps = keep;
             }
             specs.push_back(s);
             which.push_back(i);
@@ -1213,12 +1274,14 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
         c->gs_vec = Lease<double>(c->pool, (size_t)dim);
         SectorResult& r = res[best];
         const DevSector Si = make_sector_mt(c, c->mt, nu, nd, true);
-        Lease<double> cf(c->pool, (size_t)r.nstep);
+        Lease<double> cf(c->pool, (size_t)r.nstep), cw(c->pool, (size_t)r.nstep);
+        std::vector<double> hw;
         if (keep) {
-            std::vector<double> hc(r.nstep);              // sum_k coeff_k w_k, w_k = v_k / b_k
-            for (int k = 0; k < r.nstep; k++) hc[k] = r.coeff[k] / (k == 0 ? r.norm0 : r.b[k]);
-            CK(cudaMemcpyAsync(cf.p, hc.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
-            launch_keep_combine(kept[best].p, Si, r.nstep, cf.p, c->gs_vec.p, c->stream);
+            hw = keep_weights(r, r.b.data());
+            CK(cudaMemcpyAsync(cw.p, hw.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
+        }
+        if (keep && r.nstep <= keep) {
+            launch_keep_combine(kept[best].p, Si, r.nstep, cw.p, c->gs_vec.p, true, c->stream);
             c->launches += 1;
             CKLAUNCH();
         } else {
@@ -1236,6 +1299,14 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             ev[0].eig = eig.p;
             ev[0].a = ab.p;
             ev[0].b = ab.p + maxnstep;
+            if (keep) {                                   // the kept steps but the last, which the run begins with
+                launch_keep_combine(kept[best].p, Si, keep - 1, cw.p, eig.p, false, c->stream);
+                c->launches += 1;
+                ev[0].resume = keep;
+                ev[0].v_at = kept[best].p + (size_t)(keep - 1) * vec_size(nu, nd);
+                ev[0].v_before = kept[best].p + (size_t)(keep - 2) * vec_size(nu, nd);
+                ev[0].b_before = (keep == 2) ? r.norm0 : r.b[keep - 2];
+            }
             run_jobs(c, ev);
             launch_to_natural(eig.p, Si, c->gs_vec.p, c->stream);
             c->launches += 1;
@@ -1659,10 +1730,47 @@ struct BatchInst {
     int best = -1, gs_up = 0, gs_dn = 0;
     double e0 = 0.0;
     Lease<double> gsvec;
+    Lease<double> kept;            // every step's v_k of every sector's scan, sector by sector; else empty
 };
 
+// Doubles of one step's v_k over all of an instance's sectors.
+long long scan_states(const BatchInst& I)
+{
+    long long n = 0;
+    for (size_t s = 0; s < I.sec.size() / 2; s++)
+        n += lz_vec_size((int)edzt_binom(I.model.nsite, I.sec[2 * s]), (int)edzt_binom(I.model.nsite, I.sec[2 * s + 1]));
+    return n;
+}
+
+// Let the scans of instances [i0, i1) keep their v_k, as long as `limit` bytes
+// last, so that no eigenvector pass has to rerun the winner's recurrence (16
+// instances of nsite 8 to 11: 16.5 -> 15.1 ms; 8 served ones of nsite 8 to 12:
+// 20.3 -> 17.9 ms).  All steps or none: the reruns of a wave share one launch,
+// whose length is that of the longest.
+void keep_scans(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxnstep, double limit)
+{
+    for (int i = i0; i < i1; i++) {
+        const long long n = scan_states(B[i]);
+        if (keep_steps(c, n, maxnstep, limit) < maxnstep) continue;
+        B[i].kept = keep_lease(c, (size_t)n * maxnstep);
+        if (!B[i].kept.p) return;
+        limit -= (double)n * maxnstep * sizeof(double);
+    }
+}
+
+// Point the scan of sector `sec` of an instance at its kept vectors, if it has any.
+void keep_in(const BatchInst& I, int sec, int maxnstep, JobSpec& j)
+{
+    if (!I.kept.p) return;
+    j.keep = I.kept.p;
+    for (int s = 0; s < sec; s++)
+        j.keep += maxnstep * lz_vec_size((int)edzt_binom(I.model.nsite, I.sec[2 * s]), (int)edzt_binom(I.model.nsite, I.sec[2 * s + 1]));
+    j.keep_steps = maxnstep;
+}
+
 void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxnstep, int nw,
-                const double* omega_dev, std::vector<double>& Gall, const std::vector<size_t>& goff)
+                const double* omega_dev, std::vector<double>& Gall, const std::vector<size_t>& goff,
+                double keep_limit)
 {
     for (int i = i0; i < i1; i++) {
         B[i].mt = std::make_unique<ModelTables>();
@@ -1695,6 +1803,8 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
         specs[q].a = ab.p + (size_t)(2 * q) * maxnstep;
         specs[q].b = ab.p + (size_t)(2 * q + 1) * maxnstep;
     }
+    keep_scans(c, B, i0, i1, maxnstep, keep_limit);
+    for (int q = 0; q < nj; q++) keep_in(B[own[q].inst], own[q].sector, maxnstep, specs[q]);
     run_jobs(c, specs);
     std::vector<double> hab((size_t)std::max(nj, 1) * 2 * maxnstep);
     CK(cudaMemcpyAsync(hab.data(), ab.p, sizeof(double) * hab.size(), cudaMemcpyDeviceToHost, c->stream));
@@ -1703,6 +1813,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     parallel_for(nj, 1 + 2000 / maxnstep, [&](int q) {   // a thread costs about 2,000 rows of tridiagonals
         SectorResult& r = res[q];
         r.nstep = specs[q].nstep;
+        r.norm0 = specs[q].norm0;
         if (r.nstep < 1) return;
         r.coeff.resize(r.nstep);
         r.ok = edzt::lowest_eigenpair(r.nstep, hab.data() + (size_t)(2 * q) * maxnstep,
@@ -1719,7 +1830,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     }
     // ---- eigenvector pass of every winner (lanczos_solver.f90:213-300)
     std::vector<JobSpec> ev;
-    std::vector<Lease<double>> eigs;          // the eigenvectors in internal order
+    std::vector<Lease<double>> eigs(i1 - i0); // the eigenvectors in internal order, where no v_k were kept
     Lease<double> coeffs(c->pool, (size_t)std::max(i1 - i0, 1) * maxnstep);
     std::vector<double> hcoef((size_t)std::max(i1 - i0, 1) * maxnstep, 0.0);
     for (int i = i0; i < i1; i++) {
@@ -1731,7 +1842,12 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
         I.e0 = res[q].e;
         I.gsvec = Lease<double>(c->pool, (size_t)sector_dim_ns(I.model.nsite, I.gs_up, I.gs_dn));
         const int ns = I.model.nsite;
-        eigs.emplace_back(c->pool, (size_t)lz_vec_size((int)edzt_binom(ns, I.gs_up), (int)edzt_binom(ns, I.gs_dn)));
+        if (I.kept.p) {
+            const std::vector<double> w = keep_weights(res[q], hab.data() + (size_t)(2 * q + 1) * maxnstep);
+            std::copy(w.begin(), w.end(), hcoef.begin() + (size_t)(i - i0) * maxnstep);
+            continue;
+        }
+        eigs[i - i0] = Lease<double>(c->pool, (size_t)lz_vec_size((int)edzt_binom(ns, I.gs_up), (int)edzt_binom(ns, I.gs_dn)));
         std::copy(res[q].coeff.begin(), res[q].coeff.end(), hcoef.begin() + (size_t)(i - i0) * maxnstep);
         JobSpec j;
         j.mt = I.mt.get();
@@ -1741,7 +1857,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
         j.key = specs[q].key;
         j.maxnstep = res[q].nstep;
         j.coeff = coeffs.p + (size_t)(i - i0) * maxnstep;
-        j.eig = eigs.back().p;
+        j.eig = eigs[i - i0].p;
         j.a = specs[q].a;            // the coefficients of the scan, still on the device
         j.b = specs[q].b;
         ev.push_back(j);
@@ -1751,7 +1867,11 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     for (int i = i0; i < i1; i++) {   // normalise (lanczos_solver.f90:291)
         const long long n = sector_dim_ns(B[i].model.nsite, B[i].gs_up, B[i].gs_dn);
         const DevSector Si = make_sector_mt(c, *B[i].mt, B[i].gs_up, B[i].gs_dn, true);
-        launch_to_natural(eigs[i - i0].p, Si, B[i].gsvec.p, c->stream);
+        if (B[i].kept.p)
+            launch_keep_combine(specs[win[i]].keep, Si, res[win[i]].nstep, coeffs.p + (size_t)(i - i0) * maxnstep,
+                                B[i].gsvec.p, true, c->stream);
+        else launch_to_natural(eigs[i - i0].p, Si, B[i].gsvec.p, c->stream);
+        B[i].kept.reset();
         launch_dot(B[i].gsvec.p, B[i].gsvec.p, n, c->dot_part->as<double>(), c->scal->as<double>(), c->stream);
         launch_scale_inv_sqrt(B[i].gsvec.p, n, c->scal->as<double>(), c->stream);
         c->launches += 4;
@@ -1812,9 +1932,13 @@ void init_inst(const edzt_instance& in, BatchInst& I)
     I.footprint = std::max(gsb, cfb) + 64 * maxd;
 }
 
-// Device memory a batch leaves cached for the next call: allocating and freeing
-// it anew took most of a small batch's time.
+// Device memory a batch leaves cached for the next call (allocating and freeing
+// it anew took most of a small batch's time): 2 GiB, or a sixteenth of what was
+// free when the context was created.  Half of that is for kept v_k: freeing and
+// allocating a block anew costs 4 to 6 ms, more than the reruns that kept
+// vectors save in most batches.
 constexpr size_t kBatchKeep = (size_t)2 << 30;
+size_t batch_cache(const edzt_ctx* c) { return std::max(kBatchKeep, c->free_at_create / 16); }
 
 void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int maxnstep, int nw, const double* omega,
                       int* isector, double* e0, double* G_cl, size_t budget)
@@ -1829,6 +1953,7 @@ void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int max
     }
     long long all = 0;
     for (const BatchInst& I : B) all += I.footprint;
+    const bool asked = budget != 0;
     if (budget == 0 && all <= (long long)kBatchKeep) {
         budget = kBatchKeep;                              // one wave; no need to ask what is free
     } else if (budget == 0) {
@@ -1842,8 +1967,10 @@ void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int max
         int i1 = i0;
         long long sum = 0;
         while (i1 < ninst && (i1 == i0 || sum + B[i1].footprint <= (long long)budget)) sum += B[i1++].footprint;
-        solve_wave(c, B, i0, i1, maxnstep, nw, om.d, Gall, goff);
-        c->pool.trim_to(kBatchKeep);
+        double keep = 0.5 * (double)batch_cache(c);
+        if (asked) keep = std::min(keep, (double)budget - (double)sum);
+        solve_wave(c, B, i0, i1, maxnstep, nw, om.d, Gall, goff, keep);
+        c->pool.trim_to(batch_cache(c));
         i0 = i1;
     }
     for (int i = 0; i < ninst; i++) {
@@ -1872,7 +1999,7 @@ void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int max
 struct LiveJob {
     JobSpec spec;
     DevSector S{};
-    Lease<double> y, v0, v1;
+    Lease<double> y, v0, v1;               // v0, v1: where the v_k are not kept
     LzState st[2] = {};                    // by phase parity, between slices
     int k = 0;                             // steps done (host view, from the last slice)
     bool done = false;
@@ -1895,6 +2022,7 @@ struct ServReq {
     Lease<double> gab;                     // [nruns][2][maxnstep] Green's-run coefficients (device)
     std::vector<double> G;                 // G_cl(nw, norb, nspin), complex interleaved
     std::vector<std::unique_ptr<LiveJob>> jobs;   // the live runs of the current phase
+    long long kept_bytes = 0;              // of the kept vectors, while the scan runs
     std::string error;
 };
 
@@ -1905,6 +2033,7 @@ struct edzt_server {
     int maxnstep = 0, nw = 0;
     std::unique_ptr<DevBuf> omega;
     long long budget = 0, reserved = 0, next_id = 1;
+    long long kept = 0;                    // of reserved: bytes of kept vectors
     double step_ms = 25.0;                 // time budget of one step
     int last_cls = -1;                     // class served by the last step
     std::map<int, double> ms_per_phase;    // measured phase time by class
@@ -1914,6 +2043,30 @@ struct edzt_server {
 };
 
 namespace {
+
+// Let an admitted request's scan keep its v_k: within a 32nd of the memory free
+// at creation and an eighth of the budget over all requests, so that what is
+// kept hardly ever holds up an admission.
+void keep_request(edzt_server* sv, ServReq& q)
+{
+    const long long n = scan_states(q.I), bytes = n * sv->maxnstep * (long long)sizeof(double);
+    const double limit = std::min((double)sv->c->free_at_create / 32, (double)sv->budget / 8);
+    if (sv->reserved + bytes > sv->budget) return;
+    if (keep_steps(sv->c, n, sv->maxnstep, limit - (double)sv->kept) < sv->maxnstep) return;
+    q.I.kept = keep_lease(sv->c, (size_t)n * sv->maxnstep);
+    if (!q.I.kept.p) return;
+    q.kept_bytes = bytes;
+    sv->kept += bytes;
+    sv->reserved += bytes;
+}
+
+void drop_kept(edzt_server* sv, ServReq& q)
+{
+    q.I.kept.reset();
+    sv->kept -= q.kept_bytes;
+    sv->reserved -= q.kept_bytes;
+    q.kept_bytes = 0;
+}
 
 // Size class of a request: its nsite, the requests up to nsite 11 together.
 int size_class(const BatchInst& I) { return std::max(I.model.nsite, 11); }
@@ -1925,8 +2078,10 @@ std::unique_ptr<LiveJob> make_live(edzt_ctx* c, const JobSpec& spec)
     L->S = make_sector_mt(c, spec.mt ? *spec.mt : c->mt, spec.nu, spec.nd, true);
     const size_t n = (size_t)lz_vec_size(L->S.up.count, L->S.dn.count);
     L->y = Lease<double>(c->pool, n);
-    L->v0 = Lease<double>(c->pool, n);
-    L->v1 = Lease<double>(c->pool, n);
+    if (!spec.keep) {
+        L->v0 = Lease<double>(c->pool, n);
+        L->v1 = Lease<double>(c->pool, n);
+    }
     L->st[1].active = 1;                                 // the state before the first phase (parity 1)
     if (spec.mode == LZ_COEFF) {
         CK(cudaMemsetAsync(spec.a, 0, sizeof(double) * spec.maxnstep, c->stream));
@@ -1947,8 +2102,9 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases)
         LzJob& J = jobs[j];
         fill_job(J, L.spec, L.S);
         J.Y = L.y.p;
-        J.V[0] = L.v0.p;
+        J.V[0] = L.spec.keep ? L.spec.keep : L.v0.p;
         J.V[1] = L.v1.p;
+        J.keep = L.spec.keep_steps;
     }
     std::vector<LzState> st(2 * (size_t)nj);
     for (int j = 0; j < nj; j++) std::memcpy(&st[2 * (size_t)j], v[j]->st, 2 * sizeof(LzState));
@@ -1986,6 +2142,7 @@ void server_admit(edzt_server* sv)
         sv->reserved += q.I.footprint;
         q.I.mt = std::make_unique<ModelTables>();
         set_tables_model(c, *q.I.mt, q.I.model);
+        keep_request(sv, q);
         const int ns = (int)q.I.sec.size() / 2;
         q.ab = Lease<double>(c->pool, (size_t)std::max(ns, 1) * 2 * sv->maxnstep);
         q.cls = size_class(q.I);
@@ -2005,6 +2162,7 @@ void server_admit(edzt_server* sv)
             j.maxnstep = sv->maxnstep;
             j.a = q.ab.p + (size_t)(2 * s) * sv->maxnstep;
             j.b = q.ab.p + (size_t)(2 * s + 1) * sv->maxnstep;
+            keep_in(q.I, s, sv->maxnstep, j);
             q.job_of_sector[s] = (int)q.jobs.size();
             q.jobs.push_back(make_live(c, j));
         }
@@ -2020,75 +2178,18 @@ bool phase_done(const ServReq& q)
     return true;
 }
 
-// Scan finished: the tridiagonal ground state of every sector, the winner
-// (ground_state.f90:62-68, 1e-10 tie band) and its eigenvector pass.
-void after_scan(edzt_server* sv, ServReq& q)
-{
-    edzt_ctx* c = sv->c;
-    const int maxnstep = sv->maxnstep;
-    const int nsec = (int)q.I.sec.size() / 2;
-    q.hab.assign((size_t)std::max(nsec, 1) * 2 * maxnstep, 0.0);
-    CK(cudaMemcpyAsync(q.hab.data(), q.ab.p, sizeof(double) * q.hab.size(), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    q.res.assign(nsec, SectorResult{});
-    for (int s = 0; s < nsec; s++) {
-        const int jq = q.job_of_sector[s];
-        if (jq < 0) continue;
-        SectorResult& r = q.res[s];
-        r.nstep = q.jobs[jq]->spec.nstep;
-        if (r.nstep < 1) continue;
-        r.coeff.resize(r.nstep);
-        r.ok = edzt::lowest_eigenpair(r.nstep, q.hab.data() + (size_t)(2 * s) * maxnstep,
-                                      q.hab.data() + (size_t)(2 * s + 1) * maxnstep, &r.e, r.coeff.data()) == 0;
-    }
-    int w = -1;
-    for (int s = 0; s < nsec; s++) {
-        if (!q.res[s].ok) continue;
-        const double tie = 1.0e-10 * std::max(1.0, std::fabs(w < 0 ? 0.0 : q.res[w].e));
-        if (w < 0 || q.res[s].e < q.res[w].e - tie) w = s;
-    }
-    q.jobs.clear();
-    if (w < 0) { q.error = "no sector produced a ground state"; q.phase = 4; return; }
-    q.win = w;
-    q.I.best = w;
-    q.I.gs_up = q.I.sec[2 * w]; q.I.gs_dn = q.I.sec[2 * w + 1];
-    q.I.e0 = q.res[w].e;
-    q.I.gsvec = Lease<double>(c->pool, (size_t)sector_dim_ns(q.I.model.nsite, q.I.gs_up, q.I.gs_dn));
-    q.coef = Lease<double>(c->pool, (size_t)q.res[w].nstep);
-    CK(cudaMemcpyAsync(q.coef.p, q.res[w].coeff.data(), sizeof(double) * q.res[w].nstep, cudaMemcpyHostToDevice,
-                       c->stream));
-    JobSpec j;                                            // eigenvector pass (lanczos_solver.f90:213-300)
-    j.mt = q.I.mt.get();
-    j.nu = q.I.gs_up; j.nd = q.I.gs_dn;
-    j.mode = LZ_EIGVEC;
-    j.init = LZ_INIT_HASH;
-    j.key = edzt_stream_key(q.I.seed, (uint64_t)w);
-    j.maxnstep = q.res[w].nstep;
-    j.coeff = q.coef.p;
-    q.eig = Lease<double>(c->pool, (size_t)lz_vec_size((int)edzt_binom(q.I.model.nsite, q.I.gs_up),
-                                                       (int)edzt_binom(q.I.model.nsite, q.I.gs_dn)));
-    j.eig = q.eig.p;
-    j.a = q.ab.p + (size_t)(2 * w) * maxnstep;
-    j.b = q.ab.p + (size_t)(2 * w + 1) * maxnstep;
-    q.jobs.push_back(make_live(c, j));
-    q.phase = 2;
-}
-
-// Eigenvector pass finished: normalise it (lanczos_solver.f90:291) and start
+// The winner's vector is there: normalise it (lanczos_solver.f90:291) and start
 // the c / c^+ runs (dmft_green.f90:204-250).
-void after_eigvec(edzt_server* sv, ServReq& q)
+void start_green(edzt_server* sv, ServReq& q)
 {
     edzt_ctx* c = sv->c;
     const int maxnstep = sv->maxnstep;
     BatchInst& I = q.I;
     const long long n = sector_dim_ns(I.model.nsite, I.gs_up, I.gs_dn);
-    const DevSector Si = make_sector_mt(c, *I.mt, I.gs_up, I.gs_dn, true);
-    launch_to_natural(q.eig.p, Si, I.gsvec.p, c->stream);
     launch_dot(I.gsvec.p, I.gsvec.p, n, c->dot_part->as<double>(), c->scal->as<double>(), c->stream);
     launch_scale_inv_sqrt(I.gsvec.p, n, c->scal->as<double>(), c->stream);
-    c->launches += 4;
+    c->launches += 3;
     CKLAUNCH();
-    q.eig.reset();
     const bool even = !(I.nspin == 2 || I.gs_up != I.gs_dn);
     q.runs = cluster_runs(I.model.norb, even, I.gs_up, I.gs_dn);
     q.gab = Lease<double>(c->pool, std::max<size_t>(q.runs.size(), 1) * 2 * maxnstep);
@@ -2118,6 +2219,85 @@ void after_eigvec(edzt_server* sv, ServReq& q)
         q.jobs.push_back(make_live(c, j));
     }
     q.phase = 3;
+}
+
+// Scan finished: the tridiagonal ground state of every sector, the winner
+// (ground_state.f90:62-68, 1e-10 tie band) and its eigenvector pass.
+void after_scan(edzt_server* sv, ServReq& q)
+{
+    edzt_ctx* c = sv->c;
+    const int maxnstep = sv->maxnstep;
+    const int nsec = (int)q.I.sec.size() / 2;
+    q.hab.assign((size_t)std::max(nsec, 1) * 2 * maxnstep, 0.0);
+    CK(cudaMemcpyAsync(q.hab.data(), q.ab.p, sizeof(double) * q.hab.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    q.res.assign(nsec, SectorResult{});
+    for (int s = 0; s < nsec; s++) {
+        const int jq = q.job_of_sector[s];
+        if (jq < 0) continue;
+        SectorResult& r = q.res[s];
+        r.nstep = q.jobs[jq]->spec.nstep;
+        r.norm0 = q.jobs[jq]->spec.norm0;
+        if (r.nstep < 1) continue;
+        r.coeff.resize(r.nstep);
+        r.ok = edzt::lowest_eigenpair(r.nstep, q.hab.data() + (size_t)(2 * s) * maxnstep,
+                                      q.hab.data() + (size_t)(2 * s + 1) * maxnstep, &r.e, r.coeff.data()) == 0;
+    }
+    int w = -1;
+    for (int s = 0; s < nsec; s++) {
+        if (!q.res[s].ok) continue;
+        const double tie = 1.0e-10 * std::max(1.0, std::fabs(w < 0 ? 0.0 : q.res[w].e));
+        if (w < 0 || q.res[s].e < q.res[w].e - tie) w = s;
+    }
+    const double* kept = (w >= 0 && q.I.kept.p) ? q.jobs[q.job_of_sector[w]]->spec.keep : nullptr;
+    q.jobs.clear();
+    if (w < 0) { q.error = "no sector produced a ground state"; q.phase = 4; return; }
+    q.win = w;
+    q.I.best = w;
+    q.I.gs_up = q.I.sec[2 * w]; q.I.gs_dn = q.I.sec[2 * w + 1];
+    q.I.e0 = q.res[w].e;
+    q.I.gsvec = Lease<double>(c->pool, (size_t)sector_dim_ns(q.I.model.nsite, q.I.gs_up, q.I.gs_dn));
+    q.coef = Lease<double>(c->pool, (size_t)q.res[w].nstep);
+    if (kept) {
+        const std::vector<double> wt = keep_weights(q.res[w], q.hab.data() + (size_t)(2 * w + 1) * maxnstep);
+        CK(cudaMemcpyAsync(q.coef.p, wt.data(), sizeof(double) * wt.size(), cudaMemcpyHostToDevice, c->stream));
+        const DevSector Si = make_sector_mt(c, *q.I.mt, q.I.gs_up, q.I.gs_dn, true);
+        launch_keep_combine(kept, Si, q.res[w].nstep, q.coef.p, q.I.gsvec.p, true, c->stream);
+        c->launches += 1;
+        CKLAUNCH();
+        drop_kept(sv, q);
+        start_green(sv, q);
+        return;
+    }
+    CK(cudaMemcpyAsync(q.coef.p, q.res[w].coeff.data(), sizeof(double) * q.res[w].nstep, cudaMemcpyHostToDevice,
+                       c->stream));
+    JobSpec j;                                            // eigenvector pass (lanczos_solver.f90:213-300)
+    j.mt = q.I.mt.get();
+    j.nu = q.I.gs_up; j.nd = q.I.gs_dn;
+    j.mode = LZ_EIGVEC;
+    j.init = LZ_INIT_HASH;
+    j.key = edzt_stream_key(q.I.seed, (uint64_t)w);
+    j.maxnstep = q.res[w].nstep;
+    j.coeff = q.coef.p;
+    q.eig = Lease<double>(c->pool, (size_t)lz_vec_size((int)edzt_binom(q.I.model.nsite, q.I.gs_up),
+                                                       (int)edzt_binom(q.I.model.nsite, q.I.gs_dn)));
+    j.eig = q.eig.p;
+    j.a = q.ab.p + (size_t)(2 * w) * maxnstep;
+    j.b = q.ab.p + (size_t)(2 * w + 1) * maxnstep;
+    q.jobs.push_back(make_live(c, j));
+    q.phase = 2;
+}
+
+// Eigenvector pass finished: its result in the reference's order.
+void after_eigvec(edzt_server* sv, ServReq& q)
+{
+    edzt_ctx* c = sv->c;
+    const DevSector Si = make_sector_mt(c, *q.I.mt, q.I.gs_up, q.I.gs_dn, true);
+    launch_to_natural(q.eig.p, Si, q.I.gsvec.p, c->stream);
+    c->launches += 1;
+    CKLAUNCH();
+    q.eig.reset();
+    start_green(sv, q);
 }
 
 // Green's runs finished: continued fractions and G_cl.
@@ -2218,6 +2398,7 @@ int server_step(edzt_server* sv)
             ServReq& q = **it;
             q.jobs.clear();
             q.I.gsvec.reset(); q.I.mt.reset(); q.ab.reset(); q.coef.reset(); q.eig.reset(); q.gab.reset();
+            drop_kept(sv, q);
             sv->reserved -= q.I.footprint;
             sv->finished[q.id] = std::move(*it);
             it = sv->active.erase(it);
@@ -2815,6 +2996,14 @@ int edzt_set_fault_test(edzt_ctx* c, int pass_cap, double wait_seconds, int stal
         c->dbg_pass_cap = pass_cap;
         c->dbg_wait_ns = (unsigned long long)(wait_seconds * 1e9);
         c->dbg_stall_cta = stall_cta;
+    });
+}
+
+int edzt_set_keep_limit_test(edzt_ctx* c, double bytes)
+{
+    return guarded(c, [&] {
+        arg_check(bytes >= 0.0, "bad limit");
+        c->dbg_keep_limit = bytes;
     });
 }
 

@@ -53,7 +53,7 @@ int edzt_max_hops(const DevModel& m, int sigma, int n);
 // sum_{k=1..nstep} coeff[k-1] v_k, accumulated in step order as the
 // eigenvector pass does.
 void launch_keep_combine(const double* keep, const DevSector& S, int nstep, const double* coeff, double* out,
-                         cudaStream_t s);
+                         bool natural, cudaStream_t s);
 // out (the reference's order) = v (a run's vector).
 void launch_to_natural(const double* v, const DevSector& S, double* out, cudaStream_t s);
 // y = H x, or y += H x (accumulate), of a sector in the reference's string order.
@@ -147,7 +147,7 @@ struct LzState {
 struct LzJob {
     DevSector S;          // spin tables in internal order
     double* Y;            // y_k; between a step's phases D, the down-hop part of H v_k
-    double* V[2];         // v_k, unnormalised: step k at V[k & 1]; keep: step k at V[0] + (k - 1) * lz_vec_size
+    double* V[2];         // v_k, unnormalised, by lz_v
     double* eig;          // EIGVEC: output eigenvector (unnormalised)
     const double* coeff;  // EIGVEC: ground eigenvector of the tridiagonal [nstep]
     double* a;            // [maxnstep] a(1..), written as steps are accepted
@@ -155,7 +155,8 @@ struct LzJob {
     int maxnstep;         // COEFF: LanczosSteps; EIGVEC: nstep of the coefficient pass
     int mode;
     int init;
-    int keep;             // 1: every step's v is kept ([maxnstep] vectors at V[0])
+    int keep;             // first steps whose v is kept, in lz_keep_slots vectors at V[0] (0: none)
+    int resume;           // EIGVEC: the first step, its v and the one before given (0: step 1, from the start vector)
     LzPhase ph[2];
     LzState* st;          // [2] the run's state by phase parity (kept across launches of a sliced run)
     uint64_t key;         // LZ_INIT_HASH
@@ -174,11 +175,15 @@ __host__ __device__ inline unsigned lz_index(int id, int iu, int ndp)
 // Doubles of one vector of a run.
 __host__ __device__ inline long long lz_vec_size(int nup, int ndn) { return (long long)lz_pad(nup) * lz_pad(ndn); }
 
-// v_k of a run (k = 0: never read).
-__host__ __device__ inline double* lz_v(const LzJob& J, int k)
+// v_k of a run (k = 0: never read): two buffers in turn, or one slot for each
+// of the first `keep` steps and two behind them in turn for the others.
+__host__ __device__ inline double* lz_v(const LzJob& J, int k, long long size)
 {
-    return J.keep ? J.V[0] + (k > 0 ? k - 1 : 0) * lz_vec_size(J.S.up.count, J.S.dn.count) : J.V[k & 1];
+    if (!J.keep) return J.V[k & 1];
+    const int i = k > 0 ? k - 1 : 0;
+    return J.V[0] + (i < J.keep ? i : J.keep + ((i - J.keep) & 1)) * size;
 }
+__host__ __device__ constexpr int lz_keep_slots(int keep, int maxnstep) { return keep < maxnstep ? keep + 2 : maxnstep; }
 
 struct LzBatch {
     int njobs;

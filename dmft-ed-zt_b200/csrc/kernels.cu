@@ -126,7 +126,8 @@ void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, c
 // src/lanczos_solver.f90:213-300, without rerunning the recurrence).
 // ---------------------------------------------------------------------------
 // A run's vectors are read in storage order (lz_index), coalesced, eight of
-// them in flight per thread; the results go to the reference's order.
+// them in flight per thread; the results go to the reference's order, or stay
+// in storage order where the recurrence goes on from them.
 // Storage position e of a run's vector as its place in the reference's order (-1: padding).
 __device__ __forceinline__ long long natural_of(unsigned e, int nup, int ndn, const int32_t* __restrict__ natu,
                                                 const int32_t* __restrict__ natd)
@@ -138,7 +139,7 @@ __device__ __forceinline__ long long natural_of(unsigned e, int nup, int ndn, co
 }
 
 __global__ void __launch_bounds__(256) k_keep_combine(const double* __restrict__ keep, int nup, int ndn, int nstep,
-                                                      const double* __restrict__ coeff,
+                                                      const double* __restrict__ coeff, int natural,
                                                       const int32_t* __restrict__ natu,
                                                       const int32_t* __restrict__ natd, double* __restrict__ out)
 {
@@ -148,20 +149,21 @@ __global__ void __launch_bounds__(256) k_keep_combine(const double* __restrict__
         double acc = 0.0;
 #pragma unroll 8
         for (int k = 0; k < nstep; k++) acc = fma(__ldg(coeff + k), __ldcs(v + k * stride), acc);
-        const long long o = natural_of((unsigned)e, nup, ndn, natu, natd);
+        const long long o = natural ? natural_of((unsigned)e, nup, ndn, natu, natd) : e;
         if (o >= 0) out[o] = acc;
     }
 }
 
 void launch_keep_combine(const double* keep, const DevSector& S, int nstep, const double* coeff, double* out,
-                         cudaStream_t s)
+                         bool natural, cudaStream_t s)
 {
     if (S.dim <= 0 || nstep <= 0) return;
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const long long blocks = std::min<long long>((S.dim + 255) / 256, 8LL * nsm);
-    k_keep_combine<<<(unsigned)blocks, 256, 0, s>>>(keep, S.up.count, S.dn.count, nstep, coeff, S.up.nat, S.dn.nat, out);
+    k_keep_combine<<<(unsigned)blocks, 256, 0, s>>>(keep, S.up.count, S.dn.count, nstep, coeff, natural, S.up.nat,
+                                                    S.dn.nat, out);
 }
 
 __global__ void __launch_bounds__(256) k_to_natural(const double* __restrict__ v, int nup, int ndn,

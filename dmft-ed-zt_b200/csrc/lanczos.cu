@@ -52,10 +52,13 @@
 // one another, and a small run's phases are synchronised over its own few
 // CTAs.
 //
-// The v_k of a run are ping-pong buffers, or (LzJob::keep) one slot per
-// step, so that the eigenvector can be summed from them afterwards.  The
-// eigenvector pass (LZ_EIGVEC) instead reruns the recurrence with the stored
-// a, b (src/lanczos_solver.f90:213-300) and accumulates sum_k coeff_k w_k.
+// The v_k of a run are ping-pong buffers, or (LzJob::keep) one slot for each
+// of its first steps, so that the eigenvector can be summed from them
+// afterwards.  The eigenvector pass (LZ_EIGVEC) reruns the recurrence with the
+// stored a, b (src/lanczos_solver.f90:213-300) and accumulates
+// sum_k coeff_k w_k: all of it, or (LzJob::resume) from the last kept step on,
+// whose column phase stages the kept v_k, so every later vector has the bits
+// of the scan's.
 //
 // A launch may be a slice of longer runs (LzBatch::slice): when its phase
 // budget runs out, a closing pass opens every unfinished run's next step
@@ -137,6 +140,8 @@ struct LzShared {
     int* status;
     unsigned long long wait_ns;
     double sum;                              // this CTA's partial sum of the last phase
+    double *vk, *vp;                         // v_k, v_{k-1}
+    long long vsize;                         // doubles of a vector
     double rb, rp;                           // 1 / S.b_cur, 1 / S.b_prev (0 before the second step)
     int job, phase;                          // what J and S hold
     int ok;
@@ -194,6 +199,7 @@ __device__ __forceinline__ bool begin_job(int j, int p, bool closing)
             C.amp_up = C.wint + C.J.S.P * C.J.S.P;
             C.amp_dn = C.amp_up + C.J.S.up.namp;
             C.dg = C.amp_dn + C.J.S.dn.namp;
+            C.vsize = lz_vec_size(C.J.S.up.count, C.J.S.dn.count);
         }
         __syncthreads();
         stage_table(C.J.S.wint, C.J.S.P * C.J.S.P, C.wint);
@@ -279,6 +285,8 @@ __device__ __forceinline__ bool begin_job(int j, int p, bool closing)
                     atomicOr(word, kDone);
                 }
             }
+            C.vk = lz_v(C.J, k, C.vsize);
+            C.vp = lz_v(C.J, k - 1, C.vsize);
             C.rb = 1.0 / n.b_cur;
             C.rp = (k >= 2 && ph == 1) ? 1.0 / n.b_prev : 0.0;
             C.job = j;
@@ -315,6 +323,7 @@ __device__ __forceinline__ void end_job(int ph, double acc)
 // t, t + 1, ...: stage v_k on their columns of every row, store it, sum v^2,
 // write the down-hop part of H v_k over y.  Returns this thread's share of
 // the sum.
+// col_init: step 1 from the start vector, or a resumed step from its kept v_k.
 template <int PW>
 __device__ __noinline__ double col_init(int np)
 {
@@ -322,19 +331,24 @@ __device__ __noinline__ double col_init(int np)
     LzShared& C = lz_shared();
     const int nup = C.J.S.up.count, ndn = C.J.S.dn.count, ndp = lz_pad(ndn), ps = ndp * PW, n = ndp * H;
     double* ws = C.chunk;
-    double* vk = lz_v(C.J, 1);
+    double* vk = C.vk;
+    const bool kept = C.S.k > 1;
     double acc = 0.0;
     for (int q = 0; q < np; q++)
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
             const int id = i / (4 * H) * 4 + 2 * (i & 1), cc = (i >> 1) & (PW - 1), c = C.c0[q] + cc;
             double2 v = make_double2(0.0, 0.0);
-            if (c < nup && id < ndn) v.x = init_value(C.J, id, c);
-            if (c < nup && id + 1 < ndn) v.y = init_value(C.J, id + 1, c);
+            const unsigned o = (unsigned)(C.c0[q] / 4 * 4 * ndp) + (H == 2 ? 2u * i : (unsigned)(i / 4 * 16 + (C.c0[q] & 2) * 4 + i % 4 * 2));
+            if (kept) {
+                v = __ldcg(reinterpret_cast<const double2*>(vk + o));
+            } else {
+                if (c < nup && id < ndn) v.x = init_value(C.J, id, c);
+                if (c < nup && id + 1 < ndn) v.y = init_value(C.J, id + 1, c);
+                __stcg(reinterpret_cast<double2*>(vk + o), v);
+            }
             double* d = ws + q * ps + id * PW + cc;
             d[0] = v.x;
             d[PW] = v.y;
-            const unsigned o = (unsigned)(C.c0[q] / 4 * 4 * ndp) + (H == 2 ? 2u * i : (unsigned)(i / 4 * 16 + (C.c0[q] & 2) * 4 + i % 4 * 2));
-            __stcg(reinterpret_cast<double2*>(vk + o), v);
             acc = fma(v.x, v.x, acc);
             acc = fma(v.y, v.y, acc);
         }
@@ -351,7 +365,7 @@ __device__ __forceinline__ double col_tile(int np, int t_next)
     const DevSpin& dn = C.J.S.dn;
     const int nup = C.J.S.up.count, ndn = dn.count, k = C.S.k, ndp = lz_pad(ndn), ps = ndp * PW;
     double* ws = C.chunk;                              // [NP][ndp][PW]
-    double* __restrict__ vk = lz_v(C.J, k);
+    double* __restrict__ vk = C.vk;
     double* __restrict__ yd = C.J.Y;
     // Staged item i of plane q: 16 bytes, two rows of one column.  A slab of
     // four columns is one contiguous run of blocks (a slab of two the halves
@@ -374,10 +388,10 @@ __device__ __forceinline__ double col_tile(int np, int t_next)
         acc = fma(v.x, v.x, acc);
         acc = fma(v.y, v.y, acc);
     };
-    if (k == 1) {
+    if (k == 1 || k == C.J.resume) {
         acc = col_init<PW>(np);
     } else {
-        const double* __restrict__ vp = lz_v(C.J, k - 1);
+        const double* __restrict__ vp = C.vp;
         const double am = -C.S.a_prev, bp = C.S.b_cur, rp = C.rb;
         constexpr int U = T > 256 ? 4 : 3;       // pairs of y and of v_{k-1} in flight per thread
 #pragma unroll 1
@@ -443,8 +457,8 @@ __device__ __forceinline__ double row_tile(int r0, int np)
     double acc = 0.0;
     const DevSpin& up = C.J.S.up;
     const int nup = up.count, ndn = C.J.S.dn.count, k = C.S.k, ndp = lz_pad(ndn), P = C.J.S.P;
-    const double* __restrict__ vk = lz_v(C.J, k);
-    const double* __restrict__ vp = lz_v(C.J, k - 1);
+    const double* __restrict__ vk = C.vk;
+    const double* __restrict__ vp = C.vp;
     double* __restrict__ yd = C.J.Y;
     const double bk = C.S.b_cur, rb = C.rb, bp = C.S.b_prev, rp = C.rp;
     const bool first = (k == 1);
@@ -540,8 +554,8 @@ __device__ __forceinline__ double long_row(int r0)
     LzShared& C = lz_shared();
     const DevSpin& up = C.J.S.up;
     const int nup = up.count, k = C.S.k, ndp = lz_pad(C.J.S.dn.count), P = C.J.S.P;
-    const double* __restrict__ vk = lz_v(C.J, k);
-    const double* __restrict__ vp = lz_v(C.J, k - 1);
+    const double* __restrict__ vk = C.vk;
+    const double* __restrict__ vp = C.vp;
     const double bk = C.S.b_cur, rb = C.rb, bp = C.S.b_prev, rp = C.rp;
     double* xs = C.chunk;                                // [nup]
     double acc = 0.0;

@@ -154,10 +154,15 @@ int edzt_diag_arpack(edzt_ctx *ctx, int ne_up, int ne_dn, uint64_t seed, uint64_
 #define EDZT_DIAG_ARPACK 2
 int edzt_set_diag_solver(edzt_ctx *ctx, int diag_solver);
 
-/* Whether ground_state's fused scan keeps every step's Lanczos vectors for
- * the eigenvector (edzt_ground_state): 1 (default) when they fit in half of
- * the device memory free at context creation, 0 never (the winner's recurrence is run again, as
- * src/lanczos_solver.f90:213-300 does).  Anything else EDZT_ERR_ARG. */
+/* Whether a fused scan keeps its Lanczos vectors for the eigenvector: 1
+ * (default) or 0 never (the winner's recurrence is run again, as
+ * src/lanczos_solver.f90:213-300 does).  Anything else EDZT_ERR_ARG.
+ * edzt_ground_state and edzt_solve keep every step's vector, or of the first
+ * steps as many as fit if that is at least half of them (only the others are
+ * run again), in at most half of the device memory free at context creation.
+ * The batched form keeps what fits in a 32nd of it (and in hbm_budget beside
+ * the instances), a server in a 32nd of it and an eighth of its budget.
+ * Where the memory is not to be had, the recurrence is run again. */
 int edzt_set_keep_vectors(edzt_ctx *ctx, int keep);
 
 /* ground_state (src/ground_state.f90:1-81): scans sectors[nsector][2] =
@@ -312,6 +317,10 @@ int edzt_clear_tuning(edzt_ctx *ctx);
  * out and the call returns EDZT_ERR_TIMEOUT.  All zero / -1: normal
  * operation.  The context stays usable after either error. */
 int edzt_set_fault_test(edzt_ctx *ctx, int pass_cap, double wait_seconds, int stall_cta);
+
+/* Test of the kept Lanczos vectors: at most `bytes` of them per scan, besides
+ * the limits that hold anyway (0: only those). */
+int edzt_set_keep_limit_test(edzt_ctx *ctx, double bytes);
 
 /* ---- the DMFT loop around the solver (host code, dmft_loop.cpp) ----------
  * The caller of the path, restated so that a whole DMFT run needs no
