@@ -183,6 +183,8 @@ struct OpsTable {
     uint4* hpk = nullptr;
     int32_t* sub = nullptr;
     uint8_t *hcnt = nullptr, *imp = nullptr;
+    SpinBuild build{};                      // what its launch gets
+    bool built = false;
 };
 
 // The model-dependent tables of one impurity model: per-spin operator tables
@@ -196,11 +198,12 @@ struct ModelTables {
     std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> ops;    // strings in the reference's order
     std::map<std::pair<int, int>, std::unique_ptr<OpsTable>> iops;   // strings in internal order
     std::map<std::pair<int, int>, DevSector> hx;                     // sectors looked up for H.v
-    std::vector<char> host;                 // wint, jcnt and jt as uploaded
+    std::vector<char> host;                 // wint, jt, the model and jcnt as uploaded
     Lease<char> block;                      // the same on the device
     double* wint = nullptr;
     int* jcnt = nullptr;
     JTrans* jt = nullptr;
+    DevModel* dmodel = nullptr;
 };
 
 }  // namespace
@@ -285,11 +288,16 @@ StrTable& int_table_ns(edzt_ctx* c, int ns, int n, int norb)
 
 StrTable& str_table(edzt_ctx* c, int n) { return str_table_ns(c, nsite_of(c), n); }
 
-// The operator tables of (n, sigma), strings in the reference's order or (internal) in internal order.
-OpsTable& ops_table_mt(edzt_ctx* c, ModelTables& mt, int n, int sigma, bool internal)
+// The operator tables of (n, sigma), strings in the reference's order or
+// (internal) in internal order.  One that is not built yet goes on the list
+// `todo`, for build_ops.
+OpsTable& ops_table_mt(edzt_ctx* c, ModelTables& mt, int n, int sigma, bool internal, std::vector<OpsTable*>& todo)
 {
     auto& ref = (internal ? mt.iops : mt.ops)[std::make_pair(n, sigma)];
-    if (ref) return *ref;
+    if (ref) {
+        if (!ref->built) todo.push_back(ref.get());
+        return *ref;
+    }
     const int norb = mt.model.norb, nbath = mt.model.nbath;
     StrTable& st = internal ? int_table_ns(c, mt.model.nsite, n, norb) : str_table_ns(c, mt.model.nsite, n);
     auto t = std::make_unique<OpsTable>();
@@ -315,12 +323,25 @@ OpsTable& ops_table_mt(edzt_ctx* c, ModelTables& mt, int n, int sigma, bool inte
     t->hcnt = reinterpret_cast<uint8_t*>(d + o_hcnt);
     t->imp = reinterpret_cast<uint8_t*>(d + o_imp);
     t->sub = mt.has_j ? reinterpret_cast<int32_t*>(d + o_sub) : nullptr;
-    launch_build_spin_ops(mt.model, sigma, st.count, st.str->as<uint32_t>(), st.rank->as<int32_t>(), t->hw, t->e1,
-                          t->hcnt, reinterpret_cast<uint32_t*>(t->hpk), t->amp, t->imp, t->sub, c->stream);
-    c->launches += 1;
-    CKLAUNCH();
+    t->build = SpinBuild{mt.dmodel, st.str->as<uint32_t>(), st.rank->as<int32_t>(), t->e1, t->hcnt,
+                         reinterpret_cast<uint32_t*>(t->hpk), t->amp, t->imp, t->sub, sigma, st.count, t->hw};
     ref = std::move(t);
+    todo.push_back(ref.get());
     return *ref;
+}
+
+// Build the listed tables (some may be listed twice).
+void build_ops(edzt_ctx* c, const std::vector<OpsTable*>& todo)
+{
+    std::vector<SpinBuild> b;
+    for (OpsTable* t : todo) {
+        if (t->built) continue;
+        t->built = true;
+        b.push_back(t->build);
+    }
+    if (b.empty()) return;
+    c->launches += launch_build_spin_ops(b.data(), (int)b.size(), c->stream);
+    CKLAUNCH();
 }
 
 bool sector_valid_ns(int ns, int nu, int nd) { return nu >= 0 && nd >= 0 && nu <= ns && nd <= ns; }
@@ -336,15 +357,19 @@ bool sector_valid(const edzt_ctx* c, int nu, int nd) { return sector_valid_ns(ns
 long long sector_dim(const edzt_ctx* c, int nu, int nd) { return sector_dim_ns(nsite_of(c), nu, nd); }
 
 // The sector of (nu, nd) with its tables in the reference's string order, or
-// (internal) in the internal order of the Lanczos runs.
-DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd, bool internal)
+// (internal) in the internal order of the Lanczos runs.  With a list `later`
+// the caller builds the tables put on it (build_ops) before their use.
+DevSector make_sector_mt(edzt_ctx* c, ModelTables& mt, int nu, int nd, bool internal,
+                         std::vector<OpsTable*>* later = nullptr)
 {
+    std::vector<OpsTable*> now, &todo = later ? *later : now;
     DevSector S{};
     const int ns = mt.model.nsite, norb = mt.model.norb;
     StrTable& su = internal ? int_table_ns(c, ns, nu, norb) : str_table_ns(c, ns, nu);
     StrTable& sd = internal ? int_table_ns(c, ns, nd, norb) : str_table_ns(c, ns, nd);
-    OpsTable& ou = ops_table_mt(c, mt, nu, 0, internal);
-    OpsTable& od = ops_table_mt(c, mt, nd, 1, internal);
+    OpsTable& ou = ops_table_mt(c, mt, nu, 0, internal, todo);
+    OpsTable& od = ops_table_mt(c, mt, nd, 1, internal, todo);
+    build_ops(c, now);
     auto fill = [&](DevSpin& sp, StrTable& st, OpsTable& o) {
         sp.count = st.count;
         sp.hw = o.hw;
@@ -382,8 +407,11 @@ const DevSector& make_sector(edzt_ctx* c, int nu, int nd)
 {
     auto it = c->mt.hx.find(std::make_pair(nu, nd));
     if (it != c->mt.hx.end()) return it->second;
-    make_sector_mt(c, c->mt, nu, nd, true);
-    return c->mt.hx.emplace(std::make_pair(nu, nd), make_sector_mt(c, c->mt, nu, nd, false)).first->second;
+    std::vector<OpsTable*> todo;
+    make_sector_mt(c, c->mt, nu, nd, true, &todo);
+    const DevSector S = make_sector_mt(c, c->mt, nu, nd, false, &todo);
+    build_ops(c, todo);
+    return c->mt.hx.emplace(std::make_pair(nu, nd), S).first->second;
 }
 
 // Interaction tables over impurity occupation patterns (pu, pd).
@@ -442,14 +470,17 @@ void build_model_tables(edzt_ctx* c, ModelTables& mt)
         }
     mt.has_j = any_j;
     const size_t nw = sizeof(double) * P * P, nj = sizeof(JTrans) * jt.size();   // 8-byte multiples, jcnt last
-    mt.host.resize(nw + nj + sizeof(int) * P * P);
+    const size_t nm = sizeof(DevModel);
+    mt.host.resize(nw + nj + nm + sizeof(int) * P * P);
     std::memcpy(mt.host.data(), w.data(), nw);
     std::memcpy(mt.host.data() + nw, jt.data(), nj);
-    std::memcpy(mt.host.data() + nw + nj, jc.data(), sizeof(int) * P * P);
+    std::memcpy(mt.host.data() + nw + nj, &m, nm);
+    std::memcpy(mt.host.data() + nw + nj + nm, jc.data(), sizeof(int) * P * P);
     mt.block = Lease<char>(c->pool, mt.host.size());
     mt.wint = reinterpret_cast<double*>(mt.block.p);
     mt.jt = reinterpret_cast<JTrans*>(mt.block.p + nw);
-    mt.jcnt = reinterpret_cast<int*>(mt.block.p + nw + nj);
+    mt.dmodel = reinterpret_cast<DevModel*>(mt.block.p + nw + nj);
+    mt.jcnt = reinterpret_cast<int*>(mt.block.p + nw + nj + nm);
     CK(cudaMemcpyAsync(mt.block.p, mt.host.data(), mt.host.size(), cudaMemcpyHostToDevice, c->stream));
 }
 
@@ -707,10 +738,11 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     std::vector<Lease<double>> bufs;
     bufs.reserve((size_t)nj * 3);
     int max_steps = 0;
+    std::vector<OpsTable*> todo;
     for (int j = 0; j < nj; j++) {
         JobSpec& s = specs[j];
         LzJob& J = jobs[j];
-        fill_job(J, s, make_sector_mt(c, s.mt ? *s.mt : c->mt, s.nu, s.nd, true));
+        fill_job(J, s, make_sector_mt(c, s.mt ? *s.mt : c->mt, s.nu, s.nd, true, &todo));
         auto vec = [&] {
             bufs.emplace_back(c->pool, (size_t)lz_vec_size(J.S.up.count, J.S.dn.count));
             return bufs.back().p;
@@ -728,6 +760,7 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
         }
         max_steps = std::max(max_steps, J.maxnstep);
     }
+    build_ops(c, todo);
     std::vector<LzState> st(2 * (size_t)nj);
     std::memset(st.data(), 0, sizeof(LzState) * st.size());
     for (int j = 0; j < nj; j++) {                                   // the state before phase 0 (parity 1)
@@ -881,16 +914,38 @@ void normalise(edzt_ctx* c, double* vec, long long n)
     c->launches += 3;
 }
 
-double finish_eigvec(edzt_ctx* c, const DevSector& S, double* vec, double e0)
+// ||H v - E0 v||^2 of a normalised v.
+double residual(edzt_ctx* c, const DevSector& S, double* vec, double e0)
 {
     const long long n = S.dim;
-    normalise(c, vec, n);
     Lease<double> v(c->pool, (size_t)n);
     launch_hx(S, vec, v.p, 0, c->stream);
     launch_axpy(v.p, vec, n, nullptr, e0, -1.0, c->stream);
     c->launches += 2;
     CKLAUNCH();
     return plain_dot(c, v.p, v.p, n);
+}
+
+double finish_eigvec(edzt_ctx* c, const DevSector& S, double* vec, double e0)
+{
+    normalise(c, vec, S.dim);
+    return residual(c, S, vec, e0);
+}
+
+// A run's vector sum over nstep vectors from v on, in the reference's order.
+VecSum natural_sum(const DevSector& S, const double* v, const double* coeff, int nstep, double* out)
+{
+    return VecSum{v, coeff, out, S.up.nat, S.dn.nat, S.up.count, S.dn.count, nstep, 1, nullptr};
+}
+
+// Form the sums and normalise them (lanczos_solver.f90:291).
+void normalised_sums(edzt_ctx* c, std::vector<VecSum>& r)
+{
+    if (r.empty()) return;
+    Lease<double> part(c->pool, r.size() * kVecSumBlocks);
+    for (size_t i = 0; i < r.size(); i++) r[i].part = part.p + i * kVecSumBlocks;
+    c->launches += launch_vec_sum_normalised(r.data(), (int)r.size(), c->stream);
+    CKLAUNCH();
 }
 
 // ---------------------------------------------------------------------------
@@ -1281,9 +1336,8 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             CK(cudaMemcpyAsync(cw.p, hw.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
         }
         if (keep && r.nstep <= keep) {
-            launch_keep_combine(kept[best].p, Si, r.nstep, cw.p, c->gs_vec.p, true, c->stream);
-            c->launches += 1;
-            CKLAUNCH();
+            std::vector<VecSum> vs{natural_sum(Si, kept[best].p, cw.p, r.nstep, c->gs_vec.p)};
+            normalised_sums(c, vs);
         } else {
             Lease<double> ab(c->pool, (size_t)2 * maxnstep), eig(c->pool, (size_t)vec_size(nu, nd));
             CK(cudaMemcpyAsync(cf.p, r.coeff.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
@@ -1300,22 +1354,21 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             ev[0].a = ab.p;
             ev[0].b = ab.p + maxnstep;
             if (keep) {                                   // the kept steps but the last, which the run begins with
-                launch_keep_combine(kept[best].p, Si, keep - 1, cw.p, eig.p, false, c->stream);
-                c->launches += 1;
+                VecSum vs = natural_sum(Si, kept[best].p, cw.p, keep - 1, eig.p);
+                vs.natural = 0;
+                c->launches += launch_vec_sum(&vs, 1, c->stream);
+                CKLAUNCH();
                 ev[0].resume = keep;
                 ev[0].v_at = kept[best].p + (size_t)(keep - 1) * vec_size(nu, nd);
                 ev[0].v_before = kept[best].p + (size_t)(keep - 2) * vec_size(nu, nd);
                 ev[0].b_before = (keep == 2) ? r.norm0 : r.b[keep - 2];
             }
             run_jobs(c, ev);
-            launch_to_natural(eig.p, Si, c->gs_vec.p, c->stream);
-            c->launches += 1;
-            CKLAUNCH();
+            std::vector<VecSum> vs{natural_sum(Si, eig.p, nullptr, 1, c->gs_vec.p)};
+            normalised_sums(c, vs);
         }
         for (auto& k : kept) k = Lease<double>();
-        if (want_residual) c->gs_residual = finish_eigvec(c, make_sector(c, nu, nd), c->gs_vec.p, r.e);
-        else normalise(c, c->gs_vec.p, dim);
-        CKLAUNCH();
+        if (want_residual) c->gs_residual = residual(c, make_sector(c, nu, nd), c->gs_vec.p, r.e);
         c->gs_up = nu; c->gs_dn = nd; c->gs_isector = best; c->gs_e0 = r.e;
     } else {
         // plain engine: diag_lanczos per sector, eigenvector for every sector
@@ -1864,20 +1917,17 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     }
     CK(cudaMemcpyAsync(coeffs.p, hcoef.data(), sizeof(double) * hcoef.size(), cudaMemcpyHostToDevice, c->stream));
     run_jobs(c, ev);
-    for (int i = i0; i < i1; i++) {   // normalise (lanczos_solver.f90:291)
-        const long long n = sector_dim_ns(B[i].model.nsite, B[i].gs_up, B[i].gs_dn);
+    std::vector<VecSum> vs;
+    for (int i = i0; i < i1; i++) {
         const DevSector Si = make_sector_mt(c, *B[i].mt, B[i].gs_up, B[i].gs_dn, true);
         if (B[i].kept.p)
-            launch_keep_combine(specs[win[i]].keep, Si, res[win[i]].nstep, coeffs.p + (size_t)(i - i0) * maxnstep,
-                                B[i].gsvec.p, true, c->stream);
-        else launch_to_natural(eigs[i - i0].p, Si, B[i].gsvec.p, c->stream);
-        B[i].kept.reset();
-        launch_dot(B[i].gsvec.p, B[i].gsvec.p, n, c->dot_part->as<double>(), c->scal->as<double>(), c->stream);
-        launch_scale_inv_sqrt(B[i].gsvec.p, n, c->scal->as<double>(), c->stream);
-        c->launches += 4;
+            vs.push_back(natural_sum(Si, specs[win[i]].keep, coeffs.p + (size_t)(i - i0) * maxnstep, res[win[i]].nstep,
+                                     B[i].gsvec.p));
+        else vs.push_back(natural_sum(Si, eigs[i - i0].p, nullptr, 1, B[i].gsvec.p));
     }
+    normalised_sums(c, vs);
+    for (int i = i0; i < i1; i++) B[i].kept.reset();
     eigs.clear();
-    CKLAUNCH();
     // ---- Green's function runs of every instance (dmft_green.f90:47-126)
     std::vector<GreenRun> runs;
     std::vector<size_t> r0(B.size(), 0);
@@ -2071,11 +2121,12 @@ void drop_kept(edzt_server* sv, ServReq& q)
 // Size class of a request: its nsite, the requests up to nsite 11 together.
 int size_class(const BatchInst& I) { return std::max(I.model.nsite, 11); }
 
-std::unique_ptr<LiveJob> make_live(edzt_ctx* c, const JobSpec& spec)
+// A live run; the tables it needs go on `todo`.
+std::unique_ptr<LiveJob> make_live(edzt_ctx* c, const JobSpec& spec, std::vector<OpsTable*>& todo)
 {
     auto L = std::make_unique<LiveJob>();
     L->spec = spec;
-    L->S = make_sector_mt(c, spec.mt ? *spec.mt : c->mt, spec.nu, spec.nd, true);
+    L->S = make_sector_mt(c, spec.mt ? *spec.mt : c->mt, spec.nu, spec.nd, true, &todo);
     const size_t n = (size_t)lz_vec_size(L->S.up.count, L->S.dn.count);
     L->y = Lease<double>(c->pool, n);
     if (!spec.keep) {
@@ -2137,6 +2188,7 @@ void server_admit(edzt_server* sv)
 {
     edzt_ctx* c = sv->c;
     while (!sv->queue.empty()) {
+        std::vector<OpsTable*> todo;
         ServReq& q = *sv->queue.front();
         if (!sv->active.empty() && sv->reserved + q.I.footprint > sv->budget) break;
         sv->reserved += q.I.footprint;
@@ -2164,8 +2216,9 @@ void server_admit(edzt_server* sv)
             j.b = q.ab.p + (size_t)(2 * s + 1) * sv->maxnstep;
             keep_in(q.I, s, sv->maxnstep, j);
             q.job_of_sector[s] = (int)q.jobs.size();
-            q.jobs.push_back(make_live(c, j));
+            q.jobs.push_back(make_live(c, j, todo));
         }
+        build_ops(c, todo);
         sv->active.push_back(std::move(sv->queue.front()));
         sv->queue.pop_front();
     }
@@ -2178,23 +2231,18 @@ bool phase_done(const ServReq& q)
     return true;
 }
 
-// The winner's vector is there: normalise it (lanczos_solver.f90:291) and start
-// the c / c^+ runs (dmft_green.f90:204-250).
+// The winner's vector is there: start the c / c^+ runs (dmft_green.f90:204-250).
 void start_green(edzt_server* sv, ServReq& q)
 {
     edzt_ctx* c = sv->c;
     const int maxnstep = sv->maxnstep;
     BatchInst& I = q.I;
-    const long long n = sector_dim_ns(I.model.nsite, I.gs_up, I.gs_dn);
-    launch_dot(I.gsvec.p, I.gsvec.p, n, c->dot_part->as<double>(), c->scal->as<double>(), c->stream);
-    launch_scale_inv_sqrt(I.gsvec.p, n, c->scal->as<double>(), c->stream);
-    c->launches += 3;
-    CKLAUNCH();
     const bool even = !(I.nspin == 2 || I.gs_up != I.gs_dn);
     q.runs = cluster_runs(I.model.norb, even, I.gs_up, I.gs_dn);
     q.gab = Lease<double>(c->pool, std::max<size_t>(q.runs.size(), 1) * 2 * maxnstep);
     CK(cudaMemsetAsync(q.gab.p, 0, sizeof(double) * std::max<size_t>(q.runs.size(), 1) * 2 * maxnstep, c->stream));
     q.jobs.clear();
+    std::vector<OpsTable*> todo;
     const int ns = I.model.nsite;
     for (size_t r = 0; r < q.runs.size(); r++) {
         GreenRun& g = q.runs[r];
@@ -2216,8 +2264,9 @@ void start_green(edzt_server* sv, ServReq& q)
         j.maxnstep = maxnstep;
         j.a = g.a; j.b = g.b;
         g.nstep = -1 - (int)q.jobs.size();              // its live run, resolved when it finishes
-        q.jobs.push_back(make_live(c, j));
+        q.jobs.push_back(make_live(c, j, todo));
     }
+    build_ops(c, todo);
     q.phase = 3;
 }
 
@@ -2262,9 +2311,8 @@ void after_scan(edzt_server* sv, ServReq& q)
         const std::vector<double> wt = keep_weights(q.res[w], q.hab.data() + (size_t)(2 * w + 1) * maxnstep);
         CK(cudaMemcpyAsync(q.coef.p, wt.data(), sizeof(double) * wt.size(), cudaMemcpyHostToDevice, c->stream));
         const DevSector Si = make_sector_mt(c, *q.I.mt, q.I.gs_up, q.I.gs_dn, true);
-        launch_keep_combine(kept, Si, q.res[w].nstep, q.coef.p, q.I.gsvec.p, true, c->stream);
-        c->launches += 1;
-        CKLAUNCH();
+        std::vector<VecSum> vs{natural_sum(Si, kept, q.coef.p, q.res[w].nstep, q.I.gsvec.p)};
+        normalised_sums(c, vs);
         drop_kept(sv, q);
         start_green(sv, q);
         return;
@@ -2284,7 +2332,9 @@ void after_scan(edzt_server* sv, ServReq& q)
     j.eig = q.eig.p;
     j.a = q.ab.p + (size_t)(2 * w) * maxnstep;
     j.b = q.ab.p + (size_t)(2 * w + 1) * maxnstep;
-    q.jobs.push_back(make_live(c, j));
+    std::vector<OpsTable*> todo;
+    q.jobs.push_back(make_live(c, j, todo));
+    build_ops(c, todo);
     q.phase = 2;
 }
 
@@ -2293,9 +2343,8 @@ void after_eigvec(edzt_server* sv, ServReq& q)
 {
     edzt_ctx* c = sv->c;
     const DevSector Si = make_sector_mt(c, *q.I.mt, q.I.gs_up, q.I.gs_dn, true);
-    launch_to_natural(q.eig.p, Si, q.I.gsvec.p, c->stream);
-    c->launches += 1;
-    CKLAUNCH();
+    std::vector<VecSum> vs{natural_sum(Si, q.eig.p, nullptr, 1, q.I.gsvec.p)};
+    normalised_sums(c, vs);
     q.eig.reset();
     start_green(sv, q);
 }
@@ -2448,9 +2497,12 @@ int edzt_ctx_ready_sector(edzt_ctx* c, int nu, int nd, DevSector* S, const char*
     if (!sector_valid(c, nu, nd)) { *why = "electron counts outside [0, nsite]"; return EDZT_ERR_ARG; }
     const int ns = nsite_of(c);
     const int norb = c->mt.model.norb;
+    auto built = [&](int n, int sigma) {
+        const auto it = c->mt.iops.find(std::make_pair(n, sigma));
+        return it != c->mt.iops.end() && it->second && it->second->built;
+    };
     const bool ready = c->int_tables.count(std::make_tuple(ns, nu, norb)) &&
-                       c->int_tables.count(std::make_tuple(ns, nd, norb)) &&
-                       c->mt.iops.count(std::make_pair(nu, 0)) && c->mt.iops.count(std::make_pair(nd, 1));
+                       c->int_tables.count(std::make_tuple(ns, nd, norb)) && built(nu, 0) && built(nd, 1);
     if (!ready) {
         *why = "the sector's tables are not built on this context: make one allocating call on the sector "
                "first (edzt_hx or edzt_lanczos_iteration)";

@@ -41,21 +41,41 @@ void launch_build_strings(int nsite, int n, uint32_t* str, int32_t* rank, cudaSt
 // Per-string tables of one spin species (sigma = 0 up, 1 down) for a model.
 // hpk: [hw/4][count] uint4 (packed hop entries, see edzt_hop_pack); amp:
 // [2*norb*nbath] (at least 2) amplitude slots.
-void launch_build_spin_ops(const DevModel& m, int sigma, int count, const uint32_t* str, const int32_t* rank,
-                           int hw, double* e1, uint8_t* hcnt, uint32_t* hpk, double* amp, uint8_t* imp,
-                           int32_t* sub, cudaStream_t s);
+// One spin table to build: operators of `count` strings of spin sigma of a
+// model (on the device).  Returns the launches made.
+struct SpinBuild {
+    const DevModel* m;
+    const uint32_t* str;
+    const int32_t* rank;
+    double* e1;
+    uint8_t* hcnt;
+    uint32_t* hpk;
+    double* amp;
+    uint8_t* imp;
+    int32_t* sub;
+    int sigma, count, hw;
+};
+constexpr int kSpinBuilds = 40;            // per launch: they travel as its argument (4 KB)
+int launch_build_spin_ops(const SpinBuild* t, int n, cudaStream_t s);
 // Largest number of allowed hops of any string with n electrons of spin sigma.
 int edzt_max_hops(const DevModel& m, int sigma, int n);
 
 // ---- kernels.cu: standalone (non-persistent) kernels ------------------------
-// Ground-state vector from the kept vectors of a coefficient run (step k at
-// (k - 1) * lz_vec_size): out (the reference's order) =
-// sum_{k=1..nstep} coeff[k-1] v_k, accumulated in step order as the
-// eigenvector pass does.
-void launch_keep_combine(const double* keep, const DevSector& S, int nstep, const double* coeff, double* out,
-                         bool natural, cudaStream_t s);
-// out (the reference's order) = v (a run's vector).
-void launch_to_natural(const double* v, const DevSector& S, double* out, cudaStream_t s);
+// Sums of a run's vectors in step order, as the eigenvector pass adds them:
+// out = sum_k coeff[k] v_k (coeff null: v_1 itself).
+struct VecSum {
+    const double* v;          // v_1; one vector after the other
+    const double* coeff;      // [nstep] on the device
+    double* out;              // the reference's order (natural) or storage order
+    const int32_t *natu, *natd;
+    int nup, ndn, nstep, natural;
+    double* part;             // [kVecSumBlocks] scratch for the norm (natural)
+};
+constexpr int kVecSums = 48;               // per launch: they travel as its argument (4 KB)
+constexpr int kVecSumBlocks = 1184;
+int launch_vec_sum(const VecSum* r, int n, cudaStream_t s);
+// The same and out / ||out|| (natural only).
+int launch_vec_sum_normalised(const VecSum* r, int n, cudaStream_t s);
 // y = H x, or y += H x (accumulate), of a sector in the reference's string order.
 void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, cudaStream_t s);
 // Whether a sector's staged row and column slab fit in shared memory.

@@ -138,51 +138,87 @@ __device__ __forceinline__ long long natural_of(unsigned e, int nup, int ndn, co
     return (iu < nup && id < ndn) ? (long long)__ldg(natd + id) * nup + __ldg(natu + iu) : -1;
 }
 
-__global__ void __launch_bounds__(256) k_keep_combine(const double* __restrict__ keep, int nup, int ndn, int nstep,
-                                                      const double* __restrict__ coeff, int natural,
-                                                      const int32_t* __restrict__ natu,
-                                                      const int32_t* __restrict__ natd, double* __restrict__ out)
+struct VecSumArgs { VecSum r[kVecSums]; };
+
+// Blocks of a sum: one per 256 elements, at most eight per SM.
+__host__ __device__ inline int vec_sum_blocks(const VecSum& r)
 {
+    const long long b = (lz_vec_size(r.nup, r.ndn) + 255) / 256;
+    return b < kVecSumBlocks ? (int)b : kVecSumBlocks;
+}
+
+// blockIdx.y: the sum.  Bound by the read of the kept vectors; the sums of a
+// batch share a launch, as one alone fills the chip only from nsite 11 on (16
+// sums of nsite 8 to 11: 820 us apart).
+__global__ void __launch_bounds__(256) k_vec_sum(const __grid_constant__ VecSumArgs A)
+{
+    __shared__ double scratch[32];
+    const VecSum& R = A.r[blockIdx.y];
+    const int nb = vec_sum_blocks(R);
+    if ((int)blockIdx.x >= nb) return;
+    const int nup = R.nup, ndn = R.ndn, nstep = R.nstep;
+    const double* __restrict__ coeff = R.coeff;
     const long long stride = lz_vec_size(nup, ndn);
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < stride; e += (long long)gridDim.x * blockDim.x) {
-        const double* v = keep + e;                      // v_1
+    double sq[1] = {0.0};
+    for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < stride; e += (long long)nb * 256) {
+        const double* v = R.v + e;                       // v_1
         double acc = 0.0;
+        if (coeff) {
 #pragma unroll 8
-        for (int k = 0; k < nstep; k++) acc = fma(__ldg(coeff + k), __ldcs(v + k * stride), acc);
-        const long long o = natural ? natural_of((unsigned)e, nup, ndn, natu, natd) : e;
-        if (o >= 0) out[o] = acc;
+            for (int k = 0; k < nstep; k++) acc = fma(__ldg(coeff + k), __ldcs(v + k * stride), acc);
+        } else {
+            acc = __ldcs(v);
+        }
+        const long long o = R.natural ? natural_of((unsigned)e, nup, ndn, R.natu, R.natd) : e;
+        if (o >= 0) {
+            R.out[o] = acc;
+            sq[0] = fma(acc, acc, sq[0]);
+        }
+    }
+    if (R.natural) {
+        block_sum<1>(sq, scratch);
+        if (threadIdx.x == 0) R.part[blockIdx.x] = sq[0];
     }
 }
 
-void launch_keep_combine(const double* keep, const DevSector& S, int nstep, const double* coeff, double* out,
-                         bool natural, cudaStream_t s)
+// out / ||out||: every block adds up the partial sums itself, in the same order.
+__global__ void __launch_bounds__(256) k_vec_norm(const __grid_constant__ VecSumArgs A)
 {
-    if (S.dim <= 0 || nstep <= 0) return;
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const long long blocks = std::min<long long>((S.dim + 255) / 256, 8LL * nsm);
-    k_keep_combine<<<(unsigned)blocks, 256, 0, s>>>(keep, S.up.count, S.dn.count, nstep, coeff, natural, S.up.nat,
-                                                    S.dn.nat, out);
+    __shared__ double scratch[32], norm;
+    const VecSum& R = A.r[blockIdx.y];
+    const int nb = vec_sum_blocks(R);
+    if ((int)blockIdx.x >= nb) return;
+    double sum[1] = {0.0};
+    for (int i = threadIdx.x; i < nb; i += 256) sum[0] += R.part[i];
+    block_sum<1>(sum, scratch);
+    if (threadIdx.x == 0) norm = sqrt(sum[0]);
+    __syncthreads();
+    const double nrm = norm;
+    const long long n = (long long)R.nup * R.ndn;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)nb * 256) R.out[i] /= nrm;
 }
 
-__global__ void __launch_bounds__(256) k_to_natural(const double* __restrict__ v, int nup, int ndn,
-                                                    const int32_t* __restrict__ natu, const int32_t* __restrict__ natd,
-                                                    double* __restrict__ out)
+static int vec_sums(const VecSum* r, int n, bool norm, cudaStream_t s)
 {
-    const long long size = lz_vec_size(nup, ndn);
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < size; e += (long long)gridDim.x * blockDim.x) {
-        const long long o = natural_of((unsigned)e, nup, ndn, natu, natd);
-        if (o >= 0) out[o] = v[e];
+    int launches = 0;
+    for (int i = 0; i < n; i += kVecSums) {
+        VecSumArgs A;
+        const int k = std::min(kVecSums, n - i);
+        int blocks = 1;
+        for (int q = 0; q < k; q++) {
+            A.r[q] = r[i + q];
+            blocks = std::max(blocks, vec_sum_blocks(A.r[q]));
+        }
+        const dim3 grid((unsigned)blocks, (unsigned)k);
+        k_vec_sum<<<grid, 256, 0, s>>>(A);
+        if (norm) k_vec_norm<<<grid, 256, 0, s>>>(A);
+        launches += norm ? 2 : 1;
     }
+    return launches;
 }
 
-void launch_to_natural(const double* v, const DevSector& S, double* out, cudaStream_t s)
-{
-    if (S.dim <= 0) return;
-    const long long blocks = std::min<long long>((S.dim + 255) / 256, 148LL * 16);
-    k_to_natural<<<(unsigned)blocks, 256, 0, s>>>(v, S.up.count, S.dn.count, S.up.nat, S.dn.nat, out);
-}
+int launch_vec_sum(const VecSum* r, int n, cudaStream_t s) { return vec_sums(r, n, false, s); }
+int launch_vec_sum_normalised(const VecSum* r, int n, cudaStream_t s) { return vec_sums(r, n, true, s); }
 
 // ---------------------------------------------------------------------------
 // Deterministic dot product (mpi_dot_product, src/numeric_utils.f90:159-170):

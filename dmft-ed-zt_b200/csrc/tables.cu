@@ -108,12 +108,21 @@ __global__ void k_build_rank(int nsite, int n, int norb, int32_t* __restrict__ r
 }
 
 // Per string of one spin species: one-body energy, hop list, impurity bits
-// and the rank of every impurity-pattern substitution.
-__global__ void k_build_spin_ops(DevModel m, int sigma, int count, const uint32_t* __restrict__ str,
-                                 const int32_t* __restrict__ rank, int hw, double* __restrict__ e1,
-                                 uint8_t* __restrict__ hcnt, uint32_t* __restrict__ hpk,
-                                 double* __restrict__ amp, uint8_t* __restrict__ imp, int32_t* __restrict__ sub)
+// and the rank of every impurity-pattern substitution.  blockIdx.y: the table;
+// all tables that a call is about to use are built by one launch (16 models of
+// 7 tables each: 110 launches of 4 us and 5 us of host time apart before).
+struct SpinBuilds { SpinBuild t[kSpinBuilds]; };
+
+__global__ void k_build_spin_ops(const __grid_constant__ SpinBuilds tabs)
 {
+    const SpinBuild& B = tabs.t[blockIdx.y];
+    const DevModel& m = *B.m;
+    const int sigma = B.sigma, count = B.count, hw = B.hw;
+    const uint32_t* __restrict__ str = B.str;
+    const int32_t* __restrict__ rank = B.rank;
+    double* __restrict__ amp = B.amp;
+    uint32_t* __restrict__ hpk = B.hpk;
+    int32_t* __restrict__ sub = B.sub;
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0) {   // amplitude slots: +V at 2c, -V at 2c+1, c = iorb*nbath + jbath
         for (int a = 0; a < m.norb; a++)
@@ -132,7 +141,7 @@ __global__ void k_build_spin_ops(DevModel m, int sigma, int count, const uint32_
         if ((u >> a) & 1u) e += m.em[a][sigma] - m.mu;
     for (int l = 0; l < nbath; l++)
         if ((u >> (norb + l)) & 1u) e += m.ek[l][sigma];
-    e1[t] = e;
+    B.e1[t] = e;
     // hybridisation hops (impurity_hamiltonian.f90:146-174), loop order iorb, jbath;
     // entry h of string t sits at uint32 index ((h/4)*count + t)*4 + h%4
     auto slot_at = [&](int h) -> uint32_t& { return hpk[((size_t)(h >> 2) * count + t) * 4 + (h & 3)]; };
@@ -155,9 +164,9 @@ __global__ void k_build_spin_ops(DevModel m, int sigma, int count, const uint32_
         }
     }
     for (int q = h; q < hw; q++) slot_at(q) = 0u;
-    hcnt[t] = (uint8_t)h;
+    B.hcnt[t] = (uint8_t)h;
     const uint32_t P = 1u << norb;
-    imp[t] = (uint8_t)(u & (P - 1u));
+    B.imp[t] = (uint8_t)(u & (P - 1u));
     if (sub) {
         for (uint32_t p = 0; p < P; p++) sub[(size_t)t * P + p] = rank[(u & ~(P - 1u)) | p];
     }
@@ -178,12 +187,20 @@ void launch_build_strings(int nsite, int n, uint32_t* str, int32_t* rank, cudaSt
     k_build_rank<<<(nst + 255) / 256, 256, 0, s>>>(nsite, n, norb, rank);
 }
 
-void launch_build_spin_ops(const DevModel& m, int sigma, int count, const uint32_t* str, const int32_t* rank,
-                           int hw, double* e1, uint8_t* hcnt, uint32_t* hpk, double* amp, uint8_t* imp,
-                           int32_t* sub, cudaStream_t s)
+int launch_build_spin_ops(const SpinBuild* t, int n, cudaStream_t s)
 {
-    const int n = count > 0 ? count : 1;   // the amplitude slots are written even for an empty table
-    k_build_spin_ops<<<(n + 127) / 128, 128, 0, s>>>(m, sigma, count, str, rank, hw, e1, hcnt, hpk, amp, imp, sub);
+    int launches = 0;
+    for (int i = 0; i < n; i += kSpinBuilds, launches++) {
+        SpinBuilds B;
+        const int k = std::min(kSpinBuilds, n - i);
+        int most = 1;                      // the amplitude slots are written even for an empty table
+        for (int q = 0; q < k; q++) {
+            B.t[q] = t[i + q];
+            most = std::max(most, t[i + q].count);
+        }
+        k_build_spin_ops<<<dim3((unsigned)(most + 127) / 128, (unsigned)k), 128, 0, s>>>(B);
+    }
+    return launches;
 }
 
 // For an impurity pattern, bath site l gives e_l hops when it is empty (the

@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from conftest import random_model
+from test_gpu_batch import _check_against_alone
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-13
@@ -88,3 +89,15 @@ def test_batch_and_server_with_kept_vectors(pkg, solver, share):
     for (s1, e1, g1), (s2, e2, g2) in zip(kept, other):
         assert s1 == s2 and e1 == e2
         assert np.abs(np.asarray(g1) - np.asarray(g2)).max() <= 1e-10
+
+
+def test_batch_of_more_instances_than_one_launch_takes(pkg, solver):
+    """52 instances: the tables (40 per launch) and the vectors' sums (48) take
+    several launches.  Against every instance alone, as the other batches are
+    (the cut of a run over the CTAs, so the order of its sums, depends on what
+    else is in the launch)."""
+    rng = np.random.default_rng(5)
+    omega = pkg.matsubara(16, 20.0)
+    insts = [dict(model=random_model(pkg, rng, 1, 4 + i % 2), sectors=[(2, 2), (2, 3)], nspin=1, seed=900 + i)
+             for i in range(52)]
+    _check_against_alone(solver, insts, solver.solve_batch(insts, 8, omega), omega, 8)
