@@ -718,6 +718,35 @@ float launch_jobs(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& s
     return ms;
 }
 
+// The same with the kernel of small runs, which need no plan.
+float launch_small(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& st, size_t smem)
+{
+    const size_t nj = jobs.size(), bytes_st = sizeof(LzState) * st.size();
+    const size_t o_jobs = (bytes_st + 255) & ~(size_t)255, size = o_jobs + sizeof(LzJob) * nj;
+    Lease<char> blob(c->pool, size);
+    bool exchange = false;
+    long long most = 0;
+    for (size_t j = 0; j < nj; j++) {
+        most = std::max(most, jobs[j].S.dim);
+        jobs[j].st = reinterpret_cast<LzState*>(blob.p) + 2 * j;
+        exchange = exchange || jobs[j].S.has_j;
+    }
+    char* h = stage_buffer(c, size);
+    std::memcpy(h + o_jobs, jobs.data(), sizeof(LzJob) * nj);
+    const LzJob* d_jobs = reinterpret_cast<const LzJob*>(blob.p + o_jobs);
+    CK(cudaMemcpyAsync(blob.p + o_jobs, h + o_jobs, sizeof(LzJob) * nj, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaEventRecord(c->ev0, c->stream));
+    CK(launch_lanczos_small(d_jobs, (int)nj, smem, exchange, most, c->stream));
+    CK(cudaEventRecord(c->ev1, c->stream));
+    c->launches += 1;
+    CK(cudaMemcpyAsync(h, blob.p, bytes_st, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    std::memcpy(st.data(), h, bytes_st);
+    float ms = 0.0f;
+    CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+    return ms;
+}
+
 void book_launch(edzt_ctx* c, const std::vector<LzJob>& jobs, double ms, double bytes)
 {
     c->st_launches += 1;
@@ -743,24 +772,31 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
         JobSpec& s = specs[j];
         LzJob& J = jobs[j];
         fill_job(J, s, make_sector_mt(c, s.mt ? *s.mt : c->mt, s.nu, s.nd, true, &todo));
-        auto vec = [&] {
-            bufs.emplace_back(c->pool, (size_t)lz_vec_size(J.S.up.count, J.S.dn.count));
-            return bufs.back().p;
-        };
-        J.Y = vec();
         if (s.keep) {
             J.keep = s.keep_steps;
             J.V[0] = s.keep;
         } else if (s.resume) {
             J.V[s.resume & 1] = s.v_at;
             J.V[(s.resume & 1) ^ 1] = s.v_before;
-        } else {
-            J.V[0] = vec();
-            J.V[1] = vec();
         }
         max_steps = std::max(max_steps, J.maxnstep);
     }
     build_ops(c, todo);
+    const LzShape* shape = force ? force : tuned_shape(c, jobs);
+    const bool plain = !shape && c->dbg_pass_cap == 0 && c->dbg_stall_cta < 0;
+    const size_t small = plain ? lz_small_smem(jobs.data(), nj) : 0;
+    for (int j = 0; j < nj && !small; j++) {
+        LzJob& J = jobs[j];
+        auto vec = [&] {
+            bufs.emplace_back(c->pool, (size_t)lz_vec_size(J.S.up.count, J.S.dn.count));
+            return bufs.back().p;
+        };
+        J.Y = vec();
+        if (!J.V[0] && !J.V[1]) {
+            J.V[0] = vec();
+            J.V[1] = vec();
+        }
+    }
     std::vector<LzState> st(2 * (size_t)nj);
     std::memset(st.data(), 0, sizeof(LzState) * st.size());
     for (int j = 0; j < nj; j++) {                                   // the state before phase 0 (parity 1)
@@ -773,7 +809,7 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     }
     int phases = 2 * max_steps + 4;     // two phases per step and the phase that closes the last one
     if (c->dbg_pass_cap > 0) phases = std::min(phases, c->dbg_pass_cap);
-    const float ms = launch_jobs(c, jobs, st, force ? force : tuned_shape(c, jobs), phases, false);
+    const float ms = small ? launch_small(c, jobs, st, small) : launch_jobs(c, jobs, st, shape, phases, false);
     double bytes = 0.0;
     for (int j = 0; j < nj; j++) {
         // the final state is the finished one of the two parity copies

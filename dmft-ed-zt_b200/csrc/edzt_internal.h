@@ -248,6 +248,11 @@ bool lz_shape_fits(const DevSector& S, const LzShape& q);
 // slots: [P.slots] partial sums; sync_words: lz_sync_bytes(njobs), zeroed.
 cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const LzJob* jobs, const long long* prefix,
                                       double* slots, unsigned* sync_words, int* status, cudaStream_t s);
+// Small coefficient runs from start to finish, one CTA each: the shared memory
+// of a launch (0: some run is not of that kind), and the launch.
+size_t lz_small_smem(const LzJob* jobs, int njobs);
+cudaError_t launch_lanczos_small(const LzJob* jobs, int njobs, size_t smem, bool exchange, long long most_states,
+                                 cudaStream_t s);
 // Sync-word buffer size (bytes) for a launch of njobs runs.
 size_t lz_sync_bytes(int njobs);
 // The device-free part of lz_plan: given every job's widths (ph[].width) and

@@ -720,6 +720,263 @@ cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const L
 }
 
 // ---------------------------------------------------------------------------
+// small runs: one CTA a run, everything in shared memory
+// ---------------------------------------------------------------------------
+// Small runs spend their steps in the persistent kernel on latency: staging,
+// arrivals, the tables' way through L2, 4.5 us a phase even for a few hundred
+// states.  Here the last two v, y, the hop lists and the tables of a run stay
+// in the shared memory of one CTA, and a step is two sums over it.  Four rows
+// of a column share the decode of an up hop; 768 threads, since 512 left the
+// issue slots idle half of the time and 1,024 run out of columns.  Bound by
+// the instructions and wavefronts of the hop sums.  A step of a lone run, in
+// us (persistent kernel): 400 states 1.9 (8.7), 1,225 3.3 (8.7), 4,900 6.5
+// (8.8), with the v_k kept 1 more; 7,056 states 9.8 (8.9), so the line lies
+// at kLzSmallStates.  Up to a state per thread, 512 threads of one row.
+constexpr long long kLzSmallStates = 6000;
+constexpr size_t kLzSmallSmemMax = kLzSmemMax - 4096;   // besides the descriptor and the sums
+
+// Where a run's parts lie in shared memory, in bytes.
+struct LzSmall {
+    int hu, hd;                   // hop lists
+    int v, wint, amp_up, amp_dn, e1u, e1d;   // v: v0, v1 and y
+    int cu, cd, pu, pd;           // hop counts, impurity patterns
+    int size;
+};
+
+__host__ __device__ inline LzSmall lz_small_layout(const DevSector& S)
+{
+    LzSmall L;
+    int o = 0;
+    auto part = [&o](long long bytes) {
+        const int at = o;
+        o += (int)((bytes + 15) / 16 * 16);
+        return at;
+    };
+    L.hu = part(4LL * S.up.hw * S.up.count);
+    L.hd = part(4LL * S.dn.hw * S.dn.count);
+    L.v = part(24LL * S.dim);
+    L.wint = part(8LL * S.P * S.P);
+    L.amp_up = part(8LL * S.up.namp);
+    L.amp_dn = part(8LL * S.dn.namp);
+    L.e1u = part(8LL * S.up.count);
+    L.e1d = part(8LL * S.dn.count);
+    L.cu = part(S.up.count);
+    L.cd = part(S.dn.count);
+    L.pu = part(S.up.count);
+    L.pd = part(S.dn.count);
+    L.size = o;
+    return L;
+}
+
+// Sum over the CTA, the same in every thread.  Alternating buffers: the next
+// sum's writes need no barrier behind this one's reads.
+template <int T>
+__device__ __forceinline__ double cta_sum(double v, double* red)
+{
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = ((int)(threadIdx.x & 31) < T / 32) ? red[threadIdx.x & 31] : 0.0;
+    return __shfl_sync(0xffffffffu, warp_sum(v), 0);
+}
+
+// T threads; R: rows of one column that a thread sums at a time.
+template <int T, int R, bool X>
+__global__ void __launch_bounds__(T) k_lanczos_small(const LzJob* __restrict__ jobs)
+{
+    __shared__ LzJob J;
+    __shared__ double red[2][32];
+    {
+        const int* src = reinterpret_cast<const int*>(jobs + blockIdx.x);
+        int* dst = reinterpret_cast<int*>(&J);
+        for (int i = threadIdx.x; i < (int)(sizeof(LzJob) / sizeof(int)); i += T) dst[i] = __ldg(src + i);
+    }
+    __syncthreads();
+    const DevSpin &up = J.S.up, &dn = J.S.dn;
+    const int nup = up.count, ndn = dn.count, n = nup * ndn, P = J.S.P, ndp = lz_pad(ndn);
+    const LzSmall L = lz_small_layout(J.S);
+    uint4* hu = reinterpret_cast<uint4*>(lz_smem + L.hu);
+    uint4* hd = reinterpret_cast<uint4*>(lz_smem + L.hd);
+    double* v = reinterpret_cast<double*>(lz_smem + L.v);
+    double* vp = v + n;
+    double* y = vp + n;
+    double* wint = reinterpret_cast<double*>(lz_smem + L.wint);
+    double* amp_up = reinterpret_cast<double*>(lz_smem + L.amp_up);
+    double* amp_dn = reinterpret_cast<double*>(lz_smem + L.amp_dn);
+    double* e1u = reinterpret_cast<double*>(lz_smem + L.e1u);
+    double* e1d = reinterpret_cast<double*>(lz_smem + L.e1d);
+    unsigned char *cu = lz_smem + L.cu, *cd = lz_smem + L.cd, *pu = lz_smem + L.pu, *pd = lz_smem + L.pd;
+    for (int i = threadIdx.x; i < up.hw / 4 * nup; i += T) hu[i] = __ldg(up.hpk + i);
+    for (int i = threadIdx.x; i < dn.hw / 4 * ndn; i += T) hd[i] = __ldg(dn.hpk + i);
+    stage_table(J.S.wint, P * P, wint);
+    stage_table(up.amp, up.namp, amp_up);
+    stage_table(dn.amp, dn.namp, amp_dn);
+    stage_table(up.e1, nup, e1u);
+    stage_table(dn.e1, ndn, e1d);
+    for (int i = threadIdx.x; i < nup; i += T) { cu[i] = __ldg(up.hcnt + i); pu[i] = __ldg(up.imp + i); }
+    for (int i = threadIdx.x; i < ndn; i += T) { cd[i] = __ldg(dn.hcnt + i); pd[i] = __ldg(dn.imp + i); }
+    // e / nup = umulhi(e, magic) for e < n: the error e * nup / 2^32 stays below 1 / nup
+    const unsigned magic = nup > 1 ? 0xffffffffu / nup + 1 : 0;
+    auto row_of = [&](int e) { return nup > 1 ? (int)__umulhi((unsigned)e, magic) : e; };
+    const long long vsize = lz_vec_size(nup, ndn);
+    const int items = (ndn + R - 1) / R * nup;
+    double a = 0.0, bk = 1.0, rb = 1.0, bp = 1.0, rp = 0.0, norm0 = 0.0;   // a_{k-1}; b_k, b_{k-1} and their reciprocals
+    int nstep = 0;
+    for (int k = 1;; k++) {
+        double* kept = J.keep ? lz_v(J, k, vsize) : nullptr;
+        double acc = 0.0;
+        auto put = [&](int e, double x) {
+            v[e] = x;
+            acc = fma(x, x, acc);
+            if (kept) {
+                const int id = row_of(e);
+                __stcg(kept + lz_index(id, e - id * nup, ndp), x);
+            }
+        };
+        if (k == 1) {
+            for (int e = threadIdx.x; e < n; e += T) {
+                const int id = row_of(e);
+                put(e, init_value(J, id, e - id * nup));
+            }
+        } else {                                         // v_k = y - a_{k-1} w_{k-1}
+            for (int e0 = threadIdx.x; e0 < n; e0 += R * T) {
+                double x[R];
+#pragma unroll
+                for (int u = 0; u < R; u++) {
+                    const int e = e0 + u * T;
+                    if (e < n) x[u] = fma(-a, div_by(vp[e], bk, rb), y[e]);
+                }
+#pragma unroll
+                for (int u = 0; u < R; u++) {
+                    const int e = e0 + u * T;
+                    if (e < n) put(e, x[u]);
+                }
+            }
+        }
+        const double nrm = sqrt(cta_sum<T>(acc, red[0]));
+        bp = bk;
+        rp = rb;
+        if (k == 1) {                                    // ||v_init|| (:128-130); b(1) = 0 (:135)
+            norm0 = nrm;
+            if (threadIdx.x == 0) J.b[0] = 0.0;
+            if (!(nrm > 0.0)) break;                     // zero start vector
+        } else if (nrm < 1.0e-16) {                      // breakdown (:161)
+            if (threadIdx.x == 0) J.b[k - 1] = 0.0;
+            break;
+        } else if (threadIdx.x == 0) {
+            J.b[k - 1] = nrm;                            // b(k) = ||v_k|| (:144,167)
+        }
+        bk = nrm;
+        rb = 1.0 / bk;
+        acc = 0.0;
+        for (int i = threadIdx.x; i < items; i += T) {   // y = H w_k - b_k w_{k-1}
+            const int blk = row_of(i), iu = i - blk * nup, r0 = blk * R;
+            const double* line[R];                       // rows past the last one repeat it
+            double s[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int id = min(r0 + r, ndn - 1);
+                line[r] = v + id * nup;
+                s[r] = (e1u[iu] + e1d[id] + wint[pu[iu] * P + pd[id]]) * line[r][iu];
+            }
+            const int hcu = cu[iu];
+            for (int h0 = 0; h0 < hcu; h0 += 4) {
+                const uint4 q = hu[(h0 >> 2) * nup + iu];
+                const uint32_t f[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int h = 0; h < 4; h++)
+                    if (h0 + h < hcu) {
+                        const double am = amp_up[edzt_hop_slot(f[h])];
+                        const int t = edzt_hop_rank(f[h]);
+#pragma unroll
+                        for (int r = 0; r < R; r++) s[r] = fma(am, line[r][t], s[r]);
+                    }
+            }
+            int hcd[R], most = 0;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                hcd[r] = cd[min(r0 + r, ndn - 1)];
+                most = max(most, hcd[r]);
+            }
+            for (int h0 = 0; h0 < most; h0 += 4)
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    if (h0 >= hcd[r]) continue;
+                    const uint4 q = hd[(h0 >> 2) * ndn + min(r0 + r, ndn - 1)];
+                    const uint32_t f[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                    for (int h = 0; h < 4; h++)
+                        if (h0 + h < hcd[r]) s[r] = fma(amp_dn[edzt_hop_slot(f[h])], v[edzt_hop_rank(f[h]) * nup + iu], s[r]);
+                }
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int id = r0 + r;
+                if (id >= ndn) break;
+                if constexpr (X) {
+                    if (J.S.has_j)
+                        s[r] = exchange_part(J.S, id, iu, pu[iu], pd[id], s[r],
+                                             [&](int id2, int iu2) { return v[id2 * nup + iu2]; });
+                }
+                double z = div_by(s[r], bk, rb);
+                if (k > 1) z = fma(-bk, div_by(vp[id * nup + iu], bp, rp), z);
+                y[id * nup + iu] = z;
+                acc = fma(div_by(line[r][iu], bk, rb), z, acc);
+            }
+        }
+        a = cta_sum<T>(acc, red[1]);                        // a(k) = <w_k, y_k> (:134,159)
+        if (threadIdx.x == 0) J.a[k - 1] = a;
+        nstep = k;
+        if (k >= J.maxnstep) break;                      // :137-141, :161-164
+        double* t = v;
+        v = vp;
+        vp = t;
+    }
+    if (threadIdx.x == 0) {
+        LzState f;
+        f.k = nstep + 1;
+        f.active = f.opened = 0;
+        f.nstep = nstep;
+        f.a_prev = a;
+        f.b_cur = bk;
+        f.b_prev = bp;
+        f.norm0 = norm0;
+        J.st[0] = f;
+        J.st[1] = f;
+    }
+}
+
+// The shared memory that a launch of k_lanczos_small needs; 0: it does not
+// take these runs.
+size_t lz_small_smem(const LzJob* jobs, int nj)
+{
+    size_t most = 0;
+    for (int j = 0; j < nj; j++) {
+        if (jobs[j].mode != LZ_COEFF || jobs[j].S.dim > kLzSmallStates) return 0;
+        most = std::max(most, (size_t)lz_small_layout(jobs[j].S).size);
+    }
+    return most <= kLzSmallSmemMax ? most : 0;
+}
+
+cudaError_t launch_lanczos_small(const LzJob* jobs, int nj, size_t smem, bool exchange, long long most, cudaStream_t s)
+{
+    using Kernel = void (*)(const LzJob*);
+    static const Kernel kernels[2][2] = {{k_lanczos_small<512, 1, false>, k_lanczos_small<512, 1, true>},
+                                         {k_lanczos_small<768, 4, false>, k_lanczos_small<768, 4, true>}};
+    static std::atomic<unsigned long long> done{0};
+    if (edzt_once_per_device(done)) {
+        for (const auto& pair : kernels)
+            for (const Kernel k : pair) {
+                const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                           (int)kLzSmallSmemMax);
+                if (e != cudaSuccess) return e;
+            }
+    }
+    const bool big = most > 512;
+    kernels[big][exchange]<<<nj, big ? 768 : 512, smem, s>>>(jobs);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
 // launch plan
 // ---------------------------------------------------------------------------
 // Per-CTA dynamic shared memory: two 512-thread CTAs per SM when every job
