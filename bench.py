@@ -567,7 +567,7 @@ def run_gpu(args):
     launches = s.launch_count() - launches0
     ks = s.kernel_stats()
     # whether the solves ran an eigenvector pass (a launch over the winning
-    # sector alone) or took the eigenvector from the scan's kept pairs
+    # sector alone) or took the eigenvector from the scan's kept vectors
     eig_pass = any(e["states"] in [float(s.dim(u, d)) for u, d in sectors] for e in s.launch_log())
     total_ms = sum(lat)
     replicas = importlib.import_module("dmft_ed_zt_b200.replicas")
@@ -627,7 +627,7 @@ def run_gpu(args):
         # Lanczos state-steps of a solve in each engine: the plain engine runs
         # the eigenvector pass of every sector as the reference does, the
         # fused engine only the winner's (or none: the eigenvector from the
-        # scan's kept pairs), so part of the ratio is skipped work
+        # scan's kept vectors), so part of the ratio is skipped work
         dims = [s.dim(u, d) for u, d in sectors]
         gdim = sum(s.dim(u + du, d + dd) for (u, d) in [max(sectors, key=lambda q: s.dim(*q))]
                    for du, dd in ((1, 0), (-1, 0)))

@@ -757,6 +757,13 @@ void book_launch(edzt_ctx* c, const std::vector<LzJob>& jobs, double ms, double 
     log_launch(c, ms, bytes, states);
 }
 
+// Whether a run may take the kernel of small ones: no shape is tuned for its
+// sector and no fault test asks for the persistent kernel.
+bool small_allowed(const edzt_ctx* c, const LzJob& J)
+{
+    return c->dbg_pass_cap == 0 && c->dbg_stall_cta < 0 && !c->tuned.count({J.S.up.count, J.S.dn.count});
+}
+
 // All runs of specs from start to finish.  Coefficient runs write a and b up
 // to their last step only: the caller zeroes them.
 void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = nullptr)
@@ -782,10 +789,22 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
         max_steps = std::max(max_steps, J.maxnstep);
     }
     build_ops(c, todo);
-    const LzShape* shape = force ? force : tuned_shape(c, jobs);
-    const bool plain = !shape && c->dbg_pass_cap == 0 && c->dbg_stall_cta < 0;
-    const size_t small = plain ? lz_small_smem(jobs.data(), nj) : 0;
-    for (int j = 0; j < nj && !small; j++) {
+    // Runs for the kernel of small ones: those of a model that are all small,
+    // so that a model's runs take the same way alone and among others.
+    std::map<const ModelTables*, size_t> small_mem;
+    for (int j = 0; j < nj; j++) {
+        const size_t need = (force || !small_allowed(c, jobs[j])) ? 0 : lz_small_smem(jobs[j].S, jobs[j].mode);
+        const auto it = small_mem.emplace(specs[j].mt, need).first;
+        it->second = (need && it->second) ? std::max(need, it->second) : 0;
+    }
+    std::vector<int> order[2];                            // jobs of either kernel
+    size_t smem = 0;
+    for (int j = 0; j < nj; j++) {
+        const size_t m = small_mem[specs[j].mt];
+        order[m > 0].push_back(j);
+        smem = std::max(smem, m);
+    }
+    for (int j : order[0]) {
         LzJob& J = jobs[j];
         auto vec = [&] {
             bufs.emplace_back(c->pool, (size_t)lz_vec_size(J.S.up.count, J.S.dn.count));
@@ -809,22 +828,33 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     }
     int phases = 2 * max_steps + 4;     // two phases per step and the phase that closes the last one
     if (c->dbg_pass_cap > 0) phases = std::min(phases, c->dbg_pass_cap);
-    const float ms = small ? launch_small(c, jobs, st, small) : launch_jobs(c, jobs, st, shape, phases, false);
-    double bytes = 0.0;
-    for (int j = 0; j < nj; j++) {
-        // the final state is the finished one of the two parity copies
-        const LzState& s0 = st[2 * (size_t)j];
-        const LzState& s1 = st[2 * (size_t)j + 1];
-        const LzState* fin = !s0.active ? &s0 : (!s1.active ? &s1 : nullptr);
-        if (!fin) throw EdztError{EDZT_ERR_NUMERIC, "Lanczos run did not finish within the pass limit"};
-        specs[j].nstep = fin->nstep;
-        specs[j].norm0 = fin->norm0;
-        const double dim = (double)jobs[j].S.dim;
-        const double init = (specs[j].init == LZ_INIT_HASH) ? 8.0 : 16.0;
-        const double per_step = (specs[j].mode == LZ_COEFF) ? 24.0 : 40.0;
-        bytes += dim * (init + per_step * specs[j].nstep);
+    for (int small = 1; small >= 0; small--) {
+        const std::vector<int>& o = order[small];
+        if (o.empty()) continue;
+        std::vector<LzJob> part;
+        std::vector<LzState> ps;
+        for (int j : o) {
+            part.push_back(jobs[j]);
+            ps.insert(ps.end(), &st[2 * (size_t)j], &st[2 * (size_t)j] + 2);
+        }
+        const float ms = small ? launch_small(c, part, ps, smem)
+                               : launch_jobs(c, part, ps, force ? force : tuned_shape(c, part), phases, false);
+        double bytes = 0.0;
+        for (size_t i = 0; i < o.size(); i++) {
+            JobSpec& s = specs[o[i]];
+            // the final state is the finished one of the two parity copies
+            const LzState& s0 = ps[2 * i];
+            const LzState& s1 = ps[2 * i + 1];
+            const LzState* fin = !s0.active ? &s0 : (!s1.active ? &s1 : nullptr);
+            if (!fin) throw EdztError{EDZT_ERR_NUMERIC, "Lanczos run did not finish within the pass limit"};
+            s.nstep = fin->nstep;
+            s.norm0 = fin->norm0;
+            const double init = (s.init == LZ_INIT_HASH) ? 8.0 : 16.0;
+            const double per_step = (s.mode == LZ_COEFF) ? 24.0 : 40.0;
+            bytes += (double)part[i].S.dim * (init + per_step * s.nstep);
+        }
+        book_launch(c, part, ms, bytes);
     }
-    book_launch(c, jobs, ms, bytes);
 }
 
 // ---------------------------------------------------------------------------
@@ -1215,6 +1245,20 @@ Lease<double> keep_lease(edzt_ctx* c, size_t n)
     }
 }
 
+// Run f.  If device memory does not suffice and drop() had kept vectors to give
+// back, run it once more without: they never make a call fail.
+template <class F, class D>
+void run_or_drop_kept(F f, D drop)
+{
+    try {
+        f();
+        return;
+    } catch (const EdztError& e) {
+        if (e.code != EDZT_ERR_OOM || !drop()) throw;
+    }
+    f();
+}
+
 struct SectorResult {
     int nstep = 0;
     double norm0 = 0.0;
@@ -1329,7 +1373,14 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             specs.push_back(s);
             which.push_back(i);
         }
-        run_jobs(c, specs);
+        run_or_drop_kept([&] { run_jobs(c, specs); },
+                         [&] {
+                             const bool had = keep > 0;
+                             keep = 0;
+                             for (auto& k : kept) k.reset();
+                             for (JobSpec& s : specs) s.keep = nullptr, s.keep_steps = 0;
+                             return had;
+                         });
         const size_t n_ab = (size_t)nsector * 2 * maxnstep;
         double* hab = reinterpret_cast<double*>(stage_buffer(c, sizeof(double) * n_ab));
         CK(cudaMemcpyAsync(hab, ab.p, sizeof(double) * n_ab, cudaMemcpyDeviceToHost, c->stream));
@@ -1894,7 +1945,16 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     }
     keep_scans(c, B, i0, i1, maxnstep, keep_limit);
     for (int q = 0; q < nj; q++) keep_in(B[own[q].inst], own[q].sector, maxnstep, specs[q]);
-    run_jobs(c, specs);
+    run_or_drop_kept([&] { run_jobs(c, specs); },
+                     [&] {
+                         bool had = false;
+                         for (int i = i0; i < i1; i++) {
+                             had = had || B[i].kept.p;
+                             B[i].kept.reset();
+                         }
+                         for (JobSpec& j : specs) j.keep = nullptr, j.keep_steps = 0;
+                         return had;
+                     });
     std::vector<double> hab((size_t)std::max(nj, 1) * 2 * maxnstep);
     CK(cudaMemcpyAsync(hab.data(), ab.p, sizeof(double) * hab.size(), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -2130,11 +2190,20 @@ struct edzt_server {
 
 namespace {
 
+void drop_kept(edzt_server* sv, ServReq& q)
+{
+    q.I.kept.reset();
+    sv->kept -= q.kept_bytes;
+    sv->reserved -= q.kept_bytes;
+    q.kept_bytes = 0;
+}
+
 // Let an admitted request's scan keep its v_k: within a 32nd of the memory free
 // at creation and an eighth of the budget over all requests, so that what is
 // kept hardly ever holds up an admission.
 void keep_request(edzt_server* sv, ServReq& q)
 {
+    drop_kept(sv, q);                                     // of an admission that failed
     const long long n = scan_states(q.I), bytes = n * sv->maxnstep * (long long)sizeof(double);
     const double limit = std::min((double)sv->c->free_at_create / 32, (double)sv->budget / 8);
     if (sv->reserved + bytes > sv->budget) return;
@@ -2144,14 +2213,6 @@ void keep_request(edzt_server* sv, ServReq& q)
     q.kept_bytes = bytes;
     sv->kept += bytes;
     sv->reserved += bytes;
-}
-
-void drop_kept(edzt_server* sv, ServReq& q)
-{
-    q.I.kept.reset();
-    sv->kept -= q.kept_bytes;
-    sv->reserved -= q.kept_bytes;
-    q.kept_bytes = 0;
 }
 
 // Size class of a request: its nsite, the requests up to nsite 11 together.
@@ -2177,10 +2238,27 @@ std::unique_ptr<LiveJob> make_live(edzt_ctx* c, const JobSpec& spec, std::vector
     return L;
 }
 
+// The largest shared memory that the runs of a request's phase take in the
+// kernel of small ones; 0: they are for the persistent kernel (some run is
+// larger, or all their steps at once, 4 us each, would outlast a server step).
+size_t small_request(const edzt_server* sv, const ServReq& q)
+{
+    size_t most = 0;
+    for (const auto& j : q.jobs) {
+        LzJob J;
+        fill_job(J, j->spec, j->S);
+        const size_t need = small_allowed(sv->c, J) ? lz_small_smem(J.S, J.mode) : 0;
+        if (!need || 0.004 * J.maxnstep > sv->step_ms) return 0;
+        most = std::max(most, need);
+    }
+    return most;
+}
+
 // One slice: at most `phases` phases (even) of every live run in v, in one
-// persistent launch; runs that finish are marked done with nstep and norm0.
+// persistent launch, or (small: the shared memory) all their steps in the
+// kernel of small runs; runs that finish are marked done with nstep and norm0.
 // Returns the launch's device time in ms.
-float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases)
+float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, size_t small = 0)
 {
     const int nj = (int)v.size();
     std::vector<LzJob> jobs(nj);
@@ -2197,7 +2275,8 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases)
     for (int j = 0; j < nj; j++) std::memcpy(&st[2 * (size_t)j], v[j]->st, 2 * sizeof(LzState));
     int budget = std::max(2, phases & ~1);
     if (c->dbg_pass_cap > 0) budget = std::min(budget, std::max(2, c->dbg_pass_cap & ~1));
-    const float ms = launch_jobs(c, jobs, st, tuned_shape(c, jobs), budget, true);
+    const float ms = small ? launch_small(c, jobs, st, small)
+                           : launch_jobs(c, jobs, st, tuned_shape(c, jobs), budget, true);
     for (int j = 0; j < nj; j++) std::memcpy(v[j]->st, &st[2 * (size_t)j], 2 * sizeof(LzState));
     double bytes = 0.0;
     for (int j = 0; j < nj; j++) {
@@ -2237,23 +2316,32 @@ void server_admit(edzt_server* sv)
         q.phase = 1;
         // the scan: one run per sector (ground_state.f90:28-73)
         const int nsite = q.I.model.nsite;
-        q.job_of_sector.assign(ns, -1);
-        for (int s = 0; s < ns; s++) {
-            const int nu = q.I.sec[2 * s], nd = q.I.sec[2 * s + 1];
-            if (sector_dim_ns(nsite, nu, nd) <= 0) continue;
-            JobSpec j;
-            j.mt = q.I.mt.get();
-            j.nu = nu; j.nd = nd;
-            j.mode = LZ_COEFF;
-            j.init = LZ_INIT_HASH;
-            j.key = edzt_stream_key(q.I.seed, (uint64_t)s);
-            j.maxnstep = sv->maxnstep;
-            j.a = q.ab.p + (size_t)(2 * s) * sv->maxnstep;
-            j.b = q.ab.p + (size_t)(2 * s + 1) * sv->maxnstep;
-            keep_in(q.I, s, sv->maxnstep, j);
-            q.job_of_sector[s] = (int)q.jobs.size();
-            q.jobs.push_back(make_live(c, j, todo));
-        }
+        run_or_drop_kept(
+            [&] {
+                q.job_of_sector.assign(ns, -1);
+                for (int s = 0; s < ns; s++) {
+                    const int nu = q.I.sec[2 * s], nd = q.I.sec[2 * s + 1];
+                    if (sector_dim_ns(nsite, nu, nd) <= 0) continue;
+                    JobSpec j;
+                    j.mt = q.I.mt.get();
+                    j.nu = nu; j.nd = nd;
+                    j.mode = LZ_COEFF;
+                    j.init = LZ_INIT_HASH;
+                    j.key = edzt_stream_key(q.I.seed, (uint64_t)s);
+                    j.maxnstep = sv->maxnstep;
+                    j.a = q.ab.p + (size_t)(2 * s) * sv->maxnstep;
+                    j.b = q.ab.p + (size_t)(2 * s + 1) * sv->maxnstep;
+                    keep_in(q.I, s, sv->maxnstep, j);
+                    q.job_of_sector[s] = (int)q.jobs.size();
+                    q.jobs.push_back(make_live(c, j, todo));
+                }
+            },
+            [&] {
+                const bool had = q.I.kept.p;
+                q.jobs.clear();
+                drop_kept(sv, q);
+                return had;
+            });
         build_ops(c, todo);
         sv->active.push_back(std::move(sv->queue.front()));
         sv->queue.pop_front();
@@ -2450,23 +2538,32 @@ int server_step(edzt_server* sv)
         sv->last_cls = cls;
         double left = sv->step_ms;
         for (int round = 0; round < 64; round++) {
-            std::vector<LiveJob*> v;
+            std::vector<LiveJob*> v, few;                 // runs of the persistent kernel, and small ones
             long long dims = 0;
+            size_t smem = 0;
             for (auto& up : sv->active) {
                 if (up->cls != cls || up->phase >= 4) continue;
-                for (auto& j : up->jobs)
-                    if (!j->done) { v.push_back(j.get()); dims += j->S.dim; }
+                const size_t small = small_request(sv, *up);
+                smem = std::max(smem, small);
+                for (auto& j : up->jobs) {
+                    if (j->done) continue;
+                    (small ? few : v).push_back(j.get());
+                    if (!small) dims += j->S.dim;
+                }
             }
-            if (v.empty()) break;
+            if (v.empty() && few.empty()) break;
+            if (!few.empty()) left -= run_slice(c, few, 0, smem);
             auto est = sv->ms_per_phase.find(cls);
             const double mpp = (est != sv->ms_per_phase.end()) ? est->second : 0.01 + (double)dims * 40.0 / 4.0e9;
             int phases = (int)std::min(4096.0, std::max(2.0, left / std::max(mpp, 1e-4)));
             phases &= ~1;
             if (phases < 2) phases = 2;
-            const float ms = run_slice(c, v, phases);
-            const double per = ms / phases;
-            sv->ms_per_phase[cls] = (est != sv->ms_per_phase.end()) ? 0.5 * (est->second + per) : per;
-            left -= ms;
+            if (!v.empty()) {
+                const float ms = run_slice(c, v, phases);
+                const double per = ms / phases;
+                sv->ms_per_phase[cls] = (est != sv->ms_per_phase.end()) ? 0.5 * (est->second + per) : per;
+                left -= ms;
+            }
             for (auto& up : sv->active) {                     // requests move on as their phase's runs finish
                 if (up->cls != cls || up->phase >= 4 || !phase_done(*up)) continue;
                 if (up->phase == 1) after_scan(sv, *up);

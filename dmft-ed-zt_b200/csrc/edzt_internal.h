@@ -249,8 +249,9 @@ bool lz_shape_fits(const DevSector& S, const LzShape& q);
 cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const LzJob* jobs, const long long* prefix,
                                       double* slots, unsigned* sync_words, int* status, cudaStream_t s);
 // Small coefficient runs from start to finish, one CTA each: the shared memory
-// of a launch (0: some run is not of that kind), and the launch.
-size_t lz_small_smem(const LzJob* jobs, int njobs);
+// that a run takes (0: it is not of that kind), and a launch with the most that
+// any of its runs takes.
+size_t lz_small_smem(const DevSector& S, int mode);
 cudaError_t launch_lanczos_small(const LzJob* jobs, int njobs, size_t smem, bool exchange, long long most_states,
                                  cudaStream_t s);
 // Sync-word buffer size (bytes) for a launch of njobs runs.

@@ -730,9 +730,10 @@ cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const L
 // issue slots idle half of the time and 1,024 run out of columns.  Bound by
 // the instructions and wavefronts of the hop sums.  A step of a lone run, in
 // us (persistent kernel): 400 states 1.9 (8.7), 1,225 3.3 (8.7), 4,900 6.5
-// (8.8), with the v_k kept 1 more; 7,056 states 9.8 (8.9), so the line lies
-// at kLzSmallStates.  Up to a state per thread, 512 threads of one row.
-constexpr long long kLzSmallStates = 6000;
+// (8.8), 7,056 9.8 (8.9), with the v_k kept up to a fifth more.  The line lies
+// where a step still takes less than half: with larger runs in the same call
+// these come in a launch of their own, before the others'.
+constexpr long long kLzSmallStates = 2000;
 constexpr size_t kLzSmallSmemMax = kLzSmemMax - 4096;   // besides the descriptor and the sums
 
 // Where a run's parts lie in shared memory, in bytes.
@@ -945,16 +946,11 @@ __global__ void __launch_bounds__(T) k_lanczos_small(const LzJob* __restrict__ j
     }
 }
 
-// The shared memory that a launch of k_lanczos_small needs; 0: it does not
-// take these runs.
-size_t lz_small_smem(const LzJob* jobs, int nj)
+size_t lz_small_smem(const DevSector& S, int mode)
 {
-    size_t most = 0;
-    for (int j = 0; j < nj; j++) {
-        if (jobs[j].mode != LZ_COEFF || jobs[j].S.dim > kLzSmallStates) return 0;
-        most = std::max(most, (size_t)lz_small_layout(jobs[j].S).size);
-    }
-    return most <= kLzSmallSmemMax ? most : 0;
+    if (mode != LZ_COEFF || S.dim > kLzSmallStates) return 0;
+    const size_t size = (size_t)lz_small_layout(S).size;
+    return size <= kLzSmallSmemMax ? size : 0;
 }
 
 cudaError_t launch_lanczos_small(const LzJob* jobs, int nj, size_t smem, bool exchange, long long most, cudaStream_t s)

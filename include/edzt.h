@@ -290,17 +290,19 @@ int edzt_server_result(edzt_server *srv, long long id, int *done, int *isector, 
 int edzt_server_cancel(edzt_server *srv, long long id);
 void edzt_server_destroy(edzt_server *srv);
 /* Device-memory footprint (bytes) a request holds at its peak in the batched
- * and served forms: the sector scan's pair and down-hop buffers (40 B per
- * state of every sector) or its Green's runs', whichever is larger, plus its
- * ground state. */
+ * and served forms: the sector scan's vectors (24 B per state of
+ * every sector, rows and columns padded to fours) or its Green's runs',
+ * whichever is larger, plus its ground state.  Kept vectors
+ * (edzt_set_keep_vectors) come on top where there is room for them. */
 int edzt_instance_footprint(const edzt_instance *inst, long long *bytes);
 
-/* Autotuner (north_star's tuned stripe width; no counterpart in the
+/* Autotuner (the stripe width among others; no counterpart in the
  * reference): times short Lanczos runs (`steps` steps, 2..1000) of the
  * context's model on sector (ne_up, ne_dn) for every tile shape of the
- * persistent kernel that fits -- columns per slab of the column phase (the
- * stripe width: 2, 4, 8 or 16), rows per tile of the row phase (1, 2, 4 or
- * 8), one CTA of 512 or two of 256 threads per SM -- and records the fastest
+ * persistent kernel that fits -- columns per tile of the column phase (the
+ * stripe width) by rows per tile of the row phase, 16 x 8, 8 x 8, 8 x 4,
+ * 4 x 4, 2 x 2 or 2 x 1, one CTA of 512 or two of 256 threads per SM -- and
+ * records the fastest
  * on the context for that sector shape; later launches on the context use it
  * for every run of that shape (results unchanged but for rounding).
  * Outputs (nullable): the chosen shape and its time per Lanczos step.
