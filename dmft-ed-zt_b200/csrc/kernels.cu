@@ -140,16 +140,17 @@ __device__ __forceinline__ long long natural_of(unsigned e, int nup, int ndn, co
 
 struct VecSumArgs { VecSum r[kVecSums]; };
 
-// Blocks of a sum: one per 256 elements, at most eight per SM.
+// Blocks of a sum: one per 256 pairs of elements, at most eight per SM.
 __host__ __device__ inline int vec_sum_blocks(const VecSum& r)
 {
-    const long long b = (lz_vec_size(r.nup, r.ndn) + 255) / 256;
+    const long long b = (lz_vec_size(r.nup, r.ndn) / 2 + 255) / 256;
     return b < kVecSumBlocks ? (int)b : kVecSumBlocks;
 }
 
-// blockIdx.y: the sum.  Bound by the read of the kept vectors; the sums of a
-// batch share a launch, as one alone fills the chip only from nsite 11 on (16
-// sums of nsite 8 to 11: 820 us apart).
+// blockIdx.y: the sum.  Bound by the read of the kept vectors: eight loads of 16
+// bytes in flight per thread (of 8 bytes: 285 steps of nsite 15, 94 GB, took 6
+// ms more).  The sums of a batch share a launch, as one alone fills the chip
+// only from nsite 11 on (16 sums of nsite 8 to 11: 820 us apart).
 __global__ void __launch_bounds__(256) k_vec_sum(const __grid_constant__ VecSumArgs A)
 {
     __shared__ double scratch[32];
@@ -158,21 +159,30 @@ __global__ void __launch_bounds__(256) k_vec_sum(const __grid_constant__ VecSumA
     if ((int)blockIdx.x >= nb) return;
     const int nup = R.nup, ndn = R.ndn, nstep = R.nstep;
     const double* __restrict__ coeff = R.coeff;
-    const long long stride = lz_vec_size(nup, ndn);
+    const long long pairs = lz_vec_size(nup, ndn) / 2;   // two rows of a column
     double sq[1] = {0.0};
-    for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < stride; e += (long long)nb * 256) {
-        const double* v = R.v + e;                       // v_1
-        double acc = 0.0;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < pairs; i += (long long)nb * 256) {
+        const double2* v = reinterpret_cast<const double2*>(R.v) + i;   // of v_1
+        double2 acc = make_double2(0.0, 0.0);
         if (coeff) {
 #pragma unroll 8
-            for (int k = 0; k < nstep; k++) acc = fma(__ldg(coeff + k), __ldcs(v + k * stride), acc);
+            for (int k = 0; k < nstep; k++) {
+                const double2 x = __ldcs(v + k * pairs);
+                const double c = __ldg(coeff + k);
+                acc.x = fma(c, x.x, acc.x);
+                acc.y = fma(c, x.y, acc.y);
+            }
         } else {
             acc = __ldcs(v);
         }
-        const long long o = R.natural ? natural_of((unsigned)e, nup, ndn, R.natu, R.natd) : e;
-        if (o >= 0) {
-            R.out[o] = acc;
-            sq[0] = fma(acc, acc, sq[0]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const unsigned e = (unsigned)(2 * i + h);
+            const long long o = R.natural ? natural_of(e, nup, ndn, R.natu, R.natd) : e;
+            if (o < 0) continue;
+            const double z = h ? acc.y : acc.x;
+            R.out[o] = z;
+            sq[0] = fma(z, z, sq[0]);
         }
     }
     if (R.natural) {
