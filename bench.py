@@ -648,14 +648,14 @@ def run_gpu(args):
                 "kernel": "k_lanczos (persistent fused Lanczos)", "peak_source": peak_src,
                 "launches": ks["launches"], "avg_launch_ms": ks["ms"] / max(ks["launches"], 1),
                 "algorithmic_bytes_per_launch": ks["bytes"] / max(ks["launches"], 1),
-                "eigenvector": "eigenvector pass" if eig_pass else "from the scan's kept Lanczos pairs",
+                "eigenvector": "eigenvector pass" if eig_pass else "from the scan's kept Lanczos vectors",
                 "note": "24 B/state per coefficient step, 40 B/state per eigenvector step; the "
-                        "ground-state scan (9 sectors, 252 MB of pair buffers and D) exceeds L2, the "
+                        "ground-state scan (9 sectors, 151 MB of vectors, and what it keeps) exceeds L2, the "
                         "eigenvector and Green's-function launches are L2-resident"}
     roofline["traffic"] = read_traffic(args.traffic_file)
     # the launches of one solve separately, told apart by the states they
     # carry: the ground-state scan (every sector), the eigenvector pass of the
-    # winner (absent when the scan kept its Lanczos pairs), the c/c^+ runs
+    # winner (absent when the scan kept its Lanczos vectors), the c/c^+ runs
     log = s.launch_log()
     scan_states = float(sum(s.dim(u, d) for u, d in sectors))
     kinds = {}
@@ -674,7 +674,7 @@ def run_gpu(args):
         gbs = by / (ms / 1000.0) / 1e9 if ms > 0 else 0.0
         per.append({"launch": name, "launches": len(ent), "avg_ms": ms, "algorithmic_bytes": by,
                     "achieved_GBs": gbs, "frac": gbs / peak if peak else None, "states": st_,
-                    "pair_and_D_bytes": 40.0 * st_})
+                    "vector_bytes": 24.0 * st_})
     if per:
         roofline["per_launch"] = per
 

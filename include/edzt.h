@@ -313,9 +313,9 @@ int edzt_clear_tuning(edzt_ctx *ctx);
 
 /* Fault tests (no counterpart in the reference; no GPU fault is involved):
  * pass_cap > 0 caps the passes of a persistent launch (a run that needs more
- * fails with EDZT_ERR_NUMERIC); wait_seconds > 0 shortens the grid-barrier
- * wait limit (default 5 s); stall_cta >= 0 makes that CTA leave the launch
- * without arriving at the next grid barrier, so the others' bounded wait runs
+ * fails with EDZT_ERR_NUMERIC); wait_seconds > 0 shortens the wait limit
+ * of a run's arrivals (default 5 s); stall_cta >= 0 makes that CTA leave the
+ * launch without arriving, so the others' bounded wait runs
  * out and the call returns EDZT_ERR_TIMEOUT.  All zero / -1: normal
  * operation.  The context stays usable after either error. */
 int edzt_set_fault_test(edzt_ctx *ctx, int pass_cap, double wait_seconds, int stall_cta);
