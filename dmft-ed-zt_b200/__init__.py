@@ -52,7 +52,7 @@ EXPORTS = (
     "edzt_kernel_stats", "edzt_reset_stats", "edzt_kernel_launch_log", "edzt_lanczos_iteration_noalloc", "edzt_solve_batch",
     "edzt_cluster_green_matrix", "edzt_gs_occupancy", "edzt_green_real", "edzt_server_create", "edzt_server_submit", "edzt_server_step", "edzt_server_result", "edzt_server_destroy",
     "edzt_server_cancel", "edzt_server_set_step_ms", "edzt_tune_sector", "edzt_clear_tuning",
-    "edzt_instance_footprint", "edzt_set_fault_test", "edzt_set_keep_limit_test", "edzt_diag_arpack",
+    "edzt_instance_footprint", "edzt_set_fault_test", "edzt_set_keep_limit_test", "edzt_set_memory_limit_test", "edzt_diag_arpack",
     "edzt_set_diag_solver", "edzt_set_keep_vectors", "edzt_hybridization", "edzt_local_green_bethe", "edzt_fit_bath", "edzt_dmft_bethe",
 )
 # ground_state's diag_solver values (src/ground_state.f90:53-60).
@@ -192,6 +192,7 @@ def load_library(path: str = LIB_PATH):
     L.edzt_instance_footprint.argtypes = [_vp, C.POINTER(C.c_longlong)]
     L.edzt_set_fault_test.argtypes = [_vp, C.c_int, C.c_double, C.c_int]
     L.edzt_set_keep_limit_test.argtypes = [_vp, C.c_double]
+    L.edzt_set_memory_limit_test.argtypes = [_vp, C.c_double]
     L.edzt_diag_lanczos.argtypes = [_vp, C.c_int, C.c_int, C.c_int, C.c_uint64, C.c_uint64, _dp, _vp, _dp]
     L.edzt_diag_arpack.argtypes = [_vp, C.c_int, C.c_int, C.c_uint64, C.c_uint64, _dp, _vp, _vp, _vp, _ip]
     L.edzt_set_diag_solver.argtypes = [_vp, C.c_int]
@@ -576,6 +577,11 @@ class Solver:
         """Test of the kept vectors (edzt_set_keep_limit_test); 0 restores the
         normal limits."""
         self._check(self._L.edzt_set_keep_limit_test(self._h, float(nbytes)))
+
+    def set_memory_limit_test(self, nbytes=0.0):
+        """Test of running out of device memory (edzt_set_memory_limit_test);
+        0: no limit."""
+        self._check(self._L.edzt_set_memory_limit_test(self._h, float(nbytes)))
 
     def footprint(self, inst) -> int:
         """Device bytes a request holds at its peak (edzt_instance_footprint)."""

@@ -67,16 +67,11 @@ class Pool {
             free_.erase(it);
             return p;
         }
-        void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
+        void* p = try_malloc(bytes);
+        if (!p) {
             trim();
-            e = cudaMalloc(&p, bytes);
-            if (e != cudaSuccess) {
-                cudaGetLastError();
-                throw EdztError{EDZT_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes failed"};
-            }
+            p = try_malloc(bytes);
+            if (!p) throw EdztError{EDZT_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes failed"};
         }
         used_[p] = bytes;
         return p;
@@ -98,6 +93,7 @@ class Pool {
         while (cached > keep && !free_.empty()) {
             auto it = std::prev(free_.end());
             cached -= it->first;
+            held_ -= it->first;
             cudaFree(it->second);
             free_.erase(it);
         }
@@ -107,9 +103,25 @@ class Pool {
         trim();
         for (auto& kv : used_) cudaFree(kv.first);
         used_.clear();
+        held_ = 0;
     }
+    // Test of running out of memory: blocks of at most `bytes` altogether (0: what the device has).
+    void set_limit(size_t bytes) { limit_ = bytes; }
 
   private:
+    void* try_malloc(size_t bytes)
+    {
+        if (limit_ && held_ + bytes > limit_) return nullptr;
+        void* p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        held_ += bytes;
+        return p;
+    }
+
+    size_t held_ = 0, limit_ = 0;           // bytes of all blocks; the test's limit
     std::multimap<size_t, void*> free_;
     std::map<void*, size_t> used_;
 };
@@ -2198,12 +2210,23 @@ void drop_kept(edzt_server* sv, ServReq& q)
     q.kept_bytes = 0;
 }
 
+// Undo an admission: the request is as it was queued.
+void take_back(edzt_server* sv, ServReq& q)
+{
+    q.jobs.clear();
+    q.job_of_sector.clear();
+    q.ab.reset();
+    drop_kept(sv, q);
+    q.I.mt.reset();
+    q.phase = 0;
+    sv->reserved -= q.I.footprint;
+}
+
 // Let an admitted request's scan keep its v_k: within a 32nd of the memory free
 // at creation and an eighth of the budget over all requests, so that what is
 // kept hardly ever holds up an admission.
 void keep_request(edzt_server* sv, ServReq& q)
 {
-    drop_kept(sv, q);                                     // of an admission that failed
     const long long n = scan_states(q.I), bytes = n * sv->maxnstep * (long long)sizeof(double);
     const double limit = std::min((double)sv->c->free_at_create / 32, (double)sv->budget / 8);
     if (sv->reserved + bytes > sv->budget) return;
@@ -2299,50 +2322,70 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, size_t small 
     return ms;
 }
 
-void server_admit(edzt_server* sv)
+// Build a request's tables and the live runs of its scan, one per sector
+// (ground_state.f90:28-73).
+void admit_request(edzt_server* sv, ServReq& q)
 {
     edzt_ctx* c = sv->c;
+    std::vector<OpsTable*> todo;
+    q.I.mt = std::make_unique<ModelTables>();
+    set_tables_model(c, *q.I.mt, q.I.model);
+    keep_request(sv, q);
+    const int ns = (int)q.I.sec.size() / 2;
+    q.ab = Lease<double>(c->pool, (size_t)std::max(ns, 1) * 2 * sv->maxnstep);
+    q.cls = size_class(q.I);
+    const int nsite = q.I.model.nsite;
+    run_or_drop_kept(
+        [&] {
+            q.job_of_sector.assign(ns, -1);
+            for (int s = 0; s < ns; s++) {
+                const int nu = q.I.sec[2 * s], nd = q.I.sec[2 * s + 1];
+                if (sector_dim_ns(nsite, nu, nd) <= 0) continue;
+                JobSpec j;
+                j.mt = q.I.mt.get();
+                j.nu = nu; j.nd = nd;
+                j.mode = LZ_COEFF;
+                j.init = LZ_INIT_HASH;
+                j.key = edzt_stream_key(q.I.seed, (uint64_t)s);
+                j.maxnstep = sv->maxnstep;
+                j.a = q.ab.p + (size_t)(2 * s) * sv->maxnstep;
+                j.b = q.ab.p + (size_t)(2 * s + 1) * sv->maxnstep;
+                keep_in(q.I, s, sv->maxnstep, j);
+                q.job_of_sector[s] = (int)q.jobs.size();
+                q.jobs.push_back(make_live(c, j, todo));
+            }
+        },
+        [&] {
+            const bool had = q.I.kept.p;
+            q.jobs.clear();
+            drop_kept(sv, q);
+            return had;
+        });
+    build_ops(c, todo);
+    q.phase = 1;
+}
+
+// Admit the requests that fit.  An admission that fails leaves nothing behind:
+// no live run may outlast the tables it points at.  The request stays queued,
+// for when others have given memory back; with no others the failure is the
+// step's.
+void server_admit(edzt_server* sv)
+{
     while (!sv->queue.empty()) {
-        std::vector<OpsTable*> todo;
         ServReq& q = *sv->queue.front();
         if (!sv->active.empty() && sv->reserved + q.I.footprint > sv->budget) break;
         sv->reserved += q.I.footprint;
-        q.I.mt = std::make_unique<ModelTables>();
-        set_tables_model(c, *q.I.mt, q.I.model);
-        keep_request(sv, q);
-        const int ns = (int)q.I.sec.size() / 2;
-        q.ab = Lease<double>(c->pool, (size_t)std::max(ns, 1) * 2 * sv->maxnstep);
-        q.cls = size_class(q.I);
-        q.phase = 1;
-        // the scan: one run per sector (ground_state.f90:28-73)
-        const int nsite = q.I.model.nsite;
-        run_or_drop_kept(
-            [&] {
-                q.job_of_sector.assign(ns, -1);
-                for (int s = 0; s < ns; s++) {
-                    const int nu = q.I.sec[2 * s], nd = q.I.sec[2 * s + 1];
-                    if (sector_dim_ns(nsite, nu, nd) <= 0) continue;
-                    JobSpec j;
-                    j.mt = q.I.mt.get();
-                    j.nu = nu; j.nd = nd;
-                    j.mode = LZ_COEFF;
-                    j.init = LZ_INIT_HASH;
-                    j.key = edzt_stream_key(q.I.seed, (uint64_t)s);
-                    j.maxnstep = sv->maxnstep;
-                    j.a = q.ab.p + (size_t)(2 * s) * sv->maxnstep;
-                    j.b = q.ab.p + (size_t)(2 * s + 1) * sv->maxnstep;
-                    keep_in(q.I, s, sv->maxnstep, j);
-                    q.job_of_sector[s] = (int)q.jobs.size();
-                    q.jobs.push_back(make_live(c, j, todo));
-                }
-            },
-            [&] {
-                const bool had = q.I.kept.p;
-                q.jobs.clear();
-                drop_kept(sv, q);
-                return had;
-            });
-        build_ops(c, todo);
+        try {
+            sv->active.reserve(sv->active.size() + 1);
+            admit_request(sv, q);
+        } catch (const EdztError& e) {
+            take_back(sv, q);
+            if (e.code == EDZT_ERR_OOM && !sv->active.empty()) break;
+            throw;
+        } catch (...) {
+            take_back(sv, q);
+            throw;
+        }
         sv->active.push_back(std::move(sv->queue.front()));
         sv->queue.pop_front();
     }
@@ -3189,6 +3232,14 @@ int edzt_set_keep_limit_test(edzt_ctx* c, double bytes)
     return guarded(c, [&] {
         arg_check(bytes >= 0.0, "bad limit");
         c->dbg_keep_limit = bytes;
+    });
+}
+
+int edzt_set_memory_limit_test(edzt_ctx* c, double bytes)
+{
+    return guarded(c, [&] {
+        arg_check(bytes >= 0.0 && bytes < 1e15, "bad limit");
+        c->pool.set_limit((size_t)bytes);
     });
 }
 

@@ -324,6 +324,11 @@ int edzt_set_fault_test(edzt_ctx *ctx, int pass_cap, double wait_seconds, int st
  * the limits that hold anyway (0: only those). */
 int edzt_set_keep_limit_test(edzt_ctx *ctx, double bytes);
 
+/* Test of running out of device memory, without taking any from others: the
+ * context's blocks, in use or cached, hold at most `bytes` altogether, and an
+ * allocation beyond that fails as one that the device refuses (0: no limit). */
+int edzt_set_memory_limit_test(edzt_ctx *ctx, double bytes);
+
 /* ---- the DMFT loop around the solver (host code, dmft_loop.cpp) ----------
  * The caller of the path, restated so that a whole DMFT run needs no
  * Fortran: the Bethe-lattice loop of src/dmft.f90:38-137 with the bath fit

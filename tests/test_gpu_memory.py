@@ -1,0 +1,84 @@
+"""Running out of device memory, made on the host: a limit on what a context's
+blocks hold (edzt_set_memory_limit_test) makes an allocation fail as one that
+the device refuses.  Kept Lanczos vectors never make a call fail that succeeds
+without them; a batch that does not fit at once runs in waves; a failed
+admission or server step leaves the server as it was; a later call gets what
+an earlier one left cached."""
+
+import numpy as np
+import pytest
+
+from conftest import random_model
+from test_gpu_keep import _states
+
+pytestmark = pytest.mark.gpu
+KB = 1024.0
+
+
+def _run(pkg, f):
+    """f() or None when it ran out of memory."""
+    try:
+        return f()
+    except pkg.EDError as e:
+        assert e.code == pkg.EDZT_ERR_OOM
+        return None
+
+
+def _instances(pkg, sizes, one_sector=False):
+    rng = np.random.default_rng(23)
+    out = []
+    for i, ns in enumerate(sizes):
+        n = ns // 2
+        out.append(dict(model=random_model(pkg, rng, 1, ns - 1, spin_dep=True),
+                        sectors=[(n, n)] if one_sector else [(n, n), (n, n + 1), (n + 1, n)], nspin=1 + i % 2,
+                        seed=70 + i))
+    return out
+
+
+def _same(got, ref):
+    for (s1, e1, g1), (s2, e2, g2) in zip(got, ref, strict=True):
+        assert s1 == s2 and abs(e1 - e2) <= 1e-10 * max(1.0, abs(e2))
+        assert np.abs(np.asarray(g1) - np.asarray(g2)).max() <= 1e-8
+
+
+def _serve(pkg, sv, insts, ids=None, steps=400):
+    """Results of the requests, or None where a step ran out of memory."""
+    ids = [sv.submit(i) for i in insts] if ids is None else ids
+    res = [None] * len(ids)
+    for _ in range(steps):
+        if _run(pkg, sv.step) is None:
+            return None, ids
+        res = [r or sv.result(i) for r, i in zip(res, ids)]
+        if all(res):
+            return [(r["isector"], r["e0"], r["G_cl"]) for r in res], ids
+    raise AssertionError("the server did not finish")
+
+
+def test_failed_admission_leaves_the_request_queued(pkg):
+    """Admissions that run out of memory, one step after the other, then memory:
+    the requests are solved as if nothing had been, and both at a time, as the
+    budget allows."""
+    insts, omega = _instances(pkg, [9, 9]), pkg.matsubara(16, 20.0)
+    with pkg.Solver(0) as s:
+        ref = []
+        for i in insts:
+            s.set_model(i["model"])
+            r = s.solve(i["sectors"], 20, omega, nspin=i["nspin"], seed=i["seed"])
+            ref.append((r["isector"], r["e0"], r["G_cl"]))
+    with pkg.Solver(0) as s:
+        footprint = max(s.footprint(i) for i in insts)
+        sv = pkg.Server(s, 20, omega, hbm_budget=int(2.5 * footprint))
+        ids = [sv.submit(i) for i in insts]
+        vectors = 24.0 * _states(pkg, 9, insts[0]["sectors"])     # of the scan's runs: more than any limit here
+        for limit in np.linspace(8 * KB, 0.9 * vectors, 30):      # ever further into the admission
+            s.set_memory_limit_test(limit)
+            with pytest.raises(pkg.EDError) as e:
+                sv.step()
+            assert e.value.code == pkg.EDZT_ERR_OOM
+        s.set_memory_limit_test(0)
+        sv.set_step_ms(1e-3)
+        assert sv.step() == (2, 0, 0)
+        got, _ = _serve(pkg, sv, insts, ids, 4000)
+        _same(got, ref)
+        assert sv.step() == (0, 0, 0)
+        sv.close()
