@@ -2173,7 +2173,8 @@ struct ServReq {
     std::vector<int> job_of_sector;        // live scan job of each sector, -1 if none
     std::vector<double> hab;               // scan coefficients on the host
     std::vector<SectorResult> res;
-    int win = -1;                          // winning sector
+    int win = -1;                          // winning sector, once the scan's results are read
+    bool has_vec = false;                  // its vector is formed
     Lease<double> coef;                    // tridiagonal eigenvector of the winner (device)
     Lease<double> eig;                     // the winner's eigenvector in internal order
     std::vector<GreenRun> runs;
@@ -2194,6 +2195,7 @@ struct edzt_server {
     long long kept = 0;                    // of reserved: bytes of kept vectors
     double step_ms = 25.0;                 // time budget of one step
     int last_cls = -1;                     // class served by the last step
+    int stuck = 0;                         // steps in a row that got nowhere for lack of memory
     std::map<int, double> ms_per_phase;    // measured phase time by class
     std::deque<std::unique_ptr<ServReq>> queue;
     std::vector<std::unique_ptr<ServReq>> active;
@@ -2405,20 +2407,20 @@ void start_green(edzt_server* sv, ServReq& q)
     const int maxnstep = sv->maxnstep;
     BatchInst& I = q.I;
     const bool even = !(I.nspin == 2 || I.gs_up != I.gs_dn);
-    q.runs = cluster_runs(I.model.norb, even, I.gs_up, I.gs_dn);
-    q.gab = Lease<double>(c->pool, std::max<size_t>(q.runs.size(), 1) * 2 * maxnstep);
-    CK(cudaMemsetAsync(q.gab.p, 0, sizeof(double) * std::max<size_t>(q.runs.size(), 1) * 2 * maxnstep, c->stream));
-    q.jobs.clear();
+    std::vector<GreenRun> runs = cluster_runs(I.model.norb, even, I.gs_up, I.gs_dn);
+    Lease<double> gab(c->pool, std::max<size_t>(runs.size(), 1) * 2 * maxnstep);
+    CK(cudaMemsetAsync(gab.p, 0, sizeof(double) * std::max<size_t>(runs.size(), 1) * 2 * maxnstep, c->stream));
+    std::vector<std::unique_ptr<LiveJob>> jobs;
     std::vector<OpsTable*> todo;
     const int ns = I.model.nsite;
-    for (size_t r = 0; r < q.runs.size(); r++) {
-        GreenRun& g = q.runs[r];
+    for (size_t r = 0; r < runs.size(); r++) {
+        GreenRun& g = runs[r];
         g.mt = I.mt.get();
         g.gs = I.gsvec.p;
         g.gs_up = I.gs_up; g.gs_dn = I.gs_dn;
         g.e0 = I.e0;
-        g.a = q.gab.p + (2 * r) * maxnstep;
-        g.b = q.gab.p + (2 * r + 1) * maxnstep;
+        g.a = gab.p + (2 * r) * maxnstep;
+        g.b = gab.p + (2 * r + 1) * maxnstep;
         g.nstep = 0;
         if (sector_dim_ns(ns, g.nu, g.nd) <= 0) continue;
         JobSpec j;
@@ -2430,16 +2432,19 @@ void start_green(edzt_server* sv, ServReq& q)
         j.ac_src = g.gs;
         j.maxnstep = maxnstep;
         j.a = g.a; j.b = g.b;
-        g.nstep = -1 - (int)q.jobs.size();              // its live run, resolved when it finishes
-        q.jobs.push_back(make_live(c, j, todo));
+        g.nstep = -1 - (int)jobs.size();                // its live run, resolved when it finishes
+        jobs.push_back(make_live(c, j, todo));
     }
     build_ops(c, todo);
+    q.runs = std::move(runs);
+    q.gab = std::move(gab);
+    q.jobs = std::move(jobs);
     q.phase = 3;
 }
 
-// Scan finished: the tridiagonal ground state of every sector, the winner
-// (ground_state.f90:62-68, 1e-10 tie band) and its eigenvector pass.
-void after_scan(edzt_server* sv, ServReq& q)
+// Scan finished: the tridiagonal ground state of every sector and the winner
+// (ground_state.f90:62-68, 1e-10 tie band).  The runs are over with that.
+void read_scan(edzt_server* sv, ServReq& q)
 {
     edzt_ctx* c = sv->c;
     const int maxnstep = sv->maxnstep;
@@ -2465,28 +2470,23 @@ void after_scan(edzt_server* sv, ServReq& q)
         const double tie = 1.0e-10 * std::max(1.0, std::fabs(w < 0 ? 0.0 : q.res[w].e));
         if (w < 0 || q.res[s].e < q.res[w].e - tie) w = s;
     }
-    const double* kept = (w >= 0 && q.I.kept.p) ? q.jobs[q.job_of_sector[w]]->spec.keep : nullptr;
     q.jobs.clear();
     if (w < 0) { q.error = "no sector produced a ground state"; q.phase = 4; return; }
     q.win = w;
     q.I.best = w;
     q.I.gs_up = q.I.sec[2 * w]; q.I.gs_dn = q.I.sec[2 * w + 1];
     q.I.e0 = q.res[w].e;
-    q.I.gsvec = Lease<double>(c->pool, (size_t)sector_dim_ns(q.I.model.nsite, q.I.gs_up, q.I.gs_dn));
-    q.coef = Lease<double>(c->pool, (size_t)q.res[w].nstep);
-    if (kept) {
-        const std::vector<double> wt = keep_weights(q.res[w], q.hab.data() + (size_t)(2 * w + 1) * maxnstep);
-        CK(cudaMemcpyAsync(q.coef.p, wt.data(), sizeof(double) * wt.size(), cudaMemcpyHostToDevice, c->stream));
-        const DevSector Si = make_sector_mt(c, *q.I.mt, q.I.gs_up, q.I.gs_dn, true);
-        std::vector<VecSum> vs{natural_sum(Si, kept, q.coef.p, q.res[w].nstep, q.I.gsvec.p)};
-        normalised_sums(c, vs);
-        drop_kept(sv, q);
-        start_green(sv, q);
-        return;
-    }
+}
+
+// Start the winner's eigenvector pass (lanczos_solver.f90:213-300).
+void start_eigvec(edzt_server* sv, ServReq& q)
+{
+    edzt_ctx* c = sv->c;
+    const int maxnstep = sv->maxnstep, w = q.win;
+    if (!q.coef.p) q.coef = Lease<double>(c->pool, (size_t)q.res[w].nstep);
     CK(cudaMemcpyAsync(q.coef.p, q.res[w].coeff.data(), sizeof(double) * q.res[w].nstep, cudaMemcpyHostToDevice,
                        c->stream));
-    JobSpec j;                                            // eigenvector pass (lanczos_solver.f90:213-300)
+    JobSpec j;
     j.mt = q.I.mt.get();
     j.nu = q.I.gs_up; j.nd = q.I.gs_dn;
     j.mode = LZ_EIGVEC;
@@ -2494,26 +2494,46 @@ void after_scan(edzt_server* sv, ServReq& q)
     j.key = edzt_stream_key(q.I.seed, (uint64_t)w);
     j.maxnstep = q.res[w].nstep;
     j.coeff = q.coef.p;
-    q.eig = Lease<double>(c->pool, (size_t)lz_vec_size((int)edzt_binom(q.I.model.nsite, q.I.gs_up),
-                                                       (int)edzt_binom(q.I.model.nsite, q.I.gs_dn)));
+    if (!q.eig.p)
+        q.eig = Lease<double>(c->pool, (size_t)lz_vec_size((int)edzt_binom(q.I.model.nsite, q.I.gs_up),
+                                                           (int)edzt_binom(q.I.model.nsite, q.I.gs_dn)));
     j.eig = q.eig.p;
     j.a = q.ab.p + (size_t)(2 * w) * maxnstep;
     j.b = q.ab.p + (size_t)(2 * w + 1) * maxnstep;
     std::vector<OpsTable*> todo;
-    q.jobs.push_back(make_live(c, j, todo));
+    std::unique_ptr<LiveJob> L = make_live(c, j, todo);
     build_ops(c, todo);
+    q.jobs.push_back(std::move(L));
     q.phase = 2;
 }
 
-// Eigenvector pass finished: its result in the reference's order.
-void after_eigvec(edzt_server* sv, ServReq& q)
+// The winner's vector from the scan's kept v_k.
+void vector_from_kept(edzt_server* sv, ServReq& q)
+{
+    edzt_ctx* c = sv->c;
+    const int maxnstep = sv->maxnstep, w = q.win;
+    JobSpec scan;
+    keep_in(q.I, w, maxnstep, scan);
+    if (!q.coef.p) q.coef = Lease<double>(c->pool, (size_t)q.res[w].nstep);
+    const std::vector<double> wt = keep_weights(q.res[w], q.hab.data() + (size_t)(2 * w + 1) * maxnstep);
+    CK(cudaMemcpyAsync(q.coef.p, wt.data(), sizeof(double) * wt.size(), cudaMemcpyHostToDevice, c->stream));
+    const DevSector Si = make_sector_mt(c, *q.I.mt, q.I.gs_up, q.I.gs_dn, true);
+    std::vector<VecSum> vs{natural_sum(Si, scan.keep, q.coef.p, q.res[w].nstep, q.I.gsvec.p)};
+    normalised_sums(c, vs);
+    drop_kept(sv, q);
+    q.has_vec = true;
+}
+
+// The winner's vector from its eigenvector pass, in the reference's order.
+void vector_from_pass(edzt_server* sv, ServReq& q)
 {
     edzt_ctx* c = sv->c;
     const DevSector Si = make_sector_mt(c, *q.I.mt, q.I.gs_up, q.I.gs_dn, true);
     std::vector<VecSum> vs{natural_sum(Si, q.eig.p, nullptr, 1, q.I.gsvec.p)};
     normalised_sums(c, vs);
+    q.jobs.clear();
     q.eig.reset();
-    start_green(sv, q);
+    q.has_vec = true;
 }
 
 // Green's runs finished: continued fractions and G_cl.
@@ -2563,6 +2583,30 @@ void after_green(edzt_server* sv, ServReq& q)
     q.phase = 4;
 }
 
+// The runs of the request's phase have finished: on to the next.  Where memory
+// runs out on the way the request keeps what it has reached (the winner, its
+// vector) and a later step goes on from there.
+void advance(edzt_server* sv, ServReq& q)
+{
+    if (q.phase == 3) {
+        after_green(sv, q);
+        return;
+    }
+    if (q.win < 0) read_scan(sv, q);
+    if (q.phase == 4) return;
+    if (!q.has_vec) {
+        if (!q.I.gsvec.p)
+            q.I.gsvec = Lease<double>(sv->c->pool, (size_t)sector_dim_ns(q.I.model.nsite, q.I.gs_up, q.I.gs_dn));
+        if (q.phase == 1 && !q.I.kept.p) {
+            start_eigvec(sv, q);
+            return;
+        }
+        if (q.phase == 1) vector_from_kept(sv, q);
+        else vector_from_pass(sv, q);
+    }
+    start_green(sv, q);
+}
+
 // One step: admit what fits, then serve the next size class in turn.
 int server_step(edzt_server* sv)
 {
@@ -2580,7 +2624,22 @@ int server_step(edzt_server* sv)
         const int cls = (it == classes.end()) ? classes.front() : *it;
         sv->last_cls = cls;
         double left = sv->step_ms;
+        std::string short_of;                             // what a request waits for memory with
+        bool moved = false;
+        auto advance_done = [&] {
+            for (auto& up : sv->active) {
+                if (up->cls != cls || up->phase >= 4 || !phase_done(*up)) continue;
+                try {
+                    advance(sv, *up);
+                    moved = true;
+                } catch (const EdztError& e) {            // the others go on
+                    if (e.code != EDZT_ERR_OOM) throw;
+                    short_of = e.msg;
+                }
+            }
+        };
         for (int round = 0; round < 64; round++) {
+            advance_done();
             std::vector<LiveJob*> v, few;                 // runs of the persistent kernel, and small ones
             long long dims = 0;
             size_t smem = 0;
@@ -2595,6 +2654,7 @@ int server_step(edzt_server* sv)
                 }
             }
             if (v.empty() && few.empty()) break;
+            moved = true;
             if (!few.empty()) left -= run_slice(c, few, 0, smem);
             auto est = sv->ms_per_phase.find(cls);
             const double mpp = (est != sv->ms_per_phase.end()) ? est->second : 0.01 + (double)dims * 40.0 / 4.0e9;
@@ -2607,14 +2667,12 @@ int server_step(edzt_server* sv)
                 sv->ms_per_phase[cls] = (est != sv->ms_per_phase.end()) ? 0.5 * (est->second + per) : per;
                 left -= ms;
             }
-            for (auto& up : sv->active) {                     // requests move on as their phase's runs finish
-                if (up->cls != cls || up->phase >= 4 || !phase_done(*up)) continue;
-                if (up->phase == 1) after_scan(sv, *up);
-                else if (up->phase == 2) after_eigvec(sv, *up);
-                else if (up->phase == 3) after_green(sv, *up);
-            }
             if (left <= 0.0) break;
         }
+        advance_done();
+        // no class got on since: nobody is left to give memory back
+        sv->stuck = (moved || short_of.empty()) ? 0 : sv->stuck + 1;
+        if (sv->stuck >= (int)classes.size()) throw EdztError{EDZT_ERR_OOM, short_of};
     }
     CK(cudaStreamSynchronize(c->stream));
     int nfin = 0;                                             // retire finished requests, free their memory

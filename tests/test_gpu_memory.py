@@ -82,3 +82,33 @@ def test_failed_admission_leaves_the_request_queued(pkg):
         _same(got, ref)
         assert sv.step() == (0, 0, 0)
         sv.close()
+
+
+def test_server_goes_on_after_a_step_without_memory(pkg):
+    """Limits from the scan's vectors on, 16 KB apart: memory runs out between
+    the phases of the requests.  With memory again the server finishes them."""
+    insts, omega = _instances(pkg, [9, 6]), pkg.matsubara(16, 20.0)
+    vectors = 24.0 * _states(pkg, 9, insts[0]["sectors"])
+
+    def call(limit):
+        with pkg.Solver(0) as s:
+            s.set_keep_vectors(0)
+            sv = pkg.Server(s, 20, omega)
+            sv.set_step_ms(1000.0)                       # a step takes a request through
+            ids, failed = [sv.submit(i) for i in insts], 0
+            s.set_memory_limit_test(limit)
+            for _ in range(4):
+                failed += _run(pkg, sv.step) is None
+            s.set_memory_limit_test(0)
+            got, _ = _serve(pkg, sv, insts, ids)
+            assert sv.step() == (0, 0, 0)
+            sv.close()
+            return failed, got
+
+    _, ref = call(0)
+    failures = []
+    for k in range(60):
+        failed, got = call(vectors + 16 * KB * k)
+        failures.append(failed)
+        _same(got, ref)
+    assert max(failures) > 0 and min(failures) == 0
