@@ -2182,6 +2182,7 @@ struct ServReq {
     std::vector<double> G;                 // G_cl(nw, norb, nspin), complex interleaved
     std::vector<std::unique_ptr<LiveJob>> jobs;   // the live runs of the current phase
     long long kept_bytes = 0;              // of the kept vectors, while the scan runs
+    bool may_keep = true;                  // until it had to give its kept vectors up
     std::string error;
 };
 
@@ -2231,7 +2232,7 @@ void keep_request(edzt_server* sv, ServReq& q)
 {
     const long long n = scan_states(q.I), bytes = n * sv->maxnstep * (long long)sizeof(double);
     const double limit = std::min((double)sv->c->free_at_create / 32, (double)sv->budget / 8);
-    if (sv->reserved + bytes > sv->budget) return;
+    if (!q.may_keep || sv->reserved + bytes > sv->budget) return;
     if (keep_steps(sv->c, n, sv->maxnstep, limit - (double)sv->kept) < sv->maxnstep) return;
     q.I.kept = keep_lease(sv->c, (size_t)n * sv->maxnstep);
     if (!q.I.kept.p) return;
@@ -2597,14 +2598,45 @@ void advance(edzt_server* sv, ServReq& q)
     if (!q.has_vec) {
         if (!q.I.gsvec.p)
             q.I.gsvec = Lease<double>(sv->c->pool, (size_t)sector_dim_ns(q.I.model.nsite, q.I.gs_up, q.I.gs_dn));
-        if (q.phase == 1 && !q.I.kept.p) {
+        if (q.phase == 1 && q.I.kept.p) {
+            try {
+                vector_from_kept(sv, q);
+            } catch (const EdztError& e) {                // no room beside them: run the recurrence again
+                if (e.code != EDZT_ERR_OOM) throw;
+                drop_kept(sv, q);
+                sv->c->pool.trim();
+            }
+        }
+        if (q.phase == 1 && !q.has_vec) {
             start_eigvec(sv, q);
             return;
         }
-        if (q.phase == 1) vector_from_kept(sv, q);
-        else vector_from_pass(sv, q);
+        if (q.phase == 2) vector_from_pass(sv, q);
     }
     start_green(sv, q);
+}
+
+// Give up the kept vectors of all requests: one whose scan is read takes the
+// eigenvector pass, one whose scan still fills them goes back to the queue,
+// ahead of the others, and starts anew without.  False: there were none.
+bool give_up_kept(edzt_server* sv)
+{
+    bool had = false;
+    for (size_t i = sv->active.size(); i-- > 0;) {
+        ServReq& q = *sv->active[i];
+        if (!q.I.kept.p || q.phase >= 4) continue;
+        had = true;
+        if (q.win >= 0) {
+            drop_kept(sv, q);
+            continue;
+        }
+        take_back(sv, q);
+        q.may_keep = false;
+        sv->queue.push_front(std::move(sv->active[i]));
+        sv->active.erase(sv->active.begin() + (long)i);
+    }
+    if (had) sv->c->pool.trim();
+    return had;
 }
 
 // One step: admit what fits, then serve the next size class in turn.
@@ -2654,15 +2686,30 @@ int server_step(edzt_server* sv)
                 }
             }
             if (v.empty() && few.empty()) break;
-            moved = true;
-            if (!few.empty()) left -= run_slice(c, few, 0, smem);
+            auto slice = [&](std::vector<LiveJob*>& runs, int phases, size_t small) {
+                try {
+                    const float ms = run_slice(c, runs, phases, small);
+                    moved = true;
+                    return ms;
+                } catch (const EdztError& e) {
+                    if (e.code != EDZT_ERR_OOM) throw;
+                    short_of = e.msg;
+                    return -1.0f;
+                }
+            };
+            if (!few.empty()) {
+                const float ms = slice(few, 0, smem);
+                if (ms < 0.0f) break;
+                left -= ms;
+            }
             auto est = sv->ms_per_phase.find(cls);
             const double mpp = (est != sv->ms_per_phase.end()) ? est->second : 0.01 + (double)dims * 40.0 / 4.0e9;
             int phases = (int)std::min(4096.0, std::max(2.0, left / std::max(mpp, 1e-4)));
             phases &= ~1;
             if (phases < 2) phases = 2;
             if (!v.empty()) {
-                const float ms = run_slice(c, v, phases);
+                const float ms = slice(v, phases, 0);
+                if (ms < 0.0f) break;
                 const double per = ms / phases;
                 sv->ms_per_phase[cls] = (est != sv->ms_per_phase.end()) ? 0.5 * (est->second + per) : per;
                 left -= ms;
@@ -2670,9 +2717,12 @@ int server_step(edzt_server* sv)
             if (left <= 0.0) break;
         }
         advance_done();
-        // no class got on since: nobody is left to give memory back
+        // no class got on since: nothing but kept vectors is left to give memory back
         sv->stuck = (moved || short_of.empty()) ? 0 : sv->stuck + 1;
-        if (sv->stuck >= (int)classes.size()) throw EdztError{EDZT_ERR_OOM, short_of};
+        if (sv->stuck >= (int)classes.size()) {
+            if (!give_up_kept(sv)) throw EdztError{EDZT_ERR_OOM, short_of};
+            sv->stuck = 0;
+        }
     }
     CK(cudaStreamSynchronize(c->stream));
     int nfin = 0;                                             // retire finished requests, free their memory

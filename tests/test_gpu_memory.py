@@ -112,3 +112,29 @@ def test_server_goes_on_after_a_step_without_memory(pkg):
         failures.append(failed)
         _same(got, ref)
     assert max(failures) > 0 and min(failures) == 0
+
+
+@pytest.mark.parametrize("second", [False, True])
+def test_server_gives_kept_vectors_up(pkg, second):
+    """Memory goes to others while a scan fills its kept vectors (and a second
+    request waits): what is left serves the requests without them, so they are
+    given up."""
+    insts, omega = _instances(pkg, [9, 9][:1 + second]), pkg.matsubara(16, 20.0)
+
+    def call(limited):
+        with pkg.Solver(0) as s:
+            sv = pkg.Server(s, 20, omega)
+            sv.set_step_ms(1e-3)
+            s.set_keep_vectors(int(limited))
+            ids = [sv.submit(insts[0])]
+            assert sv.step() == (1, 0, 0)                # the scan is on its way
+            if limited:                                  # 2.7 MB a request; 8 MB are held, 7.8 MB of them kept
+                s.set_memory_limit_test(1.5 * s.footprint(insts[0]))
+            ids += [sv.submit(i) for i in insts[1:]]
+            got, _ = _serve(pkg, sv, insts, ids, 4000)
+            sv.close()
+            return got
+
+    ref, got = call(False), call(True)
+    assert got is not None
+    _same(got, ref)
