@@ -1258,7 +1258,8 @@ Lease<double> keep_lease(edzt_ctx* c, size_t n)
 }
 
 // Run f.  If device memory does not suffice and drop() had kept vectors to give
-// back, run it once more without: they never make a call fail.
+// back to the device, run it once more without: they never make a call fail.
+// Everything that is allocated while they are held runs under this.
 template <class F, class D>
 void run_or_drop_kept(F f, D drop)
 {
@@ -1362,6 +1363,13 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
         if (!keep)
             for (auto& k : kept) k = Lease<double>();
     }
+    auto drop_kept = [&] {
+        const bool had = keep > 0;
+        keep = 0;
+        for (auto& k : kept) k.reset();
+        if (had) c->pool.trim();
+        return had;
+    };
     if (c->engine == EDZT_ENGINE_FUSED) {
         std::vector<JobSpec> specs;
         std::vector<int> which;
@@ -1387,11 +1395,8 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
         }
         run_or_drop_kept([&] { run_jobs(c, specs); },
                          [&] {
-                             const bool had = keep > 0;
-                             keep = 0;
-                             for (auto& k : kept) k.reset();
                              for (JobSpec& s : specs) s.keep = nullptr, s.keep_steps = 0;
-                             return had;
+                             return drop_kept();
                          });
         const size_t n_ab = (size_t)nsector * 2 * maxnstep;
         double* hab = reinterpret_cast<double*>(stage_buffer(c, sizeof(double) * n_ab));
@@ -1425,47 +1430,51 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
         if (best < 0) throw EdztError{EDZT_ERR_NUMERIC, "no sector produced a ground state"};
         const int nu = sectors[2 * best], nd = sectors[2 * best + 1];
         const long long dim = sector_dim(c, nu, nd);
-        c->gs_vec = Lease<double>(c->pool, (size_t)dim);
         SectorResult& r = res[best];
-        const DevSector Si = make_sector_mt(c, c->mt, nu, nd, true);
-        Lease<double> cf(c->pool, (size_t)r.nstep), cw(c->pool, (size_t)r.nstep);
-        std::vector<double> hw;
-        if (keep) {
-            hw = keep_weights(r, r.b.data());
-            CK(cudaMemcpyAsync(cw.p, hw.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
-        }
-        if (keep && r.nstep <= keep) {
-            std::vector<VecSum> vs{natural_sum(Si, kept[best].p, cw.p, r.nstep, c->gs_vec.p)};
-            normalised_sums(c, vs);
-        } else {
-            Lease<double> ab(c->pool, (size_t)2 * maxnstep), eig(c->pool, (size_t)vec_size(nu, nd));
-            CK(cudaMemcpyAsync(cf.p, r.coeff.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
-            CK(cudaMemcpyAsync(ab.p, r.a.data(), sizeof(double) * maxnstep, cudaMemcpyHostToDevice, c->stream));
-            CK(cudaMemcpyAsync(ab.p + maxnstep, r.b.data(), sizeof(double) * maxnstep, cudaMemcpyHostToDevice, c->stream));
-            std::vector<JobSpec> ev(1);
-            ev[0].nu = nu; ev[0].nd = nd;
-            ev[0].mode = LZ_EIGVEC;
-            ev[0].init = LZ_INIT_HASH;
-            ev[0].key = edzt_stream_key(seed, stream_of(best));
-            ev[0].maxnstep = r.nstep;
-            ev[0].coeff = cf.p;
-            ev[0].eig = eig.p;
-            ev[0].a = ab.p;
-            ev[0].b = ab.p + maxnstep;
-            if (keep) {                                   // the kept steps but the last, which the run begins with
-                VecSum vs = natural_sum(Si, kept[best].p, cw.p, keep - 1, eig.p);
-                vs.natural = 0;
-                c->launches += launch_vec_sum(&vs, 1, c->stream);
-                CKLAUNCH();
-                ev[0].resume = keep;
-                ev[0].v_at = kept[best].p + (size_t)(keep - 1) * vec_size(nu, nd);
-                ev[0].v_before = kept[best].p + (size_t)(keep - 2) * vec_size(nu, nd);
-                ev[0].b_before = (keep == 2) ? r.norm0 : r.b[keep - 2];
+        auto form_vector = [&] {
+            c->gs_vec.reset();
+            c->gs_vec = Lease<double>(c->pool, (size_t)dim);
+            const DevSector Si = make_sector_mt(c, c->mt, nu, nd, true);
+            Lease<double> cf(c->pool, (size_t)r.nstep), cw(c->pool, (size_t)r.nstep);
+            std::vector<double> hw;
+            if (keep) {
+                hw = keep_weights(r, r.b.data());
+                CK(cudaMemcpyAsync(cw.p, hw.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
             }
-            run_jobs(c, ev);
-            std::vector<VecSum> vs{natural_sum(Si, eig.p, nullptr, 1, c->gs_vec.p)};
-            normalised_sums(c, vs);
-        }
+            if (keep && r.nstep <= keep) {
+                std::vector<VecSum> vs{natural_sum(Si, kept[best].p, cw.p, r.nstep, c->gs_vec.p)};
+                normalised_sums(c, vs);
+            } else {
+                Lease<double> ab(c->pool, (size_t)2 * maxnstep), eig(c->pool, (size_t)vec_size(nu, nd));
+                CK(cudaMemcpyAsync(cf.p, r.coeff.data(), sizeof(double) * r.nstep, cudaMemcpyHostToDevice, c->stream));
+                CK(cudaMemcpyAsync(ab.p, r.a.data(), sizeof(double) * maxnstep, cudaMemcpyHostToDevice, c->stream));
+                CK(cudaMemcpyAsync(ab.p + maxnstep, r.b.data(), sizeof(double) * maxnstep, cudaMemcpyHostToDevice, c->stream));
+                std::vector<JobSpec> ev(1);
+                ev[0].nu = nu; ev[0].nd = nd;
+                ev[0].mode = LZ_EIGVEC;
+                ev[0].init = LZ_INIT_HASH;
+                ev[0].key = edzt_stream_key(seed, stream_of(best));
+                ev[0].maxnstep = r.nstep;
+                ev[0].coeff = cf.p;
+                ev[0].eig = eig.p;
+                ev[0].a = ab.p;
+                ev[0].b = ab.p + maxnstep;
+                if (keep) {                                   // the kept steps but the last, which the run begins with
+                    VecSum vs = natural_sum(Si, kept[best].p, cw.p, keep - 1, eig.p);
+                    vs.natural = 0;
+                    c->launches += launch_vec_sum(&vs, 1, c->stream);
+                    CKLAUNCH();
+                    ev[0].resume = keep;
+                    ev[0].v_at = kept[best].p + (size_t)(keep - 1) * vec_size(nu, nd);
+                    ev[0].v_before = kept[best].p + (size_t)(keep - 2) * vec_size(nu, nd);
+                    ev[0].b_before = (keep == 2) ? r.norm0 : r.b[keep - 2];
+                }
+                run_jobs(c, ev);
+                std::vector<VecSum> vs{natural_sum(Si, eig.p, nullptr, 1, c->gs_vec.p)};
+                normalised_sums(c, vs);
+            }
+        };
+        run_or_drop_kept(form_vector, drop_kept);
         for (auto& k : kept) k = Lease<double>();
         if (want_residual) c->gs_residual = residual(c, make_sector(c, nu, nd), c->gs_vec.p, r.e);
         c->gs_up = nu; c->gs_dn = nd; c->gs_isector = best; c->gs_e0 = r.e;
@@ -1957,16 +1966,17 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
     }
     keep_scans(c, B, i0, i1, maxnstep, keep_limit);
     for (int q = 0; q < nj; q++) keep_in(B[own[q].inst], own[q].sector, maxnstep, specs[q]);
-    run_or_drop_kept([&] { run_jobs(c, specs); },
-                     [&] {
-                         bool had = false;
-                         for (int i = i0; i < i1; i++) {
-                             had = had || B[i].kept.p;
-                             B[i].kept.reset();
-                         }
-                         for (JobSpec& j : specs) j.keep = nullptr, j.keep_steps = 0;
-                         return had;
-                     });
+    auto drop_kept = [&] {
+        bool had = false;
+        for (int i = i0; i < i1; i++) {
+            had = had || B[i].kept.p;
+            B[i].kept.reset();
+        }
+        for (JobSpec& j : specs) j.keep = nullptr, j.keep_steps = 0;
+        if (had) c->pool.trim();
+        return had;
+    };
+    run_or_drop_kept([&] { run_jobs(c, specs); }, drop_kept);
     std::vector<double> hab((size_t)std::max(nj, 1) * 2 * maxnstep);
     CK(cudaMemcpyAsync(hab.data(), ab.p, sizeof(double) * hab.size(), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1990,52 +2000,55 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
         if (w < 0 || res[q].e < res[w].e - tie) win[i] = q;
     }
     // ---- eigenvector pass of every winner (lanczos_solver.f90:213-300)
-    std::vector<JobSpec> ev;
-    std::vector<Lease<double>> eigs(i1 - i0); // the eigenvectors in internal order, where no v_k were kept
-    Lease<double> coeffs(c->pool, (size_t)std::max(i1 - i0, 1) * maxnstep);
-    std::vector<double> hcoef((size_t)std::max(i1 - i0, 1) * maxnstep, 0.0);
-    for (int i = i0; i < i1; i++) {
-        const int q = win[i];
-        if (q < 0) throw EdztError{EDZT_ERR_NUMERIC, "instance " + std::to_string(i) + ": no sector produced a ground state"};
-        BatchInst& I = B[i];
-        I.best = own[q].sector;
-        I.gs_up = specs[q].nu; I.gs_dn = specs[q].nd;
-        I.e0 = res[q].e;
-        I.gsvec = Lease<double>(c->pool, (size_t)sector_dim_ns(I.model.nsite, I.gs_up, I.gs_dn));
-        const int ns = I.model.nsite;
-        if (I.kept.p) {
-            const std::vector<double> w = keep_weights(res[q], hab.data() + (size_t)(2 * q + 1) * maxnstep);
-            std::copy(w.begin(), w.end(), hcoef.begin() + (size_t)(i - i0) * maxnstep);
-            continue;
+    auto form_vectors = [&] {
+        std::vector<JobSpec> ev;
+        std::vector<Lease<double>> eigs(i1 - i0); // the eigenvectors in internal order, where no v_k were kept
+        Lease<double> coeffs(c->pool, (size_t)std::max(i1 - i0, 1) * maxnstep);
+        std::vector<double> hcoef((size_t)std::max(i1 - i0, 1) * maxnstep, 0.0);
+        for (int i = i0; i < i1; i++) {
+            const int q = win[i];
+            if (q < 0) throw EdztError{EDZT_ERR_NUMERIC, "instance " + std::to_string(i) + ": no sector produced a ground state"};
+            BatchInst& I = B[i];
+            I.best = own[q].sector;
+            I.gs_up = specs[q].nu; I.gs_dn = specs[q].nd;
+            I.e0 = res[q].e;
+            I.gsvec.reset();
+            I.gsvec = Lease<double>(c->pool, (size_t)sector_dim_ns(I.model.nsite, I.gs_up, I.gs_dn));
+            const int ns = I.model.nsite;
+            if (I.kept.p) {
+                const std::vector<double> w = keep_weights(res[q], hab.data() + (size_t)(2 * q + 1) * maxnstep);
+                std::copy(w.begin(), w.end(), hcoef.begin() + (size_t)(i - i0) * maxnstep);
+                continue;
+            }
+            eigs[i - i0] = Lease<double>(c->pool, (size_t)lz_vec_size((int)edzt_binom(ns, I.gs_up), (int)edzt_binom(ns, I.gs_dn)));
+            std::copy(res[q].coeff.begin(), res[q].coeff.end(), hcoef.begin() + (size_t)(i - i0) * maxnstep);
+            JobSpec j;
+            j.mt = I.mt.get();
+            j.nu = I.gs_up; j.nd = I.gs_dn;
+            j.mode = LZ_EIGVEC;
+            j.init = LZ_INIT_HASH;
+            j.key = specs[q].key;
+            j.maxnstep = res[q].nstep;
+            j.coeff = coeffs.p + (size_t)(i - i0) * maxnstep;
+            j.eig = eigs[i - i0].p;
+            j.a = specs[q].a;            // the coefficients of the scan, still on the device
+            j.b = specs[q].b;
+            ev.push_back(j);
         }
-        eigs[i - i0] = Lease<double>(c->pool, (size_t)lz_vec_size((int)edzt_binom(ns, I.gs_up), (int)edzt_binom(ns, I.gs_dn)));
-        std::copy(res[q].coeff.begin(), res[q].coeff.end(), hcoef.begin() + (size_t)(i - i0) * maxnstep);
-        JobSpec j;
-        j.mt = I.mt.get();
-        j.nu = I.gs_up; j.nd = I.gs_dn;
-        j.mode = LZ_EIGVEC;
-        j.init = LZ_INIT_HASH;
-        j.key = specs[q].key;
-        j.maxnstep = res[q].nstep;
-        j.coeff = coeffs.p + (size_t)(i - i0) * maxnstep;
-        j.eig = eigs[i - i0].p;
-        j.a = specs[q].a;            // the coefficients of the scan, still on the device
-        j.b = specs[q].b;
-        ev.push_back(j);
-    }
-    CK(cudaMemcpyAsync(coeffs.p, hcoef.data(), sizeof(double) * hcoef.size(), cudaMemcpyHostToDevice, c->stream));
-    run_jobs(c, ev);
-    std::vector<VecSum> vs;
-    for (int i = i0; i < i1; i++) {
-        const DevSector Si = make_sector_mt(c, *B[i].mt, B[i].gs_up, B[i].gs_dn, true);
-        if (B[i].kept.p)
-            vs.push_back(natural_sum(Si, specs[win[i]].keep, coeffs.p + (size_t)(i - i0) * maxnstep, res[win[i]].nstep,
-                                     B[i].gsvec.p));
-        else vs.push_back(natural_sum(Si, eigs[i - i0].p, nullptr, 1, B[i].gsvec.p));
-    }
-    normalised_sums(c, vs);
+        CK(cudaMemcpyAsync(coeffs.p, hcoef.data(), sizeof(double) * hcoef.size(), cudaMemcpyHostToDevice, c->stream));
+        run_jobs(c, ev);
+        std::vector<VecSum> vs;
+        for (int i = i0; i < i1; i++) {
+            const DevSector Si = make_sector_mt(c, *B[i].mt, B[i].gs_up, B[i].gs_dn, true);
+            if (B[i].kept.p)
+                vs.push_back(natural_sum(Si, specs[win[i]].keep, coeffs.p + (size_t)(i - i0) * maxnstep, res[win[i]].nstep,
+                                         B[i].gsvec.p));
+            else vs.push_back(natural_sum(Si, eigs[i - i0].p, nullptr, 1, B[i].gsvec.p));
+        }
+        normalised_sums(c, vs);
+    };
+    run_or_drop_kept(form_vectors, drop_kept);
     for (int i = i0; i < i1; i++) B[i].kept.reset();
-    eigs.clear();
     // ---- Green's function runs of every instance (dmft_green.f90:47-126)
     std::vector<GreenRun> runs;
     std::vector<size_t> r0(B.size(), 0);

@@ -24,6 +24,40 @@ def _run(pkg, f):
         return None
 
 
+def _limits(kept):
+    """Limits around the kept vectors' size, 8 KB apart, and from little to plenty."""
+    return sorted({kept + 8 * KB * k for k in range(130)} | {float(x) for x in np.geomspace(64 * KB, 2 * kept, 12)})
+
+
+# The tolerance is that of the kept vectors' tests for m steps: (m + 4) 2^-53
+# sqrt(m) < 1e-13 for m <= 60.
+@pytest.mark.parametrize("sectors,steps,share", [([(4, 5), (5, 4), (4, 4)], 20, 1.0), ([(4, 4)], 40, 1.0),
+                                                 ([(4, 4)], 40, 0.6)])
+def test_kept_vectors_never_make_a_ground_state_fail(pkg, sectors, steps, share):
+    m = random_model(pkg, np.random.default_rng(17), 1, 8, spin_dep=True)
+    kept = 8.0 * _states(pkg, 9, sectors) * (steps if share == 1.0 else int(share * steps))
+
+    def call(limit, keep):
+        with pkg.Solver(0) as s:
+            s.set_model(m)
+            s.set_keep_vectors(keep)
+            if share < 1.0:
+                s.set_keep_limit_test(kept)
+            s.set_memory_limit_test(limit)
+            return _run(pkg, lambda: s.ground_state(sectors, steps, seed=3))
+
+    ref = call(0, 0)
+    outcomes = set()
+    for limit in _limits(kept):
+        without, with_ = call(limit, 0), call(limit, 1)
+        outcomes.add((without is not None, with_ is not None))
+        if with_ is not None:
+            assert with_["isector"] == ref["isector"] and with_["e0"] == ref["e0"]
+            assert np.abs(with_["vec"] - ref["vec"]).max() <= 1e-13
+    assert (True, False) not in outcomes
+    assert (True, True) in outcomes and (False, False) in outcomes
+
+
 def _instances(pkg, sizes, one_sector=False):
     rng = np.random.default_rng(23)
     out = []
@@ -39,6 +73,27 @@ def _same(got, ref):
     for (s1, e1, g1), (s2, e2, g2) in zip(got, ref, strict=True):
         assert s1 == s2 and abs(e1 - e2) <= 1e-10 * max(1.0, abs(e2))
         assert np.abs(np.asarray(g1) - np.asarray(g2)).max() <= 1e-8
+
+
+def _batch(pkg, insts, steps, limit, keep, budget):
+    with pkg.Solver(0) as s:
+        s.set_keep_vectors(keep)
+        s.set_memory_limit_test(limit)
+        b = _run(pkg, lambda: s.solve_batch(insts, steps, pkg.matsubara(16, 20.0), hbm_budget=budget))
+    return b and list(zip(b["isector"], b["e0"], b["G_cl"]))
+
+
+def test_kept_vectors_never_make_a_batch_fail(pkg):
+    insts, steps = _instances(pkg, [9, 9, 9], one_sector=True), 30
+    kept = 8.0 * steps * _states(pkg, 9, [(4, 4)])
+    ref = _batch(pkg, insts, steps, 0, 0, 1 << 30)
+    outcomes = set()
+    for limit in _limits(2 * kept):
+        without, with_ = (_batch(pkg, insts, steps, limit, keep, 1 << 30) for keep in (0, 1))
+        outcomes.add((without is not None, with_ is not None))
+        if with_ is not None:
+            _same(with_, ref)
+    assert (True, False) not in outcomes and (True, True) in outcomes
 
 
 def _serve(pkg, sv, insts, ids=None, steps=400):
