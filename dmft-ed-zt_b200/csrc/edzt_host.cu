@@ -56,6 +56,25 @@ void arg_check(bool ok, const char* what)
 class Pool {
   public:
     ~Pool() { release_all(); }
+    // A new block; cached ones are given back to the device where memory is short.
+    void* grow(size_t bytes)
+    {
+        void* p = try_malloc(bytes);
+        if (!p) {
+            trim();
+            p = try_malloc(bytes);
+            if (!p) throw EdztError{EDZT_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes failed"};
+        }
+        held_ += bytes;
+        return p;
+    }
+    // The same for a buffer that its owner frees.
+    void* apart(size_t bytes)
+    {
+        void* p = grow(bytes);
+        held_ -= bytes;
+        return p;
+    }
     void* get(size_t bytes)
     {
         bytes = (bytes + 255) & ~(size_t)255;
@@ -67,12 +86,7 @@ class Pool {
             free_.erase(it);
             return p;
         }
-        void* p = try_malloc(bytes);
-        if (!p) {
-            trim();
-            p = try_malloc(bytes);
-            if (!p) throw EdztError{EDZT_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes failed"};
-        }
+        void* p = grow(bytes);
         used_[p] = bytes;
         return p;
     }
@@ -117,7 +131,6 @@ class Pool {
             cudaGetLastError();
             return nullptr;
         }
-        held_ += bytes;
         return p;
     }
 
@@ -153,6 +166,7 @@ struct DevBuf {
     void* p = nullptr;
     DevBuf() = default;
     explicit DevBuf(size_t bytes) { CK(cudaMalloc(&p, bytes > 0 ? bytes : 16)); }
+    DevBuf(Pool& pool, size_t bytes) : p(pool.apart(bytes > 0 ? bytes : 16)) {}
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { if (p) cudaFree(p); }
@@ -274,9 +288,9 @@ std::unique_ptr<StrTable> build_str_table(edzt_ctx* c, int ns, int n, int norb)
     t->n = n;
     t->count = (int)edzt_binom(ns, n);
     const size_t cnt = (size_t)std::max(t->count, 1);
-    t->str = std::make_unique<DevBuf>(sizeof(uint32_t) * cnt);
-    t->rank = std::make_unique<DevBuf>(sizeof(int32_t) * ((size_t)1 << ns));
-    if (norb > 0) t->nat = std::make_unique<DevBuf>(sizeof(int32_t) * cnt);
+    t->str = std::make_unique<DevBuf>(c->pool, sizeof(uint32_t) * cnt);
+    t->rank = std::make_unique<DevBuf>(c->pool, sizeof(int32_t) * ((size_t)1 << ns));
+    if (norb > 0) t->nat = std::make_unique<DevBuf>(c->pool, sizeof(int32_t) * cnt);
     launch_build_strings(ns, n, t->str->as<uint32_t>(), t->rank->as<int32_t>(), c->stream, norb,
                          t->nat ? t->nat->as<int32_t>() : nullptr);
     c->launches += 2;
@@ -3214,7 +3228,7 @@ int edzt_server_create(edzt_ctx* c, int maxnstep, int nw, const double* omega, s
         sv->c = c;
         sv->maxnstep = maxnstep;
         sv->nw = nw;
-        sv->omega = std::make_unique<DevBuf>(sizeof(double) * std::max(nw, 1));
+        sv->omega = std::make_unique<DevBuf>(c->pool, sizeof(double) * std::max(nw, 1));
         if (nw > 0) CK(cudaMemcpy(sv->omega->p, omega, sizeof(double) * nw, cudaMemcpyDefault));
         if (hbm_budget == 0) {
             size_t fr = 0, tot = 0;

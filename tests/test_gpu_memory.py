@@ -193,3 +193,15 @@ def test_server_gives_kept_vectors_up(pkg, second):
     ref, got = call(False), call(True)
     assert got is not None
     _same(got, ref)
+
+
+def test_string_tables_get_what_earlier_calls_left_cached(pkg):
+    """A scan leaves blocks cached; the string tables of a later model take
+    their place when there is no other memory."""
+    with pkg.Solver(0) as s:
+        s.set_model(random_model(pkg, np.random.default_rng(2), 1, 9))
+        s.ground_state([(5, 5)], 60, seed=1)             # 63,504 states, 60 steps: 30 MB kept
+        s.set_model(random_model(pkg, np.random.default_rng(2), 1, 15))
+        s.set_memory_limit_test(2048 * KB)               # the last ground state (500 KB) and the tables
+        up, dn = s.generate_basis(8, 1)                  # rank tables of 2^16 strings, 256 KB each
+        assert up.size == 12870 and dn.size == 16
