@@ -119,6 +119,13 @@ class Pool {
         used_.clear();
         held_ = 0;
     }
+    // Device memory that is free, under the test's limit.
+    size_t available() const
+    {
+        size_t fr = 0, tot = 0;
+        CK(cudaMemGetInfo(&fr, &tot));
+        return limit_ ? std::min(fr, limit_ - std::min(held_, limit_)) : fr;
+    }
     // Test of running out of memory: blocks of at most `bytes` altogether (0: what the device has).
     void set_limit(size_t bytes) { limit_ = bytes; }
 
@@ -2139,13 +2146,11 @@ void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int max
     long long all = 0;
     for (const BatchInst& I : B) all += I.footprint;
     const bool asked = budget != 0;
-    if (budget == 0 && all <= (long long)kBatchKeep) {
-        budget = kBatchKeep;                              // one wave; no need to ask what is free
-    } else if (budget == 0) {
-        size_t fr = 0, tot = 0;
-        CK(cudaMemGetInfo(&fr, &tot));
-        budget = fr / 10 * 8;
-    }
+    // A small batch tries one wave without asking what is free: the query can
+    // wait on the driver behind other processes' queries.
+    bool queried = asked || all > (long long)kBatchKeep;
+    if (!queried) budget = kBatchKeep;
+    else if (!asked) budget = c->pool.available() / 10 * 8;
     InVec om(c, omega, nw);
     std::vector<double> Gall(std::max(goff[ninst], (size_t)1), 0.0);
     for (int i0 = 0; i0 < ninst;) {   // waves that fit the device-memory budget
@@ -2154,7 +2159,20 @@ void solve_batch_impl(edzt_ctx* c, int ninst, const edzt_instance* inst, int max
         while (i1 < ninst && (i1 == i0 || sum + B[i1].footprint <= (long long)budget)) sum += B[i1++].footprint;
         double keep = 0.5 * (double)batch_cache(c);
         if (asked) keep = std::min(keep, (double)budget - (double)sum);
-        solve_wave(c, B, i0, i1, maxnstep, nw, om.d, Gall, goff, keep);
+        try {
+            solve_wave(c, B, i0, i1, maxnstep, nw, om.d, Gall, goff, keep);
+        } catch (const EdztError& e) {
+            if (e.code != EDZT_ERR_OOM || queried) throw;
+            for (int i = i0; i < i1; i++) {               // it does not fit at once: waves of what is free
+                B[i].gsvec.reset();
+                B[i].kept.reset();
+                B[i].mt.reset();
+            }
+            c->pool.trim();
+            budget = c->pool.available() / 10 * 8;
+            queried = true;
+            continue;
+        }
         c->pool.trim_to(batch_cache(c));
         i0 = i1;
     }

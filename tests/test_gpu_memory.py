@@ -96,6 +96,19 @@ def test_kept_vectors_never_make_a_batch_fail(pkg):
     assert (True, False) not in outcomes and (True, True) in outcomes
 
 
+@pytest.mark.parametrize("share", [0.3, 0.5, 0.9])
+def test_batch_that_does_not_fit_at_once_runs_in_waves(pkg, share):
+    """Without a budget of the caller's a batch takes what there is: instances
+    that fit one by one are solved, whatever their sum."""
+    insts = _instances(pkg, [9, 9, 10, 9, 10, 9])
+    with pkg.Solver(0) as s:
+        total = float(sum(s.footprint(i) for i in insts))
+    ref = _batch(pkg, insts, 30, 0, 1, 0)
+    got = _batch(pkg, insts, 30, share * total + 512 * KB, 1, 0)
+    assert got is not None
+    _same(got, ref)
+
+
 def _serve(pkg, sv, insts, ids=None, steps=400):
     """Results of the requests, or None where a step ran out of memory."""
     ids = [sv.submit(i) for i in insts] if ids is None else ids
