@@ -661,6 +661,12 @@ void log_launch(edzt_ctx* c, double ms, double bytes, double states)
     c->log_states.push_back(states);
 }
 
+// A form of the kernel of small runs (0: none) and the shared memory of its runs.
+struct SmallKernel {
+    int form = 0;
+    size_t smem = 0;
+};
+
 // The run's descriptor but for its vectors and state.
 void fill_job(LzJob& J, const JobSpec& s, const DevSector& S)
 {
@@ -751,25 +757,19 @@ float launch_jobs(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& s
     return ms;
 }
 
-// The same with the kernel of small runs, which need no plan.
-float launch_small(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& st, size_t smem)
+// The same with a form of the kernel of small runs, which need no plan.
+float launch_small(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& st, const SmallKernel& K)
 {
     const size_t nj = jobs.size(), bytes_st = sizeof(LzState) * st.size();
     const size_t o_jobs = (bytes_st + 255) & ~(size_t)255, size = o_jobs + sizeof(LzJob) * nj;
     Lease<char> blob(c->pool, size);
-    bool exchange = false;
-    long long most = 0;
-    for (size_t j = 0; j < nj; j++) {
-        most = std::max(most, jobs[j].S.dim);
-        jobs[j].st = reinterpret_cast<LzState*>(blob.p) + 2 * j;
-        exchange = exchange || jobs[j].S.has_j;
-    }
+    for (size_t j = 0; j < nj; j++) jobs[j].st = reinterpret_cast<LzState*>(blob.p) + 2 * j;
     char* h = stage_buffer(c, size);
     std::memcpy(h + o_jobs, jobs.data(), sizeof(LzJob) * nj);
     const LzJob* d_jobs = reinterpret_cast<const LzJob*>(blob.p + o_jobs);
     CK(cudaMemcpyAsync(blob.p + o_jobs, h + o_jobs, sizeof(LzJob) * nj, cudaMemcpyHostToDevice, c->stream));
     CK(cudaEventRecord(c->ev0, c->stream));
-    CK(launch_lanczos_small(d_jobs, (int)nj, smem, exchange, most, c->stream));
+    CK(launch_lanczos_small(d_jobs, (int)nj, K.smem, K.form, c->stream));
     CK(cudaEventRecord(c->ev1, c->stream));
     c->launches += 1;
     CK(cudaMemcpyAsync(h, blob.p, bytes_st, cudaMemcpyDeviceToHost, c->stream));
@@ -795,6 +795,19 @@ void book_launch(edzt_ctx* c, const std::vector<LzJob>& jobs, double ms, double 
 bool small_allowed(const edzt_ctx* c, const LzJob& J)
 {
     return c->dbg_pass_cap == 0 && c->dbg_stall_cta < 0 && !c->tuned.count({J.S.up.count, J.S.dn.count});
+}
+
+// Count a run in with the others of its model: K becomes the form for all of
+// them, or -1 (the persistent kernel) when one is not small.
+void small_include(SmallKernel& K, const LzJob& J)
+{
+    const size_t need = lz_small_smem(J.S, J.mode);
+    if (K.form < 0 || need == 0) {
+        K = SmallKernel{-1, 0};
+        return;
+    }
+    K.form = std::max(K.form, lz_small_form(J.S));
+    K.smem = std::max(K.smem, need);
 }
 
 // All runs of specs from start to finish.  Coefficient runs write a and b up
@@ -823,19 +836,21 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     }
     build_ops(c, todo);
     // Runs for the kernel of small ones: those of a model that are all small,
-    // so that a model's runs take the same way alone and among others.
-    std::map<const ModelTables*, size_t> small_mem;
+    // in the form for that model, so that a model's runs take the same way
+    // alone and among others.
+    std::map<const ModelTables*, SmallKernel> kernel_of;
     for (int j = 0; j < nj; j++) {
-        const size_t need = (force || !small_allowed(c, jobs[j])) ? 0 : lz_small_smem(jobs[j].S, jobs[j].mode);
-        const auto it = small_mem.emplace(specs[j].mt, need).first;
-        it->second = (need && it->second) ? std::max(need, it->second) : 0;
+        SmallKernel& K = kernel_of.emplace(specs[j].mt, SmallKernel{}).first->second;
+        if (force || !small_allowed(c, jobs[j])) K.form = -1;
+        small_include(K, jobs[j]);
     }
-    std::vector<int> order[2];                            // jobs of either kernel
-    size_t smem = 0;
+    std::vector<int> order[kSmallForms + 1];              // jobs by kernel; 0: the persistent one
+    size_t smem[kSmallForms + 1] = {};
     for (int j = 0; j < nj; j++) {
-        const size_t m = small_mem[specs[j].mt];
-        order[m > 0].push_back(j);
-        smem = std::max(smem, m);
+        const SmallKernel& K = kernel_of[specs[j].mt];
+        const int f = std::max(K.form, 0);
+        order[f].push_back(j);
+        smem[f] = std::max(smem[f], K.smem);
     }
     for (int j : order[0]) {
         LzJob& J = jobs[j];
@@ -861,8 +876,8 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     }
     int phases = 2 * max_steps + 4;     // two phases per step and the phase that closes the last one
     if (c->dbg_pass_cap > 0) phases = std::min(phases, c->dbg_pass_cap);
-    for (int small = 1; small >= 0; small--) {
-        const std::vector<int>& o = order[small];
+    for (int f = kSmallForms; f >= 0; f--) {
+        const std::vector<int>& o = order[f];
         if (o.empty()) continue;
         std::vector<LzJob> part;
         std::vector<LzState> ps;
@@ -870,8 +885,8 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
             part.push_back(jobs[j]);
             ps.insert(ps.end(), &st[2 * (size_t)j], &st[2 * (size_t)j] + 2);
         }
-        const float ms = small ? launch_small(c, part, ps, smem)
-                               : launch_jobs(c, part, ps, force ? force : tuned_shape(c, part), phases, false);
+        const float ms = f ? launch_small(c, part, ps, SmallKernel{f, smem[f]})
+                           : launch_jobs(c, part, ps, force ? force : tuned_shape(c, part), phases, false);
         double bytes = 0.0;
         for (size_t i = 0; i < o.size(); i++) {
             JobSpec& s = specs[o[i]];
@@ -2309,27 +2324,27 @@ std::unique_ptr<LiveJob> make_live(edzt_ctx* c, const JobSpec& spec, std::vector
     return L;
 }
 
-// The largest shared memory that the runs of a request's phase take in the
-// kernel of small ones; 0: they are for the persistent kernel (some run is
-// larger, or all their steps at once, 4 us each, would outlast a server step).
-size_t small_request(const edzt_server* sv, const ServReq& q)
+// The kernel of small runs for those of a request's phase; form 0: they are for
+// the persistent kernel (some run is larger, or all their steps at once, 4 us
+// each, would outlast a server step).
+SmallKernel small_request(const edzt_server* sv, const ServReq& q)
 {
-    size_t most = 0;
+    SmallKernel K;
     for (const auto& j : q.jobs) {
         LzJob J;
         fill_job(J, j->spec, j->S);
-        const size_t need = small_allowed(sv->c, J) ? lz_small_smem(J.S, J.mode) : 0;
-        if (!need || 0.004 * J.maxnstep > sv->step_ms) return 0;
-        most = std::max(most, need);
+        if (!small_allowed(sv->c, J) || 0.004 * J.maxnstep > sv->step_ms) K.form = -1;
+        small_include(K, J);
+        if (K.form < 0) return SmallKernel{};
     }
-    return most;
+    return K;
 }
 
 // One slice: at most `phases` phases (even) of every live run in v, in one
-// persistent launch, or (small: the shared memory) all their steps in the
-// kernel of small runs; runs that finish are marked done with nstep and norm0.
-// Returns the launch's device time in ms.
-float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, size_t small = 0)
+// persistent launch, or (small.form) all their steps in the kernel of small
+// runs; runs that finish are marked done with nstep and norm0.  Returns the
+// launch's device time in ms.
+float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, const SmallKernel& small = {})
 {
     const int nj = (int)v.size();
     std::vector<LzJob> jobs(nj);
@@ -2346,8 +2361,8 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, size_t small 
     for (int j = 0; j < nj; j++) std::memcpy(&st[2 * (size_t)j], v[j]->st, 2 * sizeof(LzState));
     int budget = std::max(2, phases & ~1);
     if (c->dbg_pass_cap > 0) budget = std::min(budget, std::max(2, c->dbg_pass_cap & ~1));
-    const float ms = small ? launch_small(c, jobs, st, small)
-                           : launch_jobs(c, jobs, st, tuned_shape(c, jobs), budget, true);
+    const float ms = small.form ? launch_small(c, jobs, st, small)
+                                : launch_jobs(c, jobs, st, tuned_shape(c, jobs), budget, true);
     for (int j = 0; j < nj; j++) std::memcpy(v[j]->st, &st[2 * (size_t)j], 2 * sizeof(LzState));
     double bytes = 0.0;
     for (int j = 0; j < nj; j++) {
@@ -2717,21 +2732,23 @@ int server_step(edzt_server* sv)
         };
         for (int round = 0; round < 64; round++) {
             advance_done();
-            std::vector<LiveJob*> v, few;                 // runs of the persistent kernel, and small ones
+            std::vector<LiveJob*> runs[kSmallForms + 1], &v = runs[0];   // by kernel; 0: the persistent one
             long long dims = 0;
-            size_t smem = 0;
+            size_t smem[kSmallForms + 1] = {}, live = 0;
             for (auto& up : sv->active) {
                 if (up->cls != cls || up->phase >= 4) continue;
-                const size_t small = small_request(sv, *up);
-                smem = std::max(smem, small);
+                const SmallKernel K = small_request(sv, *up);
+                smem[K.form] = std::max(smem[K.form], K.smem);
                 for (auto& j : up->jobs) {
                     if (j->done) continue;
-                    (small ? few : v).push_back(j.get());
-                    if (!small) dims += j->S.dim;
+                    runs[K.form].push_back(j.get());
+                    live++;
+                    if (!K.form) dims += j->S.dim;
                 }
             }
-            if (v.empty() && few.empty()) break;
-            auto slice = [&](std::vector<LiveJob*>& runs, int phases, size_t small) {
+            if (live == 0) break;
+            bool short_slice = false;
+            auto slice = [&](std::vector<LiveJob*>& runs, int phases, const SmallKernel& small) {
                 try {
                     const float ms = run_slice(c, runs, phases, small);
                     moved = true;
@@ -2739,22 +2756,21 @@ int server_step(edzt_server* sv)
                 } catch (const EdztError& e) {
                     if (e.code != EDZT_ERR_OOM) throw;
                     short_of = e.msg;
-                    return -1.0f;
+                    short_slice = true;
+                    return 0.0f;
                 }
             };
-            if (!few.empty()) {
-                const float ms = slice(few, 0, smem);
-                if (ms < 0.0f) break;
-                left -= ms;
-            }
+            for (int f = 1; f <= kSmallForms; f++)
+                if (!runs[f].empty() && !short_slice) left -= slice(runs[f], 0, SmallKernel{f, smem[f]});
+            if (short_slice) break;
             auto est = sv->ms_per_phase.find(cls);
             const double mpp = (est != sv->ms_per_phase.end()) ? est->second : 0.01 + (double)dims * 40.0 / 4.0e9;
             int phases = (int)std::min(4096.0, std::max(2.0, left / std::max(mpp, 1e-4)));
             phases &= ~1;
             if (phases < 2) phases = 2;
             if (!v.empty()) {
-                const float ms = slice(v, phases, 0);
-                if (ms < 0.0f) break;
+                const float ms = slice(v, phases, SmallKernel{});
+                if (short_slice) break;
                 const double per = ms / phases;
                 sv->ms_per_phase[cls] = (est != sv->ms_per_phase.end()) ? 0.5 * (est->second + per) : per;
                 left -= ms;

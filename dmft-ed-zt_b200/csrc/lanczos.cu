@@ -953,22 +953,25 @@ size_t lz_small_smem(const DevSector& S, int mode)
     return size <= kLzSmallSmemMax ? size : 0;
 }
 
-cudaError_t launch_lanczos_small(const LzJob* jobs, int nj, size_t smem, bool exchange, long long most, cudaStream_t s)
+// Forms 1, 3: up to 512 states, a thread an element; 2, 4: more, four rows of a
+// column a thread; 3, 4 with exchange terms.  Chosen by a model's runs alone,
+// not by what else is in the launch: the forms differ in the last bits.
+int lz_small_form(const DevSector& S) { return 1 + (S.dim > 512 ? 1 : 0) + (S.has_j ? 2 : 0); }
+
+cudaError_t launch_lanczos_small(const LzJob* jobs, int nj, size_t smem, int form, cudaStream_t s)
 {
     using Kernel = void (*)(const LzJob*);
-    static const Kernel kernels[2][2] = {{k_lanczos_small<512, 1, false>, k_lanczos_small<512, 1, true>},
-                                         {k_lanczos_small<768, 4, false>, k_lanczos_small<768, 4, true>}};
+    static const Kernel kernels[kSmallForms] = {k_lanczos_small<512, 1, false>, k_lanczos_small<768, 4, false>,
+                                                k_lanczos_small<512, 1, true>, k_lanczos_small<768, 4, true>};
     static std::atomic<unsigned long long> done{0};
     if (edzt_once_per_device(done)) {
-        for (const auto& pair : kernels)
-            for (const Kernel k : pair) {
-                const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           (int)kLzSmallSmemMax);
-                if (e != cudaSuccess) return e;
-            }
+        for (const Kernel k : kernels) {
+            const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)kLzSmallSmemMax);
+            if (e != cudaSuccess) return e;
+        }
     }
-    const bool big = most > 512;
-    kernels[big][exchange]<<<nj, big ? 768 : 512, smem, s>>>(jobs);
+    kernels[form - 1]<<<nj, form % 2 ? 512 : 768, smem, s>>>(jobs);
     return cudaGetLastError();
 }
 
