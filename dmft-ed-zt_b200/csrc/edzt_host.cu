@@ -631,6 +631,8 @@ struct JobSpec {
     double* v_at = nullptr;          // its v, which is kept, and
     double* v_before = nullptr;      // the one before (overwritten by later ones),
     double b_before = 0.0;           // and the norm of that
+    int form = 0;                    // EIGVEC: the scan's; COEFF: set to the kernel that ran (0: the
+                                     // persistent one, else a form of the kernel of small runs)
     // results
     int nstep = 0;
     double norm0 = 0.0;
@@ -801,7 +803,7 @@ bool small_allowed(const edzt_ctx* c, const LzJob& J)
 // them, or -1 (the persistent kernel) when one is not small.
 void small_include(SmallKernel& K, const LzJob& J)
 {
-    const size_t need = lz_small_smem(J.S, J.mode);
+    const size_t need = lz_small_smem(J.S);
     if (K.form < 0 || need == 0) {
         K = SmallKernel{-1, 0};
         return;
@@ -840,6 +842,7 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     // alone and among others.
     std::map<const ModelTables*, SmallKernel> kernel_of;
     for (int j = 0; j < nj; j++) {
+        if (specs[j].mode != LZ_COEFF) continue;          // an eigenvector pass goes where its scan went
         SmallKernel& K = kernel_of.emplace(specs[j].mt, SmallKernel{}).first->second;
         if (force || !small_allowed(c, jobs[j])) K.form = -1;
         small_include(K, jobs[j]);
@@ -847,8 +850,9 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     std::vector<int> order[kSmallForms + 1];              // jobs by kernel; 0: the persistent one
     size_t smem[kSmallForms + 1] = {};
     for (int j = 0; j < nj; j++) {
-        const SmallKernel& K = kernel_of[specs[j].mt];
-        const int f = std::max(K.form, 0);
+        SmallKernel K{specs[j].form, specs[j].form ? lz_small_smem(jobs[j].S) : 0};
+        if (specs[j].mode == LZ_COEFF) K = kernel_of[specs[j].mt];
+        const int f = specs[j].form = std::max(K.form, 0);
         order[f].push_back(j);
         smem[f] = std::max(smem[f], K.smem);
     }
@@ -1310,6 +1314,7 @@ void run_or_drop_kept(F f, D drop)
 
 struct SectorResult {
     int nstep = 0;
+    int form = 0;                    // JobSpec::form of the scan
     double norm0 = 0.0;
     double e = HUGE_VAL;
     std::vector<double> a, b, coeff;
@@ -1442,6 +1447,7 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
             const int i = which[q];
             SectorResult& r = res[i];
             r.nstep = specs[q].nstep;
+            r.form = specs[q].form;
             r.norm0 = specs[q].norm0;
             r.a.assign(hab + (size_t)(2 * i) * maxnstep, hab + (size_t)(2 * i + 1) * maxnstep);
             r.b.assign(hab + (size_t)(2 * i + 1) * maxnstep, hab + (size_t)(2 * i + 2) * maxnstep);
@@ -1495,7 +1501,8 @@ void ground_state_impl(edzt_ctx* c, int nsector, const int* sectors, int maxnste
                 ev[0].eig = eig.p;
                 ev[0].a = ab.p;
                 ev[0].b = ab.p + maxnstep;
-                if (keep) {                                   // the kept steps but the last, which the run begins with
+                ev[0].form = r.form;
+                if (keep && !r.form) {                        // the kept steps but the last, which the run begins with
                     VecSum vs = natural_sum(Si, kept[best].p, cw.p, keep - 1, eig.p);
                     vs.natural = 0;
                     c->launches += launch_vec_sum(&vs, 1, c->stream);
@@ -2069,6 +2076,7 @@ void solve_wave(edzt_ctx* c, std::vector<BatchInst>& B, int i0, int i1, int maxn
             j.eig = eigs[i - i0].p;
             j.a = specs[q].a;            // the coefficients of the scan, still on the device
             j.b = specs[q].b;
+            j.form = specs[q].form;
             ev.push_back(j);
         }
         CK(cudaMemcpyAsync(coeffs.p, hcoef.data(), sizeof(double) * hcoef.size(), cudaMemcpyHostToDevice, c->stream));
@@ -2333,6 +2341,7 @@ SmallKernel small_request(const edzt_server* sv, const ServReq& q)
     for (const auto& j : q.jobs) {
         LzJob J;
         fill_job(J, j->spec, j->S);
+        if (J.mode != LZ_COEFF) return SmallKernel{j->spec.form, j->spec.form ? lz_small_smem(J.S) : 0};
         if (!small_allowed(sv->c, J) || 0.004 * J.maxnstep > sv->step_ms) K.form = -1;
         small_include(K, J);
         if (K.form < 0) return SmallKernel{};
@@ -2377,6 +2386,7 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, const SmallKe
         L.k = std::max(L.k, k_now);
         if (fin) {
             L.done = true;
+            L.spec.form = small.form;
             L.spec.nstep = fin->nstep;
             L.spec.norm0 = fin->norm0;
         }
@@ -2519,6 +2529,7 @@ void read_scan(edzt_server* sv, ServReq& q)
         if (jq < 0) continue;
         SectorResult& r = q.res[s];
         r.nstep = q.jobs[jq]->spec.nstep;
+        r.form = q.jobs[jq]->spec.form;
         r.norm0 = q.jobs[jq]->spec.norm0;
         if (r.nstep < 1) continue;
         r.coeff.resize(r.nstep);
@@ -2561,6 +2572,7 @@ void start_eigvec(edzt_server* sv, ServReq& q)
     j.eig = q.eig.p;
     j.a = q.ab.p + (size_t)(2 * w) * maxnstep;
     j.b = q.ab.p + (size_t)(2 * w + 1) * maxnstep;
+    j.form = q.res[w].form;
     std::vector<OpsTable*> todo;
     std::unique_ptr<LiveJob> L = make_live(c, j, todo);
     build_ops(c, todo);

@@ -248,12 +248,12 @@ bool lz_shape_fits(const DevSector& S, const LzShape& q);
 // slots: [P.slots] partial sums; sync_words: lz_sync_bytes(njobs), zeroed.
 cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const LzJob* jobs, const long long* prefix,
                                       double* slots, unsigned* sync_words, int* status, cudaStream_t s);
-// Small coefficient runs from start to finish, one CTA each: the shared memory
-// that a run takes (0: it is not of that kind), its form of the kernel (the
+// Small runs from start to finish, one CTA each: the shared memory that a run
+// takes (0: it is not of that kind), its form of the kernel (the
 // forms sum in different orders: a model's runs all take the largest of
 // theirs), and a launch with the most shared memory that any of its runs takes.
 constexpr int kSmallForms = 4;
-size_t lz_small_smem(const DevSector& S, int mode);
+size_t lz_small_smem(const DevSector& S);
 int lz_small_form(const DevSector& S);
 cudaError_t launch_lanczos_small(const LzJob* jobs, int njobs, size_t smem, int form, cudaStream_t s);
 // Sync-word buffer size (bytes) for a launch of njobs runs.

@@ -58,7 +58,9 @@
 // stored a, b (src/lanczos_solver.f90:213-300) and accumulates
 // sum_k coeff_k w_k: all of it, or (LzJob::resume) from the last kept step on,
 // whose column phase stages the kept v_k, so every later vector has the bits
-// of the scan's.
+// of the scan's.  It runs in the kernel that the scan ran in (JobSpec::form):
+// in another one's summation order the fixed coefficients lose the vectors'
+// norm once they have converged.
 //
 // A launch may be a slice of longer runs (LzBatch::slice): when its phase
 // budget runs out, a closing pass opens every unfinished run's next step
@@ -821,6 +823,9 @@ __global__ void __launch_bounds__(T) k_lanczos_small(const LzJob* __restrict__ j
     auto row_of = [&](int e) { return nup > 1 ? (int)__umulhi((unsigned)e, magic) : e; };
     const long long vsize = lz_vec_size(nup, ndn);
     const int items = (ndn + R - 1) / R * nup;
+    // The eigenvector pass takes the scan's steps again, all of them in this
+    // form of the kernel: a, b and every vector have the scan's bits.
+    const bool coeff = J.mode == LZ_COEFF;
     double a = 0.0, bk = 1.0, rb = 1.0, bp = 1.0, rp = 0.0, norm0 = 0.0;   // a_{k-1}; b_k, b_{k-1} and their reciprocals
     int nstep = 0;
     for (int k = 1;; k++) {
@@ -859,12 +864,12 @@ __global__ void __launch_bounds__(T) k_lanczos_small(const LzJob* __restrict__ j
         rp = rb;
         if (k == 1) {                                    // ||v_init|| (:128-130); b(1) = 0 (:135)
             norm0 = nrm;
-            if (threadIdx.x == 0) J.b[0] = 0.0;
+            if (coeff && threadIdx.x == 0) J.b[0] = 0.0;
             if (!(nrm > 0.0)) break;                     // zero start vector
         } else if (nrm < 1.0e-16) {                      // breakdown (:161)
-            if (threadIdx.x == 0) J.b[k - 1] = 0.0;
+            if (coeff && threadIdx.x == 0) J.b[k - 1] = 0.0;
             break;
-        } else if (threadIdx.x == 0) {
+        } else if (coeff && threadIdx.x == 0) {
             J.b[k - 1] = nrm;                            // b(k) = ||v_k|| (:144,167)
         }
         bk = nrm;
@@ -921,11 +926,16 @@ __global__ void __launch_bounds__(T) k_lanczos_small(const LzJob* __restrict__ j
                 double z = div_by(s[r], bk, rb);
                 if (k > 1) z = fma(-bk, div_by(vp[id * nup + iu], bp, rp), z);
                 y[id * nup + iu] = z;
-                acc = fma(div_by(line[r][iu], bk, rb), z, acc);
+                const double w = div_by(line[r][iu], bk, rb);
+                acc = fma(w, z, acc);
+                if (!coeff) {                            // += coeff_k w_k, this thread's element in every step
+                    double* e = J.eig + lz_index(id, iu, ndp);
+                    __stcg(e, fma(__ldg(J.coeff + k - 1), w, k == 1 ? 0.0 : __ldcg(e)));
+                }
             }
         }
         a = cta_sum<T>(acc, red[1]);                        // a(k) = <w_k, y_k> (:134,159)
-        if (threadIdx.x == 0) J.a[k - 1] = a;
+        if (coeff && threadIdx.x == 0) J.a[k - 1] = a;
         nstep = k;
         if (k >= J.maxnstep) break;                      // :137-141, :161-164
         double* t = v;
@@ -946,9 +956,9 @@ __global__ void __launch_bounds__(T) k_lanczos_small(const LzJob* __restrict__ j
     }
 }
 
-size_t lz_small_smem(const DevSector& S, int mode)
+size_t lz_small_smem(const DevSector& S)
 {
-    if (mode != LZ_COEFF || S.dim > kLzSmallStates) return 0;
+    if (S.dim > kLzSmallStates) return 0;
     const size_t size = (size_t)lz_small_layout(S).size;
     return size <= kLzSmallSmemMax ? size : 0;
 }

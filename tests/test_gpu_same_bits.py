@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from conftest import random_model
+from test_gpu_keep import _states
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +37,57 @@ def test_small_models_do_not_see_their_company(pkg, solver, others):
         one = solver.solve(inst["sectors"], steps, omega, nspin=inst["nspin"], seed=inst["seed"])
         assert batch["e0"][i] == one["e0"] and np.array_equal(batch["G_cl"][i], one["G_cl"]), i
         assert served[i]["e0"] == one["e0"] and np.array_equal(served[i]["G_cl"], one["G_cl"]), i
+
+
+def _tolerance(steps):
+    """Both ways sum coeff_k w_k of the same w_k in the same order: a term
+    differs by at most two roundings and the sums add one a step, so an element
+    by (steps + 4) 2^-53 sum_k |coeff_k| |w_k|, where the sum over k is at most
+    2 (0.5 to 1.2 in a restatement of these runs).  The normalisation divides
+    it by the sum's norm, which is 1 until copies of converged states come in
+    and anything of order one then (0.02 to 1.4 there): 1e-4 is left for it,
+    and a factor of two for the norms' own difference."""
+    return (steps + 4) * 2.0**-53 * 2.0 * 2.0 / 1e-4
+
+
+@pytest.mark.parametrize("nsite,sector", [(6, (3, 3)), (7, (3, 4))])
+@pytest.mark.parametrize("steps", [80, 150, 300])
+def test_small_scan_run_again(pkg, solver, nsite, sector, steps):
+    """400 and 1,225 states far beyond convergence, where a second run in any
+    other arithmetic loses the vectors' norm."""
+    for seed in range(6):
+        solver.set_model(random_model(pkg, np.random.default_rng(500 + seed), 1, nsite - 1))
+        per_step = 8.0 * _states(pkg, nsite, [sector])
+        got = []
+        try:
+            for keep, limit in ((1, 0.0), (0, 0.0), (1, per_step * (steps // 2 + 4))):
+                solver.set_keep_vectors(keep)
+                solver.set_keep_limit_test(limit)
+                got.append(solver.ground_state([sector], steps, seed=seed))
+        finally:
+            solver.set_keep_vectors(1)
+            solver.set_keep_limit_test(0)
+        for r in got[1:]:
+            assert r["e0"] == got[0]["e0"]
+            assert np.abs(r["vec"] - got[0]["vec"]).max() <= _tolerance(steps), (seed, steps)
+
+
+def test_small_winner_of_a_larger_scan_run_again(pkg, solver):
+    """A scan with a sector for the persistent kernel takes all of the model's
+    runs there: the small winner's second run goes there too."""
+    for seed in range(3):
+        m = random_model(pkg, np.random.default_rng(700 + seed), 1, 7)
+        m.ek += 3.0                                      # few electrons: (1, 1) of 64 states or (2, 2) of 784
+        m.mu = 0.0
+        solver.set_model(m)
+        steps, sectors = 150, [(1, 1), (2, 2), (4, 4)]
+        got = []
+        try:
+            for keep in (1, 0):
+                solver.set_keep_vectors(keep)
+                got.append(solver.ground_state(sectors, steps, seed=seed))
+        finally:
+            solver.set_keep_vectors(1)
+        assert got[0]["sector"] != (4, 4)
+        assert got[0]["e0"] == got[1]["e0"]
+        assert np.abs(got[0]["vec"] - got[1]["vec"]).max() <= _tolerance(steps)
