@@ -549,7 +549,8 @@ __device__ __forceinline__ double row_tile(int r0, int np)
 }
 
 // Row phase of one row, for lines so long that two do not fit (13,400 up
-// strings or more: nsite 17 and beyond).
+// strings or more: nsite 17 and beyond).  It sums in row_tile's order: the
+// eigenvector pass of a shorter sector of the same scan runs there.
 template <bool X, int T>
 __device__ __forceinline__ double long_row(int r0)
 {
@@ -571,14 +572,15 @@ __device__ __forceinline__ double long_row(int r0)
         const unsigned o = lz_index(r0, iu, ndp);
         const int hc = __ldg(up.hcnt + iu), pu = __ldg(up.imp + iu);
         const double v = xs[iu];
-        double y = fma(__ldg(up.e1 + iu) + e1d + C.wint[pu * P + pd], v, __ldcg(C.J.Y + o));
+        double y = 0.0;
         for (int h = 0; h < hc; h++) {
             const uint32_t e = __ldg(reinterpret_cast<const uint32_t*>(up.hpk) + ((size_t)(h >> 2) * nup + iu) * 4 + (h & 3));
             y = fma(C.amp_up[edzt_hop_slot(e)], xs[edzt_hop_rank(e)], y);
         }
+        y = fma(__ldg(up.e1 + iu) + (e1d + C.wint[pu * P + pd]), v, y);
         if constexpr (X) { if (C.J.S.has_j) y = exchange_part(C.J.S, r0, iu, pu, pd, y, fetch); }
         const double w = div_by(v, bk, rb);
-        y = fma(-bk, k == 1 ? 0.0 : div_by(__ldcg(vp + o), bp, rp), div_by(y, bk, rb));
+        y = fma(-bk, k == 1 ? 0.0 : div_by(__ldcg(vp + o), bp, rp), div_by(y + __ldcg(C.J.Y + o), bk, rb));
         __stcg(C.J.Y + o, y);
         acc = fma(w, y, acc);
         if (C.J.mode != LZ_COEFF) {

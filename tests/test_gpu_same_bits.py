@@ -91,3 +91,23 @@ def test_small_winner_of_a_larger_scan_run_again(pkg, solver):
         assert got[0]["sector"] != (4, 4)
         assert got[0]["e0"] == got[1]["e0"]
         assert np.abs(got[0]["vec"] - got[1]["vec"]).max() <= _tolerance(steps)
+
+
+def test_short_winner_of_a_scan_with_long_lines_run_again(pkg, solver):
+    """Lines of 24,310 strings make the scan of every sector take rows one by
+    one; the second run of (2, 1), 2,312 states, takes tiles of rows."""
+    rng = np.random.default_rng(81)
+    for seed in range(3):
+        m = random_model(pkg, rng, 1, 16)
+        m.ek += 3.0                                      # every electron costs: the emptier sector wins
+        m.mu = 0.0
+        solver.set_model(m)
+        steps, got = 120, []
+        try:
+            for keep in (1, 0):
+                solver.set_keep_vectors(keep)
+                got.append(solver.ground_state([(8, 1), (2, 1)], steps, seed=seed))
+        finally:
+            solver.set_keep_vectors(1)
+        assert got[0]["sector"] == (2, 1) and got[0]["e0"] == got[1]["e0"]
+        assert np.abs(got[0]["vec"] - got[1]["vec"]).max() <= _tolerance(steps), seed
