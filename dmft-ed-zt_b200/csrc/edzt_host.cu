@@ -16,11 +16,11 @@
 #include <atomic>
 #include <algorithm>
 #include <deque>
-#include <thread>
 #include <tuple>
 #include <cuda_runtime.h>
 #include "../../include/edzt.h"
 #include "edzt_internal.h"
+#include "host_threads.h"
 #include "tridiag.h"
 
 namespace {
@@ -1250,24 +1250,6 @@ void diag_arpack_impl(edzt_ctx* c, const DevSector& S, uint64_t key, double* vec
         }
     }
     R.eigval = theta[0];
-}
-
-// f(0) ... f(n - 1) on the host's threads, a thread for every per_thread of them.
-template <class F>
-void parallel_for(int n, int per_thread, F&& f)
-{
-    const int nt = std::max(1, std::min(n / per_thread, (int)std::thread::hardware_concurrency()));
-    if (nt == 1) {
-        for (int i = 0; i < n; i++) f(i);
-        return;
-    }
-    std::atomic<int> next{0};
-    std::vector<std::thread> th;
-    for (int t = 0; t < nt; t++)
-        th.emplace_back([&] {
-            for (int i = next++; i < n; i = next++) f(i);
-        });
-    for (auto& x : th) x.join();
 }
 
 // How many of its maxnstep steps a scan over `states` states (as stored) may
