@@ -546,6 +546,7 @@ DevModel model_from(int norb, int nbath, const double* em, const double* ek, con
 
 void set_tables_model(edzt_ctx* c, ModelTables& mt, const DevModel& m)
 {
+    mt.valid = false;                                     // until the tables are this model's
     mt.ops.clear();
     mt.iops.clear();
     mt.hx.clear();

@@ -218,3 +218,23 @@ def test_string_tables_get_what_earlier_calls_left_cached(pkg):
         s.set_memory_limit_test(2048 * KB)               # the last ground state (500 KB) and the tables
         up, dn = s.generate_basis(8, 1)                  # rank tables of 2^16 strings, 256 KB each
         assert up.size == 12870 and dn.size == 16
+
+
+def test_model_that_was_not_set_is_not_used(pkg):
+    """Four orbitals' tables that do not fit: no model is set, not half of one."""
+    m = random_model(pkg, np.random.default_rng(4), 1, 5)
+    with pkg.Solver(0) as s:
+        s.set_model(m)
+        e0 = s.ground_state([(3, 3)], 20, seed=1)["e0"]
+    with pkg.Solver(0) as s:
+        s.set_model(m)
+        s.set_memory_limit_test(1)
+        with pytest.raises(pkg.EDError) as e:
+            s.set_model(random_model(pkg, np.random.default_rng(4), 4, 2, J=0.5))
+        assert e.value.code == pkg.EDZT_ERR_OOM
+        s.set_memory_limit_test(0)
+        with pytest.raises(pkg.EDError) as e:
+            s.hx(3, 3, np.ones(400))
+        assert e.value.code == pkg.EDZT_ERR_STATE
+        s.set_model(m)
+        assert s.ground_state([(3, 3)], 20, seed=1)["e0"] == e0
