@@ -2848,7 +2848,13 @@ int edzt_ctx_ready_sector(edzt_ctx* c, int nu, int nd, DevSector* S, const char*
                "first (edzt_hx or edzt_lanczos_iteration)";
         return EDZT_ERR_STATE;
     }
-    *S = make_sector_mt(c, c->mt, nu, nd, true);   // only looks the tables up
+    try {
+        *S = make_sector_mt(c, c->mt, nu, nd, true);   // only looks the tables up
+    } catch (const EdztError& e) {                     // a sector that the kernels do not take
+        c->err = e.msg;
+        *why = c->err.c_str();
+        return e.code;
+    }
     return EDZT_OK;
 }
 
