@@ -999,8 +999,8 @@ int plain_lanczos(edzt_ctx* c, const DevSector& S, const double* v_init, int max
             launch_axpy(eig, w.p, n, nullptr, coeff[k - 1], 1.0, c->stream);
             c->launches += 1;
         }
-        launch_hx(S, w.p, v.p, 1, c->stream);                            // :158
-        c->launches += 2;
+        launch_hx(S, w.p, v.p, 1, c->stream);                                  // :158
+        c->launches += 1;
         if (!coeff) a[k - 1] = plain_dot(c, w.p, v.p, n);                      // :159
         if (k >= maxnstep) { nstep = k; break; }                               // :161-164
         launch_axpy(v.p, w.p, n, nullptr, a[k - 1], -1.0, c->stream);          // :166
