@@ -52,7 +52,7 @@ EXPORTS = (
     "edzt_kernel_stats", "edzt_reset_stats", "edzt_kernel_launch_log", "edzt_lanczos_iteration_noalloc", "edzt_solve_batch",
     "edzt_cluster_green_matrix", "edzt_gs_occupancy", "edzt_green_real", "edzt_server_create", "edzt_server_submit", "edzt_server_step", "edzt_server_result", "edzt_server_destroy",
     "edzt_server_cancel", "edzt_server_set_step_ms", "edzt_tune_sector", "edzt_clear_tuning",
-    "edzt_instance_footprint", "edzt_set_fault_test", "edzt_set_keep_limit_test", "edzt_set_memory_limit_test", "edzt_diag_arpack",
+    "edzt_instance_footprint", "edzt_set_fault_test", "edzt_set_keep_limit_test", "edzt_set_memory_limit_test", "edzt_trim", "edzt_diag_arpack",
     "edzt_set_diag_solver", "edzt_set_keep_vectors", "edzt_hybridization", "edzt_local_green_bethe", "edzt_fit_bath", "edzt_dmft_bethe",
 )
 # ground_state's diag_solver values (src/ground_state.f90:53-60).
@@ -167,6 +167,7 @@ def load_library(path: str = LIB_PATH):
     L.edzt_version.restype = C.c_char_p
     L.edzt_set_model.argtypes = [_vp, C.c_int, C.c_int, _vp, _vp, _vp] + [C.c_double] * 5
     L.edzt_set_engine.argtypes = [_vp, C.c_int]
+    L.edzt_trim.argtypes = [_vp]
     L.edzt_basis.argtypes = [_vp, C.c_int, C.c_int, _ip, _ip, _vp, _vp]
     L.edzt_basis_rank.argtypes = [_vp, C.c_int, _vp]
     L.edzt_sector_dim.argtypes = [_vp, C.c_int, C.c_int]
@@ -349,6 +350,11 @@ class Solver:
 
     def set_engine(self, engine: int):
         self._check(self._L.edzt_set_engine(self._h, int(engine)))
+
+    def trim(self):
+        """Give the device memory that the context holds cached between calls
+        back (edzt_trim); the model and the resident ground state stay."""
+        self._check(self._L.edzt_trim(self._h))
 
     def launch_count(self) -> int:
         return int(self._L.edzt_launch_count(self._h))

@@ -2990,6 +2990,14 @@ int edzt_set_model(edzt_ctx* c, int norb, int nbath, const double* em, const dou
     });
 }
 
+int edzt_trim(edzt_ctx* c)
+{
+    return guarded(c, [&] {
+        CK(cudaStreamSynchronize(c->stream));
+        c->pool.trim();
+    });
+}
+
 long long edzt_sector_dim(edzt_ctx* c, int ne_up, int ne_dn)
 {
     if (!c || !c->mt.valid) return 0;

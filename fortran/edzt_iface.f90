@@ -84,6 +84,10 @@ module edzt_iface
       type(c_ptr), value :: ctx
       integer(c_int), value :: diag_solver                    ! 1 Lanczos, 2 ARPACK
     end function
+    integer(c_int) function edzt_trim(ctx) bind(C, name="edzt_trim")
+      import :: c_int, c_ptr
+      type(c_ptr), value :: ctx
+    end function
     integer(c_int) function edzt_set_keep_vectors(ctx, keep) bind(C, name="edzt_set_keep_vectors")
       import :: c_int, c_ptr
       type(c_ptr), value :: ctx

@@ -68,6 +68,15 @@ const char *edzt_version(void);
 int edzt_set_model(edzt_ctx *ctx, int norb, int nbath, const double *em, const double *ek,
                    const double *vmk, double U, double Up, double Jex, double Jp, double mu);
 
+/* Device memory between calls.  A context keeps the blocks of a call for the
+ * next one: what edzt_ground_state and edzt_solve worked with, kept Lanczos
+ * vectors among it (up to half of the memory free at its creation, see
+ * edzt_set_keep_vectors), and after a batch 2 GiB or a sixteenth of that
+ * memory, whichever is more.  Its own allocations take those blocks back
+ * before they fail.  edzt_trim gives them to the device, for others to use; the
+ * model, the tables and the resident ground state stay. */
+int edzt_trim(edzt_ctx *ctx);
+
 /* Selects the Lanczos engine (EDZT_ENGINE_*). */
 int edzt_set_engine(edzt_ctx *ctx, int engine);
 
