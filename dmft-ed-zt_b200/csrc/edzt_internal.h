@@ -1,11 +1,11 @@
 // edzt_internal.h — host-side declarations shared by the CUDA translation
 // units of libedzt (not part of the public C ABI; see include/edzt.h).
 #pragma once
-#include <atomic>
 #include <cstdint>
 #include <vector>
 #include <cuda_runtime.h>
 #include "edzt_device.cuh"
+#include "host_threads.h"
 
 // Impurity model as the kernels see it.  Shapes follow the reference's
 // Fortran arrays em(norb,2), ek(nbath,2), vmk(norb,nbath,2)
@@ -18,15 +18,15 @@ struct DevModel {
     double U, Up, Jex, Jp, mu;
 };
 
-// True the first time it is called for the current device with this set of
-// flags: per-device one-time set-up such as a kernel's shared-memory
-// attribute, which cudaFuncSetAttribute sets for the current device only.
-inline bool edzt_once_per_device(std::atomic<unsigned long long>& done)
+// Set-up of the current device such as a kernel's shared-memory attribute, which
+// cudaFuncSetAttribute sets for that device only: f() the first time, done
+// before any thread's call returns.
+template <class F>
+inline void edzt_once_per_device(OnceEach& done, F&& f)
 {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return true;
-    const unsigned long long bit = 1ull << dev;
-    return (done.fetch_or(bit) & bit) == 0;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+    done.run(dev, f);
 }
 
 // ---- tables.cu -------------------------------------------------------------

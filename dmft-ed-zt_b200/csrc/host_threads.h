@@ -1,4 +1,4 @@
-// host_threads.h — a parallel loop on the host's threads.
+// host_threads.h — a parallel loop on the host's threads; set-up done once per device.
 #pragma once
 #include <algorithm>
 #include <atomic>
@@ -36,3 +36,19 @@ void parallel_for(int n, int per_thread, F&& f)
     for (auto& t : others) t.join();
     if (failed) std::rethrow_exception(failed);
 }
+
+// f() once for each index (a device): a caller that finds it begun by another
+// thread waits until it is done.
+class OnceEach {
+  public:
+    template <class F>
+    void run(int i, F&& f)
+    {
+        if (i < 0 || i >= kMost) f();
+        else std::call_once(once_[i], f);
+    }
+
+  private:
+    static constexpr int kMost = 64;
+    std::once_flag once_[kMost];
+};

@@ -82,11 +82,11 @@ static size_t hx_tile_smem(const DevSector& S, int R, int PL)
 template <int R, int PL, int T, int NB>
 static void launch_hx_tile(const DevSector& S, const double* x, double* y, int accumulate, int grid, cudaStream_t s)
 {
-    static std::atomic<unsigned long long> attr_set{0};
-    if (edzt_once_per_device(attr_set)) {
+    static OnceEach attr_set;
+    edzt_once_per_device(attr_set, [] {
         cudaFuncSetAttribute(k_hx_tile<false, R, PL, T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax);
         cudaFuncSetAttribute(k_hx_tile<true, R, PL, T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax);
-    }
+    });
     const size_t sm = hx_tile_smem(S, R, PL);
     if (accumulate) k_hx_tile<true, R, PL, T, NB><<<grid, T, sm, s>>>(S, x, y);
     else k_hx_tile<false, R, PL, T, NB><<<grid, T, sm, s>>>(S, x, y);

@@ -975,14 +975,11 @@ cudaError_t launch_lanczos_small(const LzJob* jobs, int nj, size_t smem, int for
     using Kernel = void (*)(const LzJob*);
     static const Kernel kernels[kSmallForms] = {k_lanczos_small<512, 1, false>, k_lanczos_small<768, 4, false>,
                                                 k_lanczos_small<512, 1, true>, k_lanczos_small<768, 4, true>};
-    static std::atomic<unsigned long long> done{0};
-    if (edzt_once_per_device(done)) {
-        for (const Kernel k : kernels) {
-            const cudaError_t e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)kLzSmallSmemMax);
-            if (e != cudaSuccess) return e;
-        }
-    }
+    static OnceEach done;
+    edzt_once_per_device(done, [&] {                      // where it fails the launch does
+        for (const Kernel k : kernels)
+            cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLzSmallSmemMax);
+    });
     kernels[form - 1]<<<nj, form % 2 ? 512 : 768, smem, s>>>(jobs);
     return cudaGetLastError();
 }

@@ -1,5 +1,7 @@
-// parallel_for (dmft-ed-zt_b200/csrc/host_threads.h) where no thread can be
-// had and where the function throws.  Prints "ok" and returns 0.
+// dmft-ed-zt_b200/csrc/host_threads.h: set-up done once, before any thread goes
+// on; parallel_for where no thread can be had and where the function throws.
+// Prints "ok" and returns 0.
+#include <chrono>
 #include <cstdio>
 #include <stdexcept>
 #include <vector>
@@ -18,8 +20,28 @@ static int run(int n)
     return bad;
 }
 
+// Threads that meet at one index's set-up and see it done.
+static int once(int threads)
+{
+    OnceEach each;
+    std::atomic<int> begun{0}, done{0}, early{0};
+    std::vector<std::thread> th;
+    for (int t = 0; t < threads; t++)
+        th.emplace_back([&] {
+            each.run(3, [&] {
+                begun++;
+                std::this_thread::sleep_for(std::chrono::milliseconds(50));
+                done++;
+            });
+            early += done == 0;
+        });
+    for (auto& t : th) t.join();
+    return begun != 1 || done != 1 || early != 0;
+}
+
 int main()
 {
+    if (once(8)) { std::printf("once\n"); return 5; }
     for (int n : {0, 1, 2, 7, 1000})
         if (run(n)) { std::printf("n %d\n", n); return 1; }
     int caught = 0;
