@@ -714,7 +714,7 @@ def run_gpu(args):
 def run_case(spec, steps):
     """Small single-kernel workloads for ncu captures and kernel A/B timing,
     on the half-filled sector of the hv leg's single-orbital model at nsite NS:
-      hx:NS   four y = H x calls (k_hx); the last one is timed
+      hx:NS   four y = H x calls (k_hx_tile); the last one is timed
       lz:NS   lanczos_iteration of 5, then of `steps` steps (k_lanczos); the
               second launch is timed
       solve   one impurity solve of the bench workload (nsite 12, 9 sectors)

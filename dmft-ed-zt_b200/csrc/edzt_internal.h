@@ -207,7 +207,6 @@ __host__ __device__ constexpr int lz_keep_slots(int keep, int maxnstep) { return
 
 struct LzBatch {
     int njobs;
-    int grid;                     // set by the launch
     size_t fixed;                 // shared memory before the staged tile; set by the launch
     int max_phases;               // phase budget of the launch (even for a slice)
     unsigned long long wait_ns;   // wait limit of a job's arrivals (0: the default 5 s)

@@ -66,9 +66,6 @@ __device__ __forceinline__ HopList hop_list(const DevSpin& sp, int t)
     return L;
 }
 
-// Values per line of one plane for tiles of W lines across.
-__host__ __device__ constexpr int plane_width(int W) { return W >= 4 ? 4 : 2; }
-
 // acc[p] += a * (two values at l of plane p), planes ps doubles apart.
 template <int NP>
 __device__ __forceinline__ void plane_axpy(double a, const double* __restrict__ l, int ps, double2 (&acc)[NP])

@@ -29,16 +29,19 @@
 // What bounds it: the load/store pipe (hop values from shared memory, 2 x 8
 // bytes a hop and state, 1.1-1.2 times the conflict-free wavefronts) and the
 // latency of staging and of the arrivals, then DRAM (64 bytes a state and
-// step once the vectors exceed L2).  Registers decide the rest: with 128 of
-// them nothing spills; 80 for half as many threads again spilled and lost a
-// sixth, tile functions called instead of inlined a third.  Measured per step
-// against slabs of the reference's string order staged as (y, w) pairs under
-// grid-wide barriers: 9 sectors of nsite 12 146 -> 124 us, 4 sectors of nsite
-// 13 280 -> 196 us, one sector of nsite 14 279 -> 212 us, of nsite 15
-// 1,092 -> 930 us, of nsite 8 13.6 -> 9.4 us.  With the hop lists of the row
-// phase loaded ahead, a CTA serving one run where that comes out even (lz_cut)
-// and no look-up of its range left in a phase: 100, 185, 202, 809 and 8.9 us,
-// 9 sectors of nsite 10 30 -> 15.
+// step once the vectors exceed L2).  Registers decide the rest: all 128 of a
+// thread are in use, and the tiles of eight lines and more spill a little (8 x
+// 8 columns by rows, 512 threads: 116 bytes stored and 148 loaded, 136 and 252
+// with exchange terms; 256 threads 20 and 20, 96 and 136; smaller tiles 0 to
+// 30, but 76 and 124 for 8 x 4 with exchange terms); 80 registers for half as
+// many threads again lost a sixth, tile functions called instead of inlined a
+// third.  Measured per step against slabs of the reference's string order
+// staged as (y, w) pairs under grid-wide barriers: 9 sectors of nsite 12
+// 146 -> 124 us, 4 sectors of nsite 13 280 -> 196 us, one sector of nsite 14
+// 279 -> 212 us, of nsite 15 1,092 -> 930 us, of nsite 8 13.6 -> 9.4 us.  With
+// the hop lists of the row phase loaded ahead, a CTA serving one run where that
+// comes out even (lz_cut) and no look-up of its range left in a phase: 100, 185,
+// 202, 809 and 8.9 us, 9 sectors of nsite 10 30 -> 15.
 //
 // The tiles of all jobs of a phase form one list, cut into one contiguous
 // range per CTA at equal modelled cost (lz_plan); within a job the column
@@ -716,7 +719,6 @@ cudaError_t launch_lanczos_persistent(const LzPlan& P, const LzBatch& B, const L
                                       double* slots, unsigned* sync_words, int* status, cudaStream_t s)
 {
     LzBatch b = B;
-    b.grid = P.grid;
     b.fixed = P.fixed;
     void* args[] = {(void*)&b, (void*)&jobs, (void*)&prefix, (void*)&slots, (void*)&sync_words, (void*)&status};
     return cudaLaunchCooperativeKernel((const void*)lz_kernel(P), dim3(P.grid), dim3(P.block), args,
@@ -987,8 +989,7 @@ cudaError_t launch_lanczos_small(const LzJob* jobs, int nj, size_t smem, int for
 // ---------------------------------------------------------------------------
 // launch plan
 // ---------------------------------------------------------------------------
-// Per-CTA dynamic shared memory: two 512-thread CTAs per SM when every job
-// fits, else one.
+// Most dynamic shared memory of a CTA of 256 threads, two of which share an SM.
 static constexpr size_t kLzSmemTwoPerSm = 113 * 1024;
 // Fixed cost of a tile in states, for cutting the tile list into CTA ranges
 static constexpr double kLzTileCost = 256.0;

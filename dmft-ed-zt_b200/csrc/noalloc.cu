@@ -152,7 +152,9 @@ void run(edzt_ctx* c, int ne_up, int ne_dn, const double* v_init, int maxnstep, 
     J.mode = LZ_COEFF;
     J.init = LZ_INIT_COPY;
     J.st = d_state;
-    // the same tile shapes, grid and shared memory as the allocating path
+    // the persistent kernel's plan, also for sectors of at most 2,000 states, whose
+    // runs take the kernel of small ones on the allocating path (and there differ
+    // from these in the last bits)
     std::vector<long long> prefix;
     const LzPlan P = lz_plan(device, &J, 1, prefix);
     if (P.grid <= 0) throw Fail{EDZT_ERR_CUDA, "persistent kernel cannot be resident (shared memory too large)"};
@@ -191,7 +193,7 @@ void run(edzt_ctx* c, int ne_up, int ne_dn, const double* v_init, int maxnstep, 
     NA_CK(cudaMemcpyAsync(b, d_b, sizeof(double) * maxnstep, cudaMemcpyDefault, st));
     NA_CK(cudaStreamSynchronize(st));
     if (status == EDZT_DEV_BARRIER_TIMEOUT)
-        throw Fail{EDZT_ERR_TIMEOUT, "persistent Lanczos kernel: grid barrier wait timed out"};
+        throw Fail{EDZT_ERR_TIMEOUT, "persistent Lanczos kernel: the wait for a run's arrivals timed out"};
     if (status != 0) throw Fail{EDZT_ERR_CUDA, "persistent Lanczos kernel reported status " + std::to_string(status)};
     const LzState* fin = !hs[0].active ? &hs[0] : (!hs[1].active ? &hs[1] : nullptr);
     if (!fin) throw Fail{EDZT_ERR_NUMERIC, "Lanczos run did not finish within the pass limit"};

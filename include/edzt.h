@@ -171,7 +171,8 @@ int edzt_set_diag_solver(edzt_ctx *ctx, int diag_solver);
  * run again), in at most half of the device memory free at context creation.
  * The batched form keeps what fits in a 32nd of it (and in hbm_budget beside
  * the instances), a server in a 32nd of it and an eighth of its budget.
- * Where the memory is not to be had, the recurrence is run again. */
+ * Where the memory is not to be had, the recurrence is run again: kept
+ * vectors never make a call fail. */
 int edzt_set_keep_vectors(edzt_ctx *ctx, int keep);
 
 /* ground_state (src/ground_state.f90:1-81): scans sectors[nsector][2] =
@@ -180,13 +181,11 @@ int edzt_set_keep_vectors(edzt_ctx *ctx, int keep);
  * on the device for edzt_cluster_green_ftn.  Sector i starts Lanczos from
  * stream i of `seed`.  gsvec (nullable, host or device) receives the vector
  * (gs%vec, src/eigpair.f90:5-9); e_sector (nullable) [nsector] the per-sector
- * lowest energies.  Device memory: when (maxnstep + 1) * 16 bytes per state
- * of all sectors fit in half of the device memory that was free when the
- * context was created, the scan keeps every
- * step's Lanczos vectors and the ground-state vector is their sum (one pass);
- * otherwise the winner's recurrence is run again, as the reference's
- * lanczos_ground_state does.  Both form the same sum; the rerun sums
- * ||v_init|| again, so the two agree to rounding. */
+ * lowest energies.  Device memory: the scan keeps its Lanczos vectors, 8 bytes
+ * per state and step, as edzt_set_keep_vectors tells, and the ground-state
+ * vector is their sum (one pass); steps that were not kept are run again, as
+ * the reference's lanczos_ground_state does, in the scan's arithmetic.  Both
+ * form the same sum of the same vectors, in the same order, to rounding. */
 int edzt_ground_state(edzt_ctx *ctx, int nsector, const int *sectors, int maxnstep, uint64_t seed,
                       int *isector, double *e0, double *gsvec, double *e_sector);
 
@@ -252,8 +251,10 @@ typedef struct edzt_instance {
  * src/dmft.f90:76-78) for ninst independent instances of uneven Fock
  * dimension: the sector scans of all instances run in one persistent launch,
  * then all eigenvector passes, then all c / c^+ runs, in waves whose device
- * memory stays within hbm_budget bytes (0: 80% of the free memory).  Each
- * instance's results are those of edzt_solve on it alone, to rounding.
+ * memory stays within hbm_budget bytes (0: a batch of up to 2 GiB is tried in
+ * one wave, others, and that one where it does not fit, take 80% of the free
+ * memory).  Each instance's results are those of edzt_solve on it alone, to
+ * rounding.
  * isector, e0: [ninst] (nullable); G_cl (nullable, host or device): the
  * instances' G_cl(nw, norb, nspin) complex arrays, concatenated in order. */
 int edzt_solve_batch(edzt_ctx *ctx, int ninst, const edzt_instance *inst, int maxnstep, int nw,
@@ -261,9 +262,12 @@ int edzt_solve_batch(edzt_ctx *ctx, int ninst, const edzt_instance *inst, int ma
 
 /* Served form: continuous batching of impurity solves on one context.
  * Requests (edzt_instance, copied at submit) wait in a queue and are
- * admitted by their device-memory footprint (the sector scan's 40 B per
+ * admitted by their device-memory footprint (the sector scan's 24 B per
  * state, or the Green's runs') while the admitted ones fit hbm_budget (0: 80%
  * of the free memory; a request is always admitted when nothing else runs).
+ * Where device memory runs out all the same, requests wait for others to give
+ * some back, ahead of that for kept vectors; a step returns EDZT_ERR_OOM when
+ * nothing can get on, and a later one goes on from there.
  * A request goes through three phases -- sector scan, eigenvector pass, c / c^+
  * runs plus continued fractions -- whose Lanczos runs live on the device
  * across launches.  Requests fall in size classes (by nsite; up to nsite 11
