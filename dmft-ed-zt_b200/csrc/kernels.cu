@@ -103,7 +103,12 @@ bool hx_fits(int nup, int ndn)
 // with 4 / 2 / 1 rows 48.6 / 50.4 / 50.3, nsite 14 166 / 162 / 174, nsite 15
 // 859 / 610 / 594).  Threads: 512, two CTAs per SM; four rows of 1,500 strings
 // or more run 256 threads three times (80 registers: 48.6 against 53.1), rows
-// of 8,000 or more 1,024 (2,677 against 2,732).
+// of 8,000 or more 1,024 (2,677 against 2,732).  Rows of up to 200 strings take
+// 128 threads, of up to 32 a warp, for as many CTAs as an SM holds: 512 threads
+// are then mostly idle, and many rows come in many waves (us a call, 512 threads
+// and now: (2,8) of nsite 16 67 and 36, (2,6) of nsite 17 71 and 45, (1,8) of
+// nsite 16 64 and 22, (0,8) 53 and 20; with 220 strings, (3,6) of nsite 12, 128
+// threads take 21.7 where 512 take 20.2).
 void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, cudaStream_t s)
 {
     const int nup = S.up.count, ndn = S.dn.count;
@@ -114,7 +119,9 @@ void launch_hx(const DevSector& S, const double* x, double* y, int accumulate, c
     int R = std::min(nup >= 8000 ? 1 : nup >= 3000 ? 2 : 4, std::max(1, ndn / nsm));
     if (R == 3) R = 2;
     const int grid = (ndn + R - 1) / R;
-    if (R == 4 && nup >= 1500) launch_hx_tile<4, 2, 256, 3>(S, x, y, accumulate, grid, s);
+    if (R == 4 && nup <= 32) launch_hx_tile<4, 2, 32, 32>(S, x, y, accumulate, grid, s);
+    else if (R == 4 && nup <= 200) launch_hx_tile<4, 2, 128, 8>(S, x, y, accumulate, grid, s);
+    else if (R == 4 && nup >= 1500) launch_hx_tile<4, 2, 256, 3>(S, x, y, accumulate, grid, s);
     else if (R == 4) launch_hx_tile<4, 2, 512, 2>(S, x, y, accumulate, grid, s);
     else if (R == 2) launch_hx_tile<2, 2, 512, 2>(S, x, y, accumulate, grid, s);
     else if (nup >= 8000) launch_hx_tile<1, 1, 1024, 1>(S, x, y, accumulate, grid, s);
