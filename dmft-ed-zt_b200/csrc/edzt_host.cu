@@ -938,7 +938,9 @@ edzt_ctx::Tuned tune_sector(edzt_ctx* c, int nu, int nd, int steps)
     edzt_ctx::Tuned best{{0, 0, 0}, HUGE_VAL};
     run({2, 1, 512});                                     // warm-up
     for (const LzShape q : {LzShape{16, 8, 256}, LzShape{16, 8, 512}, LzShape{8, 8, 256}, LzShape{8, 8, 512}, LzShape{8, 4, 256},
-                            LzShape{8, 4, 512}, LzShape{4, 4, 256}, LzShape{4, 4, 512}, LzShape{2, 2, 256}, LzShape{2, 2, 512}, LzShape{2, 1, 512}}) {
+                            LzShape{8, 4, 512}, LzShape{8, 2, 512}, LzShape{8, 1, 512}, LzShape{4, 8, 512}, LzShape{4, 4, 256},
+                            LzShape{4, 4, 512}, LzShape{4, 2, 512}, LzShape{4, 1, 512}, LzShape{2, 8, 512}, LzShape{2, 4, 512},
+                            LzShape{2, 2, 256}, LzShape{2, 2, 512}, LzShape{2, 1, 512}}) {
         if (!lz_shape_fits(S, q)) continue;
         const double ms = run(q);
         if (ms < best.ms_per_step) best = {q, ms};

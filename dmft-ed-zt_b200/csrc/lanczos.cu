@@ -30,12 +30,11 @@
 // bytes a hop and state, 1.1-1.2 times the conflict-free wavefronts) and the
 // latency of staging and of the arrivals, then DRAM (64 bytes a state and
 // step once the vectors exceed L2).  Registers decide the rest: all 128 of a
-// thread are in use, and the tiles of eight lines and more spill a little (8 x
-// 8 columns by rows, 512 threads: 116 bytes stored and 148 loaded, 136 and 252
-// with exchange terms; 256 threads 20 and 20, 96 and 136; smaller tiles 0 to
-// 30, but 76 and 124 for 8 x 4 with exchange terms); 80 registers for half as
-// many threads again lost a sixth, tile functions called instead of inlined a
-// third.  Measured per step against slabs of the reference's string order
+// thread are in use, and the largest tiles spill a little (8 x 8 columns by
+// rows, 512 threads: 116 bytes stored and 148 loaded; 256 threads 20 and 20; with
+// exchange terms 76 to 152 and 124 to 252 for tiles of eight columns or rows;
+// others 0 to 28); 80 registers for half as many threads again lost a sixth, tile
+// functions called instead of inlined a third.  Measured per step against slabs of the reference's string order
 // staged as (y, w) pairs under grid-wide barriers: 9 sectors of nsite 12
 // 146 -> 124 us, 4 sectors of nsite 13 280 -> 196 us, one sector of nsite 14
 // 279 -> 212 us, of nsite 15 1,092 -> 930 us, of nsite 8 13.6 -> 9.4 us.  With
@@ -684,23 +683,33 @@ int lz_debug_bad(long long* out4)
 
 using LzKernel = void (*)(LzBatch, const LzJob*, const long long*, double*, unsigned*, int*);
 
-// The kernel of a tile shape: wc columns by r rows.
+// The kernel of a tile shape: wc columns by r rows (two CTAs of half the
+// threads only of shapes that have a use for them).
 static LzKernel lz_kernel(const LzPlan& P)
 {
 #define EDZT_LZ(c, w, nc, nr, pw, pr)                                                                    \
-    if (P.wc == c && P.r == w) {                                                                         \
-        if (P.block == kLzThreads)                                                                       \
-            return P.exchange ? k_lanczos<nc, nr, pw, pr, true, kLzThreads>                              \
-                              : k_lanczos<nc, nr, pw, pr, false, kLzThreads>;                            \
+    if (P.wc == c && P.r == w && P.block == kLzThreads)                                                  \
+        return P.exchange ? k_lanczos<nc, nr, pw, pr, true, kLzThreads>                                  \
+                          : k_lanczos<nc, nr, pw, pr, false, kLzThreads>;
+#define EDZT_LZ2(c, w, nc, nr, pw, pr)                                                                   \
+    EDZT_LZ(c, w, nc, nr, pw, pr)                                                                        \
+    if (P.wc == c && P.r == w && P.block == kLzThreads / 2)                                              \
         return P.exchange ? k_lanczos<nc, nr, pw, pr, true, kLzThreads / 2>                              \
-                          : k_lanczos<nc, nr, pw, pr, false, kLzThreads / 2>;                            \
-    }
-    EDZT_LZ(16, 8, 4, 2, 4, 4)
-    EDZT_LZ(8, 8, 2, 2, 4, 4)
-    EDZT_LZ(8, 4, 2, 1, 4, 4)
-    EDZT_LZ(4, 4, 1, 1, 4, 4)
-    EDZT_LZ(2, 2, 1, 1, 2, 2)
-    EDZT_LZ(2, 1, 1, 1, 2, 1)
+                          : k_lanczos<nc, nr, pw, pr, false, kLzThreads / 2>;
+    EDZT_LZ2(16, 8, 4, 2, 4, 4)
+    EDZT_LZ2(8, 8, 2, 2, 4, 4)
+    EDZT_LZ2(8, 4, 2, 1, 4, 4)
+    EDZT_LZ(8, 2, 2, 1, 4, 2)
+    EDZT_LZ(8, 1, 2, 1, 4, 1)
+    EDZT_LZ(4, 8, 1, 2, 4, 4)
+    EDZT_LZ2(4, 4, 1, 1, 4, 4)
+    EDZT_LZ(4, 2, 1, 1, 4, 2)
+    EDZT_LZ(4, 1, 1, 1, 4, 1)
+    EDZT_LZ(2, 8, 1, 2, 2, 4)
+    EDZT_LZ(2, 4, 1, 1, 2, 4)
+    EDZT_LZ2(2, 2, 1, 1, 2, 2)
+    EDZT_LZ2(2, 1, 1, 1, 2, 1)
+#undef EDZT_LZ2
 #undef EDZT_LZ
     return nullptr;
 }
@@ -997,6 +1006,8 @@ static constexpr double kLzTileCost = 256.0;
 // this much work in states, or an uneven share of the whole
 static constexpr double kLzSwitchCost = 2000.0;
 static constexpr double kLzUneven = 1.15;
+// Lines of which a few are taken two at a time
+static constexpr int kLzLongLine = 500;
 // Time of a tile with two CTAs on the SM over its time with one
 static constexpr double kLzPairSlowdown = 1.75;
 
@@ -1024,9 +1035,13 @@ static double lz_load(const LzJob* jobs, int nj, int G, const std::vector<long l
 LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, const LzShape* force)
 {
     LzPlan P;
-    int tables = 0, lines_up = 0, lines_dn = 0;
+    int tables = 0, lines_up = 0, lines_dn = 0, nsm = 0;
+    long long columns = 0, rows = 0;                     // in groups of four
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
     for (int j = 0; j < nj; j++) {
         const DevSector& S = jobs[j].S;
+        columns += (S.up.count + 3) / 4;
+        rows += (S.dn.count + 3) / 4;
         lines_up = std::max(lines_up, S.up.count);
         lines_dn = std::max(lines_dn, S.dn.count);
         tables = std::max(tables, table_doubles(S.P, std::max(S.up.namp, S.dn.namp)));
@@ -1060,18 +1075,30 @@ LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, 
         return F;
     }
     // The widest tiles that fit one CTA per SM: a hop is decoded once for the
-    // lines of a tile (nsite 14: eight lines 202 us a step, four 250).  Tiles
-    // of eight lines may also run two CTAs per SM, which overlap one's staging
+    // lines of a tile (nsite 14: eight lines 202 us a step, four 250).  Columns
+    // and rows each by the length of their own lines: rows of 12,870 strings
+    // leave tiles of two, but columns of 16 strings are best taken eight at a
+    // time (us a step, 2 x 2 and 8 x 2: (8,1) of nsite 16 111 and 68, (8,2) 120
+    // and 76; 2 x 2 and 2 x 8: (0,8) 101 and 60, (2,6) of nsite 17 113 and 70).
+    // Where fours of long rows, or columns, occupy half of the SMs at most, they
+    // are taken two at a time, by twice as many CTAs (8 x 8 and 8 x 2: (7,1) of
+    // nsite 14 36 and 27, (7,2) 36 and 28, (6,3) of nsite 12 20.1 and 17.5; 2 x 8:
+    // (2,7) of nsite 14 35 and 26); lines of 252 strings gain nothing from it.
+    // Tiles of eight lines may also run two CTAs per SM, which overlap one's staging
     // with the other's hop sums but halve what a CTA gets through: taken when
     // the busiest CTA's load, in passes over a tile, times kLzPairSlowdown is
     // less than one CTA per SM has (us a step, one / two CTAs: 9 sectors of
     // nsite 12 106 / 99, of nsite 10 18.2 / 15.5; one sector of nsite 12
     // 23 / 31; 2 sectors of nsite 13 92 / 110).
-    if (!shape(P, 8, 8, kLzThreads) && !shape(P, 4, 4, kLzThreads) && !shape(P, 2, 2, kLzThreads))
-        shape(P, 2, 1, kLzThreads);
+    int wc = 8, r = 8;
+    while (wc > 2 && P.fixed + lz_col_smem(lines_dn, wc) > kLzSmemMax) wc /= 2;
+    while (r > 1 && P.fixed + lz_row_smem(lines_up, r) > kLzSmemMax) r /= 2;
+    if (lines_dn >= kLzLongLine && 2 * columns <= nsm) wc = std::min(wc, 2);
+    if (lines_up >= kLzLongLine && 2 * rows <= nsm) r = std::min(r, 2);
+    shape(P, wc, r, kLzThreads);
     cut(P, prefix);
     LzPlan Q = P;
-    if (P.wc == 8 && shape(Q, 8, 8, kLzThreads / 2)) {
+    if (P.wc == 8 && P.r == 8 && shape(Q, 8, 8, kLzThreads / 2)) {
         const double one = lz_load(jobs, nj, P.grid, prefix);
         std::vector<long long> pre;
         cut(Q, pre);

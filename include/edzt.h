@@ -313,10 +313,9 @@ int edzt_instance_footprint(const edzt_instance *inst, long long *bytes);
  * reference): times short Lanczos runs (`steps` steps, 2..1000) of the
  * context's model on sector (ne_up, ne_dn) for every tile shape of the
  * persistent kernel that fits -- columns per tile of the column phase (the
- * stripe width) by rows per tile of the row phase, 16 x 8, 8 x 8, 8 x 4,
- * 4 x 4, 2 x 2 or 2 x 1, one CTA of 512 or two of 256 threads per SM -- and
- * records the fastest
- * on the context for that sector shape; later launches on the context use it
+ * stripe width) by rows per tile of the row phase, 16 x 8 and 8, 4 or 2 by 8,
+ * 4, 2 or 1, one CTA of 512 or (some) two of 256 threads per SM -- and records
+ * the fastest on the context for that sector shape; later launches on the context use it
  * for every run of that shape (results unchanged but for rounding).
  * Outputs (nullable): the chosen shape and its time per Lanczos step.
  * edzt_clear_tuning forgets every recorded shape. */
