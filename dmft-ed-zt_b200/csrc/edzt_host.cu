@@ -265,6 +265,9 @@ struct edzt_ctx {
     size_t stage_bytes = 0;
     // persistent-kernel statistics
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // a second stream for launches side by side (made when first needed)
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_done = nullptr;
     long long st_launches = 0;
     double st_ms = 0.0, st_bytes = 0.0;
     // small host-visible scratch for the plain engine
@@ -664,12 +667,6 @@ void log_launch(edzt_ctx* c, double ms, double bytes, double states)
     c->log_states.push_back(states);
 }
 
-// A form of the kernel of small runs (0: none) and the shared memory of its runs.
-struct SmallKernel {
-    int form = 0;
-    size_t smem = 0;
-};
-
 // The run's descriptor but for its vectors and state.
 void fill_job(LzJob& J, const JobSpec& s, const DevSector& S)
 {
@@ -760,23 +757,58 @@ float launch_jobs(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& s
     return ms;
 }
 
-// The same with a form of the kernel of small runs, which need no plan.
-float launch_small(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& st, const SmallKernel& K)
+// The same with the kernel of small runs, which need no plan: form[j] is that of
+// jobs[j].  Each form is a launch; two go side by side, on the context's stream
+// and one that starts and ends with it.  Returns the device time in ms.
+float launch_small(edzt_ctx* c, std::vector<LzJob>& jobs, std::vector<LzState>& st, const std::vector<int>& form)
 {
     const size_t nj = jobs.size(), bytes_st = sizeof(LzState) * st.size();
     const size_t o_jobs = (bytes_st + 255) & ~(size_t)255, size = o_jobs + sizeof(LzJob) * nj;
     Lease<char> blob(c->pool, size);
-    for (size_t j = 0; j < nj; j++) jobs[j].st = reinterpret_cast<LzState*>(blob.p) + 2 * j;
     char* h = stage_buffer(c, size);
-    std::memcpy(h + o_jobs, jobs.data(), sizeof(LzJob) * nj);
-    const LzJob* d_jobs = reinterpret_cast<const LzJob*>(blob.p + o_jobs);
-    CK(cudaMemcpyAsync(blob.p + o_jobs, h + o_jobs, sizeof(LzJob) * nj, cudaMemcpyHostToDevice, c->stream));
+    LzJob* hj = reinterpret_cast<LzJob*>(h + o_jobs);
+    int first[kSmallForms + 2] = {};                      // of each form's jobs on the device
+    size_t smem[kSmallForms + 1] = {};
+    for (int f = 1, i = 0; f <= kSmallForms; f++) {
+        first[f] = i;
+        for (size_t j = 0; j < nj; j++) {
+            if (form[j] != f) continue;
+            jobs[j].st = reinterpret_cast<LzState*>(blob.p) + 2 * j;
+            std::memcpy(hj + i++, &jobs[j], sizeof(LzJob));
+            smem[f] = std::max(smem[f], lz_small_smem(jobs[j].S));
+        }
+        first[f + 1] = i;
+    }
+    const LzJob* dj = reinterpret_cast<const LzJob*>(blob.p + o_jobs);
+    CK(cudaMemcpyAsync(blob.p + o_jobs, hj, sizeof(LzJob) * nj, cudaMemcpyHostToDevice, c->stream));
     CK(cudaEventRecord(c->ev0, c->stream));
-    CK(launch_lanczos_small(d_jobs, (int)nj, K.smem, K.form, c->stream));
+    struct Side {                                         // nothing of it outlasts the call
+        cudaStream_t s = nullptr;
+        ~Side() { if (s) cudaStreamSynchronize(s); }
+    } side;
+    int n = 0;
+    for (int f = 1; f <= kSmallForms; f++) {
+        if (first[f + 1] == first[f]) continue;
+        cudaStream_t on = c->stream;
+        if (n++ % 2 == 1) {
+            if (!c->side) {
+                if (!c->side_done) CK(cudaEventCreateWithFlags(&c->side_done, cudaEventDisableTiming));
+                CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+            }
+            if (!side.s) CK(cudaStreamWaitEvent(c->side, c->ev0, 0));
+            on = side.s = c->side;
+        }
+        CK(launch_lanczos_small(dj + first[f], first[f + 1] - first[f], smem[f], f, on));
+        c->launches += 1;
+    }
+    if (side.s) {
+        CK(cudaEventRecord(c->side_done, side.s));
+        CK(cudaStreamWaitEvent(c->stream, c->side_done, 0));
+    }
     CK(cudaEventRecord(c->ev1, c->stream));
-    c->launches += 1;
     CK(cudaMemcpyAsync(h, blob.p, bytes_st, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    side.s = nullptr;
     std::memcpy(st.data(), h, bytes_st);
     float ms = 0.0f;
     CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
@@ -800,17 +832,11 @@ bool small_allowed(const edzt_ctx* c, const LzJob& J)
     return c->dbg_pass_cap == 0 && c->dbg_stall_cta < 0 && !c->tuned.count({J.S.up.count, J.S.dn.count});
 }
 
-// Count a run in with the others of its model: K becomes the form for all of
+// Count a run in with the others of its model: form becomes that for all of
 // them, or -1 (the persistent kernel) when one is not small.
-void small_include(SmallKernel& K, const LzJob& J)
+void small_include(int& form, const LzJob& J)
 {
-    const size_t need = lz_small_smem(J.S);
-    if (K.form < 0 || need == 0) {
-        K = SmallKernel{-1, 0};
-        return;
-    }
-    K.form = std::max(K.form, lz_small_form(J.S));
-    K.smem = std::max(K.smem, need);
+    form = (form < 0 || lz_small_smem(J.S) == 0) ? -1 : std::max(form, lz_small_form(J.S));
 }
 
 // All runs of specs from start to finish.  Coefficient runs write a and b up
@@ -841,21 +867,17 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     // Runs for the kernel of small ones: those of a model that are all small,
     // in the form for that model, so that a model's runs take the same way
     // alone and among others.
-    std::map<const ModelTables*, SmallKernel> kernel_of;
+    std::map<const ModelTables*, int> form_of;
     for (int j = 0; j < nj; j++) {
         if (specs[j].mode != LZ_COEFF) continue;          // an eigenvector pass goes where its scan went
-        SmallKernel& K = kernel_of.emplace(specs[j].mt, SmallKernel{}).first->second;
-        if (force || !small_allowed(c, jobs[j])) K.form = -1;
-        small_include(K, jobs[j]);
+        int& form = form_of.emplace(specs[j].mt, 0).first->second;
+        if (force || !small_allowed(c, jobs[j])) form = -1;
+        small_include(form, jobs[j]);
     }
-    std::vector<int> order[kSmallForms + 1];              // jobs by kernel; 0: the persistent one
-    size_t smem[kSmallForms + 1] = {};
+    std::vector<int> order[2];                            // jobs of the persistent kernel, and small ones
     for (int j = 0; j < nj; j++) {
-        SmallKernel K{specs[j].form, specs[j].form ? lz_small_smem(jobs[j].S) : 0};
-        if (specs[j].mode == LZ_COEFF) K = kernel_of[specs[j].mt];
-        const int f = specs[j].form = std::max(K.form, 0);
-        order[f].push_back(j);
-        smem[f] = std::max(smem[f], K.smem);
+        if (specs[j].mode == LZ_COEFF) specs[j].form = std::max(form_of[specs[j].mt], 0);
+        order[specs[j].form > 0].push_back(j);
     }
     for (int j : order[0]) {
         LzJob& J = jobs[j];
@@ -881,17 +903,19 @@ void run_jobs(edzt_ctx* c, std::vector<JobSpec>& specs, const LzShape* force = n
     }
     int phases = 2 * max_steps + 4;     // two phases per step and the phase that closes the last one
     if (c->dbg_pass_cap > 0) phases = std::min(phases, c->dbg_pass_cap);
-    for (int f = kSmallForms; f >= 0; f--) {
-        const std::vector<int>& o = order[f];
+    for (int small = 1; small >= 0; small--) {
+        const std::vector<int>& o = order[small];
         if (o.empty()) continue;
         std::vector<LzJob> part;
         std::vector<LzState> ps;
+        std::vector<int> form;
         for (int j : o) {
             part.push_back(jobs[j]);
+            form.push_back(specs[j].form);
             ps.insert(ps.end(), &st[2 * (size_t)j], &st[2 * (size_t)j] + 2);
         }
-        const float ms = f ? launch_small(c, part, ps, SmallKernel{f, smem[f]})
-                           : launch_jobs(c, part, ps, force ? force : tuned_shape(c, part), phases, false);
+        const float ms = small ? launch_small(c, part, ps, form)
+                               : launch_jobs(c, part, ps, force ? force : tuned_shape(c, part), phases, false);
         double bytes = 0.0;
         for (size_t i = 0; i < o.size(); i++) {
             JobSpec& s = specs[o[i]];
@@ -2317,35 +2341,36 @@ std::unique_ptr<LiveJob> make_live(edzt_ctx* c, const JobSpec& spec, std::vector
     return L;
 }
 
-// The kernel of small runs for those of a request's phase; form 0: they are for
-// the persistent kernel (some run is larger, or all their steps at once, 4 us
-// each, would outlast a server step).
-SmallKernel small_request(const edzt_server* sv, const ServReq& q)
+// The form of the kernel of small runs for those of a request's phase; 0: they
+// are for the persistent kernel (some run is larger, or all their steps at once,
+// 4 us each, would outlast a server step).
+int small_request(const edzt_server* sv, const ServReq& q)
 {
-    SmallKernel K;
+    int form = 0;
     for (const auto& j : q.jobs) {
         LzJob J;
         fill_job(J, j->spec, j->S);
-        if (J.mode != LZ_COEFF) return SmallKernel{j->spec.form, j->spec.form ? lz_small_smem(J.S) : 0};
-        if (!small_allowed(sv->c, J) || 0.004 * J.maxnstep > sv->step_ms) K.form = -1;
-        small_include(K, J);
-        if (K.form < 0) return SmallKernel{};
+        if (J.mode != LZ_COEFF) return j->spec.form;
+        if (!small_allowed(sv->c, J) || 0.004 * J.maxnstep > sv->step_ms) form = -1;
+        small_include(form, J);
     }
-    return K;
+    return std::max(form, 0);
 }
 
 // One slice: at most `phases` phases (even) of every live run in v, in one
-// persistent launch, or (small.form) all their steps in the kernel of small
-// runs; runs that finish are marked done with nstep and norm0.  Returns the
-// launch's device time in ms.
-float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, const SmallKernel& small = {})
+// persistent launch, or (phases 0) all their steps in the kernel of small runs;
+// runs that finish are marked done with nstep and norm0.  Returns the launch's
+// device time in ms.
+float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases)
 {
     const int nj = (int)v.size();
     std::vector<LzJob> jobs(nj);
+    std::vector<int> form(nj);
     for (int j = 0; j < nj; j++) {
         LiveJob& L = *v[j];
         LzJob& J = jobs[j];
         fill_job(J, L.spec, L.S);
+        form[j] = L.spec.form;
         J.Y = L.y.p;
         J.V[0] = L.spec.keep ? L.spec.keep : L.v0.p;
         J.V[1] = L.v1.p;
@@ -2355,8 +2380,8 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, const SmallKe
     for (int j = 0; j < nj; j++) std::memcpy(&st[2 * (size_t)j], v[j]->st, 2 * sizeof(LzState));
     int budget = std::max(2, phases & ~1);
     if (c->dbg_pass_cap > 0) budget = std::min(budget, std::max(2, c->dbg_pass_cap & ~1));
-    const float ms = small.form ? launch_small(c, jobs, st, small)
-                                : launch_jobs(c, jobs, st, tuned_shape(c, jobs), budget, true);
+    const float ms = phases == 0 ? launch_small(c, jobs, st, form)
+                                 : launch_jobs(c, jobs, st, tuned_shape(c, jobs), budget, true);
     for (int j = 0; j < nj; j++) std::memcpy(v[j]->st, &st[2 * (size_t)j], 2 * sizeof(LzState));
     double bytes = 0.0;
     for (int j = 0; j < nj; j++) {
@@ -2371,7 +2396,6 @@ float run_slice(edzt_ctx* c, std::vector<LiveJob*>& v, int phases, const SmallKe
         L.k = std::max(L.k, k_now);
         if (fin) {
             L.done = true;
-            L.spec.form = small.form;
             L.spec.nstep = fin->nstep;
             L.spec.norm0 = fin->norm0;
         }
@@ -2729,25 +2753,23 @@ int server_step(edzt_server* sv)
         };
         for (int round = 0; round < 64; round++) {
             advance_done();
-            std::vector<LiveJob*> runs[kSmallForms + 1], &v = runs[0];   // by kernel; 0: the persistent one
+            std::vector<LiveJob*> v, few;                 // runs of the persistent kernel, and small ones
             long long dims = 0;
-            size_t smem[kSmallForms + 1] = {}, live = 0;
             for (auto& up : sv->active) {
                 if (up->cls != cls || up->phase >= 4) continue;
-                const SmallKernel K = small_request(sv, *up);
-                smem[K.form] = std::max(smem[K.form], K.smem);
+                const int form = small_request(sv, *up);
                 for (auto& j : up->jobs) {
                     if (j->done) continue;
-                    runs[K.form].push_back(j.get());
-                    live++;
-                    if (!K.form) dims += j->S.dim;
+                    j->spec.form = form;
+                    (form ? few : v).push_back(j.get());
+                    if (!form) dims += j->S.dim;
                 }
             }
-            if (live == 0) break;
+            if (v.empty() && few.empty()) break;
             bool short_slice = false;
-            auto slice = [&](std::vector<LiveJob*>& runs, int phases, const SmallKernel& small) {
+            auto slice = [&](std::vector<LiveJob*>& runs, int phases) {
                 try {
-                    const float ms = run_slice(c, runs, phases, small);
+                    const float ms = run_slice(c, runs, phases);
                     moved = true;
                     return ms;
                 } catch (const EdztError& e) {
@@ -2757,8 +2779,7 @@ int server_step(edzt_server* sv)
                     return 0.0f;
                 }
             };
-            for (int f = 1; f <= kSmallForms; f++)
-                if (!runs[f].empty() && !short_slice) left -= slice(runs[f], 0, SmallKernel{f, smem[f]});
+            if (!few.empty()) left -= slice(few, 0);
             if (short_slice) break;
             auto est = sv->ms_per_phase.find(cls);
             const double mpp = (est != sv->ms_per_phase.end()) ? est->second : 0.01 + (double)dims * 40.0 / 4.0e9;
@@ -2766,7 +2787,7 @@ int server_step(edzt_server* sv)
             phases &= ~1;
             if (phases < 2) phases = 2;
             if (!v.empty()) {
-                const float ms = slice(v, phases, SmallKernel{});
+                const float ms = slice(v, phases);
                 if (short_slice) break;
                 const double per = ms / phases;
                 sv->ms_per_phase[cls] = (est != sv->ms_per_phase.end()) ? 0.5 * (est->second + per) : per;
@@ -2909,6 +2930,8 @@ void edzt_ctx_destroy(edzt_ctx* c)
     if (c->stage) cudaFreeHost(c->stage);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
+    if (c->side_done) cudaEventDestroy(c->side_done);
+    if (c->side) cudaStreamDestroy(c->side);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
