@@ -260,8 +260,9 @@ size_t lz_sync_bytes(int njobs);
 // The device-free part of lz_plan: given every job's widths (ph[].width) and
 // the grid G, the phases' tile lists, CTA ranges, participants and the column
 // phase's slab order (prefix as lz_plan describes it), the tiles per phase
-// (total) and the number of partial-sum slots (returned).
-long long lz_cut(LzJob* jobs, int njobs, int G, std::vector<long long>& prefix, long long total[2]);
+// (total) and the number of partial-sum slots (returned).  slow: time of a
+// tile's lines over what they take a CTA that has the SM to itself.
+long long lz_cut(LzJob* jobs, int njobs, int G, std::vector<long long>& prefix, long long total[2], double slow = 1.0);
 // The slab order regrouped so that the slabs of a tile of several planes are neighbours.
 void lz_group_slabs(const LzJob* jobs, int njobs, int G, std::vector<long long>& prefix);
 

@@ -1000,36 +1000,44 @@ cudaError_t launch_lanczos_small(const LzJob* jobs, int nj, size_t smem, int for
 // ---------------------------------------------------------------------------
 // Most dynamic shared memory of a CTA of 256 threads, two of which share an SM.
 static constexpr size_t kLzSmemTwoPerSm = 113 * 1024;
-// Fixed cost of a tile in states, for cutting the tile list into CTA ranges
+// Fixed cost of a list position in states, for cutting the list into CTA ranges
 static constexpr double kLzTileCost = 256.0;
-// A CTA that serves two jobs in a phase reloads tables and waits twice: worth
-// this much work in states, or an uneven share of the whole
-static constexpr double kLzSwitchCost = 2000.0;
-static constexpr double kLzUneven = 1.15;
 // Lines of which a few are taken two at a time
 static constexpr int kLzLongLine = 500;
-// Time of a tile with two CTAs on the SM over its time with one
+// Time of a tile's lines with two CTAs on the SM over their time with one
 static constexpr double kLzPairSlowdown = 1.75;
+// What a pass over a tile takes besides its lines (staging round, barriers), and
+// a job besides its passes (tables, the wait for its arrivals), in lines of 7 ns
+static constexpr double kLzPassLines = 200.0, kLzJobLines = 600.0;
 
-// Load of the busiest CTA, both phases: passes over a tile times its lines,
-// a partly filled tile 0.8 of a pass.
-static double lz_load(const LzJob* jobs, int nj, int G, const std::vector<long long>& prefix)
+// Load of the busiest CTA of a phase whose CTAs take the ranges `range`, in
+// lines: those of its passes (a partly filled tile 0.8 of a pass), `slow` times
+// as long as for a CTA that has the SM to itself, its passes and its jobs.
+static double phase_load(const LzJob* jobs, int nj, int G, int ph, const long long* range, double slow)
 {
-    double sum = 0.0;
-    for (int ph = 0; ph < 2; ph++) {
-        const long long* range = prefix.data() + 2 * (size_t)(nj + 1) + (size_t)ph * (G + 1);
-        std::vector<double> load((size_t)G, 0.0);
-        for (int j = 0; j < nj; j++) {
+    double most = 0.0;
+    int j = 0;
+    for (int b = 0; b < G; b++) {
+        double load = 0.0;
+        for (long long t = range[b]; t < range[b + 1];) {
+            while (jobs[j].ph[ph].tile0 + jobs[j].ph[ph].ntiles <= t) j++;
             const LzPhase& Q = jobs[j].ph[ph];
-            const int lines = (ph == 0) ? jobs[j].S.dn.count : jobs[j].S.up.count;
-            for (int b = Q.part0; b < Q.part0 + Q.npart; b++) {
-                const long long n = std::min(range[b + 1], Q.tile0 + Q.ntiles) - std::max(range[b], Q.tile0);
-                load[b] += lines * ((double)(n / Q.planes) + (n % Q.planes ? 0.8 : 0.0));
-            }
+            const int lines = (ph == 0) ? jobs[j].S.dn.count : jobs[j].S.up.count, planes = std::max(1, Q.planes);
+            const int n = (int)(std::min(range[b + 1], Q.tile0 + Q.ntiles) - t);
+            const double full = n / planes, rest = n % planes ? 1.0 : 0.0;
+            load += slow * lines * (full + 0.8 * rest) + kLzPassLines * (full + rest) + kLzJobLines;
+            t += n;
         }
-        sum += *std::max_element(load.begin(), load.end());
+        most = std::max(most, load);
     }
-    return sum;
+    return most;
+}
+
+// Both phases of a plan.
+static double lz_load(const LzJob* jobs, int nj, int G, const std::vector<long long>& prefix, double slow)
+{
+    const long long* range = prefix.data() + 2 * (size_t)(nj + 1);
+    return phase_load(jobs, nj, G, 0, range, slow) + phase_load(jobs, nj, G, 1, range + G + 1, slow);
 }
 
 LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, const LzShape* force)
@@ -1065,7 +1073,7 @@ LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, 
         }
         Q.grid = lz_grid_size(device, Q);
         if (Q.grid <= 0) return;
-        Q.slots = lz_cut(jobs, nj, Q.grid, pre, Q.total);
+        Q.slots = lz_cut(jobs, nj, Q.grid, pre, Q.total, Q.block < kLzThreads ? kLzPairSlowdown : 1.0);
         lz_group_slabs(jobs, nj, Q.grid, pre);
         pre.resize(pre.size() + kMaxPlanes, 0);          // the kernel reads whole tiles of slab numbers
     };
@@ -1086,8 +1094,8 @@ LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, 
     // (2,7) of nsite 14 35 and 26); lines of 252 strings gain nothing from it.
     // Tiles of eight lines may also run two CTAs per SM, which overlap one's staging
     // with the other's hop sums but halve what a CTA gets through: taken when
-    // the busiest CTA's load, in passes over a tile, times kLzPairSlowdown is
-    // less than one CTA per SM has (us a step, one / two CTAs: 9 sectors of
+    // the busiest CTA's load (lz_load) is less then than with one CTA per SM (us
+    // a step, one / two CTAs: 9 sectors of
     // nsite 12 106 / 99, of nsite 10 18.2 / 15.5; one sector of nsite 12
     // 23 / 31; 2 sectors of nsite 13 92 / 110).
     int wc = 8, r = 8;
@@ -1099,14 +1107,16 @@ LzPlan lz_plan(int device, LzJob* jobs, int nj, std::vector<long long>& prefix, 
     cut(P, prefix);
     LzPlan Q = P;
     if (P.wc == 8 && P.r == 8 && shape(Q, 8, 8, kLzThreads / 2)) {
-        const double one = lz_load(jobs, nj, P.grid, prefix);
+        const double one = lz_load(jobs, nj, P.grid, prefix, 1.0);
         std::vector<long long> pre;
+        std::vector<LzPhase> mine;                       // the jobs' phases of P
+        for (int j = 0; j < nj; j++) mine.insert(mine.end(), jobs[j].ph, jobs[j].ph + 2);
         cut(Q, pre);
-        if (Q.grid > P.grid && kLzPairSlowdown * lz_load(jobs, nj, Q.grid, pre) < one) {
+        if (Q.grid > P.grid && lz_load(jobs, nj, Q.grid, pre, kLzPairSlowdown) < one) {
             prefix.swap(pre);
             return Q;
         }
-        cut(P, prefix);                                  // the jobs' phases of the plan that is kept
+        for (int j = 0; j < nj; j++) std::copy_n(mine.data() + 2 * j, 2, jobs[j].ph);
     }
     return P;
 }
@@ -1141,7 +1151,7 @@ void lz_group_slabs(const LzJob* jobs, int nj, int G, std::vector<long long>& pr
     }
 }
 
-long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, long long total[2])
+long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, long long total[2], double slow)
 {
     long long slots = 0;
     prefix.assign(2 * (size_t)(nj + 1) + 2 * (size_t)(G + 1), 0);
@@ -1158,30 +1168,40 @@ long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, lon
         const long long T = pre[nj];
         total[ph] = T;
         // CTA ranges: with no more tiles than CTAs, CTA b takes tile b; else
-        // each job gets CTAs in proportion to its cost (a tile costs its
-        // states plus a fixed amount for its staging round and barriers),
-        // so that a CTA serves one job and need not reload its tables or
-        // wait for two; where that leaves some CTA with much more than its
-        // share, and with more jobs than CTAs, the list is cut where the
-        // running cost crosses b/G of the total, every CTA keeping at least
-        // one tile.
+        // either the list is cut where the running cost (a tile costs its
+        // states plus a fixed amount) crosses b/G of the total, every CTA
+        // keeping at least one tile, or (with no more jobs than CTAs) each job
+        // gets CTAs in proportion to its cost, so that a CTA serves one job and
+        // need not reload its tables or wait for two: whichever leaves the
+        // busiest CTA less to do (phase_load).  All sectors of a model at once
+        // show it, as do batches of uneven sizes (us a step when that went by
+        // the states alone, and by phase_load: nsite 11 341 and 156, nsite 12 928
+        // and 440, nsite 10 48 both; 40 batches and served sets of 3 to 16 models
+        // of 6 to 12 sites 10% less, none more than 1.5% more).
         long long* range = prefix.data() + 2 * (size_t)(nj + 1) + (size_t)ph * (G + 1);
         if (T <= G) {
             for (int b = 0; b <= G; b++) range[b] = std::min<long long>(b, T);
         } else {
-            std::vector<double> cost((size_t)nj, 0.0), cum((size_t)T + 1, 0.0);
+            // a job's positions cost the same but for a last one of fewer lines
+            std::vector<double> cost((size_t)nj, 0.0), each((size_t)nj, 0.0), cum((size_t)nj + 1, 0.0);
             for (int j = 0; j < nj; j++) {
                 const LzPhase& Q = jobs[j].ph[ph];
-                const long long lines = (ph == 0) ? jobs[j].S.dn.count : jobs[j].S.up.count;
-                const int count = (ph == 0) ? jobs[j].S.up.count : jobs[j].S.dn.count;
-                for (int i = 0; i < Q.ntiles; i++) {
-                    const int w = std::min(Q.width, count - i * Q.width);
-                    cum[Q.tile0 + i + 1] = cum[Q.tile0 + i] + (double)lines * w + kLzTileCost;
-                }
-                cost[j] = cum[Q.tile0 + Q.ntiles] - cum[Q.tile0];
+                const double lines = (ph == 0) ? jobs[j].S.dn.count : jobs[j].S.up.count;
+                const double count = (ph == 0) ? jobs[j].S.up.count : jobs[j].S.dn.count;
+                each[j] = lines * Q.width + kLzTileCost;
+                cost[j] = lines * count + kLzTileCost * Q.ntiles;
+                cum[j + 1] = cum[j] + cost[j];
             }
             std::vector<int> share;
-            double worst = HUGE_VAL;
+            range[0] = 0;
+            range[G] = T;
+            for (int b = 1, j = 0; b < G; b++) {
+                const double target = cum[nj] * b / G;
+                while (j + 1 < nj && cum[j + 1] <= target) j++;
+                const LzPhase& Q = jobs[j].ph[ph];
+                const long long t = Q.tile0 + std::min<long long>(Q.ntiles - 1, (long long)((target - cum[j]) / each[j]));
+                range[b] = std::min(std::max(t, range[b - 1] + 1), T - (G - b));
+            }
             if (nj <= G) {                               // CTAs one by one to the job whose CTAs have the most to do
                 share.assign((size_t)nj, 1);
                 std::priority_queue<std::pair<double, int>> load;
@@ -1204,28 +1224,14 @@ long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, lon
                     for (const auto& f : full) load.push(f);
                     if (j < 0) break;
                 }
-                worst = 0.0;
-                for (int j = 0; j < nj; j++) {
-                    const int nt = jobs[j].ph[ph].ntiles;
-                    worst = std::max(worst, cost[j] / nt * ((nt + share[j] - 1) / share[j]));
-                }
-            }
-            if (worst <= kLzUneven * cum[T] / G + kLzSwitchCost) {
+                std::vector<long long> own((size_t)G + 1);
                 int b = 0;
                 for (int j = 0; j < nj; j++)
                     for (int q = 0; q < share[j]; q++)
-                        range[b++] = jobs[j].ph[ph].tile0 + (long long)jobs[j].ph[ph].ntiles * q / share[j];
-                range[G] = T;
-            } else {
-                range[0] = 0;
-                range[G] = T;
-                long long t = 0;
-                for (int b = 1; b < G; b++) {
-                    const double target = cum[T] * b / G;
-                    while (t < T && cum[t + 1] <= target) t++;
-                    range[b] = std::min(std::max(t, range[b - 1] + 1), T - (G - b));
-                    t = range[b];
-                }
+                        own[b++] = jobs[j].ph[ph].tile0 + (long long)jobs[j].ph[ph].ntiles * q / share[j];
+                own[G] = T;
+                if (phase_load(jobs, nj, G, ph, own.data(), slow) <= phase_load(jobs, nj, G, ph, range, slow))
+                    std::copy(own.begin(), own.end(), range);
             }
         }
         // participants of a job: the CTAs whose range meets its tiles (a contiguous run)
