@@ -1005,9 +1005,15 @@ static constexpr double kLzTileCost = 256.0;
 // Lines of which a few are taken two at a time
 static constexpr int kLzLongLine = 500;
 // Time of a tile's lines with two CTAs on the SM over their time with one
-static constexpr double kLzPairSlowdown = 1.75;
+static constexpr double kLzPairSlowdown = 2.037;
 // What a pass over a tile takes besides its lines (staging round, barriers), and
-// a job besides its passes (tables, the wait for its arrivals), in lines of 7 ns
+// a job besides its passes (tables, the wait for its arrivals), in lines of 6 ns.
+// Fitted to 111 launches of 1 to 169 runs of nsite 6 to 13, timed with one and
+// with two CTAs per SM.  The line is drawn between two that lie close: 9 runs of
+// nsite 12 (99.8 us a step with two, 105 with one) and two runs of 924 and 495 by
+// 792 strings (32.8 and 30.9).  Three in four of the others are taken right to
+// 1%, all to 10% but (4,5) of nsite 9's four (12.6 instead of 10.8); lines alone
+// at 1.75 missed a quarter by 5 to 59%.
 static constexpr double kLzPassLines = 200.0, kLzJobLines = 600.0;
 
 // Load of the busiest CTA of a phase whose CTAs take the ranges `range`, in
@@ -1177,7 +1183,7 @@ long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, lon
         // show it, as do batches of uneven sizes (us a step when that went by
         // the states alone, and by phase_load: nsite 11 341 and 156, nsite 12 928
         // and 440, nsite 10 48 both; 40 batches and served sets of 3 to 16 models
-        // of 6 to 12 sites 10% less, none more than 1.5% more).
+        // of 6 to 12 sites 9% less kernel time, none more than 1.3% more).
         long long* range = prefix.data() + 2 * (size_t)(nj + 1) + (size_t)ph * (G + 1);
         if (T <= G) {
             for (int b = 0; b <= G; b++) range[b] = std::min<long long>(b, T);
