@@ -1002,6 +1002,12 @@ cudaError_t launch_lanczos_small(const LzJob* jobs, int nj, size_t smem, int for
 static constexpr size_t kLzSmemTwoPerSm = 113 * 1024;
 // Fixed cost of a list position in states, for cutting the list into CTA ranges
 static constexpr double kLzTileCost = 256.0;
+// A CTA that serves two jobs in a phase reloads tables and waits twice: worth
+// this much work in states, or an uneven share of the whole, where the loads of
+// both cuts are this close
+static constexpr double kLzSwitchCost = 2000.0;
+static constexpr double kLzUneven = 1.15;
+static constexpr double kLzClose = 1.1;
 // Lines of which a few are taken two at a time
 static constexpr int kLzLongLine = 500;
 // Time of a tile's lines with two CTAs on the SM over their time with one
@@ -1179,7 +1185,10 @@ long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, lon
         // keeping at least one tile, or (with no more jobs than CTAs) each job
         // gets CTAs in proportion to its cost, so that a CTA serves one job and
         // need not reload its tables or wait for two: whichever leaves the
-        // busiest CTA less to do (phase_load).  All sectors of a model at once
+        // busiest CTA less to do (phase_load), and where that is close the
+        // latter, unless its costliest CTA has much more than its share (two
+        // runs of nsite 12, 924 and 495 by 792 strings: 30.8 us a step instead
+        // of 29.8; kLzClose from 1.1 to 1.25 the same, 1.05 too narrow).  All sectors of a model at once
         // show it, as do batches of uneven sizes (us a step when that went by
         // the states alone, and by phase_load: nsite 11 341 and 156, nsite 12 928
         // and 440, nsite 10 48 both; 40 batches and served sets of 3 to 16 models
@@ -1236,7 +1245,15 @@ long long lz_cut(LzJob* jobs, int nj, int G, std::vector<long long>& prefix, lon
                     for (int q = 0; q < share[j]; q++)
                         own[b++] = jobs[j].ph[ph].tile0 + (long long)jobs[j].ph[ph].ntiles * q / share[j];
                 own[G] = T;
-                if (phase_load(jobs, nj, G, ph, own.data(), slow) <= phase_load(jobs, nj, G, ph, range, slow))
+                const double one = phase_load(jobs, nj, G, ph, own.data(), slow);
+                const double even = phase_load(jobs, nj, G, ph, range, slow);
+                double worst = 0.0;
+                for (int j = 0; j < nj; j++) {
+                    const int nt = jobs[j].ph[ph].ntiles;
+                    worst = std::max(worst, cost[j] / nt * ((nt + share[j] - 1) / share[j]));
+                }
+                const bool close = one < kLzClose * even && even < kLzClose * one;
+                if (close ? worst <= kLzUneven * cum[nj] / G + kLzSwitchCost : one < even)
                     std::copy(own.begin(), own.end(), range);
             }
         }
