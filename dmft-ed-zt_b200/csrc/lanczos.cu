@@ -1017,9 +1017,9 @@ static constexpr double kLzPairSlowdown = 2.037;
 // Fitted to 111 launches of 1 to 169 runs of nsite 6 to 13, timed with one and
 // with two CTAs per SM.  The line is drawn between two that lie close: 9 runs of
 // nsite 12 (99.8 us a step with two, 105 with one) and two runs of 924 and 495 by
-// 792 strings (32.8 and 30.9).  Three in four of the others are taken right to
-// 1%, all to 10% but (4,5) of nsite 9's four (12.6 instead of 10.8); lines alone
-// at 1.75 missed a quarter by 5 to 59%.
+// 792 strings (32.8 and 30.9).  96 of the 111 are taken right to 1%, four are
+// missed by 5 to 17% (the c / c^+ runs of ten models of nsite 6 to 9: 12.6 instead
+// of 10.8); lines alone at 1.75 miss 28 by more than 5%, one by 145%.
 static constexpr double kLzPassLines = 200.0, kLzJobLines = 600.0;
 
 // Load of the busiest CTA of a phase whose CTAs take the ranges `range`, in
